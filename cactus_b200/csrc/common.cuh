@@ -146,18 +146,23 @@ __host__ __device__ static inline TiledDims tiled_dims(int wtype, int64_t K, int
 // Rows beyond N and blocks beyond K/32 are zero.
 constexpr float ACT_MAGIC = 12582912.0f;   // 1.5 * 2^23 = as_float(0x4B400000)
 __host__ __device__ static inline int act_scale_index(int j, int col) { return ((j * 4 + (col >> 1)) * 4) + (col & 1); }
-// Products of ACT_F8_MIN_N and more columns also carry what the tcgen05 kernel (mmq_tc.cu) reads: after the scale plane
-// two more quant planes in K-major core-matrix order (per n-tile and block two 8-column x 16-byte matrices, elements
-// 0..15 then 16..31), holding each quant a = 16 h + l (h = a >> 4, l = a & 15) as two e4m3 bytes -- `hi` the byte whose
-// value is h * 2^-5, `lo` the byte l, whose value is l * 2^-9 (the subnormals and first binade of e4m3 are the
-// integers 0..15 times 2^-9) -- and a second scale plane with {D[2cp], D[2cp+1], C[2cp], C[2cp+1]} at the same float
-// indices, D = d * 2^18 and C = -8 * d * sum(a) (the kernel multiplies unsigned weight nibbles u = q + 8).
-constexpr int ACT_F8_MIN_N = 16;
+// b200_mul_mat_q, which knows the weights' shape when it quantises, may put behind them what the tcgen05 kernel (mmq_tc.cu)
+// multiplies: the fp16 operands d * a as rn(d * a) and the exact remainder, [column chunk][block group][rn | remainder]
+// [n-tile of the chunk], 2 KB each -- what a CTA needs of one block group is one contiguous piece.  The 2 KB are in the
+// core-matrix order of the MMA's B descriptor: 16 matrices of 8 columns x 8 values of K, 128 bytes each, the matrices of
+// block j at 4j .. 4j + 3.  Within a block K is in the order in which the T16 weight words yield it: matrix
+// c = 2 (i & 1) + half, value 2t + (i >> 1) is element 16 half + 4t + i (t = 0..3, i = 0..3).
+// n-tiles per column chunk: at most 8 (64 columns), an even number, the chunks as equal as that allows
+__host__ __device__ static inline int act_chunk_nt(int64_t n_nt) {
+    const int64_t chunks = (n_nt + 7) / 8;
+    return (int) (((n_nt + chunks - 1) / chunks + 1) & ~(int64_t) 1);
+}
 struct ActDims {
     int64_t N, K, nb, nbp, n_bg, n_nt;
     size_t d_offset;     // byte offset of the scale plane
-    size_t hi_offset, lo_offset, s2_offset;   // the e4m3 planes and their scale plane (0 when absent)
     size_t total_bytes;
+    size_t b_offset, b_bytes;   // the tcgen05 kernel's operands, where they are wanted
+    int chunk_nt;               // their n-tiles per column chunk
 };
 
 __host__ __device__ static inline ActDims act_dims(int64_t K, int64_t N) {
@@ -170,13 +175,9 @@ __host__ __device__ static inline ActDims act_dims(int64_t K, int64_t N) {
     a.n_nt = (N + 7) / 8;
     a.d_offset = (size_t) a.n_nt * a.nbp * 256;
     a.total_bytes = a.d_offset + (size_t) a.n_nt * a.n_bg * 256;
-    a.hi_offset = a.lo_offset = a.s2_offset = 0;
-    if (N >= ACT_F8_MIN_N) {   // every offset below follows from d_offset alone: the scale planes are a quarter of a quant plane
-        a.hi_offset = a.total_bytes;
-        a.lo_offset = a.hi_offset + a.d_offset;
-        a.s2_offset = a.lo_offset + a.d_offset;
-        a.total_bytes = a.s2_offset + a.d_offset / 4;
-    }
+    a.chunk_nt = act_chunk_nt(a.n_nt);
+    a.b_offset = a.total_bytes;   // = d_offset + d_offset / 4: the scale plane is a quarter of the quant plane
+    a.b_bytes = (size_t) ((a.n_nt + a.chunk_nt - 1) / a.chunk_nt) * a.n_bg * a.chunk_nt * 4096;
     return a;
 }
 
@@ -213,18 +214,12 @@ __device__ __forceinline__ double rms_block_sum(double sum) {
     return tot;
 }
 
-// e4m3 byte of h * 2^-5 for the signed nibble h (index = h & 15)
-__device__ __forceinline__ uint32_t e4m3_hi_byte(uint32_t nib) {
-    const uint64_t tab = (nib & 8) ? 0x90989CA0A2A4A6A8ull : 0x262422201C181000ull;   // h = -8..-1 | h = 0..7, lowest byte first
-    return (uint32_t) (tab >> (8 * (nib & 7))) & 0xffu;
-}
 // Stores one lane's share (4 quants, element group j of 8) of a quantised block (row n, block b).  LAYOUT 0: the
-// reference's block_q8_0 stream; 1: B8 tiles in mma.sync B-fragment order; 2: B8 tiles as K-major core matrices;
-// 3: layout 1 plus the e4m3 planes of ACT_F8_MIN_N (qsum = the sum of the block's 32 quants).
-// Lane j == 0 also stores the block scale (layouts 1/2/3: the f32 pair {d, -d * 12582912}; zero for padding).
+// reference's block_q8_0 stream; 1: B8 tiles in mma.sync B-fragment order; 2: those plus the tcgen05 kernel's operands.
+// Lane j == 0 also stores the block scale (layouts 1 and 2: the f32 pair {d, -d * 12582912}; zero for padding).
 template <int LAYOUT>
 __device__ __forceinline__ void q8_store(uint8_t *__restrict__ out, size_t d_offset, int64_t nb, int64_t nbp, int64_t n, int64_t b, int j,
-                                         uint32_t packed, __half d, bool real, int qsum = 0) {
+                                         uint32_t packed, __half d, bool real, int chunk_nt = 2) {
     if (LAYOUT == 0) {
         uint8_t *blkp = out + (n * nb + b) * 34;
         if (j == 0) *reinterpret_cast<__half *>(blkp) = d;
@@ -234,33 +229,28 @@ __device__ __forceinline__ void q8_store(uint8_t *__restrict__ out, size_t d_off
     } else {
         const int64_t nt = n >> 3;
         const int g = (int) (n & 7);
-        const int t = j & 3;
+        const int t = j & 3, half = j >> 2;
         uint8_t *tile = out + (nt * nbp + b) * 256;
-        if (LAYOUT == 1 || LAYOUT == 3) {
-            *reinterpret_cast<uint32_t *>(tile + (g * 4 + t) * 8 + (j >= 4 ? 4 : 0)) = packed;
-            if (LAYOUT == 3) {
-                const size_t hi_off = d_offset + d_offset / 4, lo_off = hi_off + d_offset;
-                const size_t at = (size_t) (nt * nbp + b) * 256 + (j >> 2) * 128 + g * 16 + t * 4;
-                const uint32_t nib = (packed >> 4) & 0x0F0F0F0Fu;
-                const uint32_t hi = e4m3_hi_byte(nib & 0xff) | (e4m3_hi_byte((nib >> 8) & 0xff) << 8) | (e4m3_hi_byte((nib >> 16) & 0xff) << 16) |
-                                    (e4m3_hi_byte(nib >> 24) << 24);
-                *reinterpret_cast<uint32_t *>(out + hi_off + at) = hi;
-                *reinterpret_cast<uint32_t *>(out + lo_off + at) = packed & 0x0F0F0F0Fu;
+        *reinterpret_cast<uint32_t *>(tile + (g * 4 + t) * 8 + half * 4) = packed;
+        if (LAYOUT == 2) {
+            const int c = (int) nt / chunk_nt;
+            uint8_t *m = out + d_offset + d_offset / 4 + ((c * (nbp >> 2) + (b >> 2)) * 2 * chunk_nt + ((int) nt - c * chunk_nt)) * 2048 + (b & 3) * 512 + half * 128 + g * 16 + t * 4;
+            const __half2 d2 = __half2half2(real ? d : __ushort_as_half((unsigned short) 0));
+            const uint32_t u = packed ^ 0x80808080u;   // a + 128: 0x6400 | (a + 128) is the fp16 1152 + a
+#pragma unroll
+            for (int o = 0; o < 2; ++o) {              // elements o and o + 2
+                const uint32_t x = __byte_perm(u, 0x64646464u, o ? 0x4341 : 0x4240);
+                const __half2 a2 = __hadd2(*reinterpret_cast<const __half2 *>(&x), __float2half2_rn(-1152.0f));
+                const __half2 hi = __hmul2(a2, d2), lo = __hfma2(a2, d2, __hneg2(hi));
+                *reinterpret_cast<__half2 *>(m + o * 256) = hi;
+                *reinterpret_cast<__half2 *>(m + o * 256 + chunk_nt * 2048) = lo;
             }
-        } else {
-            // two 8-column x 16-byte core matrices: elements 0..15 of each column, then elements 16..31
-            *reinterpret_cast<uint32_t *>(tile + (j >> 2) * 128 + g * 16 + t * 4) = packed;
         }
         if (j == 0) {
             float *dp = reinterpret_cast<float *>(out + d_offset) + (nt * (nbp >> 2) + (b >> 2)) * 64 + act_scale_index((int) (b & 3), g);
             const float df = real ? __half2float(d) : 0.0f;
             dp[0] = df;
             dp[2] = -df * ACT_MAGIC;
-            if (LAYOUT == 3) {
-                float *dp2 = reinterpret_cast<float *>(out + d_offset + d_offset / 4 + 2 * d_offset) + (dp - reinterpret_cast<float *>(out + d_offset));
-                dp2[0] = df * 262144.0f;
-                dp2[2] = __fmul_rn((float) (-8 * qsum), df);
-            }
         }
     }
 }
@@ -268,7 +258,7 @@ __device__ __forceinline__ void q8_store(uint8_t *__restrict__ out, size_t d_off
 // quantises the 4 values of one lane of an 8-lane block group (all 8 lanes of the group must call it) and stores them
 template <int LAYOUT>
 __device__ __forceinline__ void q8_quantize_store(const float (&v)[4], uint8_t *__restrict__ out, size_t d_offset, int64_t nb, int64_t nbp,
-                                                  int64_t n, int64_t b, int j, bool real, int variant) {
+                                                  int64_t n, int64_t b, int j, bool real, int variant, int chunk_nt = 2) {
     float amax = fmaxf(fmaxf(fabsf(v[0]), fabsf(v[1])), fmaxf(fabsf(v[2]), fabsf(v[3])));
     const unsigned grp = 0xFFu << (threadIdx.x & 24);  // the 8 lanes that share this block
     amax = fmaxf(amax, __shfl_xor_sync(grp, amax, 1));
@@ -278,19 +268,9 @@ __device__ __forceinline__ void q8_quantize_store(const float (&v)[4], uint8_t *
     float id;
     q8_scales(amax, variant, &d, &id);
     uint32_t packed = 0;
-    int qsum = 0;
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        const int q = q8_round(v[i], id, variant);
-        qsum += q;
-        packed |= ((uint32_t) (q & 0xff)) << (8 * i);
-    }
-    if (LAYOUT == 3) {
-        qsum += __shfl_xor_sync(grp, qsum, 1);
-        qsum += __shfl_xor_sync(grp, qsum, 2);
-        qsum += __shfl_xor_sync(grp, qsum, 4);
-    }
-    q8_store<LAYOUT>(out, d_offset, nb, nbp, n, b, j, packed, d, real, qsum);
+    for (int i = 0; i < 4; ++i) packed |= ((uint32_t) (q8_round(v[i], id, variant) & 0xff)) << (8 * i);
+    q8_store<LAYOUT>(out, d_offset, nb, nbp, n, b, j, packed, d, real, chunk_nt);
 }
 
 // the same for one value per lane: the 32 lanes of a (fully active) warp hold one block in element order
@@ -303,19 +283,13 @@ __device__ __forceinline__ void q8_quantize_store_warp(float v, uint8_t *__restr
     __half d;
     float id;
     q8_scales(amax, variant, &d, &id);
-    const int qi = q8_round(v, id, variant);
-    int qsum = qi;
-    if (LAYOUT == 3) {
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) qsum += __shfl_xor_sync(0xffffffffu, qsum, o);
-    }
-    const uint32_t q = (uint32_t) (qi & 0xff);
+    const uint32_t q = (uint32_t) (q8_round(v, id, variant) & 0xff);
     uint32_t packed = q;
     packed |= __shfl_down_sync(0xffffffffu, q, 1) << 8;
     packed |= __shfl_down_sync(0xffffffffu, q, 2) << 16;
     packed |= __shfl_down_sync(0xffffffffu, q, 3) << 24;
     const int lane = threadIdx.x & 31;
-    if ((lane & 3) == 0) q8_store<LAYOUT>(out, d_offset, nb, nbp, n, b, lane >> 2, packed, d, real, qsum);
+    if ((lane & 3) == 0) q8_store<LAYOUT>(out, d_offset, nb, nbp, n, b, lane >> 2, packed, d, real);
 }
 
 }  // namespace b200

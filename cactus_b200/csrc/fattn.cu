@@ -19,8 +19,6 @@
 
 namespace b200 {
 
-int act_layout(int64_t N);   // quantize.cu: which B8 layout the mul_mat kernels expect for N columns
-
 
 constexpr int FA_THREADS = 128;
 #ifndef FA_MIN_CTAS
@@ -134,7 +132,7 @@ struct FattnParams {
     uint8_t *qout;   // optional: the output rows quantised to Q8_0 in the B8 activation layout of the mul_mat that follows
     size_t q_d_offset;
     int64_t q_nb, q_nbp;
-    int q_canon, q_variant;
+    int q_variant;
     float *partial;  // [Nq][H][nsplit][D + 2]
     int nsplit, hgroups;
     int w0;          // > 0: a token gets ceil(words / w0) KV splits (at most nsplit), so long sequences are cut, short ones are not;
@@ -183,10 +181,9 @@ __device__ __forceinline__ int fattn_target_words(const FattnParams &p, int ctas
 // Called by the 32 lanes of a warp with 32 consecutive elements of one output row: quantises them as one Q8_0 block of
 // column n.  A real call (not inlined): the attention kernel sits at its register limit and its main loop must not pay
 // for this code.
-__device__ __noinline__ void fattn_quant_block(uint8_t *qout, size_t d_offset, int64_t nb, int64_t nbp, int canon, int variant, int64_t n, int64_t b,
+__device__ __noinline__ void fattn_quant_block(uint8_t *qout, size_t d_offset, int64_t nb, int64_t nbp, int variant, int64_t n, int64_t b,
                                                float val, bool real) {
-    if (canon) q8_quantize_store_warp<3>(val, qout, d_offset, nb, nbp, n, b, real, variant);
-    else q8_quantize_store_warp<1>(val, qout, d_offset, nb, nbp, n, b, real, variant);
+    q8_quantize_store_warp<1>(val, qout, d_offset, nb, nbp, n, b, real, variant);
 }
 
 // One output element; a warp calls this for 32 consecutive d of one (token, head).  With QUANT the row is also (or only)
@@ -200,9 +197,9 @@ __device__ __forceinline__ void fattn_store_out(const FattnParams &p, int64_t j,
     }
     if (p.dst) p.dst[(j * p.H + head) * D + d] = val;
     const int64_t b = (head * D + d) >> 5;
-    fattn_quant_block(p.qout, p.q_d_offset, p.q_nb, p.q_nbp, p.q_canon, p.q_variant, j, b, val, true);
+    fattn_quant_block(p.qout, p.q_d_offset, p.q_nb, p.q_nbp, p.q_variant, j, b, val, true);
     if (j == p.Nq - 1) {
-        for (int64_t n = p.Nq; n < ((p.Nq + 7) & ~(int64_t) 7); ++n) fattn_quant_block(p.qout, p.q_d_offset, p.q_nb, p.q_nbp, p.q_canon, p.q_variant, n, b, 0.0f, false);
+        for (int64_t n = p.Nq; n < ((p.Nq + 7) & ~(int64_t) 7); ++n) fattn_quant_block(p.qout, p.q_d_offset, p.q_nb, p.q_nbp, p.q_variant, n, b, 0.0f, false);
     }
 }
 
@@ -732,7 +729,7 @@ static int flash_attn_impl(bool parity, int64_t D, int64_t H, int64_t Hkv, int64
     p.dst = dst; p.partial = (float *) scratch; p.nsplit = ns; p.hgroups = hgroups; p.w0 = w0;
     const ActDims ad = act_dims(H * D, Nq);
     p.qout = (uint8_t *) act; p.q_d_offset = ad.d_offset; p.q_nb = ad.nb; p.q_nbp = ad.nbp;
-    p.q_canon = act_layout(Nq) == 3 ? 1 : 0; p.q_variant = variant;
+    p.q_variant = variant;
     p.order = index ? (const int32_t *) ((const char *) index + index_order_offset(Nq, p.nw)) : nullptr;
     p.plan = index ? (const int32_t *) ((const char *) index + index_plan_offset(Nq, p.nw)) : nullptr;
     p.slots = FA_MIN_CTAS * fa_sm_count();

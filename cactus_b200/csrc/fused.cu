@@ -9,12 +9,9 @@
 
 namespace b200 {
 
-int act_layout(int64_t N);
-
 // One CTA per (padded) token row, one pass: a thread keeps its groups of 4 elements in registers from the load to the
 // quantised store.  The sum of squares is accumulated in the order rms_norm_kernel uses (rms_block_sum), so the
 // scale -- and with it every quantised value -- is bit-identical to the unfused chain.
-template <int LAYOUT>
 // (x, res and h carry no __restrict__: a graph allocator may hand the same memory to the residual and to the normalised output)
 __global__ void __launch_bounds__(1024) add_rms_norm_quantize_kernel(float *x, int64_t x_nb_row, const float *res,
                                                                     int64_t res_nb_row, const float *__restrict__ w, float *h,
@@ -63,12 +60,11 @@ __global__ void __launch_bounds__(1024) add_rms_norm_quantize_kernel(float *x, i
             }
             if (hr) *reinterpret_cast<float4 *>(hr + gi * 4) = make_float4(o[0], o[1], o[2], o[3]);
         }
-        q8_quantize_store<LAYOUT>(o, out, d_offset, nb, nbp, n, gi >> 3, (int) (gi & 7), real, variant);
+        q8_quantize_store<1>(o, out, d_offset, nb, nbp, n, gi >> 3, (int) (gi & 7), real, variant);
     }
 }
 
 // silu(gate) * up, quantised; the same index space as quantize_q8_0_kernel
-template <int LAYOUT>
 __global__ void __launch_bounds__(256) silu_mul_quantize_kernel(const float *gate, const float *up, int64_t nb_row,
                                                                float *dst, int64_t dst_nb_row,
                                                                int64_t N, int64_t n_rows_padded, int64_t nb, int64_t nbp,
@@ -93,7 +89,7 @@ __global__ void __launch_bounds__(256) silu_mul_quantize_kernel(const float *gat
         }
         if (dst) *reinterpret_cast<float4 *>(reinterpret_cast<char *>(dst) + n * dst_nb_row + (b * 32 + j * 4) * 4) = make_float4(v[0], v[1], v[2], v[3]);
     }
-    q8_quantize_store<LAYOUT>(v, out, d_offset, nb, nbp, n, b, j, real, variant);
+    q8_quantize_store<1>(v, out, d_offset, nb, nbp, n, b, j, real, variant);
 }
 
 // One CTA per token: the angles as rope_norm_kernel builds them, q rotated into qo (which may be q itself, with the same
@@ -179,13 +175,8 @@ int b200_add_rms_norm_quantize(float *x, int64_t x_nb_row, const float *residual
     const unsigned threads = rms_threads(d);
     cudaStream_t st = (cudaStream_t) stream;
     const int early = rows <= pdl_early_rows() ? 1 : 0;
-    if (act_layout(rows) == 3) {
-        launch_pdl(add_rms_norm_quantize_kernel<3>, dim3(grid), dim3(threads), 0, st, x, x_nb_row, residual, residual_nb_row, w, h, h_nb_row, d, rows, eps, a.nb, a.nbp,
-                                                                  (uint8_t *) scratch, a.d_offset, variant, early);
-    } else {
-        launch_pdl(add_rms_norm_quantize_kernel<1>, dim3(grid), dim3(threads), 0, st, x, x_nb_row, residual, residual_nb_row, w, h, h_nb_row, d, rows, eps, a.nb, a.nbp,
-                                                                  (uint8_t *) scratch, a.d_offset, variant, early);
-    }
+    launch_pdl(add_rms_norm_quantize_kernel, dim3(grid), dim3(threads), 0, st, x, x_nb_row, residual, residual_nb_row, w, h, h_nb_row, d, rows, eps, a.nb, a.nbp,
+               (uint8_t *) scratch, a.d_offset, variant, early);
     return check_launch("add_rms_norm_quantize");
 }
 
@@ -203,11 +194,7 @@ int b200_silu_mul_quantize(const float *gate, const float *up, int64_t nb_row, f
     const unsigned grid = (unsigned) ((threads + 255) / 256);
     cudaStream_t st = (cudaStream_t) stream;
     const int early = N <= pdl_early_rows() ? 1 : 0;
-    if (act_layout(N) == 3) {
-        launch_pdl(silu_mul_quantize_kernel<3>, dim3(grid), dim3(256), 0, st, gate, up, nb_row, dst, dst_nb_row, N, rows_padded, a.nb, a.nbp, (uint8_t *) scratch, a.d_offset, variant, early);
-    } else {
-        launch_pdl(silu_mul_quantize_kernel<1>, dim3(grid), dim3(256), 0, st, gate, up, nb_row, dst, dst_nb_row, N, rows_padded, a.nb, a.nbp, (uint8_t *) scratch, a.d_offset, variant, early);
-    }
+    launch_pdl(silu_mul_quantize_kernel, dim3(grid), dim3(256), 0, st, gate, up, nb_row, dst, dst_nb_row, N, rows_padded, a.nb, a.nbp, (uint8_t *) scratch, a.d_offset, variant, early);
     return check_launch("silu_mul_quantize");
 }
 

@@ -149,7 +149,7 @@ constexpr int MMQ_PLAIN = 0, MMQ_PEER = 1, MMQ_STREAMK = 2, MMQ_STREAMK_SEG = 3;
 template <int WTYPE, int NTW, int WN, int MT, int WM, int STAGES, int MINB, int MODE = MMQ_PLAIN>
 __global__ void __launch_bounds__(WM * WN * 32, MINB) mmq_kernel(TiledDims dims, const uint8_t *__restrict__ w, ActDims act,
                                                           const uint8_t *__restrict__ aq, float *__restrict__ dst,
-                                                          int64_t dst_nb_row, float *__restrict__ partial, int ksplit, int canon, int cluster, PeerDst peers) {
+                                                          int64_t dst_nb_row, float *__restrict__ partial, int ksplit, int cluster, PeerDst peers) {
     pdl_prologue();
     using S = MmqCfg<WTYPE, NTW, WN, MT, WM, STAGES>;
     constexpr int MMQ_STAGES = STAGES;
@@ -358,14 +358,8 @@ __global__ void __launch_bounds__(WM * WN * 32, MINB) mmq_kernel(TiledDims dims,
             }
             const int ntl = wn * NTW + 2 * np;
             uint2 b0, b1;
-            if (canon) {   // activations kept as two 8-column x 16-byte core matrices per block (the tcgen05 kernel's order)
-                const uint8_t *q0 = Bs + ntl * 1024 + j * 256 + g * 16 + t * 4, *q1 = q0 + 1024;
-                b0 = make_uint2(*reinterpret_cast<const uint32_t *>(q0), *reinterpret_cast<const uint32_t *>(q0 + 128));
-                b1 = make_uint2(*reinterpret_cast<const uint32_t *>(q1), *reinterpret_cast<const uint32_t *>(q1 + 128));
-            } else {
-                b0 = reinterpret_cast<const uint2 *>(Bs + ntl * 1024 + j * 256)[lane];
-                b1 = reinterpret_cast<const uint2 *>(Bs + (ntl + 1) * 1024 + j * 256)[lane];
-            }
+            b0 = reinterpret_cast<const uint2 *>(Bs + ntl * 1024 + j * 256)[lane];
+            b1 = reinterpret_cast<const uint2 *>(Bs + (ntl + 1) * 1024 + j * 256)[lane];
             sc[buf][0] = *reinterpret_cast<const uint2 *>(Ss + ntl * 256 + (j * 4 + t) * 16);
             sc[buf][1] = *reinterpret_cast<const uint2 *>(Ss + (ntl + 1) * 256 + (j * 4 + t) * 16);
 #pragma unroll
@@ -652,9 +646,9 @@ struct MmqVariant {
     int cta_tiles;   // 16-row tiles per CTA
     int cta_nt;      // 8-column tiles per CTA
     int ctas_per_sm; // resident CTAs per SM (filled on first use)
-    int (*launch)(const TiledDims &, const uint8_t *, const ActDims &, const uint8_t *, float *, int64_t, float *, int, int, int, const PeerDst &, cudaStream_t);
+    int (*launch)(const TiledDims &, const uint8_t *, const ActDims &, const uint8_t *, float *, int64_t, float *, int, int, const PeerDst &, cudaStream_t);
     int (*max_clusters)(int);   // resident clusters of `ksplit` CTAs on this device (0 = cannot be launched that way)
-    int (*launch_streamk)(const TiledDims &, const uint8_t *, const ActDims &, const uint8_t *, float *, int64_t, void *, int, int, int, const PeerDst &, cudaStream_t);
+    int (*launch_streamk)(const TiledDims &, const uint8_t *, const ActDims &, const uint8_t *, float *, int64_t, void *, int, int, const PeerDst &, cudaStream_t);
     size_t streamk_slot_bytes;  // one partial tile of a CTA in the stream-K workspace
 };
 
@@ -670,27 +664,27 @@ static size_t streamk_counter_bytes(int64_t n_groups) { return (size_t) ((n_grou
 // the block groups of a head in the head/tail deal
 template <int WTYPE, int NTW, int WN, int MT, int WM, int STAGES, int MINB>
 static int launch_variant_streamk(const TiledDims &d, const uint8_t *w, const ActDims &a, const uint8_t *aq, float *dst, int64_t dst_nb_row,
-                                  void *workspace, int ctas, int head, int canon, const PeerDst &segs, cudaStream_t st) {
+                                  void *workspace, int ctas, int head, const PeerDst &segs, cudaStream_t st) {
     using S = MmqCfg<WTYPE, NTW, WN, MT, WM, STAGES>;
     const int n_groups = (int) (d.n_rt / S::CTA_TILES);
     launch_pdl(zero_u32_kernel, dim3((unsigned) ((n_groups + 255) / 256)), dim3(256), 0, st, (unsigned *) workspace, n_groups);
     if (int e = check_launch("mmq stream-K counters")) return e;
     if (segs.n_seg > 1) launch_pdl(mmq_kernel<WTYPE, NTW, WN, MT, WM, STAGES, MINB, MMQ_STREAMK_SEG>, dim3((unsigned) ctas), dim3(S::THREADS), S::TOTAL, st, d, w, a,
-                                   aq, dst, dst_nb_row, (float *) workspace, head, canon, 0, segs);   // segs: row ranges only, never peers
+                                   aq, dst, dst_nb_row, (float *) workspace, head, 0, segs);   // segs: row ranges only, never peers
     else launch_pdl(mmq_kernel<WTYPE, NTW, WN, MT, WM, STAGES, MINB, MMQ_STREAMK>, dim3((unsigned) ctas), dim3(S::THREADS), S::TOTAL, st, d, w, a, aq, dst,
-                    dst_nb_row, (float *) workspace, head, canon, 0, PeerDst{});
+                    dst_nb_row, (float *) workspace, head, 0, PeerDst{});
     return check_launch("mmq stream-K");
 }
 
 template <int WTYPE, int NTW, int WN, int MT, int WM, int STAGES, int MINB>
 static int launch_variant(const TiledDims &d, const uint8_t *w, const ActDims &a, const uint8_t *aq, float *dst, int64_t dst_nb_row,
-                          float *partial, int ksplit, int canon, int cluster, const PeerDst &peers, cudaStream_t st) {
+                          float *partial, int ksplit, int cluster, const PeerDst &peers, cudaStream_t st) {
     using S = MmqCfg<WTYPE, NTW, WN, MT, WM, STAGES>;
     dim3 grid((unsigned) ((d.n_rt + S::CTA_TILES - 1) / S::CTA_TILES), (unsigned) ((a.n_nt + S::NT - 1) / S::NT), (unsigned) ksplit);
     const bool peer = peers.n > 0 || peers.n_seg > 1;
     if (!cluster) {
-        if (peer) launch_pdl(mmq_kernel<WTYPE, NTW, WN, MT, WM, STAGES, MINB, MMQ_PEER>, grid, dim3(S::THREADS), S::TOTAL, st, d, w, a, aq, dst, dst_nb_row, partial, ksplit, canon, 0, peers);
-        else launch_pdl(mmq_kernel<WTYPE, NTW, WN, MT, WM, STAGES, MINB, MMQ_PLAIN>, grid, dim3(S::THREADS), S::TOTAL, st, d, w, a, aq, dst, dst_nb_row, partial, ksplit, canon, 0, peers);
+        if (peer) launch_pdl(mmq_kernel<WTYPE, NTW, WN, MT, WM, STAGES, MINB, MMQ_PEER>, grid, dim3(S::THREADS), S::TOTAL, st, d, w, a, aq, dst, dst_nb_row, partial, ksplit, 0, peers);
+        else launch_pdl(mmq_kernel<WTYPE, NTW, WN, MT, WM, STAGES, MINB, MMQ_PLAIN>, grid, dim3(S::THREADS), S::TOTAL, st, d, w, a, aq, dst, dst_nb_row, partial, ksplit, 0, peers);
         return check_launch("mmq");
     }
     cudaLaunchConfig_t cfg = {};
@@ -707,16 +701,17 @@ static int launch_variant(const TiledDims &d, const uint8_t *w, const ActDims &a
     attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = pdl_enabled() ? 2 : 1;
-    cudaError_t e = peer ? cudaLaunchKernelEx(&cfg, mmq_kernel<WTYPE, NTW, WN, MT, WM, STAGES, MINB, MMQ_PEER>, d, w, a, aq, dst, dst_nb_row, partial, ksplit, canon, 1, peers)
-                         : cudaLaunchKernelEx(&cfg, mmq_kernel<WTYPE, NTW, WN, MT, WM, STAGES, MINB, MMQ_PLAIN>, d, w, a, aq, dst, dst_nb_row, partial, ksplit, canon, 1, peers);
+    cudaError_t e = peer ? cudaLaunchKernelEx(&cfg, mmq_kernel<WTYPE, NTW, WN, MT, WM, STAGES, MINB, MMQ_PEER>, d, w, a, aq, dst, dst_nb_row, partial, ksplit, 1, peers)
+                         : cudaLaunchKernelEx(&cfg, mmq_kernel<WTYPE, NTW, WN, MT, WM, STAGES, MINB, MMQ_PLAIN>, d, w, a, aq, dst, dst_nb_row, partial, ksplit, 1, peers);
     if (e != cudaSuccess) return set_error(B200_E_CUDA, "mmq cluster launch: %s", cudaGetErrorString(e));
     count_launch();
     return B200_OK;
 }
 
-template <int WTYPE, int NTW, int WN, int MT, int WM, int STAGES, int MINB>
+template <int WTYPE, int NTW, int WN, int MT, int WM, int STAGES, int MINB, int MODEL>
 static int max_clusters_variant(int ksplit) {
     using S = MmqCfg<WTYPE, NTW, WN, MT, WM, STAGES>;
+    constexpr int MODEL_SMEM = 227 * 1024 / (MODEL + 1);   // with more than this, MODEL CTAs fit and not one more
     static int cache[64][9];   // per device and cluster size: 0 = not asked yet, -1 = none, else the count
     static std::mutex mu;
     int dev = 0;
@@ -728,7 +723,7 @@ static int max_clusters_variant(int ksplit) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(1, 1, (unsigned) ksplit);
     cfg.blockDim = dim3(S::THREADS);
-    cfg.dynamicSmemBytes = S::TOTAL;
+    cfg.dynamicSmemBytes = S::TOTAL > MODEL_SMEM ? S::TOTAL : MODEL_SMEM;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeClusterDimension;
     attr[0].val.clusterDim.x = 1;
@@ -745,26 +740,29 @@ static int max_clusters_variant(int ksplit) {
     return n;
 }
 
-template <int WTYPE, int NTW, int WN, int MT, int WM, int STAGES = 4, int MINB = 1>
+// MODEL: the CTAs per SM that the split model (choose_ksplit, streamk_ctas) counts with, where they are fewer than fit.  How K is
+// split is part of the result's last bits, so the split of a shape does not follow a change in register use.
+template <int WTYPE, int NTW, int WN, int MT, int WM, int STAGES = 4, int MINB = 1, int MODEL = 8>
 static MmqVariant make_variant() {
     using S = MmqCfg<WTYPE, NTW, WN, MT, WM, STAGES>;
     MmqVariant v;
     v.cta_tiles = S::CTA_TILES;
     v.cta_nt = S::NT;
     v.launch = launch_variant<WTYPE, NTW, WN, MT, WM, STAGES, MINB>;
-    v.max_clusters = max_clusters_variant<WTYPE, NTW, WN, MT, WM, STAGES, MINB>;
+    v.max_clusters = max_clusters_variant<WTYPE, NTW, WN, MT, WM, STAGES, MINB, MODEL>;
     v.launch_streamk = launch_variant_streamk<WTYPE, NTW, WN, MT, WM, STAGES, MINB>;
     v.streamk_slot_bytes = (size_t) S::CTA_TILES * 16 * S::NT * 8 * sizeof(float);
     cudaFuncSetAttribute(mmq_kernel<WTYPE, NTW, WN, MT, WM, STAGES, MINB, MMQ_STREAMK>, cudaFuncAttributeMaxDynamicSharedMemorySize, S::TOTAL);
     cudaFuncSetAttribute(mmq_kernel<WTYPE, NTW, WN, MT, WM, STAGES, MINB, MMQ_STREAMK_SEG>, cudaFuncAttributeMaxDynamicSharedMemorySize, S::TOTAL);
-    cudaFuncSetAttribute(mmq_kernel<WTYPE, NTW, WN, MT, WM, STAGES, MINB, MMQ_PLAIN>, cudaFuncAttributeMaxDynamicSharedMemorySize, S::TOTAL);
+    cudaFuncSetAttribute(mmq_kernel<WTYPE, NTW, WN, MT, WM, STAGES, MINB, MMQ_PLAIN>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                         S::TOTAL > 227 * 1024 / (MODEL + 1) ? S::TOTAL : 227 * 1024 / (MODEL + 1));   // (the residency query asks for that much)
     cudaFuncSetAttribute(mmq_kernel<WTYPE, NTW, WN, MT, WM, STAGES, MINB, MMQ_PEER>, cudaFuncAttributeMaxDynamicSharedMemorySize, S::TOTAL);
     int n = 0;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, mmq_kernel<WTYPE, NTW, WN, MT, WM, STAGES, MINB>, S::THREADS, S::TOTAL) != cudaSuccess || n <= 0) {
         cudaGetLastError();
         n = 1;
     }
-    v.ctas_per_sm = n;
+    v.ctas_per_sm = n < MODEL ? n : MODEL;
     return v;
 }
 
@@ -786,7 +784,7 @@ static const MmqVariant &pick_variant(int64_t N) {
     std::lock_guard<std::mutex> lock(mu);
     if (!ready[dev]) {
         MmqVariant(*t)[4] = table[dev];
-        t[0][0] = make_variant<WTYPE, 2, 1, 2, 4>();   // 128 rows x 16 cols, 4 warps
+        t[0][0] = make_variant<WTYPE, 2, 1, 2, 4, 4, 1, 3>();   // 128 rows x 16 cols, 4 warps
         t[0][1] = make_variant<WTYPE, 2, 1, 1, 4>();   //  64 rows x 16 cols
         t[0][2] = t[0][0]; t[0][3] = t[0][0];
         t[1][0] = make_variant<WTYPE, 4, 1, 2, 4>();   // 128 rows x 32 cols
@@ -861,6 +859,13 @@ int mmvq_max_n() {
     return v;
 }
 
+// The tuning switches of this kernel (B200_MMQ_STREAMK, _VARIANT, _CLASS, _CLUSTER) also select it where the tcgen05 kernel
+// would run otherwise.
+bool mmq_sync_forced() {
+    static const bool v = getenv("B200_MMQ_STREAMK") || getenv("B200_MMQ_VARIANT") || getenv("B200_MMQ_CLASS") || getenv("B200_MMQ_CLUSTER");
+    return v;
+}
+
 size_t mmq_workspace_bytes(int wtype, int64_t K, int64_t M, int64_t N) {
     if (N <= 2) return 0;   // never the tensor-core kernel (mmvq_max_n() is 2 ... 8: columns 3..8 may need it)
     // upper bound over every K split the launcher may choose (the choice depends on the device): never more
@@ -917,7 +922,7 @@ void launch_mmq_reduce(const float *partial, int ks, int64_t M, int64_t N, float
 }
 
 int launch_mmq(int wtype, const TiledDims &d, const void *w, const ActDims &a, const void *aq, float *dst, int64_t dst_nb_row,
-               void *workspace, size_t workspace_bytes, cudaStream_t st, bool canon, const PeerDst &peers) {
+               void *workspace, size_t workspace_bytes, cudaStream_t st, const PeerDst &peers) {
     const MmqVariant &v = variant_for(wtype, a.N);
     bool cluster = false;
     int ks = choose_ksplit(v, d, a.n_nt, &cluster);
@@ -928,9 +933,9 @@ int launch_mmq(int wtype, const TiledDims &d, const void *w, const ActDims &a, c
     if (peers.n == 0 && (peers.n_seg <= 1 || peers.n_wseg > 0) && workspace) {   // (the ranges of a row-split rank keep the plain grid)
         int head = 0;
         if (const int ctas = streamk_ctas(v, d, a, ks, cluster, workspace_bytes, &head))
-            return v.launch_streamk(d, (const uint8_t *) w, a, (const uint8_t *) aq, dst, dst_nb_row, workspace, ctas, head, canon ? 1 : 0, peers, st);
+            return v.launch_streamk(d, (const uint8_t *) w, a, (const uint8_t *) aq, dst, dst_nb_row, workspace, ctas, head, peers, st);
     }
-    if (int e = v.launch(d, (const uint8_t *) w, a, (const uint8_t *) aq, dst, dst_nb_row, (float *) workspace, ks, canon ? 1 : 0, cluster ? 1 : 0, peers, st)) return e;
+    if (int e = v.launch(d, (const uint8_t *) w, a, (const uint8_t *) aq, dst, dst_nb_row, (float *) workspace, ks, cluster ? 1 : 0, peers, st)) return e;
     if (ks > 1 && !cluster) {
         const int64_t total = d.M * a.N;
         launch_pdl(mmq_reduce_kernel, dim3((unsigned) ((total + 255) / 256)), dim3(256), 0, st, (const float *) workspace, ks, d.M, a.N, dst, dst_nb_row, peers);

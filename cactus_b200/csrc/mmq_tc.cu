@@ -1,51 +1,53 @@
-// MUL_MAT for a batch of activation columns on the 5th-generation tensor cores (tcgen05, TMEM accumulators).
+// MUL_MAT for a batch of activation columns on the 5th-generation tensor cores, with the block scales folded into the
+// operands so that one accumulator in tensor memory runs over K.
 //
-// Same arithmetic as mmq.cu (lm_ggml_compute_forward_mul_mat, cactus/ggml-cpu/ggml-cpu.c:1257-1449): one exact integer
-// dot product per 32-element block, then d_w[row] * d_a[col] scaling into fp32 accumulators.  What differs is where the
-// work runs:
-//   * The integer dot is computed by tcgen05.mma.kind::f8f6f4 on e4m3 operands that hold small integers.  The
-//     subnormals and the first binade of e4m3 are the integers 0..15 times 2^-9, so a weight nibble u = q + 8, zero
-//     extended to a byte, already *is* the e4m3 encoding of u * 2^-9: expanding the packed weights is a mask and an
-//     XOR.  An activation quant a = 16 h + l (h = a >> 4, l = a & 15) is two e4m3 bytes (h * 2^-5 and l * 2^-9, planes
-//     written by the quantiser), multiplied by two MMAs that accumulate.  Every product and every partial sum is an
-//     integer below 2^17 times 2^-18, so the fp32 accumulator holds the exact value of sum(u a) * 2^-18: the block dot
-//     stays bit-exact, and it arrives as a float -- no int -> float conversion in the epilogue.
-//   * sum(q a) = sum(u a) - 8 sum(a); the quantiser stores D = d_a * 2^18 and C = -8 d_a sum(a) per (column, block), so
-//     t = fma(v, D, C) = d_a * dot and y = fma(t, d_w, y) are the only two operations per value and block, issued as
-//     fma.rn.f32x2 on column pairs.
-//   * The expanded weights never touch shared memory: a thread owns one weight row, expands 4 blocks of it in registers
-//     and writes them into tensor memory (tcgen05.st), from where the MMA reads its A operand.
+// lm_ggml_compute_forward_mul_mat (cactus/ggml-cpu/ggml-cpu.c:1257-1449) computes, per output value,
+// sum over blocks b of d_w[row, b] * d_a[col, b] * dot_b with dot_b an integer.  Scaling after every block (mmq.cu) costs a
+// pass over the accumulator tile per 32 values of K; here the scales go into the operands instead:
+//   A[row, k] = d_w[row, b] * q[row, k]      (15 significant bits for Q4_0, 19 for Q8_0: 11 of the fp16 scale and the quant)
+//   B[col, k] = d_a[col, b] * a[col, k]      (19 significant bits)
+// Each is an fp16 value plus the exact fp16 remainder (x_hi = rn(x), x_lo = x - x_hi; d is a multiple of 2^-24, so the
+// remainder always fits), and the product is A_hi B_hi + A_hi B_lo + A_lo B_hi (the missing A_lo B_lo is below 2^-22 of a
+// term), accumulated in fp32 by tcgen05.mma.kind::f16.  Nothing is rounded that the reference does not round, except the
+// order of the fp32 sums.  The tensor core truncates when it accumulates, so the accumulator is emptied into shared
+// memory every TC_FLUSH block groups and the small terms (A_hi B_lo, A_lo B_hi) have columns of their own.
+// A value beyond the fp16 range (|d q| > 65504) makes the sum non-finite; such results are recomputed exactly from the
+// integers (tc_exact_value).
 //
-// A CTA (one per SM, 20 warps with fixed roles, joined by mbarriers only) owns 128 weight rows x up to 64 columns and
-// walks K in groups of 4 blocks:
-//   warps 0-3   MMA issue: warp w issues block w of every group -- two MMAs of 128 x 64 x 32 (hi plane, then lo plane
-//               accumulating) -- so the accumulator tiles in flight turn over independently of each other;
-//   warp 4      producer: five TMA tensor copies per group into a ring of stages -- the packed T16 weight tiles (one
-//               box of 8 row tiles, written with the 128-byte swizzle so that the row-per-thread reads below are
-//               conflict free), their fp16 scales, the two e4m3 activation planes and the activation scales;
-//   warps 8-11  expand: thread = weight row; four 16-byte loads give the row's 4 blocks, 32 registers go to TMEM;
-//   warps 12-19 epilogue: one per (TMEM lane quarter, 32-column half).  Accumulator tiles are read in the MMA fragment
-//               order (16x256b: a thread holds 4 rows x 4 column pairs of a block, so a 16-byte load of column scales
-//               serves 4 rows), the tile of block b+1 is in flight while block b is scaled.
-// Tensor memory: six accumulator tiles of one block (64 columns each) and four A buffers of 4 blocks (32 columns each).
+// What bounds it: the MMAs.  128 x 128 x 16 + 128 x 64 x 16 per 16 values of K take 96 clk (measured: N / 2 clk per MMA), so a
+// block group of 256 rows x 64 columns x 128 values takes 1542 clk; the kernel runs at 1800 (two row tiles), and a CTA needs
+// about 5 us to fill and empty its pipeline.  What is around the MMAs has to stay below that:
+//   * the activations arrive as B_hi / B_lo planes written once by the quantiser (act_dims: b_offset) in the core-matrix
+//     order of the MMA's B descriptor.  A CTA owns 256 weight rows (two MMA row tiles) per activation copy: 50 KB per
+//     block group, 33 B/clk per SM, below the 40 B/clk that bulk copies out of L2 reach with all SMs at it.  One copy brings
+//     all of it (a bulk copy costs its thread 75 clk, so 2 KB pieces bounded an earlier form);
+//   * the weights are turned into fp16 in registers and go straight into tensor memory (the MMA's A operand): three half2
+//     operations (2 clk each on this GPU) and 1.5 logic operations per pair of values, 768 clk per block group.  T16 tiles are
+//     in MMA fragment order, which is what tcgen05.st.16x128b takes: lane (g, t) stores the words of rows g and g + 8 as it
+//     loaded them, so there is no transposition; the order of K within a block that follows from it is the order the
+//     quantiser writes B in;
+//   * every hand-over between warps is some twenty instructions at 10-16 clk each beside busy warps, so there are few: one per
+//     half block group and role, with an A stage for each team of weight warps.
+//
+// Roles of a CTA (one per SM, 24 or 32 warps): warps 0 and 1 issue the MMAs of one row tile each, warp 2 the copies (a ring of
+// stages of one block group), two or three teams of 8 warps convert weights (the teams take the half block groups in turn; a
+// warp: 32 rows), the last four warps move the accumulators to shared memory and write results.  The two row tiles share the
+// copies only: each has its own A stages, accumulator and barriers.  Code that runs once per tile is kept small and in loops:
+// with 172 KB of (unrolled, inlined) code the kernel spent most of its time on instruction cache misses.
+//
+// Work split (TcPlan): clusters of up to 8 CTAs share the K range of one tile (256 rows x <= 64 columns) and add their parts
+// through distributed shared memory in rank order; or, when there are many tiles, one CTA per SM takes an equal and
+// contiguous share of all (tile, block group) iterations, and a tile that two or three CTAs share is added by the CTA that
+// arrives last, in K order (parts parked in the workspace; a counter per tile), so sums do not depend on timing.
+//
+// Measured against the mma.sync kernel: the table at use_tc (mul_mat.cu).
 // Every wait is bounded; on time-out the CTA raises b200_kernel_status, all roles fall through, the producer waits
-// (bounded) for its copies in flight, the issuing warps for their MMAs, the CTA frees its TMEM and returns.
-//
-// Measured on B200 (probes run on this pool; the figures that shaped the kernel and that bound it today):
-//   * tcgen05.mma 128 x 64 x 32, e4m3 or s8, issued back to back: 48.6 clk with A in shared memory, 45.5 clk with A in
-//     TMEM (the shared-memory operand fetch, not the 32 clk of arithmetic, sets the pace); 128 x 128 x 32: 64.6 clk = 8117
-//     MAC/clk/SM; s8 and e4m3 run at the same rate.  Integer-valued e4m3 operands accumulate exactly (0 mismatches in
-//     8192 dots including the extreme values).
-//   * a hand-over between warps costs 230-280 clk whatever the mechanism (mbarrier try_wait / test_wait, a polled
-//     shared-memory counter, bar.sync / bar.arrive all measured 460-560 clk per round trip), and a wait costs the
-//     waiting warp well over a hundred cycles even when the phase is already complete;
-//   * tcgen05.ld moves 253 B/clk/SM in the 16x256b shape, 476 in 16x128b, 652 in 32x32b;
-//   * a 16-byte shared-memory load whose lanes share 4 addresses occupies the SM's load unit for about 6 clk.
-// With one block (92 clk of MMA, 128 clk of FP32 work) as the unit that is handed from role to role, those costs add
-// up to about 2900 clk per group of 4 blocks where the mma.sync kernel needs 2700: the kernel passes every parity
-// case but is not the default (B200_MMQ_TC=1 selects it).
+// (bounded) for its copies in flight, the issuing warp for its MMAs, the CTA frees its tensor memory and returns.
 #include <cuda.h>
+#include <cuda_fp16.h>
 
+#include <atomic>
+#include <chrono>
 #include <cstdlib>
 #include <mutex>
 #include <unordered_map>
@@ -54,52 +56,58 @@
 
 namespace b200 {
 
-void launch_mmq_reduce(const float *partial, int ks, int64_t M, int64_t N, float *dst, int64_t dst_nb_row, cudaStream_t st);
-int launch_mmq(int wtype, const TiledDims &d, const void *w, const ActDims &a, const void *aq, float *dst, int64_t dst_nb_row,
-               void *workspace, size_t workspace_bytes, cudaStream_t st, bool canon, const PeerDst &peers);
-
-__device__ int g_tc_error = 0;   // non-zero after a bounded wait gave up
+__device__ int g_tc_error = 0;                    // non-zero after a bounded wait gave up
 __device__ unsigned g_tc_spin_limit = 1u << 20;   // try_wait rounds before a wait gives up (each may suspend for a while)
 constexpr uint32_t TC_DRAIN_LIMIT = 1u << 22;     // what a CTA that gave up still waits for: its own copies and MMAs in flight
-#ifdef B200_TC_PROFILE
-__device__ long long g_tc_prof[4][64];   // [role][iteration]: clock of CTA 0 when the role starts work on an iteration
-#define TC_PROF(role, it) do { if (blockIdx.x == 0 && blockIdx.z == 0 && lane == 0 && (it) < 64) g_tc_prof[role][it] = clock64(); } while (0)
-#else
-#define TC_PROF(role, it) do { } while (0)
-#endif
 
-constexpr int TC_THREADS = 640;   // 20 warps: 0-3 MMA issue, 4 producer (5-7 idle), 8-11 expand, 12-19 epilogue
-constexpr int TC_STAGES = 6;
-constexpr int TC_ROWS = 128, TC_COLS = 64;
-constexpr int TC_WQ = 8 * 1024, TC_WD = 8 * 128, TC_BH = 8 * 1024, TC_BL = 8 * 1024, TC_BS = 8 * 256;
-constexpr int TC_OFF_WD = TC_WQ, TC_OFF_BH = TC_OFF_WD + TC_WD, TC_OFF_BL = TC_OFF_BH + TC_BH, TC_OFF_BS = TC_OFF_BL + TC_BL;
-constexpr int TC_STAGE = TC_OFF_BS + TC_BS;   // 27648 = 27 * 1024: every stage starts on a swizzle-pattern boundary
-constexpr int TC_BAR_OFFSET = TC_STAGES * TC_STAGE;
-constexpr int TC_ACC = 6;    // accumulator tiles (one block each, 64 TMEM columns)
-constexpr int TC_ABUF = 4;   // A buffers (the 4 blocks of a group each, 32 TMEM columns)
-constexpr int TC_ISSUE_WARPS = 4, TC_EXP_WARPS = 4, TC_EPI_WARPS = 8;
-// barriers (8 bytes each)
-constexpr int BAR_FULL = 0, BAR_EMPTY = TC_STAGES, BAR_A_FULL = 2 * TC_STAGES, BAR_A_FREE = BAR_A_FULL + TC_ABUF, BAR_ACC_FULL = BAR_A_FREE + TC_ABUF,
-              BAR_ACC_FREE = BAR_ACC_FULL + TC_ACC, BAR_DRAIN = BAR_ACC_FREE + TC_ACC, TC_N_BARS = BAR_DRAIN + TC_ISSUE_WARPS;
-constexpr int TC_SMEM = TC_BAR_OFFSET + TC_N_BARS * 8 + 32;
-constexpr uint32_t TC_A_COL = 64 * TC_ACC;   // TMEM columns 0..383: accumulators, 384..511: A buffers
+constexpr int TC_RT = 16;            // 16-row tiles of a CTA at most: 256 rows, two MMA row tiles
+constexpr int TC_FLUSH = 16;         // block groups accumulated in tensor memory before they are added up in shared memory
+constexpr int TC_EPI_THREADS = 128;
 
-struct TcMaps {
-    CUtensorMap wq, wd, bh, bl, bs;
+// Geometry for up to NT tiles of 8 activation columns per CTA.
+template <int WTYPE, int NT>
+struct TcCfg {
+    static constexpr int WT = WTYPE == B200_TYPE_Q4_0 ? 1024 : 2048;   // one row tile, one block group
+    static constexpr int OFF_S = TC_RT * WT;                           // its scales: 128 bytes per row tile
+    static constexpr int OFF_B = OFF_S + TC_RT * 128;                  // B_hi: 2 KB per column tile, then B_lo
+    static constexpr int STAGE = OFF_B + NT * 4096;
+    static constexpr int ACC = NT * 8 * 1024;                          // partial results, f32 [column][256 rows]
+    static constexpr int FIT = (232448 - 6144 - ACC) / STAGE;
+    static constexpr int STAGES = FIT > 8 ? 8 : FIT;
+    // tensor memory of row tile mt: an accumulator of 2 x 8 NT columns (hi | small terms) at mt * D_MT, ABUF A stages of half a block
+    // group (32 columns of A_hi, 32 of A_lo) at A_COL + mt * A_MT
+    static constexpr int D_MT = 16 * NT;
+    static constexpr int ABUF = NT < 8 ? 3 : 2;
+    static constexpr int A_MT = ABUF * 64, A_COL = 512 - 2 * A_MT;
+    // warps: 4 for MMAs and copies, a team of 8 weight warps per A stage (each waits for its own stage phase after phase, which a
+    // parity wait can tell apart), 4 for the write-back
+    static constexpr int WARP_EPI = 4 + 8 * ABUF, THREADS = 32 * (WARP_EPI + 4);
+    // barriers: FULL a stage has landed; WREAD its weights are in registers; DONE (per row tile) all MMAs on it are complete; AFULL /
+    // AFREE (row tile, A stage); ACCF the accumulator is complete, ACCE it has been read
+    static constexpr int B_FULL = 0, B_WREAD = STAGES, B_DONE = 2 * STAGES, B_AFULL = 4 * STAGES, B_AFREE = B_AFULL + 2 * ABUF, B_ACCF = B_AFREE + 2 * ABUF,
+                         B_ACCE = B_ACCF + 2, B_DRAIN = B_ACCE + 2, N_BARS = B_DRAIN + 2;
+    static constexpr int OFF_ACC = STAGES * STAGE;
+    static constexpr int BAR_OFFSET = OFF_ACC + ACC;
+    static constexpr int SH_OFFSET = BAR_OFFSET + (N_BARS * 8 + 15) / 16 * 16;   // TcShared
+    static constexpr int SMEM = SH_OFFSET + 5120;
+    static_assert(STAGE % 1024 == 0 && SMEM <= 232448 && 2 * D_MT <= A_COL && STAGES >= 2, "shared / tensor memory of an SM");
 };
 
-__device__ __forceinline__ uint64_t tc_pack2(uint32_t lo, uint32_t hi) {
-    uint64_t r;
-    asm("mov.b64 %0, {%1,%2};" : "=l"(r) : "r"(lo), "r"(hi));
-    return r;
-}
-__device__ __forceinline__ uint64_t tc_fma2(uint64_t a, uint64_t b, uint64_t c) {
-    uint64_t r;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-    return r;
-}
-// K-major, no swizzle: core matrices of 8 rows x 16 bytes; lbo = byte step between the two core matrices along K,
-// sbo = byte step between 8-row groups
+// How the iterations are dealt out (see the head comment).
+struct TcPlan {
+    int rt_per_group;   // row tiles of a CTA: 16 or 8
+    int groups, chunks; // row groups, column chunks; tile = group * chunks + chunk
+    int cs;             // > 0: clusters of cs CTAs, one tile per cluster; 0: equal shares over gridDim.x CTAs
+    unsigned long long launch_id;   // equal shares: marks the arrival counters (56 bits)
+    uint32_t share, extra;   // equal shares: CTA j takes share iterations, one more if j < extra
+    int debug;          // 32: the producer copies nothing (the test of the give-up path)
+};
+// The weights as tensor maps: 1 KB (2 KB) tiles and 128-byte scale tiles of one block group, 8 row tiles (128 rows) per copy.
+// Row ranges that come from separate tensors (PeerDst::wseg) have a pair of maps each.
+struct TcMaps {
+    CUtensorMap q[3], s[3];
+};
+
 __device__ __forceinline__ uint64_t tc_smem_desc(uint32_t addr, uint32_t lbo, uint32_t sbo) {
     return (uint64_t) ((addr >> 4) & 0x3FFF) | ((uint64_t) ((lbo >> 4) & 0x3FFF) << 16) | ((uint64_t) ((sbo >> 4) & 0x3FFF) << 32) | (1ull << 46);
 }
@@ -108,16 +116,19 @@ __device__ __forceinline__ bool tc_try(uint32_t bar, uint32_t parity) {
     asm volatile("{\n.reg .pred p;\nmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\nselp.u32 %0, 1, 0, p;\n}\n" : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
     return ok != 0;
 }
-// Bounded wait of a whole (converged) warp.  A barrier operation costs the issuing warp more than a hundred cycles even
-// when the phase is already complete, and those cycles add up within a warp, so a warp that needs several barriers at once
-// hands one to each of its first lanes: lane i < n waits for (bar[i], parity[i]), the others pass true.  false = gave up
-// (or the CTA already gave up elsewhere).
-__device__ __forceinline__ bool tc_wait_lanes(bool mine, uint32_t bar, uint32_t parity, volatile int *abort_flag, uint32_t limit) {
-    bool ok = !mine || tc_try(bar, parity);
-    if (__all_sync(0xffffffffu, ok)) return true;
+// One lane of a converged warp.  What is issued under this predicate takes its operands from uniform registers: 22 clk per
+// tcgen05.mma and 45 per commit, against 56 and 120 behind a lane number compare (measured; 75 against 107 beside busy warps).
+__device__ __forceinline__ bool tc_elect() {
+    uint32_t el;
+    asm volatile("{\n.reg .pred p;\nelect.sync _|p, 0xffffffff;\nselp.u32 %0, 1, 0, p;\n}\n" : "=r"(el));
+    return el != 0;
+}
+// Bounded wait of a whole (converged) warp; false = gave up (or the CTA already gave up elsewhere).  The loop is one function
+// for all callers: the kernel's hot code has to fit the instruction cache.
+__device__ __noinline__ bool tc_wait_slow(uint32_t bar, uint32_t parity, volatile int *abort_flag, uint32_t limit) {
+#pragma unroll 1
     for (uint32_t i = 0; i < limit; ++i) {
-        if (!ok) ok = tc_try(bar, parity);
-        if (__all_sync(0xffffffffu, ok)) return true;
+        if (tc_try(bar, parity)) return true;
         if ((i & 15u) == 15u && *abort_flag) return false;
     }
     *abort_flag = 1;
@@ -125,7 +136,7 @@ __device__ __forceinline__ bool tc_wait_lanes(bool mine, uint32_t bar, uint32_t 
     return false;
 }
 __device__ __forceinline__ bool tc_wait(uint32_t bar, uint32_t parity, volatile int *abort_flag, uint32_t limit) {
-    return tc_wait_lanes(true, bar, parity, abort_flag, limit);
+    return tc_try(bar, parity) || tc_wait_slow(bar, parity, abort_flag, limit);
 }
 __device__ __forceinline__ void tc_arrive(uint32_t bar) { asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];\n" ::"r"(bar) : "memory"); }
 __device__ __forceinline__ void tc_commit(uint32_t bar) {
@@ -139,286 +150,564 @@ __device__ __forceinline__ void tc_tma_3d(uint32_t dst, const CUtensorMap *map, 
     asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];\n"
                  ::"r"(dst), "l"(map), "r"(x), "r"(y), "r"(z), "r"(bar) : "memory");
 }
-// D[tmem] (+)= A[tmem] * B[smem], 128 x 64 x 32, e4m3 x e4m3 -> f32
-__device__ __forceinline__ void tc_mma_f8_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
-    asm volatile("{\n.reg .pred p;\nsetp.ne.b32 p, %4, 0;\ntcgen05.mma.cta_group::1.kind::f8f6f4 [%0], [%1], %2, %3, p;\n}\n"
+__device__ __forceinline__ void tc_copy(uint32_t dst, const void *src, uint32_t bytes, uint32_t bar) {
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];\n" ::"r"(dst), "l"(src), "r"(bytes), "r"(bar) : "memory");
+}
+// D[tmem] (+)= A[tmem] * B[smem], M 128, K 16, fp16 x fp16 -> f32; N comes with the instruction descriptor
+__device__ __forceinline__ void tc_mma(uint32_t d_tmem, uint32_t a_tmem, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
+    asm volatile("{\n.reg .pred p;\nsetp.ne.b32 p, %4, 0;\ntcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n}\n"
                  ::"r"(d_tmem), "r"(a_tmem), "l"(bdesc), "r"(idesc), "r"(accumulate) : "memory");
 }
+__device__ __forceinline__ uint32_t tc_h2(__half2 v) { return *reinterpret_cast<uint32_t *>(&v); }
+__device__ __forceinline__ __half2 tc_as_h2(uint32_t v) { return *reinterpret_cast<__half2 *>(&v); }
+// 16 tensor-memory lanes x 16 columns: register 2c = (row g, column 4c + t), 2c + 1 = (row g + 8, column 4c + t)
+__device__ __forceinline__ void tc_st_16x128b_x4(uint32_t taddr, const uint32_t (&a)[8]) {
+    asm volatile("tcgen05.st.sync.aligned.16x128b.x4.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};\n"
+                 ::"r"(taddr), "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(a[4]), "r"(a[5]), "r"(a[6]), "r"(a[7]) : "memory");
+}
+__device__ __forceinline__ void tc_ld_x16(uint32_t (&r)[16], uint32_t taddr) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];\n"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]),
+                   "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]) : "r"(taddr));
+}
 
-#define TC_REGS16(r, o) "=r"(r[o + 0]), "=r"(r[o + 1]), "=r"(r[o + 2]), "=r"(r[o + 3]), "=r"(r[o + 4]), "=r"(r[o + 5]), "=r"(r[o + 6]), "=r"(r[o + 7]), \
-                        "=r"(r[o + 8]), "=r"(r[o + 9]), "=r"(r[o + 10]), "=r"(r[o + 11]), "=r"(r[o + 12]), "=r"(r[o + 13]), "=r"(r[o + 14]), "=r"(r[o + 15])
-// 16 TMEM lanes x 32 columns in the mma C-fragment order: r[4k + 0,1] = (lane g, columns 8k + 2t, + 1), r[4k + 2,3] = (lane g + 8, same)
-#define TC_LD_16x32(r, o, taddr)                                                                                                  \
-    asm volatile("tcgen05.ld.sync.aligned.16x256b.x4.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];\n" \
-                 : TC_REGS16(r, o) : "r"(taddr))
+// ---- a row tile's tensor (PeerDst::wseg) and its place in it ----
+__device__ __forceinline__ void tc_weight_at(const PeerDst &peers, int rt, int &seg, int &rt_in) {
+    seg = 0;
+    rt_in = rt;
+    if (peers.n_wseg > 0) {
+        const int row = rt * 16;
+        if (row >= peers.seg_end[0]) {
+            seg = (peers.n_seg > 2 && row >= peers.seg_end[1]) ? 2 : 1;
+            rt_in -= (seg == 2 ? peers.seg_end[1] : peers.seg_end[0]) / 16;
+        }
+    }
+}
 
-// debugging switches in `mode`: bit 0 no MMAs, bit 1 no scaling FMAs, bit 2 no accumulator reads, bit 3 no weight expansion,
-// bits 4-6 leave out the activation planes / the packed weights / the scale planes of every copy
-__global__ void __launch_bounds__(TC_THREADS, 1) mmq_tc_q4_kernel(const __grid_constant__ TcMaps maps, TiledDims dims, ActDims act,
-                                                               float *__restrict__ dst, int64_t dst_nb_row,
-                                                               float *__restrict__ partial, int ksplit, int mode) {
+// A piece of work: block groups [bg, bg + len) of a tile (row group x column chunk).
+struct TcPiece {
+    uint32_t tile, group, chunk, bg, len;
+    uint32_t two;            // more than 128 rows: the second MMA row tile is in use
+    uint32_t slot0, parts;   // equal shares: where the tile's first part is parked (the others: slot 2j of the CTAs that follow), how many
+};
+constexpr int TC_MAX_PIECES = 128;
+
+// What the write-back needs of the launch and the CTA's share of the work, in shared memory.  All of it is worked out once, by
+// one thread, while the first copies are on their way: code that every role repeats costs instruction cache misses.
+struct TcShared {
+    TiledDims dims;
+    ActDims act;
+    PeerDst peers;
+    TcPlan plan;
+    const uint8_t *w, *aq;
+    float *dst;
+    int64_t dst_nb_row;
+    unsigned long long *counters;   // per tile {launch id, arrivals}
+    float4 *slots;                  // parked parts
+    uint32_t slot_n;                // float4s of one
+    uint32_t tmem;
+    int abort_flag, flag;
+    uint32_t n_pieces, n_iter;
+    TcPiece piece[TC_MAX_PIECES];
+};
+
+static_assert(sizeof(TcShared) <= 5120, "TcShared has its place in TcCfg");
+
+// One result from the integers themselves: what the reference computes, block by block.  Only for values whose folded
+// operands left the fp16 range.
+template <int WTYPE>
+__device__ __noinline__ float tc_exact_value(const TcShared *o, int row, int col) {
+    int seg, rt;
+    tc_weight_at(o->peers, row >> 4, seg, rt);
+    const uint8_t *wq = o->peers.n_wseg > 0 ? o->peers.wseg[seg] : o->w, *ws = wq + (o->peers.n_wseg > 0 ? (size_t) o->peers.wseg_qs[seg] : o->dims.qs_bytes);
+    const int r = row & 15, g = r & 7, h = r >> 3;
+    float sum = 0.0f;
+#pragma unroll 1
+    for (int b = 0; b < (int) o->dims.nb; ++b) {
+        const int64_t at = (int64_t) rt * o->dims.n_bg + (b >> 2);
+        const int j = b & 3;
+        const uint2 *a = reinterpret_cast<const uint2 *>(o->aq + ((col >> 3) * o->act.nbp + b) * 256) + (col & 7) * 4;
+        int dot = 0;
+#pragma unroll 1
+        for (int t = 0; t < 4; ++t) {
+            if (WTYPE == B200_TYPE_Q4_0) {
+                const uint32_t word = reinterpret_cast<const uint32_t *>(wq + at * 1024 + (g * 4 + t) * 32)[h * 4 + j];
+                dot = __dp4a((int) ((word << 4) & 0xF0F0F0F0u), (int) a[t].x, dot);
+                dot = __dp4a((int) (word & 0xF0F0F0F0u), (int) a[t].y, dot);
+            } else {
+                const uint32_t *word = reinterpret_cast<const uint32_t *>(wq + at * 2048 + j * 512 + (g * 4 + t) * 16);
+                dot = __dp4a((int) word[h], (int) a[t].x, dot);
+                dot = __dp4a((int) word[2 + h], (int) a[t].y, dot);
+            }
+        }
+        const float dw = __half2float(reinterpret_cast<const __half *>(ws)[at * 64 + r * 4 + j]) * (WTYPE == B200_TYPE_Q4_0 ? 0.0625f : 1.0f);
+        const float da = reinterpret_cast<const float *>(o->aq + o->act.d_offset)[((col >> 3) * o->act.n_bg + (b >> 2)) * 64 + act_scale_index(j, col & 7)];
+        sum = fmaf(dw * da, (float) dot, sum);
+    }
+    return sum;
+}
+
+// Equal shares: CTA j takes iterations [first_of(j), first_of(j + 1)) of [tile][block group].  A share that ends inside a tile
+// starts with that last piece: the CTA that completes the tile then finds it parked long before.  CTA j parks a piece that
+// starts where its share starts in slot 2j, the piece its share ends with in slot 2j + 1.
+__device__ __forceinline__ uint32_t tc_first_of(const TcPlan &p, uint32_t j) { return j * p.share + min(j, p.extra); }
+__device__ __forceinline__ uint32_t tc_cta_of(const TcPlan &p, uint32_t it) {   // the CTA that holds iteration `it`
+    const uint32_t big = p.extra * (p.share + 1);
+    return it < big ? it / (p.share + 1) : p.extra + (it - big) / p.share;
+}
+__device__ __noinline__ void tc_share(TcShared *o, const TcPlan plan, uint32_t n_bg, uint32_t n_rt) {
+    uint32_t it0, it1;
+    if (plan.cs > 0) {   // the CTAs of a cluster cut the K range of one tile
+        const uint32_t cs = (uint32_t) plan.cs, rank = blockIdx.x % cs, tile = blockIdx.x / cs * n_bg;
+        it0 = tile + rank * n_bg / cs;
+        it1 = tile + (rank + 1) * n_bg / cs;
+    } else {
+        it0 = tc_first_of(plan, blockIdx.x);
+        it1 = tc_first_of(plan, blockIdx.x + 1);
+    }
+    uint32_t n = 0, tile = it0 / n_bg, at = it0;
+    const uint32_t tile_h = it1 / n_bg, head = tile_h * n_bg > it0 ? it1 - tile_h * n_bg : 0u;
+    o->n_iter = it1 - it0;
+    if (head > 0) { at = tile_h * n_bg; tile = tile_h; }
+#pragma unroll 1
+    while (it1 > it0) {
+        TcPiece &q = o->piece[n++];
+        q.tile = tile;
+        q.group = tile / (uint32_t) plan.chunks;
+        q.chunk = tile - q.group * (uint32_t) plan.chunks;
+        q.bg = at - tile * n_bg;
+        q.len = min(it1 - at, n_bg - q.bg);
+        q.two = n_rt - q.group * (uint32_t) plan.rt_per_group > 8 && plan.rt_per_group > 8 ? 1u : 0u;
+        q.parts = 1;
+        q.slot0 = 0;
+        if (plan.cs == 0 && q.len < n_bg) {
+            const uint32_t first = tc_cta_of(plan, tile * n_bg);
+            q.parts = tc_cta_of(plan, tile * n_bg + n_bg - 1) - first + 1;
+            q.slot0 = 2 * first + (tc_first_of(plan, first) < tile * n_bg ? 1u : 0u);
+        }
+        if (n == 1 && head > 0) { at = it0; tile = it0 / n_bg; it1 -= head; }   // on to the start of the share
+        else { at += q.len; ++tile; if (at >= it1) break; }
+    }
+    o->n_pieces = n;
+}
+
+// Values that do not simply go to 16 aligned bytes: a ragged or unaligned edge, other GPUs' buffers too, or not finite
+template <int WTYPE>
+__device__ __noinline__ void tc_write_slow(const TcShared *o, int row, int row_end, int col, float4 f) {
+#pragma unroll 1
+    for (int i = 0; i < 4 && row + i < row_end; ++i) {
+        float y = i == 0 ? f.x : i == 1 ? f.y : i == 2 ? f.z : f.w;
+        if (!isfinite(y)) y = tc_exact_value<WTYPE>(o, row + i, col);
+        const int64_t off = col * o->dst_nb_row + (int64_t) (row + i) * 4 + peer_row_shift(o->peers, row + i);
+#pragma unroll 1
+        for (int p = -1; p < o->peers.n; ++p) *reinterpret_cast<float *>(reinterpret_cast<char *>(p < 0 ? o->dst : o->peers.p[p]) + off) = y;
+    }
+}
+// Where a thread's share of a tile goes: elements e0, e0 + step, ... of [column][256 rows / 4]; step is a multiple of 64, so the
+// rows stay the same and the column moves.
+struct TcOut {
+    char *to;
+    int64_t inc;
+    int row, row_end, col, col_inc, col_end;
+    bool vec;
+    __device__ __forceinline__ TcOut(const TcShared *o, const TcPiece &q, uint32_t e0, uint32_t step) {
+        row = (int) q.group * o->plan.rt_per_group * 16 + (int) (e0 & 63) * 4;
+        row_end = min((int) o->dims.M, ((int) q.group + 1) * o->plan.rt_per_group * 16);
+        col = (int) q.chunk * o->act.chunk_nt * 8 + (int) (e0 >> 6);
+        col_inc = (int) (step >> 6);
+        col_end = row < row_end ? (int) o->act.N : 0;
+        const int64_t nb = o->dst_nb_row;
+        inc = col_inc * nb;
+        to = reinterpret_cast<char *>(o->dst) + col * nb + (int64_t) row * 4 + peer_row_shift(o->peers, row);
+        vec = row + 3 < row_end && o->peers.n == 0 && ((reinterpret_cast<uintptr_t>(to) | (uintptr_t) nb) & 15) == 0;
+    }
+    template <int WTYPE>
+    __device__ __forceinline__ void put(const TcShared *o, float4 v) {
+        if (vec && isfinite((v.x + v.y) + (v.z + v.w))) *reinterpret_cast<float4 *>(to) = v;
+        else tc_write_slow<WTYPE>(o, row, row_end, col, v);
+        to += inc;
+        col += col_inc;
+    }
+};
+__device__ __forceinline__ float4 tc_lds4(uint32_t at) {
+    float4 v;
+    asm volatile("ld.shared.v4.f32 {%0,%1,%2,%3}, [%4];\n" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(at));
+    return v;
+}
+
+// The tile's parts lie in the shared memory of the cluster's CTAs: this CTA adds slice `rank` of the columns in rank order.
+template <int WTYPE>
+__device__ __noinline__ void tc_write_cluster(const TcShared *o, uint32_t acc_u32, uint32_t te, uint32_t threads) {
+    const uint32_t cs = (uint32_t) o->plan.cs, rank = blockIdx.x % cs, per4 = ((uint32_t) o->act.chunk_nt * 8 + cs - 1) / cs * 64;
+    const uint32_t end = min((uint32_t) o->act.chunk_nt * 512, (rank + 1) * per4);
+    uint32_t e = rank * per4 + te;
+    TcOut out(o, o->piece[0], e, threads);
+#pragma unroll 1
+    for (; e < end && out.col < out.col_end; e += threads) {
+        float4 x[8];
+#pragma unroll
+        for (uint32_t k = 0; k < 8; ++k) {   // all in flight at once
+            uint32_t remote;
+            x[k] = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (k < cs) {
+                asm volatile("mapa.shared::cluster.u32 %0, %1, %2;\n" : "=r"(remote) : "r"(acc_u32 + e * 16u), "r"(k));
+                asm volatile("ld.shared::cluster.v4.f32 {%0,%1,%2,%3}, [%4];\n" : "=f"(x[k].x), "=f"(x[k].y), "=f"(x[k].z), "=f"(x[k].w) : "r"(remote));
+            }
+        }
+#pragma unroll
+        for (uint32_t k = 1; k < 8; ++k) { x[0].x += x[k].x; x[0].y += x[k].y; x[0].z += x[k].z; x[0].w += x[k].w; }
+        out.template put<WTYPE>(o, x[0]);
+    }
+}
+
+// Piece q is complete in shared memory: write the tile if this is all of it or the last part to arrive, else park it.  Called by
+// `threads` threads, te = 0 ..., which meet at barrier `bar`.  A tile's counter is {launch id, arrivals}; a word without
+// this launch's id counts as zero, so the workspace needs no clearing, and the last to arrive leaves it zero for the next
+// replay of a graph.  The parts (at most three) are added in K order whoever does it.
+template <int WTYPE>
+__device__ __noinline__ void tc_finish(TcShared *o, uint32_t acc_u32, uint32_t piece, uint32_t te, uint32_t threads, uint32_t bar) {
+    const TcPiece q = o->piece[piece];
+    const uint32_t total4 = (uint32_t) o->act.chunk_nt * 512;
+    volatile int *const flag = &o->flag;
+    const uint32_t own = q.parts == 1 ? 0u : blockIdx.x - (q.slot0 >> 1);
+    bool write = true;
+    const float4 *at[3];
+#pragma unroll
+    for (uint32_t k = 0; k < 3; ++k) at[k] = k < q.parts && k != own ? o->slots + (size_t) (k == 0 ? q.slot0 : (q.slot0 & ~1u) + 2 * k) * o->slot_n : nullptr;
+    if (q.parts > 1) {
+        const unsigned long long id = o->plan.launch_id << 8;
+        unsigned long long *const arrived = o->counters + q.tile;
+        if (te == 0) {   // every other part parked already: nothing of this one has to go through memory
+            unsigned long long seen;
+            asm volatile("ld.acquire.gpu.global.u64 %0, [%1];\n" : "=l"(seen) : "l"(arrived) : "memory");
+            *flag = seen == id + q.parts - 1;
+        }
+        asm volatile("bar.sync %0, %1;\n" ::"r"(bar), "r"(threads) : "memory");
+        write = *flag != 0;
+        if (!write) {
+            float4 *to = o->slots + (size_t) (own == 0 ? q.slot0 : 2 * blockIdx.x) * o->slot_n;
+#pragma unroll 1
+            for (uint32_t e = te; e < total4; e += threads) {
+                __stcg(to + e, tc_lds4(acc_u32 + e * 16u));
+            }
+            __threadfence();
+            asm volatile("bar.sync %0, %1;\n" ::"r"(bar), "r"(threads) : "memory");
+            if (te == 0) {
+                unsigned long long old = *reinterpret_cast<volatile unsigned long long *>(arrived), seen, base;
+                do {
+                    seen = old;
+                    base = (seen ^ id) < 256 ? seen : id;
+                    old = atomicCAS(arrived, seen, base + 1);
+                } while (old != seen);
+                *flag = base == id + q.parts - 1;
+                __threadfence();
+            }
+            asm volatile("bar.sync %0, %1;\n" ::"r"(bar), "r"(threads) : "memory");
+            write = *flag != 0;
+        }
+        if (write && te == 0) *arrived = 0;
+    }
+    if (write) {
+        TcOut out(o, q, te, threads);
+#pragma unroll 1
+        for (uint32_t e = te; e < total4 && out.col < out.col_end; e += threads) {
+            float4 x[3];
+#pragma unroll
+            for (uint32_t k = 0; k < 3; ++k) {   // in flight together
+                x[k] = make_float4(0.f, 0.f, 0.f, 0.f);
+                if (at[k]) x[k] = __ldcg(at[k] + e);
+                else if (k == own) x[k] = tc_lds4(acc_u32 + e * 16u);
+            }
+            out.template put<WTYPE>(o, make_float4(x[0].x + x[1].x + x[2].x, x[0].y + x[1].y + x[2].y, x[0].z + x[1].z + x[2].z, x[0].w + x[1].w + x[2].w));
+        }
+    }
+    asm volatile("bar.sync %0, %1;\n" ::"r"(bar), "r"(threads) : "memory");   // the partial results are free again
+}
+
+template <int WTYPE, int NT>
+__global__ void __launch_bounds__((TcCfg<WTYPE, NT>::THREADS), 1) mmq_tc_kernel(TiledDims dims, const uint8_t *__restrict__ w, ActDims act, const uint8_t *__restrict__ aq,
+                                                              float *__restrict__ dst, int64_t dst_nb_row, void *__restrict__ workspace, TcPlan plan, PeerDst peers,
+                                                              const __grid_constant__ TcMaps maps) {
+    using C = TcCfg<WTYPE, NT>;
     extern __shared__ __align__(1024) uint8_t smem[];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const uint32_t smem_u32 = (uint32_t) __cvta_generic_to_shared(smem);
-    const uint32_t bars = smem_u32 + TC_BAR_OFFSET;
-    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(smem + TC_BAR_OFFSET + TC_N_BARS * 8);
-    volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_slot + 2);
+    const uint32_t bars = smem_u32 + C::BAR_OFFSET;
+    TcShared *const sh = reinterpret_cast<TcShared *>(smem + C::SH_OFFSET);
+    volatile int *const abort_flag = &sh->abort_flag;
+    float *const acc_s = reinterpret_cast<float *>(smem + C::OFF_ACC);
+    const uint32_t acc_u32 = smem_u32 + C::OFF_ACC;
 #define BAR(which, i) (bars + 8u * (uint32_t) ((which) + (i)))
-
-    const int cta_rt0 = blockIdx.x * 8;
-    const int cta_nt0 = blockIdx.y * 8;
-    const int ks = blockIdx.z;
-    const int per = (int) ((dims.n_bg + ksplit - 1) / ksplit);
-    const int bg_begin = ks * per;
-    const int bg_end = min((int) dims.n_bg, bg_begin + per);
-    const int n_iter = max(0, bg_end - bg_begin);
+    const uint32_t n_bg = (uint32_t) dims.n_bg;
     const uint32_t spin_limit = g_tc_spin_limit;
 
-    if (tid == 0) {
-        *abort_flag = 0;
-        for (int i = 0; i < TC_N_BARS; ++i) {
-            // empty: the issuing warps' commits (activation planes read), the expanding warps (packed weights read), the epilogue warps (scales read)
-            const int count = (i >= BAR_EMPTY && i < BAR_A_FULL)            ? TC_ISSUE_WARPS + TC_EXP_WARPS + TC_EPI_WARPS
-                            : (i >= BAR_A_FULL && i < BAR_A_FREE)            ? TC_EXP_WARPS
-                            : (i >= BAR_A_FREE && i < BAR_ACC_FULL)          ? TC_ISSUE_WARPS
-                            : (i >= BAR_ACC_FREE && i < BAR_DRAIN)           ? TC_EPI_WARPS : 1;
-            asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;\n" ::"r"(BAR(0, i)), "r"(count));
-        }
+    if (tid == 96) {   // warp 3 has no role of its own
+        sh->dims = dims;
+        sh->act = act;
+        sh->peers = peers;
+        sh->plan = plan;
+        sh->w = w; sh->aq = aq; sh->dst = dst; sh->dst_nb_row = dst_nb_row;
+        sh->counters = reinterpret_cast<unsigned long long *>(workspace);
+        sh->slots = reinterpret_cast<float4 *>(reinterpret_cast<char *>(workspace) + ((size_t) plan.groups * plan.chunks * 8 + 255) / 256 * 256);
+        sh->slot_n = (uint32_t) act.chunk_nt * 512;
+    }
+    if (tid == 64) {
+        sh->abort_flag = 0;
+        tc_share(sh, plan, n_bg, (uint32_t) dims.n_rt);
+    }
+    if (tid < C::N_BARS) {
+        const int i = tid;
+        const int count = (i >= C::B_WREAD && i < C::B_DONE) ? 16
+                        : (i >= C::B_AFULL && i < C::B_AFREE) || (i >= C::B_ACCE && i < C::B_DRAIN) ? 4 : 1;
+        asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;\n" ::"r"(BAR(0, i)), "r"(count));
         asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
     }
-    if (warp == 0) {   // all 512 columns (the CTA is alone on its SM)
-        const uint32_t slot = (uint32_t) __cvta_generic_to_shared(tmem_slot);
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 512;\n" ::"r"(slot) : "memory");
+    if (warp == 1) {   // all 512 columns (the CTA is alone on its SM)
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 512;\n" ::"r"((uint32_t) __cvta_generic_to_shared(&sh->tmem)) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::: "memory");
     }
     asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-    const uint32_t tmem = *tmem_slot;
+    const uint32_t tmem = sh->tmem;
     pdl_prologue();   // everything above touches no global memory
 
-    if (warp < 4) {
-        asm volatile("setmaxnreg.dec.sync.aligned.u32 40;\n");
-        // ---------------- MMA issue: warp w issues block w of every group, so the four accumulator tiles in flight turn over independently ----------------
-        const int j = warp;
-        const uint32_t idesc = (1u << 4) | ((uint32_t) (TC_COLS >> 3) << 17) | ((uint32_t) (TC_ROWS >> 4) << 24);   // e4m3 x e4m3 -> f32, K-major both
-        const uint64_t bh0 = tc_smem_desc(smem_u32 + TC_OFF_BH + j * 256, 128, 1024), bl0 = tc_smem_desc(smem_u32 + TC_OFF_BL + j * 256, 128, 1024);
-        int ti = j % TC_ACC, tpar = 0;   // accumulator tile of block 4 it + j and the parity of its use count
-        for (int it = 0; it < n_iter; ++it) {
-            const int s = it % TC_STAGES, ab = it % TC_ABUF;
-            // lane 0: the stage has landed; lane 1: the expanded weights are in TMEM; lane 2: the accumulator tile has been read
-            const uint32_t wbar = lane == 0 ? BAR(BAR_FULL, s) : lane == 1 ? BAR(BAR_A_FULL, ab) : BAR(BAR_ACC_FREE, ti);
-            const uint32_t wpar = lane == 0 ? (uint32_t) ((it / TC_STAGES) & 1) : lane == 1 ? (uint32_t) ((it / TC_ABUF) & 1) : (uint32_t) (tpar ^ 1);
-            if (!tc_wait_lanes(lane < 3, wbar, wpar, abort_flag, spin_limit)) break;
-            if (warp == 0) TC_PROF(2, it);
-            asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-            if (lane == 0) {
-                if (mode & 1) {
-                    tc_arrive(BAR(BAR_ACC_FULL, ti)); tc_arrive(BAR(BAR_A_FREE, ab)); tc_arrive(BAR(BAR_EMPTY, s));
-                } else {
-                    const uint64_t st16 = (uint64_t) ((s * TC_STAGE) >> 4);
-                    const uint32_t d_t = tmem + 64u * (uint32_t) ti, a_t = tmem + TC_A_COL + 32u * ab + 8u * j;
-                    tc_mma_f8_ts(d_t, a_t, bh0 + st16, idesc, 0u);
-                    tc_mma_f8_ts(d_t, a_t, bl0 + st16, idesc, 1u);
-                    tc_commit(BAR(BAR_ACC_FULL, ti)); tc_commit(BAR(BAR_A_FREE, ab)); tc_commit(BAR(BAR_EMPTY, s));
+    if (warp < 2) {
+        // ---------------- MMA issue for row tile mt = warp ----------------
+        const uint32_t mt = (uint32_t) warp, nt = (uint32_t) act.chunk_nt;
+        const uint32_t idesc_wide = (1u << 4) | (2 * nt << 17) | (8u << 24), idesc_hi = (1u << 4) | (nt << 17) | (8u << 24);   // f16 x f16 -> f32, K-major both, M 128
+        const uint32_t d = tmem + mt * C::D_MT, d_small = d + 8 * nt, a0 = tmem + C::A_COL + mt * C::A_MT;
+        const uint64_t bdesc0 = tc_smem_desc(smem_u32 + C::OFF_B, 128, 2048);
+        uint32_t s = 0, acc_par = 1, ab = 0, a_par = 0;   // ab: A stage
+        bool ok = true;
+#pragma unroll 1
+        for (uint32_t p = 0; p < sh->n_pieces && ok; ++p) {
+            const bool active = mt == 0 || sh->piece[p].two;
+            const uint32_t len = sh->piece[p].len;
+#pragma unroll 1
+            for (uint32_t i = 0; i < len && ok; ++i) {
+                const uint32_t acc = i % TC_FLUSH == 0 ? 0u : 1u;
+                if (acc == 0) {
+                    ok = tc_wait(BAR(C::B_ACCE, mt), acc_par, abort_flag, spin_limit);
+                    acc_par ^= 1;
                 }
+                // (that the stage has landed follows from AFULL: the weight warps waited for it)
+                const uint64_t bdesc = bdesc0 + (uint64_t) (s * (C::STAGE >> 4));
+                const bool last = i + 1 == len || (i + 1) % TC_FLUSH == 0;
+#pragma unroll
+                for (uint32_t h = 0; h < 2; ++h) {
+                    ok = ok && tc_wait(BAR(C::B_AFULL, C::ABUF * mt + ab), a_par, abort_flag, spin_limit);
+                    asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+                    if (tc_elect() && ok) {
+                        if (active) {
+#pragma unroll
+                            for (uint32_t k = 0; k < 4; ++k) {
+                                const uint64_t b = bdesc + (uint64_t) (h * 64 + k * 16);
+                                const uint32_t a = a0 + ab * 64 + 8 * k, acc_k = k == 0 ? (acc | h) : 1u;
+                                tc_mma(d, a, b, idesc_wide, acc_k);          // A_hi (B_hi | B_lo)
+                                tc_mma(d_small, a + 32, b, idesc_hi, 1u);   // A_lo B_hi, on the small terms
+                            }
+                        }
+                        tc_commit(BAR(C::B_AFREE, C::ABUF * mt + ab));
+                        if (h == 1) {
+                            tc_commit(BAR(C::B_DONE, 2 * s + mt));
+                            if (last) tc_commit(BAR(C::B_ACCF, mt));
+                        }
+                    }
+                    __syncwarp();
+                    if (++ab == C::ABUF) { ab = 0; a_par ^= 1; }
+                }
+                if (++s == C::STAGES) s = 0;
             }
-            __syncwarp();
-            ti += 4;
-            if (ti >= TC_ACC) { ti -= TC_ACC; tpar ^= 1; }
         }
-        if (lane == 0) {   // no MMA of this CTA may be in flight when its tensor memory is freed, whatever happened elsewhere
-            tc_commit(BAR(BAR_DRAIN, warp));
-            for (uint32_t spin = 0; spin < TC_DRAIN_LIMIT && !tc_try(BAR(BAR_DRAIN, warp), 0); ++spin) {}
+        // no MMA of this CTA may be in flight when its tensor memory is freed, whatever happened elsewhere.  (elect.sync picks the
+        // same lane every time, the one whose MMAs the commit has to cover.)
+        if (tc_elect()) {
+            tc_commit(BAR(C::B_DRAIN, mt));
+#pragma unroll 1
+            for (uint32_t spin = 0; spin < TC_DRAIN_LIMIT && !tc_try(BAR(C::B_DRAIN, mt), 0); ++spin) {}
         }
         __syncwarp();
-    } else if (warp < 8) {
-        asm volatile("setmaxnreg.dec.sync.aligned.u32 40;\n");
-        if (warp == 4) {
-            // ---------------- producer: lanes 0..4 = the five tensor copies of a stage ----------------
-            const CUtensorMap *map = lane == 0 ? &maps.wq : lane == 1 ? &maps.wd : lane == 2 ? &maps.bh : lane == 3 ? &maps.bl : &maps.bs;
-            const uint32_t dst_off = lane == 0 ? 0 : lane == 1 ? TC_OFF_WD : lane == 2 ? TC_OFF_BH : lane == 3 ? TC_OFF_BL : TC_OFF_BS;
-            int issued = 0;
-            for (int it = 0; it < n_iter; ++it) {
-                const int s = it % TC_STAGES, n = it / TC_STAGES;
-                if (!tc_wait_lanes(lane == 0, BAR(BAR_EMPTY, s), (uint32_t) ((n & 1) ^ 1), abort_flag, spin_limit)) break;
-                TC_PROF(0, it);
-                const uint32_t tx = TC_STAGE - ((mode & 16) ? TC_BH + TC_BL : 0) - ((mode & 32) ? TC_WQ : 0) - ((mode & 64) ? TC_WD + TC_BS : 0);
-                if (lane == 0) asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(BAR(BAR_FULL, s)), "r"(tx) : "memory");
-                __syncwarp();
-                const int bg = bg_begin + it;
-                const uint32_t to = smem_u32 + s * TC_STAGE + dst_off;
-                if (lane == 0) { if (!(mode & 32)) tc_tma_3d(to, map, 0, bg * 8, cta_rt0, BAR(BAR_FULL, s)); }      // rows / columns past the end read as zero
-                else if (lane == 1) { if (!(mode & 64)) tc_tma_2d(to, map, bg * 32, cta_rt0, BAR(BAR_FULL, s)); }
-                else if (lane < 4) { if (!(mode & 16)) tc_tma_2d(to, map, bg * 256, cta_nt0, BAR(BAR_FULL, s)); }
-                else if (lane == 4) { if (!(mode & 64)) tc_tma_2d(to, map, bg * 64, cta_nt0, BAR(BAR_FULL, s)); }
-                issued = it + 1;
+    } else if (warp == 2) {
+        // ---------------- producer: two or four tensor copies of weights, one bulk copy of activations per block group ----------------
+        uint32_t s = 0, par = 1, issued = 0;
+        bool ok = !(plan.debug & 32);
+        const uint32_t b_bytes = (uint32_t) act.chunk_nt * 4096u;
+#pragma unroll 1
+        for (uint32_t p = 0; p < sh->n_pieces && ok; ++p) {
+            const TcPiece q = sh->piece[p];
+            const int boxes = 1 + (int) q.two;   // rows past the end read as zero
+            const uint32_t bytes = (uint32_t) boxes * 8u * (C::WT + 128u) + b_bytes;
+            const CUtensorMap *qm[2], *sm[2];
+            int rt_in[2];
+#pragma unroll
+            for (int k = 0; k < 2; ++k) {
+                int seg;
+                tc_weight_at(peers, (int) q.group * plan.rt_per_group + 8 * k, seg, rt_in[k]);
+                qm[k] = &maps.q[seg];
+                sm[k] = &maps.s[seg];
             }
-            // copies in flight must land before the CTA may exit, whatever happened elsewhere
-            for (int it = max(0, issued - TC_STAGES); it < issued && lane == 0; ++it) {
-                const uint32_t bar = BAR(BAR_FULL, it % TC_STAGES), parity = (uint32_t) ((it / TC_STAGES) & 1);
-                for (uint32_t spin = 0; spin < TC_DRAIN_LIMIT && !tc_try(bar, parity); ++spin) {}
-            }
-            __syncwarp();
-        }
-    } else if (warp < 12) {
-        asm volatile("setmaxnreg.dec.sync.aligned.u32 96;\n");
-        // ---------------- expand: thread = weight row m of the CTA's 128 ----------------
-        const int m = tid - 256;
-        const int tile = m >> 4, hrow = (m >> 3) & 1, g = m & 7;
-        // the 128-byte line of (tile, g) holds the 16-byte chunks 2t + hrow = word t of blocks 0..3 of row g + 8 hrow; the TMA
-        // swizzle stores chunk c at position c ^ (line & 7) = c ^ g
-        const uint32_t line = smem_u32 + (uint32_t) ((tile * 8 + g) * 128);
-        uint32_t chunk[4];
+            const uint8_t *bsrc = aq + act.b_offset + ((int64_t) q.chunk * n_bg + q.bg) * b_bytes;
+#pragma unroll 1
+            for (uint32_t i = 0; i < q.len; ++i) {
+                const uint32_t st = smem_u32 + s * C::STAGE, bar = BAR(C::B_FULL, s);
+                if (!tc_wait(BAR(C::B_WREAD, s), par, abort_flag, spin_limit) || !tc_wait(BAR(C::B_DONE, 2 * s), par, abort_flag, spin_limit) ||
+                    !tc_wait(BAR(C::B_DONE, 2 * s + 1), par, abort_flag, spin_limit)) { ok = false; break; }
+                if (tc_elect()) {
+                    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(bar), "r"(bytes) : "memory");
+                    const int bg = (int) (q.bg + i);
 #pragma unroll
-        for (int t = 0; t < 4; ++t) chunk[t] = (uint32_t) (((2 * t + hrow) ^ g) * 16);
-        const uint32_t a_lane = tmem + ((uint32_t) (32 * (warp - 8)) << 16) + TC_A_COL;
-        for (int it = 0; it < n_iter; ++it) {
-            const int s = it % TC_STAGES, ab = it % TC_ABUF;
-            const uint32_t wbar = lane == 0 ? BAR(BAR_FULL, s) : BAR(BAR_A_FREE, ab);
-            const uint32_t wpar = lane == 0 ? (uint32_t) ((it / TC_STAGES) & 1) : (uint32_t) (((it / TC_ABUF) & 1) ^ 1);
-            if (!tc_wait_lanes(lane < 2, wbar, wpar, abort_flag, spin_limit)) break;
-            if (warp == 8) TC_PROF(1, it);
-            uint32_t r[4][4];   // r[t][j] = word t of block j
-#pragma unroll
-            for (int t = 0; t < 4; ++t)
-                asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];\n" : "=r"(r[t][0]), "=r"(r[t][1]), "=r"(r[t][2]), "=r"(r[t][3]) : "r"(line + s * TC_STAGE + chunk[t]));
-            __syncwarp();
-            if (lane == 0) tc_arrive(BAR(BAR_EMPTY, s));   // the packed weights of this stage are in registers (the arrive orders the loads before it)
-            if (!(mode & 8)) {
-                asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-#pragma unroll
-                for (int h = 0; h < 2; ++h) {
-                    uint32_t a[16];     // a[8 jj + c]: bytes 4c..4c+3 of the row of block 2h + jj, element order
-#pragma unroll
-                    for (int jj = 0; jj < 2; ++jj)
-#pragma unroll
-                        for (int t = 0; t < 4; ++t) {
-                            const uint32_t w = r[t][2 * h + jj];
-                            a[8 * jj + t] = (w & 0x0F0F0F0Fu) ^ 0x08080808u;              // elements 4t..4t+3: u = q + 8 (the nibbles hold q in two's complement)
-                            a[8 * jj + 4 + t] = ((w >> 4) & 0x0F0F0F0Fu) ^ 0x08080808u;   // elements 16+4t..
+                    for (int k = 0; k < 2; ++k) {
+                        if (k < boxes) {
+                            if (WTYPE == B200_TYPE_Q4_0) tc_tma_2d(st + (uint32_t) (k * 8 * C::WT), qm[k], bg * 256, rt_in[k], bar);
+                            else tc_tma_3d(st + (uint32_t) (k * 8 * C::WT), qm[k], 0, bg * 2, rt_in[k], bar);
+                            tc_tma_2d(st + (uint32_t) (C::OFF_S + k * 1024), sm[k], bg * 32, rt_in[k], bar);
                         }
-                    asm volatile("tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};\n"
-                                 ::"r"(a_lane + 32u * ab + 16u * h), "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(a[4]), "r"(a[5]), "r"(a[6]), "r"(a[7]), "r"(a[8]), "r"(a[9]),
-                                 "r"(a[10]), "r"(a[11]), "r"(a[12]), "r"(a[13]), "r"(a[14]), "r"(a[15]) : "memory");
+                    }
+                    tc_copy(st + C::OFF_B, bsrc + (int64_t) i * b_bytes, b_bytes, bar);
+                }
+                __syncwarp();
+                ++issued;
+                if (++s == C::STAGES) { s = 0; par ^= 1; }
+            }
+        }
+        // copies in flight must land before the CTA may exit, whatever happened elsewhere
+#pragma unroll 1
+        for (uint32_t k = issued > C::STAGES ? issued - C::STAGES : 0; k < issued && lane == 0; ++k) {
+            const uint32_t bar = BAR(C::B_FULL, k % C::STAGES), parity = (k / C::STAGES) & 1;
+#pragma unroll 1
+            for (uint32_t spin = 0; spin < TC_DRAIN_LIMIT && !tc_try(bar, parity); ++spin) {}
+        }
+        __syncwarp();
+    } else if (warp >= 4 && warp < C::WARP_EPI) {
+        // ---------------- weights: a warp owns 32 rows (two T16 tiles: the lanes of tensor memory it can reach) of every third half block group ----------------
+        const int q4 = warp & 3, mt = ((warp - 4) >> 2) & 1, team = (warp - 4) >> 3;
+        const uint32_t rt0 = (uint32_t) (mt * 8 + q4 * 2);
+        const uint32_t a_base = tmem + ((uint32_t) (32 * q4) << 16) + C::A_COL + (uint32_t) (mt * C::A_MT);
+        const uint32_t w_at = smem_u32 + rt0 * C::WT + (uint32_t) (lane * (WTYPE == B200_TYPE_Q4_0 ? 32 : 16));
+        const uint32_t s_at = smem_u32 + C::OFF_S + rt0 * 128 + (uint32_t) ((lane >> 2) * 8);
+        const bool active = mt == 0 || plan.rt_per_group > 8;
+        const uint32_t halves = 2 * sh->n_iter;
+        uint32_t s = (uint32_t) team >> 1, full_par = 0, free_par = 1;
+#pragma unroll 1
+        for (uint32_t hc = (uint32_t) team; hc < halves; hc += C::ABUF, free_par ^= 1) {
+            const uint32_t half = hc & 1, ab = (uint32_t) team;
+            if (!tc_wait(BAR(C::B_FULL, s), full_par, abort_flag, spin_limit)) break;
+            constexpr int NW = WTYPE == B200_TYPE_Q4_0 ? 4 : 8;
+            uint32_t r[2][NW];      // Q4_0: rows g, g + 8 x word t of the two blocks; Q8_0: block j: (g, t), (g + 8, t), (g, 4 + t), (g + 8, 4 + t)
+            uint32_t sc[2][2];      // the two block scales of rows g, g + 8
+#pragma unroll
+            for (int u = 0; u < 2; ++u) {
+#pragma unroll
+                for (int v = 0; v < 2; ++v) {
+                    const uint32_t at = w_at + s * C::STAGE + half * (WTYPE == B200_TYPE_Q4_0 ? 8 : 1024) + (uint32_t) (u * C::WT + v * (WTYPE == B200_TYPE_Q4_0 ? 16 : 512));
+                    if (WTYPE == B200_TYPE_Q4_0) asm volatile("ld.shared.v2.u32 {%0,%1}, [%2];\n" : "=r"(r[u][2 * v]), "=r"(r[u][2 * v + 1]) : "r"(at));
+                    else asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];\n" : "=r"(r[u][(4 * v) % NW]), "=r"(r[u][(4 * v + 1) % NW]), "=r"(r[u][(4 * v + 2) % NW]), "=r"(r[u][(4 * v + 3) % NW]) : "r"(at));
+                }
+                const uint32_t sa = s_at + s * C::STAGE + half * 4 + (uint32_t) (u * 128);
+                asm volatile("ld.shared.u32 %0, [%1];\n" : "=r"(sc[u][0]) : "r"(sa));
+                asm volatile("ld.shared.u32 %0, [%1];\n" : "=r"(sc[u][1]) : "r"(sa + 64));
+            }
+            __syncwarp();
+            if (lane == 0) tc_arrive(BAR(C::B_WREAD, s));   // the weights are in registers (the arrive orders the loads before it)
+            if (!tc_wait(BAR(C::B_AFREE, C::ABUF * mt + ab), free_par, abort_flag, spin_limit)) break;
+            asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+            const uint32_t a_to = a_base + ab * 64;
+            if (active) {
+#pragma unroll
+                for (int j = 0; j < 2; ++j) {   // block 2 half + j of both tiles
+#pragma unroll
+                    for (int u = 0; u < 2; ++u) {
+                        uint32_t hi[8], lo[8];
+#pragma unroll
+                        for (int row = 0; row < 2; ++row) {
+                            const __half2 d2 = j ? __high2half2(tc_as_h2(sc[u][row])) : __low2half2(tc_as_h2(sc[u][row]));
+#pragma unroll
+                            for (int si = 0; si < 4; ++si) {
+                                __half2 q2;
+                                if (WTYPE == B200_TYPE_Q4_0) {
+                                    // nibbles at bits 4 si and 16 + 4 si, two's complement; v = q + 8.  0x6400 | v is the fp16
+                                    // 1024 + v, 0x6400 | 16 v is 1024 + 16 v; both steps to q are exact
+                                    const uint32_t word = r[u][row * 2 + j], w8 = si < 2 ? word : word >> 8;
+                                    if ((si & 1) == 0) q2 = __hadd2(tc_as_h2((w8 & 0x000F000Fu) ^ 0x64086408u), __float2half2_rn(-1032.0f));
+                                    else q2 = __hfma2(tc_as_h2((w8 & 0x00F000F0u) ^ 0x64806480u), __float2half2_rn(0.0625f), __float2half2_rn(-72.0f));
+                                } else {
+                                    const uint32_t word = r[u][(4 * j + row + 2 * (si & 1)) % NW] ^ 0x80808080u;   // q + 128
+                                    q2 = __hadd2(tc_as_h2(__byte_perm(word, 0x64646464u, si < 2 ? 0x4240 : 0x4341)), __float2half2_rn(-1152.0f));
+                                }
+                                const __half2 x = __hmul2(q2, d2);
+                                hi[si * 2 + row] = tc_h2(x);
+                                lo[si * 2 + row] = tc_h2(__hfma2(q2, d2, __hneg2(x)));
+                            }
+                        }
+                        tc_st_16x128b_x4(a_to + ((uint32_t) (16 * u) << 16) + (uint32_t) (j * 16), hi);
+                        tc_st_16x128b_x4(a_to + ((uint32_t) (16 * u) << 16) + (uint32_t) (j * 16) + 32, lo);
+                    }
                 }
                 asm volatile("tcgen05.wait::st.sync.aligned;\n" ::: "memory");
-            }
-            asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
-            __syncwarp();
-            if (lane == 0) tc_arrive(BAR(BAR_A_FULL, ab));
-        }
-    } else {
-        asm volatile("setmaxnreg.inc.sync.aligned.u32 152;\n");
-        // -------- epilogue: rows 32 q + {g, g+8, g+16, g+24}, column pairs 32 cg + 8 k + 2 t (k < 4) --------
-        const int q = warp & 3, cg = (warp - 12) >> 2, g = lane >> 2, t = lane & 3;
-        uint64_t y[4][4];
-#pragma unroll
-        for (int r = 0; r < 4; ++r)
-#pragma unroll
-            for (int k = 0; k < 4; ++k) y[r][k] = 0ull;
-        const uint32_t t_lo = tmem + ((uint32_t) (32 * q) << 16) + 32u * cg, t_hi = t_lo + (16u << 16);
-
-        uint32_t c0[32], c1[32];   // the accumulator tiles of an even / odd block: [0..15] rows g, g+8, [16..31] rows g+16, g+24
-        // y += d_w * (D * v + C) for one block: v = 2^-18 sum(u a), D = d_a 2^18, C = -8 d_a sum(a)
-        auto scale_block = [&](const uint32_t (&cc)[32], const uint8_t *sj, const uint64_t (&dw)[4]) {
-#pragma unroll
-            for (int k = 0; k < 4; ++k) {
-                const uint4 sc = *reinterpret_cast<const uint4 *>(sj + k * 256);   // {D0, D1, C0, C1} of columns 8k + 2t, + 1
-                const uint64_t da = tc_pack2(sc.x, sc.y), ca = tc_pack2(sc.z, sc.w);
-#pragma unroll
-                for (int r = 0; r < 4; ++r) {
-                    const int i = (r >> 1) * 16 + 4 * k + 2 * (r & 1);
-                    const uint64_t tt = tc_fma2(tc_pack2(cc[i], cc[i + 1]), da, ca);
-                    y[r][k] = tc_fma2(tt, dw[r], y[r][k]);
-                }
-            }
-        };
-        auto dw_of = [&](const uint2 (&h4)[4], int j, uint64_t (&dw)[4]) {
-#pragma unroll
-            for (int r = 0; r < 4; ++r) {
-                const uint32_t h = (j < 2) ? h4[r].x : h4[r].y;
-                const __half2 h2 = *reinterpret_cast<const __half2 *>(&h);
-                const uint32_t uu = __float_as_uint((j & 1) ? __high2float(h2) : __low2float(h2));
-                dw[r] = tc_pack2(uu, uu);
-            }
-        };
-        int ti = 0, tpar = 0;   // accumulator tile of the block being loaded (or the next to be loaded) and the parity of its use count
-        bool ok = n_iter > 0 && tc_wait(BAR(BAR_ACC_FULL, 0), 0u, abort_flag, spin_limit);
-        if (ok) {
-            asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-            if (mode & 4) {
-#pragma unroll
-                for (int i = 0; i < 32; ++i) c0[i] = c1[i] = 0u;
-            } else {
-                TC_LD_16x32(c0, 0, t_lo); TC_LD_16x32(c0, 16, t_hi);
-            }
-        }
-        for (int it = 0; ok && it < n_iter; ++it) {
-            const int s = it % TC_STAGES;
-            if (warp == 12) TC_PROF(3, it);
-            const uint8_t *st = smem + s * TC_STAGE;
-            // weight scales: fp16 at 4*row + block within a tile's 128 bytes; rows {g, g+8} of tiles 2q and 2q + 1
-            const uint2 *sa = reinterpret_cast<const uint2 *>(st + TC_OFF_WD + (2 * q) * 128);
-            const uint2 h4[4] = {sa[g], sa[g + 8], sa[16 + g], sa[24 + g]};
-            const uint8_t *Ss = st + TC_OFF_BS + (4 * cg) * 256 + t * 16;
-            uint64_t dw[4];
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                // block j of this group sits in c0 (j even) or c1 (j odd); it is complete after this wait: hand its tile back
-                if (!(mode & 4)) asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
                 asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
-                __syncwarp();
-                if (lane == 0) tc_arrive(BAR(BAR_ACC_FREE, ti));
-                if (++ti == TC_ACC) { ti = 0; tpar ^= 1; }
-                // start reading the next block's tile before this one is scaled
-                if (j < 3 || it + 1 < n_iter) {
-                    ok = tc_wait(BAR(BAR_ACC_FULL, ti), (uint32_t) tpar, abort_flag, spin_limit);
-                    asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-                    if (!ok) break;
-                    const uint32_t a = 64u * (uint32_t) ti;
-                    if (!(mode & 4)) {
-                        if (j & 1) { TC_LD_16x32(c0, 0, t_lo + a); TC_LD_16x32(c0, 16, t_hi + a); }
-                        else { TC_LD_16x32(c1, 0, t_lo + a); TC_LD_16x32(c1, 16, t_hi + a); }
-                    }
-                }
-                if (!(mode & 2)) {
-                    dw_of(h4, j, dw);
-                    if (j & 1) scale_block(c1, Ss + j * 64, dw);
-                    else scale_block(c0, Ss + j * 64, dw);
-                }
             }
-            if (!ok) break;
             __syncwarp();
-            if (lane == 0) tc_arrive(BAR(BAR_EMPTY, s));
+            if (lane == 0) tc_arrive(BAR(C::B_AFULL, C::ABUF * mt + ab));
+            s += C::ABUF == 2 ? 1u : 1u + half;   // two or three halves on
+            if (s >= C::STAGES) { s -= C::STAGES; full_par ^= 1; }
         }
-        asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
-        // write back
+    } else if (warp >= C::WARP_EPI) {
+        // ---------------- accumulator -> shared memory -> result ----------------
+        const int q4 = warp & 3, et = tid - C::WARP_EPI * 32;
+        const uint32_t cols = 8 * (uint32_t) act.chunk_nt;
+        uint32_t acc_par = 0;
+        bool ok = true;
+#pragma unroll 1
+        for (uint32_t p = 0; p < sh->n_pieces && ok; ++p) {
+            const int n_mt = 1 + (int) sh->piece[p].two;
+            const uint32_t len = sh->piece[p].len;
+#pragma unroll 1
+            for (uint32_t i = 0; i < len && ok; i += TC_FLUSH, acc_par ^= 1) {
+#pragma unroll 1
+                for (int mt = 0; mt < 2; ++mt) {
+                    ok = ok && tc_wait(BAR(C::B_ACCF, mt), acc_par, abort_flag, spin_limit);
+                    if (ok && mt < n_mt) {
+                        asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+                        float *o = acc_s + mt * 128 + q4 * 32 + lane;   // the thread's row
+                        const uint32_t d_at = tmem + ((uint32_t) (32 * q4) << 16) + (uint32_t) (mt * C::D_MT);
+#pragma unroll 1
+                        for (uint32_t c = 0; c < cols; c += 16, o += 16 * 256) {
+                            uint32_t u[16], v[16];
+                            tc_ld_x16(u, d_at + c);
+                            tc_ld_x16(v, d_at + cols + c);
+                            asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
 #pragma unroll
-        for (int r = 0; r < 4; ++r) {
-            const int64_t row = (int64_t) blockIdx.x * TC_ROWS + 32 * q + 8 * r + g;
-#pragma unroll
-            for (int k = 0; k < 4; ++k) {
-                const int64_t col = (int64_t) cta_nt0 * 8 + 32 * cg + 8 * k + 2 * t;
-                uint32_t lo, hi;
-                asm("mov.b64 {%0,%1}, %2;" : "=r"(lo), "=r"(hi) : "l"(y[r][k]));
-                const float v0 = __uint_as_float(lo), v1 = __uint_as_float(hi);
-                if (row < dims.M) {
-                    if (ksplit == 1) {
-                        if (col < act.N) *reinterpret_cast<float *>(reinterpret_cast<char *>(dst) + col * dst_nb_row + row * 4) = v0;
-                        if (col + 1 < act.N) *reinterpret_cast<float *>(reinterpret_cast<char *>(dst) + (col + 1) * dst_nb_row + row * 4) = v1;
-                    } else {
-                        if (col < act.N) partial[((int64_t) ks * act.N + col) * dims.M + row] = v0;
-                        if (col + 1 < act.N) partial[((int64_t) ks * act.N + col + 1) * dims.M + row] = v1;
+                            for (int k = 0; k < 16; ++k) {
+                                const float x = __uint_as_float(u[k]) + __uint_as_float(v[k]);
+                                o[k * 256] = i == 0 ? x : o[k * 256] + x;
+                            }
+                        }
+                        asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
                     }
+                    __syncwarp();
+                    if (lane == 0) tc_arrive(BAR(C::B_ACCE, mt));
                 }
             }
+            if (!ok || p + 1 == sh->n_pieces) break;   // the last piece: all warps share what is left to do, below
+            asm volatile("bar.sync 1, 128;\n" ::: "memory");
+            tc_finish<WTYPE>(sh, acc_u32, p, (uint32_t) et, TC_EPI_THREADS, 1u);
         }
     }
-#undef BAR
     asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
-    __syncthreads();
-    if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;\n" ::"r"(tmem) : "memory");
+    pdl_trigger();
+    if (plan.cs > 0) {
+        asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;\n" ::: "memory");
+        if (!*abort_flag) tc_write_cluster<WTYPE>(sh, acc_u32, (uint32_t) tid, C::THREADS);
+        // nobody leaves while a neighbour may still read its part
+        asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;\n" ::: "memory");
+    } else {
+        __syncthreads();
+        if (sh->n_pieces > 0 && !*abort_flag) tc_finish<WTYPE>(sh, acc_u32, sh->n_pieces - 1, (uint32_t) tid, C::THREADS, 0u);
+        __syncthreads();
+    }
+#undef BAR
+    if (warp == 1) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;\n" ::"r"(tmem) : "memory");
 }
 
 static int tc_sm_count() {   // every device of a process is the same model
@@ -429,6 +718,60 @@ static int tc_sm_count() {   // every device of a process is the same model
         return v > 0 ? v : 148;
     }();
     return n;
+}
+
+using tc_kernel_fn = void (*)(TiledDims, const uint8_t *, ActDims, const uint8_t *, float *, int64_t, void *, TcPlan, PeerDst, TcMaps);
+struct TcVariant {
+    tc_kernel_fn fn;
+    int nt, smem, threads;
+    int max_clusters[9];   // resident clusters of 1..8 CTAs on the current device
+};
+template <int WTYPE, int NT>
+static void tc_make(TcVariant &v) {
+    v.fn = mmq_tc_kernel<WTYPE, NT>;
+    v.nt = NT;
+    v.smem = TcCfg<WTYPE, NT>::SMEM;
+    v.threads = TcCfg<WTYPE, NT>::THREADS;
+    cudaFuncSetAttribute(v.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, v.smem);
+    for (int cs = 1; cs <= 8; ++cs) {
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3((unsigned) cs);
+        cfg.blockDim = dim3((unsigned) v.threads);
+        cfg.dynamicSmemBytes = (size_t) v.smem;
+        cudaLaunchAttribute attr[1];
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = (unsigned) cs;
+        attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+        cfg.attrs = attr;
+        cfg.numAttrs = 1;
+        int n = 0;
+        if (cs == 1) n = tc_sm_count();
+        else if (cudaOccupancyMaxActiveClusters(&n, v.fn, &cfg) != cudaSuccess) {
+            cudaGetLastError();
+            n = 0;
+        }
+        v.max_clusters[cs] = n;
+    }
+}
+// column classes: up to 16, 32 columns, more (64-column chunks)
+static const TcVariant &tc_variant(int wtype, int64_t N) {
+    static TcVariant table[64][2][3];   // per device: kernel attributes and occupancy are per-context properties
+    static bool ready[64] = {false};
+    static std::mutex mu;
+    int dev = 0;
+    cudaGetDevice(&dev);
+    dev &= 63;
+    std::lock_guard<std::mutex> lock(mu);
+    if (!ready[dev]) {
+        tc_make<B200_TYPE_Q4_0, 2>(table[dev][0][0]);
+        tc_make<B200_TYPE_Q4_0, 4>(table[dev][0][1]);
+        tc_make<B200_TYPE_Q4_0, 8>(table[dev][0][2]);
+        tc_make<B200_TYPE_Q8_0, 2>(table[dev][1][0]);
+        tc_make<B200_TYPE_Q8_0, 4>(table[dev][1][1]);
+        tc_make<B200_TYPE_Q8_0, 8>(table[dev][1][2]);
+        ready[dev] = true;
+    }
+    return table[dev][wtype == B200_TYPE_Q4_0 ? 0 : 1][N > 32 ? 2 : (N > 16 ? 1 : 0)];
 }
 
 // ---- tensor maps ----
@@ -444,30 +787,23 @@ static tc_encode_fn tc_encoder() {
     }();
     return fn;
 }
-// 2-D view: rows of `inner_words` 32-bit words, a box of box_words x 8 rows
-static bool tc_encode(CUtensorMap *m, const void *base, uint64_t inner_words, uint64_t rows, uint32_t box_words) {
+// rows of `line_words` 32-bit words x `lines` lines x `rows`, a box of one line (2-D: `box_lines` 1) or box_lines lines, 8 rows
+static bool tc_encode(CUtensorMap *m, const void *base, uint32_t line_words, uint64_t lines, uint64_t rows, uint32_t box_lines) {
     tc_encode_fn enc = tc_encoder();
     if (!enc) return false;
-    const cuuint64_t dims[2] = {inner_words, rows};
-    const cuuint64_t strides[1] = {inner_words * 4};
-    const cuuint32_t box[2] = {box_words, 8};
-    const cuuint32_t elem[2] = {1, 1};
-    return enc(m, CU_TENSOR_MAP_DATA_TYPE_UINT32, 2, const_cast<void *>(base), dims, strides, box, elem, CU_TENSOR_MAP_INTERLEAVE_NONE,
+    const cuuint32_t elem[3] = {1, 1, 1};
+    if (box_lines == 1) {
+        const cuuint64_t dims[2] = {line_words * lines, rows}, strides[1] = {line_words * lines * 4};
+        const cuuint32_t box[2] = {line_words, 8};
+        return enc(m, CU_TENSOR_MAP_DATA_TYPE_UINT32, 2, const_cast<void *>(base), dims, strides, box, elem, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                   CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+    }
+    const cuuint64_t dims[3] = {line_words, lines, rows}, strides[2] = {line_words * 4ull, line_words * lines * 4};
+    const cuuint32_t box[3] = {line_words, box_lines, 8};
+    return enc(m, CU_TENSOR_MAP_DATA_TYPE_UINT32, 3, const_cast<void *>(base), dims, strides, box, elem, CU_TENSOR_MAP_INTERLEAVE_NONE,
                CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
-// The packed weight tiles as lines of 128 bytes (8 lines per tile): [row tile][block group * 8 + line][32 words], a box of
-// 8 row tiles x one block group's 8 lines, written with the 128-byte swizzle (16-byte chunk c of line l at c ^ (l & 7)).
-static bool tc_encode_wq(CUtensorMap *m, const void *base, uint64_t n_bg, uint64_t n_rt) {
-    tc_encode_fn enc = tc_encoder();
-    if (!enc) return false;
-    const cuuint64_t dims[3] = {32, n_bg * 8, n_rt};
-    const cuuint64_t strides[2] = {128, n_bg * 1024};
-    const cuuint32_t box[3] = {32, 8, 8};
-    const cuuint32_t elem[3] = {1, 1, 1};
-    return enc(m, CU_TENSOR_MAP_DATA_TYPE_UINT32, 3, const_cast<void *>(base), dims, strides, box, elem, CU_TENSOR_MAP_INTERLEAVE_NONE,
-               CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
-}
-// encoded maps are pure functions of (pointer, extents): keep them, a model has a few hundred weights
+// encoded maps are pure functions of (pointer, type, extents): kept, a model has a few hundred weights
 struct TcKey {
     const void *p;
     int64_t a, b;
@@ -476,85 +812,125 @@ struct TcKey {
 struct TcKeyHash {
     size_t operator()(const TcKey &k) const { return std::hash<const void *>()(k.p) ^ (size_t) (k.a * 0x9E3779B97F4A7C15ull) ^ (size_t) (k.b * 0xC2B2AE3D27D4EB4Full); }
 };
-struct TcWeightMaps { CUtensorMap q, d; };
-struct TcActMaps { CUtensorMap h, l, s; };
-static bool tc_weight_maps(const TiledDims &d, const void *w, TcWeightMaps *out) {
+struct TcPair { CUtensorMap q, s; };
+static bool tc_weight_maps(int wtype, const TiledDims &d, const void *w, CUtensorMap &q, CUtensorMap &s) {
     static std::mutex mu;
-    static std::unordered_map<TcKey, TcWeightMaps, TcKeyHash> cache;
-    const TcKey key{w, d.n_rt, d.n_bg};
+    static std::unordered_map<TcKey, TcPair, TcKeyHash> cache;
+    const TcKey key{w, d.n_rt * 16 + wtype, d.n_bg};
     std::lock_guard<std::mutex> lock(mu);
     auto it = cache.find(key);
     if (it == cache.end()) {
-        TcWeightMaps p;
-        if (!tc_encode_wq(&p.q, w, (uint64_t) d.n_bg, (uint64_t) d.n_rt)) return false;
-        if (!tc_encode(&p.d, (const uint8_t *) w + d.qs_bytes, (uint64_t) d.n_bg * 32, (uint64_t) d.n_rt, 32)) return false;
+        TcPair p;
+        if (!tc_encode(&p.q, w, 256, (uint64_t) d.n_bg * (wtype == B200_TYPE_Q4_0 ? 1 : 2), (uint64_t) d.n_rt, wtype == B200_TYPE_Q4_0 ? 1 : 2)) return false;
+        if (!tc_encode(&p.s, (const uint8_t *) w + d.qs_bytes, 32, (uint64_t) d.n_bg, (uint64_t) d.n_rt, 1)) return false;
         if (cache.size() > 65536) cache.clear();
         it = cache.emplace(key, p).first;
     }
-    *out = it->second;
-    return true;
-}
-static bool tc_act_maps(const ActDims &a, const void *aq, TcActMaps *out) {
-    static std::mutex mu;
-    static std::unordered_map<TcKey, TcActMaps, TcKeyHash> cache;
-    const TcKey key{aq, a.n_nt, a.n_bg};
-    std::lock_guard<std::mutex> lock(mu);
-    auto it = cache.find(key);
-    if (it == cache.end()) {
-        TcActMaps p;
-        if (!tc_encode(&p.h, (const uint8_t *) aq + a.hi_offset, (uint64_t) a.nbp * 64, (uint64_t) a.n_nt, 256)) return false;
-        if (!tc_encode(&p.l, (const uint8_t *) aq + a.lo_offset, (uint64_t) a.nbp * 64, (uint64_t) a.n_nt, 256)) return false;
-        if (!tc_encode(&p.s, (const uint8_t *) aq + a.s2_offset, (uint64_t) a.n_bg * 64, (uint64_t) a.n_nt, 64)) return false;
-        if (cache.size() > 65536) cache.clear();
-        it = cache.emplace(key, p).first;
-    }
-    *out = it->second;
+    q = it->second.q;
+    s = it->second.s;
     return true;
 }
 
-int launch_mmq_tc(int wtype, const TiledDims &d, const void *w, const ActDims &a, const void *aq, float *dst, int64_t dst_nb_row,
-                  void *workspace, size_t workspace_bytes, cudaStream_t st) {
-    TcWeightMaps wm;
-    TcActMaps am;
-    if (wtype != B200_TYPE_Q4_0 || a.hi_offset == 0 || !is_aligned(w, 16) || !is_aligned(aq, 16) || !tc_weight_maps(d, w, &wm) || !tc_act_maps(a, aq, &am)) {
-        return launch_mmq(wtype, d, w, a, aq, dst, dst_nb_row, workspace, workspace_bytes, st, false, PeerDst{});
-    }
-    static bool configured[64] = {false};
-    int dev = 0;
-    cudaGetDevice(&dev);
-    if (!configured[dev & 63]) {
-        cudaError_t e = cudaFuncSetAttribute(mmq_tc_q4_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, TC_SMEM);
-        if (e != cudaSuccess) return set_error(B200_E_CUDA, "mmq_tc shared memory opt-in: %s", cudaGetErrorString(e));
-        configured[dev & 63] = true;
-    }
-    static const int mode = [] {   // debugging switches, see the kernel
-        const char *e = getenv("B200_TC_DEBUG");
+static size_t tc_slot_bytes(int nt) { return (size_t) nt * 8 * 256 * 4; }
+static size_t tc_counter_bytes(int64_t tiles) { return (size_t) ((tiles * 8 + 255) / 256 * 256); }
+// workspace of the equal-share split: a counter per tile, two parked parts per CTA
+size_t mmq_tc_workspace_bytes(int64_t M, int64_t N) {
+    const int nt = N > 32 ? 8 : (N > 16 ? 4 : 2);
+    const int64_t tiles = ((M + 127) / 128) * ((N + 8 * nt - 1) / (8 * nt));
+    return tc_counter_bytes(tiles) + (size_t) tc_sm_count() * 2 * tc_slot_bytes(nt);
+}
+
+// The work split, from what was measured on B200 (clocks per block group of a CTA: the MMAs, or the copies when a CTA has only 128
+// rows; a few block groups of fixed cost to start and to finish).
+static TcPlan tc_plan(const TcVariant &v, const TiledDims &d, const ActDims &a, bool workspace) {
+    static const int forced = [] {   // tuning aid: B200_TC_PLAN = 100 * (row tiles 8 / 16) + cluster size (0: equal shares)
+        const char *e = getenv("B200_TC_PLAN");
+        return e ? atoi(e) : -1;
+    }();
+    static const int debug = [] {
+        const char *e = getenv("B200_TCF_DEBUG");
         return e ? atoi(e) : 0;
     }();
+    TcPlan best = {};
+    double best_cost = -1;
+    const int chunk_nt = a.chunk_nt, chunks = (int) ((a.n_nt + chunk_nt - 1) / chunk_nt);
+    for (int rpg = 16; rpg >= 8; rpg -= 8) {
+        const int64_t groups = (d.n_rt + rpg - 1) / rpg, tiles = groups * chunks;
+        // clocks per block group: MMAs (96 per 16 values of K and 128 rows at 64 columns), against the copies at 40 B/clk
+        const double mma = (rpg / 8) * 8 * 12.0 * chunk_nt, copy = (rpg * (d.tile_bytes + 128) + chunk_nt * 4096) / 40.0;
+        // and what the hand-overs between the warps allow
+        const double unit = std::max(std::max(mma * 1.15, copy), 1400.0) / 1000.0;
+        for (int cs = 0; cs <= 8; ++cs) {
+            double cost;
+            if (cs == 0) {
+                // few tiles would have many parts each, which one CTA would have to add (tc_finish knows three)
+                const int64_t grid = std::min<int64_t>(tc_sm_count(), tiles * d.n_bg), share = tiles * d.n_bg / grid;
+                if (!workspace || 2 * share < d.n_bg || share / d.n_bg + 4 > TC_MAX_PIECES) continue;
+                cost = (double) (tiles * d.n_bg) / tc_sm_count() * unit + 2.0 * unit + 6.0;
+            } else {
+                if (cs > d.n_bg || v.max_clusters[cs] <= 0) continue;
+                const int64_t waves = (tiles + v.max_clusters[cs] - 1) / v.max_clusters[cs];
+                cost = waves * (((d.n_bg + cs - 1) / cs) * unit + 2.0 * unit + (cs > 1 ? 3.0 : 2.0));
+            }
+            if (forced >= 0 && forced != rpg * 100 + cs) continue;
+            if (best_cost < 0 || cost < best_cost) {
+                best_cost = cost;
+                best.rt_per_group = rpg;
+                best.groups = (int) groups;
+                best.chunks = chunks;
+                best.cs = cs;
+            }
+        }
+    }
+    if (best_cost < 0) {
+        best.rt_per_group = 16;
+        best.groups = (int) ((d.n_rt + 15) / 16);
+        best.chunks = chunks;
+        best.cs = 1;
+    }
+    best.debug = debug;
+    return best;
+}
+
+int launch_mmq_tc(int wtype, const TiledDims &d, const void *w, const ActDims &a, const void *aq, float *dst, int64_t dst_nb_row,
+                  void *workspace, size_t workspace_bytes, const PeerDst &peers, cudaStream_t st) {
+    const TcVariant &v = tc_variant(wtype, a.N);
     TcMaps maps;
-    maps.wq = wm.q; maps.wd = wm.d; maps.bh = am.h; maps.bl = am.l; maps.bs = am.s;
-    const int64_t row_groups = (d.n_rt + 7) / 8, col_chunks = (a.n_nt + 7) / 8;
-    // K splits: whole waves of one CTA per SM, a few block groups of fixed cost per split
-    const int64_t ctas = row_groups * col_chunks, slots = (int64_t) tc_sm_count();
-    int ks = 1;
-    int64_t best = -1;
-    for (int k = 1; k <= 16; ++k) {
-        const int64_t per = (d.n_bg + k - 1) / k;
-        if (k > 1 && per < 2) break;
-        const int64_t cost = ((ctas * k + slots - 1) / slots) * (per + 3) + (k > 1 ? 2 : 0);
-        if (best < 0 || cost < best) { best = cost; ks = k; }
+    for (int i = 0; i < std::max(1, peers.n_wseg); ++i) {
+        const int64_t M = peers.n_wseg == 0 ? d.M : (i == peers.n_wseg - 1 ? d.M : peers.seg_end[i]) - (i > 0 ? peers.seg_end[i - 1] : 0);
+        if (!tc_weight_maps(wtype, tiled_dims(wtype, d.K, M), peers.n_wseg == 0 ? w : peers.wseg[i], maps.q[i], maps.s[i]))
+            return set_error(B200_E_CUDA, "mmq_tc: no tensor map for the weights");
     }
-    const size_t per_split = (size_t) a.N * d.M * sizeof(float);
-    if (ks > 1 && (!workspace || workspace_bytes < per_split * ks)) ks = workspace ? (int) std::max<size_t>(1, workspace_bytes / per_split) : 1;
-    dim3 grid((unsigned) row_groups, (unsigned) col_chunks, (unsigned) ks);
-    cudaError_t le = launch_pdl(mmq_tc_q4_kernel, grid, dim3(TC_THREADS), (size_t) TC_SMEM, st, maps, d, a, dst, dst_nb_row, (float *) workspace, ks, mode);
-    if (le != cudaSuccess) return set_error(B200_E_CUDA, "mmq_tc launch: %s", cudaGetErrorString(le));
-    if (int e = check_launch("mmq_tc")) return e;
-    if (ks > 1) {
-        launch_mmq_reduce((const float *) workspace, ks, d.M, a.N, dst, dst_nb_row, st);
-        return check_launch("mmq_reduce");
+    const bool ws = workspace && workspace_bytes >= mmq_tc_workspace_bytes(d.M, a.N) && d.n_rt * d.n_bg * a.n_nt < (1ll << 31);
+    TcPlan plan = tc_plan(v, d, a, ws);
+    const int tiles = plan.groups * plan.chunks;
+    static std::atomic<unsigned long long> next_id{(unsigned long long) std::chrono::steady_clock::now().time_since_epoch().count() * 0x9E3779B97F4A7C15ull};
+    plan.launch_id = (next_id.fetch_add(1) & 0xffffffffffffffull) | 1ull << 55;   // never zero
+    const int64_t total = (int64_t) tiles * d.n_bg;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned) (plan.cs == 0 ? std::min<int64_t>(tc_sm_count(), total) : (int64_t) tiles * plan.cs));
+    plan.share = (uint32_t) (total / cfg.gridDim.x);
+    plan.extra = (uint32_t) (total % cfg.gridDim.x);
+    cfg.blockDim = dim3((unsigned) v.threads);
+    cfg.dynamicSmemBytes = (size_t) v.smem;
+    cfg.stream = st;
+    cudaLaunchAttribute attr[2];
+    int n = 0;
+    if (pdl_enabled()) {
+        attr[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[n++].val.programmaticStreamSerializationAllowed = 1;
     }
-    return B200_OK;
+    if (plan.cs > 1) {
+        attr[n].id = cudaLaunchAttributeClusterDimension;
+        attr[n].val.clusterDim.x = (unsigned) plan.cs;
+        attr[n].val.clusterDim.y = attr[n].val.clusterDim.z = 1;
+        ++n;
+    }
+    cfg.attrs = attr;
+    cfg.numAttrs = (unsigned) n;
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, v.fn, d, (const uint8_t *) w, a, (const uint8_t *) aq, dst, dst_nb_row, workspace, plan, peers, maps);
+    if (e != cudaSuccess) return set_error(B200_E_CUDA, "mmq_tc launch: %s", cudaGetErrorString(e));
+    return check_launch("mmq_tc");
 }
 
 int tc_error_flag() {
@@ -570,13 +946,3 @@ void tc_set_wait_limit(unsigned rounds) {
 }
 
 }  // namespace b200
-
-namespace b200 { int tcf_error_flag(); void tcf_set_wait_limit(unsigned rounds); }
-extern "C" B200_API int b200_kernel_status(void) { return b200::tc_error_flag() | (b200::tcf_error_flag() << 1); }
-extern "C" B200_API void b200_kernel_set_wait_limit(unsigned rounds) {
-    b200::tc_set_wait_limit(rounds);
-    b200::tcf_set_wait_limit(rounds);
-}
-#ifdef B200_TC_PROFILE
-extern "C" B200_API void b200_tc_profile(long long *out) { cudaMemcpyFromSymbol(out, b200::g_tc_prof, sizeof(long long) * 256); }
-#endif

@@ -1,21 +1,24 @@
 // C ABI of MUL_MAT: argument checks and the choice between the dp4a kernel (few columns, mmvq_max_n()) and the
 // tensor-core kernels.
+#include <algorithm>
+#include <cstdlib>
 #include <mutex>
 
 #include "common.cuh"
 
 namespace b200 {
-int act_layout(int64_t N);
 int launch_mmq_tc(int wtype, const TiledDims &d, const void *w, const ActDims &a, const void *aq, float *dst, int64_t dst_nb_row,
-                  void *workspace, size_t workspace_bytes, cudaStream_t st);
-int launch_mmq_tcf(int wtype, const TiledDims &d, const void *w, const ActDims &a, const void *aq, float *dst, int64_t dst_nb_row,
-                   void *workspace, size_t workspace_bytes, cudaStream_t st, int terms);
-int mmq_tc_mode();
+                  void *workspace, size_t workspace_bytes, const PeerDst &peers, cudaStream_t st);
+size_t mmq_tc_workspace_bytes(int64_t M, int64_t N);
+int tc_error_flag();
+void tc_set_wait_limit(unsigned rounds);
+bool mmq_sync_forced();
+int launch_quantize_b8(const float *x, int64_t x_nb_row, int64_t K, int64_t N, void *scratch, int variant, int layout, cudaStream_t st);
 int mmvq_max_n();
 int launch_mmvq(int wtype, const TiledDims &d, const void *w, const ActDims &a, const void *aq, float *dst, int64_t dst_nb_row, const PeerDst &peers,
                 cudaStream_t st);
 int launch_mmq(int wtype, const TiledDims &d, const void *w, const ActDims &a, const void *aq, float *dst, int64_t dst_nb_row,
-               void *workspace, size_t workspace_bytes, cudaStream_t st, bool canon, const PeerDst &peers);
+               void *workspace, size_t workspace_bytes, cudaStream_t st, const PeerDst &peers);
 int launch_peer_signal_wait(void *const *flags_of_rank, int rank, int g, cudaStream_t st);
 size_t mmq_workspace_bytes(int wtype, int64_t K, int64_t M, int64_t N);
 }  // namespace b200
@@ -54,7 +57,35 @@ static bool shape_ok(int wtype, int64_t K, int64_t M, int64_t N) {
     return (wtype == B200_TYPE_Q4_0 || wtype == B200_TYPE_Q8_0) && K > 0 && K % 32 == 0 && M > 0 && N > 0;
 }
 
+// b200_mul_mat_q alone chooses between the two tensor-core kernels: it knows the weights' shape when it quantises, and the
+// tcgen05 kernel wants its operands laid out by the quantiser.  (Products of activations that are quantised on their own feed
+// whole models, whose results stay bit for bit what they were: every product re-quantises its input, so a last-bit
+// difference in one sum is a different rounding somewhere in the next.)
+// Measured on B200 (us, tcgen05 / mma.sync kernel): up to 32 columns the latter is as fast or faster at every size
+// (4096 x 28672: 37.7 / 38.2 at 32, 34.0 / 22.6 at 16).  From there on the tensor core wins where there is enough work to
+// fill its pipeline, which takes about 5 us to start and to finish:
+//   K x M            N = 40        64           80            256
+//   4096 x 28672     39.7 / 56.6   44.3 / 57.8   62.9 / 103.4   131 / 177
+//   14336 x 4096     27.4 / 28.6   30.1 / 28.7   35.8 / 49.0    71.1 / 91.3
+//   4096 x 6144      15.1 / 17.2   16.8 / 17.2   22.4 / 24.9    37.6 / 47.6
+//   4096 x 4096      13.5 / 12.8   13.9 / 13.0   15.8 / 17.9    24.7 / 30.8
+//   2048 x 2048       9.2 / 8.0     9.1 / 8.0    10.5 / 9.1     13.1 / 11.8
+// so: one column chunk needs 24 row groups (a K split over at most five CTAs), more chunks 8 M weights.
+// B200_MMQ_TC decides by hand (0: never, else from 9 columns on).
+static bool use_tc(int64_t K, int64_t M, int64_t N) {
+    static const int forced = [] {
+        const char *e = getenv("B200_MMQ_TC");
+        return e ? atoi(e) : -1;
+    }();
+    if (forced == 0 || N < 9 || mmq_sync_forced()) return false;
+    if (forced > 0) return true;
+    return N > 64 ? M * K >= (8 << 20) : N > 32 && M >= 6144 && K >= 1024;
+}
+
 extern "C" {
+
+int b200_kernel_status(void) { return tc_error_flag() ? 2 : 0; }
+void b200_kernel_set_wait_limit(unsigned rounds) { tc_set_wait_limit(rounds); }
 
 size_t b200_mul_mat_workspace_bytes(int wtype, int64_t K, int64_t M, int64_t N) {
     if (!shape_ok(wtype, K, M, N)) return 0;
@@ -63,7 +94,8 @@ size_t b200_mul_mat_workspace_bytes(int wtype, int64_t K, int64_t M, int64_t N) 
 
 size_t b200_mul_mat_scratch_bytes(int wtype, int64_t K, int64_t M, int64_t N) {
     if (!shape_ok(wtype, K, M, N)) return 0;
-    return b200_act_bytes(K, N) + mmq_workspace_bytes(wtype, K, M, N);
+    const ActDims a = act_dims(K, N);
+    return a.total_bytes + (use_tc(K, M, N) ? a.b_bytes + mmq_tc_workspace_bytes(M, N) : mmq_workspace_bytes(wtype, K, M, N));
 }
 
 static int mul_mat_prequant(int wtype, const void *w, int64_t K, int64_t M, const void *act, int64_t N, float *dst, int64_t dst_row_stride_bytes,
@@ -130,15 +162,7 @@ static int mul_mat_prequant(int wtype, const void *w, int64_t K, int64_t M, cons
     const TiledDims d = tiled_dims(wtype, K, M);
     const ActDims a = act_dims(K, N);
     if (N <= mmvq_max_n()) return launch_mmvq(wtype, d, w, a, act, dst, dst_row_stride_bytes, peers, (cudaStream_t) stream);
-    // the tcgen05 kernel reads the e4m3 planes, multiplies Q4_0 weights and writes one destination; everything else (Q8_0
-    // weights, a row-split product) takes the mma.sync kernel on the fragment-order plane that is always there
-    if (act_layout(N) == 3 && wtype == B200_TYPE_Q4_0 && peers.n == 0 && peers.n_seg <= 1) {
-        return launch_mmq_tc(wtype, d, w, a, act, dst, dst_row_stride_bytes, workspace, workspace_bytes, (cudaStream_t) stream);
-    }
-    if (mmq_tc_mode() >= 2 && N >= 16 && wtype == B200_TYPE_Q4_0 && peers.n == 0 && peers.n_seg <= 1) {
-        return launch_mmq_tcf(wtype, d, w, a, act, dst, dst_row_stride_bytes, workspace, workspace_bytes, (cudaStream_t) stream, mmq_tc_mode() == 2 ? 3 : 2);
-    }
-    return launch_mmq(wtype, d, w, a, act, dst, dst_row_stride_bytes, workspace, workspace_bytes, (cudaStream_t) stream, false, peers);
+    return launch_mmq(wtype, d, w, a, act, dst, dst_row_stride_bytes, workspace, workspace_bytes, (cudaStream_t) stream, peers);
 }
 
 int b200_mul_mat_q_prequant_multi(int wtype, int n_weights, const void *const *w, const int64_t *M, int64_t K, const void *act, int64_t N,
@@ -176,17 +200,25 @@ int b200_mul_mat_q_prequant_multi(int wtype, int n_weights, const void *const *w
     }
     const TiledDims d = tiled_dims(wtype, K, total);
     const ActDims a = act_dims(K, N);
-    return launch_mmq(wtype, d, w[0], a, act, dst[0], dst_row_stride_bytes, workspace, workspace_bytes, (cudaStream_t) stream, false, segs);
+    return launch_mmq(wtype, d, w[0], a, act, dst[0], dst_row_stride_bytes, workspace, workspace_bytes, (cudaStream_t) stream, segs);
 }
 
 int b200_mul_mat_q(int wtype, const void *w, int64_t K, int64_t M, const float *x, int64_t x_row_stride_bytes, int64_t N,
                    float *dst, int64_t dst_row_stride_bytes, void *scratch, size_t scratch_bytes, int variant, b200_stream_t stream) {
     B200_REQUIRE(shape_ok(wtype, K, M, N), "bad mul_mat shape/type: type %d K %lld M %lld N %lld", wtype, (long long) K, (long long) M, (long long) N);
-    const size_t ab = b200_act_bytes(K, N);
-    const size_t wb = mmq_workspace_bytes(wtype, K, M, N);
+    const ActDims a = act_dims(K, N);
+    const bool tc = use_tc(K, M, N);
+    const size_t ab = a.total_bytes + (tc ? a.b_bytes : 0), wb = tc ? mmq_tc_workspace_bytes(M, N) : mmq_workspace_bytes(wtype, K, M, N);
     if (!scratch || scratch_bytes < ab + wb) return set_error(B200_E_SCRATCH, "scratch too small: %zu < %zu", scratch_bytes, ab + wb);
-    if (int e = b200_quantize_activations(x, x_row_stride_bytes, K, N, scratch, ab, variant, stream)) return e;
-    return b200_mul_mat_q_prequant(wtype, w, K, M, scratch, N, dst, dst_row_stride_bytes, wb ? (char *) scratch + ab : nullptr, wb, stream);
+    if (!tc) {
+        if (int e = b200_quantize_activations(x, x_row_stride_bytes, K, N, scratch, ab, variant, stream)) return e;
+        return b200_mul_mat_q_prequant(wtype, w, K, M, scratch, N, dst, dst_row_stride_bytes, wb ? (char *) scratch + ab : nullptr, wb, stream);
+    }
+    B200_REQUIRE(w && x && dst && is_aligned(w, 16) && is_aligned(x, 4) && is_aligned(dst, 4) && is_aligned(scratch, 256), "null or misaligned pointer");
+    B200_REQUIRE(x_row_stride_bytes % 4 == 0 && dst_row_stride_bytes % 4 == 0 && dst_row_stride_bytes >= M * 4, "bad row stride");
+    B200_REQUIRE(variant == B200_Q8_AVX2 || variant == B200_Q8_SCALAR, "unknown quantiser variant %d", variant);
+    if (int e = launch_quantize_b8(x, x_row_stride_bytes, K, N, scratch, variant, 2, (cudaStream_t) stream)) return e;
+    return launch_mmq_tc(wtype, tiled_dims(wtype, K, M), w, a, scratch, dst, dst_row_stride_bytes, (char *) scratch + ab, wb, PeerDst{}, (cudaStream_t) stream);
 }
 
 int b200_mul_mat_q_noalloc(int wtype, const void *w, int64_t K, int64_t M, const float *x, int64_t x_row_stride_bytes, int64_t N,

@@ -9,13 +9,13 @@ namespace b200 {
 // ---------------------------------------------------------------------------------------------
 // quantize_row_q8_0 (cactus/ggml-cpu/ggml-cpu-quants.c:732-1045).  8 threads per 32-element block,
 // 4 elements each; the block maximum is reduced with three shuffles.  LAYOUT 0 writes the reference's
-// block_q8_0 stream, LAYOUT 1 the B8 scratch layout (mma.sync fragment order), LAYOUT 3 that plus the e4m3 planes in
-// the K-major core-matrix order the tcgen05 kernel's shared-memory descriptors expect (common.cuh, ACT_F8_MIN_N).
+// block_q8_0 stream, LAYOUT 1 the B8 scratch layout (mma.sync fragment order), LAYOUT 2 that plus the fp16
+// operands of the tcgen05 kernel (common.cuh).
 // ---------------------------------------------------------------------------------------------
 template <int LAYOUT>
 __global__ void __launch_bounds__(256) quantize_q8_0_kernel(const float *__restrict__ x, int64_t x_nb_row, int64_t K,
                                                            int64_t N, int64_t n_rows_padded, int64_t nb, int64_t nbp,
-                                                           uint8_t *__restrict__ out, size_t d_offset, int variant, int early) {
+                                                           uint8_t *__restrict__ out, size_t d_offset, int variant, int early, int chunk_nt) {
     pdl_prologue(early != 0);
     const int64_t gid = (int64_t) blockIdx.x * blockDim.x + threadIdx.x;
     const int j = (int) (gid & 7);             // which group of 4 elements inside the block
@@ -36,7 +36,7 @@ __global__ void __launch_bounds__(256) quantize_q8_0_kernel(const float *__restr
             v[0] = row[0]; v[1] = row[1]; v[2] = row[2]; v[3] = row[3];
         }
     }
-    q8_quantize_store<LAYOUT>(v, out, d_offset, nb, nbp, n, b, j, real, variant);
+    q8_quantize_store<LAYOUT>(v, out, d_offset, nb, nbp, n, b, j, real, variant, chunk_nt);
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -211,28 +211,10 @@ int launch_quantize_b8(const float *x, int64_t x_nb_row, int64_t K, int64_t N, v
     const int64_t threads = a.n_nt * 8 * a.nbp * 8;
     const int64_t grid = (threads + 255) / 256;
     const int early = N <= pdl_early_rows() ? 1 : 0;
-    if (layout == 3) launch_pdl(quantize_q8_0_kernel<3>, dim3((unsigned) grid), dim3(256), 0, st, x, x_nb_row, K, N, a.n_nt * 8, a.nb, a.nbp, (uint8_t *) scratch, a.d_offset, variant, early);
-    else launch_pdl(quantize_q8_0_kernel<1>, dim3((unsigned) grid), dim3(256), 0, st, x, x_nb_row, K, N, a.n_nt * 8, a.nb, a.nbp, (uint8_t *) scratch, a.d_offset, variant, early);
+    if (layout == 2) launch_pdl(quantize_q8_0_kernel<2>, dim3((unsigned) grid), dim3(256), 0, st, x, x_nb_row, K, N, a.n_nt * 8, a.nb, a.nbp, (uint8_t *) scratch, a.d_offset, variant, early, a.chunk_nt);
+    else launch_pdl(quantize_q8_0_kernel<1>, dim3((unsigned) grid), dim3(256), 0, st, x, x_nb_row, K, N, a.n_nt * 8, a.nb, a.nbp, (uint8_t *) scratch, a.d_offset, variant, early, a.chunk_nt);
     return check_launch("quantize_q8_0 (activations)");
 }
-
-// What the quantised activations of an N-column product hold: 1 = the B8 tiles in fragment order, which the dp4a and
-// mma.sync kernels read; 3 = those plus the e4m3 planes of the tcgen05 kernel (ACT_F8_MIN_N columns and more; the
-// scratch of such a product always has room for them).  The tcgen05 kernel is taken with B200_MMQ_TC=1: it passes every
-// parity case, but at the decode width of 64 columns it does not beat the mma.sync kernel yet (see mmq_tc.cu).
-// B200_MMQ_TC: 0 mma.sync kernel, 1 the per-block tcgen05 kernel (mmq_tc.cu), 2 / 3 the folded-scale tcgen05 kernel
-// (mmq_tcf.cu) with 3 / 2 product terms.
-int mmq_tc_mode() {
-    static const int mode = [] {
-        const char *e = getenv("B200_MMQ_TC");
-        int mode = e ? atoi(e) : 0;
-        if (mode < 0 || mode > 3) mode = 0;
-        return mode;
-    }();
-    return mode;
-}
-bool mmq_tc_enabled() { return mmq_tc_mode() == 1; }
-int act_layout(int64_t N) { return (N >= ACT_F8_MIN_N && mmq_tc_enabled()) ? 3 : 1; }
 
 }  // namespace b200
 
@@ -288,7 +270,7 @@ int b200_quantize_q8_0(const float *x, int64_t x_row_stride_bytes, int64_t K, in
     const int64_t nb = K / 32;
     const int64_t threads = N * nb * 8;
     quantize_q8_0_kernel<0><<<(unsigned) ((threads + 255) / 256), 256, 0, (cudaStream_t) stream>>>(
-        x, x_row_stride_bytes, K, N, N, nb, nb, (uint8_t *) dst_blocks, 0, variant, 0);
+        x, x_row_stride_bytes, K, N, N, nb, nb, (uint8_t *) dst_blocks, 0, variant, 0, 2);
     return check_launch("quantize_q8_0");
 }
 
@@ -305,7 +287,7 @@ int b200_quantize_activations(const float *x, int64_t x_row_stride_bytes, int64_
     B200_REQUIRE(is_aligned(x, 4) && x_row_stride_bytes % 4 == 0, "misaligned activations");
     B200_REQUIRE(is_aligned(scratch, 256), "scratch must be 256-byte aligned");
     if (scratch_bytes < act_dims(K, N).total_bytes) return set_error(B200_E_SCRATCH, "scratch too small: %zu < %zu", scratch_bytes, act_dims(K, N).total_bytes);
-    return launch_quantize_b8(x, x_row_stride_bytes, K, N, scratch, variant, act_layout(N), (cudaStream_t) stream);
+    return launch_quantize_b8(x, x_row_stride_bytes, K, N, scratch, variant, 1, (cudaStream_t) stream);
 }
 
 int b200_block_dots(int wtype, const void *w, int64_t K, int64_t M, const float *x, int64_t x_row_stride_bytes, int64_t N,

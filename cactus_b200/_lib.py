@@ -100,6 +100,28 @@ def lib() -> C.CDLL:
     return _lib
 
 
+_host = None
+
+
+def host():
+    """The native host path of the single-op entry points (csrc/host/ops_host.cpp); like the kernels, without a fallback."""
+    global _host
+    if _host is None:
+        import importlib.machinery
+        import importlib.util
+
+        import torch  # noqa: F401  (its libraries have to be loaded first)
+        lib()
+        path = os.path.join(HERE, "lib", "_ops_host.so")
+        if not os.path.exists(path):
+            raise B200Error(f"{path} is missing: build it with `python -m cactus_b200.build`")
+        spec = importlib.util.spec_from_file_location("_ops_host", path, loader=importlib.machinery.ExtensionFileLoader("_ops_host", path))
+        m = importlib.util.module_from_spec(spec)
+        spec.loader.exec_module(m)
+        _host = m
+    return _host
+
+
 def check(rc: int) -> None:
     if rc != 0:
         raise B200Error(f"cactus_b200 error {rc}: {lib().b200_last_error().decode()}")

@@ -13,6 +13,7 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 OUT = os.path.join(HERE, "lib")
 LIB = os.path.join(OUT, "libcactus_b200.so")
+HOST_LIB = os.path.join(OUT, "_ops_host.so")   # the Python-facing host path (needs torch's headers)
 SOURCES = ["abi.cu", "quantize.cu", "mmvq.cu", "mmq.cu", "mmq_tc.cu", "mul_mat.cu", "fattn.cu", "rowops.cu", "kvops.cu", "fused.cu", "peer.cu"]
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
@@ -61,7 +62,26 @@ def build(force: bool = False, verbose: bool = False) -> str:
                 print(log)
     if jobs or force or _stale(LIB, objs):
         run([nvcc(), "-shared", "-o", LIB, *objs, "-gencode", "arch=compute_100a,code=sm_100a", "-lcudart"])
+    build_host(force)
     return LIB
+
+
+def build_host(force: bool = False) -> str:
+    src = os.path.join(CSRC, "host", "ops_host.cpp")
+    if force or _stale(HOST_LIB, [src, os.path.join(os.path.dirname(HERE), "include", "cactus_b200.h")]):
+        import sysconfig
+
+        import torch
+        from torch.utils.cpp_extension import include_paths
+        tlib = os.path.join(os.path.dirname(torch.__file__), "lib")
+        cuda = os.path.dirname(os.path.dirname(nvcc())) if os.path.isabs(nvcc()) else "/usr/local/cuda"
+        cmd = ["g++", "-O2", "-std=c++17", "-shared", "-fPIC", "-fvisibility=hidden", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+               *[f"-I{p}" for p in (*include_paths(), sysconfig.get_paths()["include"], os.path.join(cuda, "include"))], src, "-o", HOST_LIB,
+               f"-L{OUT}", "-lcactus_b200", f"-L{tlib}", "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_python", "-Wl,-rpath,$ORIGIN"]
+        r = subprocess.run(cmd, capture_output=True, text=True)
+        if r.returncode != 0:
+            raise RuntimeError("g++ failed:\n" + " ".join(cmd) + "\n" + r.stdout + r.stderr)
+    return HOST_LIB
 
 
 if __name__ == "__main__":

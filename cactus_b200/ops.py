@@ -10,6 +10,7 @@ from __future__ import annotations
 import numpy as np
 import torch
 
+from . import _lib
 from ._lib import B200Error, check, lib
 
 Q4_0, Q8_0 = 2, 8
@@ -94,18 +95,7 @@ def quantize_row_q8_0(x: torch.Tensor, variant: int = Q8_AVX2) -> torch.Tensor:
 def mul_mat(w: QWeight, x: torch.Tensor, variant: int = Q8_AVX2, out: torch.Tensor | None = None,
             scratch: torch.Tensor | None = None) -> torch.Tensor:
     """dst[n, m] = sum_k W[m, k] x[n, k]  (ggml: dst = mul_mat(w, x) with ne = [M, N])."""
-    _need_cuda(x)
-    assert x.dtype == torch.float32 and x.dim() == 2 and x.stride(1) == 1 and x.shape[1] == w.K
-    L = lib()
-    N = x.shape[0]
-    if out is None:
-        out = torch.empty((N, w.M), dtype=torch.float32, device=x.device)
-    need = L.b200_mul_mat_scratch_bytes(w.wtype, w.K, w.M, N)
-    if scratch is None or scratch.numel() < need:
-        scratch = torch.empty(need, dtype=torch.uint8, device=x.device)
-    check(L.b200_mul_mat_q(w.wtype, w.data.data_ptr(), w.K, w.M, x.data_ptr(), x.stride(0) * 4, N, out.data_ptr(),
-                           out.stride(0) * 4, scratch.data_ptr(), scratch.numel(), variant, _stream()))
-    return out
+    return (_lib._host or _lib.host()).mul_mat(w.wtype, w.K, w.M, w.data, x, variant, out, scratch)
 
 
 def block_dots(w: QWeight, x: torch.Tensor, variant: int = Q8_AVX2) -> torch.Tensor:
@@ -124,32 +114,25 @@ def flash_attn_ext(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, mask: torc
     """q f32 [Nq, H, D]; k, v f16 [cells, Hkv, D] (the cache; the first n_kv cells are attended);
     mask f16 [>=Nq, n_kv] -> f32 [Nq, H, D].  ``parity=True`` runs the slow validation kernel that follows the
     reference's order of roundings (fp16 output accumulator) instead of the fast fp32-accumulating one."""
+    n_kv = k.shape[0] if n_kv is None else n_kv
+    if not parity:
+        return (_lib._host or _lib.host()).flash_attn_ext(q, k, v, mask, scale, max_bias, logit_softcap, n_kv)
     _need_cuda(q, k, v, mask)
     L = lib()
     Nq, H, D = q.shape
     Hkv = k.shape[1]
-    n_kv = k.shape[0] if n_kv is None else n_kv
     assert q.dtype == torch.float32 and k.dtype == torch.float16 and v.dtype == torch.float16
     assert q.stride(2) == 1 and k.stride(2) == 1 and v.stride(2) == 1
     out = torch.empty((Nq, H, D), dtype=torch.float32, device=q.device)
-    need = L.b200_flash_attn_scratch_bytes(D, H, Hkv, Nq, n_kv)
-    scratch = torch.empty(max(need, 256), dtype=torch.uint8, device=q.device)
+    index = None
     if mask is not None:
         assert mask.dtype == torch.float16 and mask.stride(1) == 1 and mask.shape[1] >= n_kv
-    if parity:
-        index = None
-        if mask is not None:
-            index = torch.empty(L.b200_mask_index_bytes(Nq, n_kv), dtype=torch.uint8, device=q.device)
-            check(L.b200_mask_index_build(mask.data_ptr(), mask.stride(0) * 2, Nq, n_kv, index.data_ptr(), index.numel(), _stream()))
-        check(L.b200_flash_attn_ext_parity(D, H, Hkv, Nq, n_kv, q.data_ptr(), q.stride(0) * 4, q.stride(1) * 4,
-                                           k.data_ptr(), k.stride(0) * 2, k.stride(1) * 2, v.data_ptr(), v.stride(0) * 2, v.stride(1) * 2,
-                                           mask.data_ptr() if mask is not None else None, mask.stride(0) * 2 if mask is not None else 0,
-                                           index.data_ptr() if index is not None else None, scale, max_bias, logit_softcap, out.data_ptr(), _stream()))
-        return out
-    check(L.b200_flash_attn_ext(D, H, Hkv, Nq, n_kv, q.data_ptr(), q.stride(0) * 4, q.stride(1) * 4,
-                                k.data_ptr(), k.stride(0) * 2, k.stride(1) * 2, v.data_ptr(), v.stride(0) * 2, v.stride(1) * 2,
-                                mask.data_ptr() if mask is not None else None, mask.stride(0) * 2 if mask is not None else 0,
-                                scale, max_bias, logit_softcap, out.data_ptr(), scratch.data_ptr(), scratch.numel(), _stream()))
+        index = torch.empty(L.b200_mask_index_bytes(Nq, n_kv), dtype=torch.uint8, device=q.device)
+        check(L.b200_mask_index_build(mask.data_ptr(), mask.stride(0) * 2, Nq, n_kv, index.data_ptr(), index.numel(), _stream()))
+    check(L.b200_flash_attn_ext_parity(D, H, Hkv, Nq, n_kv, q.data_ptr(), q.stride(0) * 4, q.stride(1) * 4,
+                                       k.data_ptr(), k.stride(0) * 2, k.stride(1) * 2, v.data_ptr(), v.stride(0) * 2, v.stride(1) * 2,
+                                       mask.data_ptr() if mask is not None else None, mask.stride(0) * 2 if mask is not None else 0,
+                                       index.data_ptr() if index is not None else None, scale, max_bias, logit_softcap, out.data_ptr(), _stream()))
     return out
 
 

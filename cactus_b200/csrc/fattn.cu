@@ -96,24 +96,56 @@ __global__ void __launch_bounds__(1024) fattn_plan_kernel(const int32_t *__restr
     __syncthreads();
     if (threadIdx.x == 0) {
         plan[0] = (int32_t) min(total_s, (long long) 0x7fffffff);
-        plan[1] = 0;   // filled by fattn_tile_vote_kernel
     }
 }
 
 // Fourth pass: how much the tokens of a ubatch share their cells.  plan[1] = the sum, over groups of 16 consecutive
 // tokens, of the number of mask words any token of the group attends to.  Against plan[0] (the same sum token by token)
 // it tells whether walking the cells once per group (fattn_tile_kernel) beats walking them once per token: a prompt's
-// tokens share nearly all their words, the tokens of a decode batch share none.
-__global__ void __launch_bounds__(256) fattn_tile_vote_kernel(const unsigned long long *__restrict__ words, int64_t Nq, int64_t nw, int32_t *__restrict__ plan) {
-    const int64_t t0 = (int64_t) blockIdx.x * 16, t1 = min(Nq, t0 + 16);
-    int cnt = 0;
+// tokens share nearly all their words, the tokens of a decode batch share none.  And the same for every tile the
+// query-tiled kernel may use (4, 8, 16 or 32 tokens): tiles whose tokens share little (decode tokens beside a prompt) are
+// flagged and listed, their tokens are walked one by one (plan[4 + k] = listed tiles of 4 << k tokens).  The line lies at
+// three tokens per word: a shared chunk costs its CTA about as much as two to three chunks of single tokens cost theirs.
+__global__ void __launch_bounds__(256) fattn_tile_vote_kernel(const unsigned long long *__restrict__ words, const int32_t *__restrict__ wcount, int64_t Nq, int64_t nw,
+                                                             int32_t *__restrict__ plan, int32_t *__restrict__ flags, int32_t *__restrict__ lists, int64_t stride) {
+    const int64_t t0 = (int64_t) blockIdx.x * 32;
+    const int n = (int) min((int64_t) 32, Nq - t0);
+    int cnt[15];   // words of: 8 groups of 4 tokens, 4 of 8, 2 of 16, 1 of 32
+#pragma unroll
+    for (int i = 0; i < 15; ++i) cnt[i] = 0;
     for (int64_t wi = threadIdx.x; wi < nw; wi += blockDim.x) {
-        unsigned long long bits = 0;
-        for (int64_t j = t0; j < t1; ++j) bits |= words[j * nw + wi];
-        cnt += bits != 0ull;
+        unsigned nz = 0;
+#pragma unroll 8
+        for (int j = 0; j < n; ++j) nz |= (words[(t0 + j) * nw + wi] != 0ull ? 1u : 0u) << j;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) cnt[i] += ((nz >> (4 * i)) & 0xfu) != 0;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) cnt[8 + i] += ((nz >> (8 * i)) & 0xffu) != 0;
+#pragma unroll
+        for (int i = 0; i < 2; ++i) cnt[12 + i] += ((nz >> (16 * i)) & 0xffffu) != 0;
+        cnt[14] += nz != 0;
     }
-    for (int o = 16; o > 0; o >>= 1) cnt += __shfl_xor_sync(0xffffffffu, cnt, o);
-    if ((threadIdx.x & 31) == 0 && cnt) atomicAdd(plan + 1, cnt);
+    __shared__ int sum[15];
+    if (threadIdx.x < 15) sum[threadIdx.x] = 0;
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < 15; ++i) {
+        int c = cnt[i];
+        for (int o = 16; o > 0; o >>= 1) c += __shfl_xor_sync(0xffffffffu, c, o);
+        if ((threadIdx.x & 31) == 0 && c) atomicAdd(sum + i, c);
+    }
+    __syncthreads();
+    if (threadIdx.x < 15) {
+        const int i = threadIdx.x, k = i < 8 ? 0 : (i < 12 ? 1 : (i < 14 ? 2 : 3)), first = k == 0 ? i : (k == 1 ? i - 8 : (k == 2 ? i - 12 : 0)), size = 4 << k;
+        if (first * size < n) {
+            if (k == 2) atomicAdd(plan + 1, sum[i]);
+            int64_t own = 0;
+            for (int j = first * size; j < min(n, (first + 1) * size); ++j) own += wcount[t0 + j];
+            const int32_t tile = (int32_t) (t0 / size + first), few = own < 3ll * sum[i] ? 1 : 0;
+            flags[k * stride + tile] = few;
+            if (few) lists[k * stride + atomicAdd(plan + 4 + k, 1)] = tile;
+        }
+    }
 }
 // the choice both attention kernels derive from the plan: true = the query-tiled kernel does the work
 __device__ __forceinline__ bool fattn_tiled_chosen(const int32_t *plan) { return 2ll * plan[1] <= (long long) plan[0]; }
@@ -137,6 +169,8 @@ struct FattnParams {
     int nsplit, hgroups;
     int w0;          // > 0: a token gets ceil(words / w0) KV splits (at most nsplit), so long sequences are cut, short ones are not;
                      // < 0: w0 is derived on the device from the mask's total word count (fattn_target_words)
+    const int32_t *tflags, *tlist, *tcount;   // query-tiled kernel: tiles whose tokens share few cells (flag per tile, list, length of the list)
+    int spread_rows;               // query-tiled kernel: grid rows whose CTAs take those tiles' tokens one by one
     const int32_t *order, *plan;   // tokens by decreasing word count; plan[0] = total words (NULL without a mask index)
     int slots;       // CTAs of this kernel the device holds at once
     int vote;        // both attention kernels were launched and the plan decides which one works (the other returns at once):
@@ -626,17 +660,21 @@ extern "C" {
 
 // index layout: words [Nq][nw] u64 | list of non-empty word indices [Nq][nw] i32 | their counts [Nq] i32 |
 // tokens by decreasing count [Nq] i32 | plan: total words i32, words summed over 16-token groups i32, 1 if the mask
-// holds values other than 0 and -inf in participating cells i32
+// holds values other than 0 and -inf in participating cells i32, unused, listed tiles of 4, 8, 16, 32 tokens 4 x i32 |
+// flag per tile, 4 x [Nq / 4] i32 | lists of flagged tiles, 4 x [Nq / 4] i32
 static size_t index_list_offset(int64_t Nq, int64_t nw) { return align_up((size_t) Nq * nw * 8, 256); }
 static size_t index_count_offset(int64_t Nq, int64_t nw) { return index_list_offset(Nq, nw) + align_up((size_t) Nq * nw * 4, 256); }
 
 static size_t index_order_offset(int64_t Nq, int64_t nw) { return index_count_offset(Nq, nw) + align_up((size_t) Nq * 4, 256); }
 static size_t index_plan_offset(int64_t Nq, int64_t nw) { return index_order_offset(Nq, nw) + align_up((size_t) Nq * 4, 256); }
 
+static size_t index_tiles_offset(int64_t Nq, int64_t nw) { return index_plan_offset(Nq, nw) + 256; }
+static int64_t index_tiles_stride(int64_t Nq) { return (Nq + 255) / 256 * 64; }   // of one flag array or list, in elements
+
 size_t b200_mask_index_bytes(int64_t Nq, int64_t n_kv) {
     if (Nq <= 0 || n_kv <= 0) return 0;
     const int64_t nw = (n_kv + 63) / 64;
-    return index_plan_offset(Nq, nw) + 256;
+    return index_tiles_offset(Nq, nw) + 8 * index_tiles_stride(Nq) * 4;
 }
 
 int b200_mask_index_build(const void *mask, int64_t mask_nb_row, int64_t Nq, int64_t n_kv, void *index, size_t index_bytes,
@@ -647,7 +685,7 @@ int b200_mask_index_build(const void *mask, int64_t mask_nb_row, int64_t Nq, int
     const int64_t nw = (n_kv + 63) / 64;
     const int64_t threads = Nq * nw * 32;
     int32_t *plan = (int32_t *) ((char *) index + index_plan_offset(Nq, nw));
-    if (!cuda_memset_ok(plan + 2, 4, (cudaStream_t) stream)) return set_error(B200_E_CUDA, "mask index: cudaMemsetAsync failed");
+    if (!cuda_memset_ok(plan, 32, (cudaStream_t) stream)) return set_error(B200_E_CUDA, "mask index: cudaMemsetAsync failed");
     mask_index_kernel<<<(unsigned) ((threads + 255) / 256), 256, 0, (cudaStream_t) stream>>>(
         (const __half *) mask, mask_nb_row, Nq, n_kv, nw, (unsigned long long *) index, plan + 2);
     if (int e = check_launch("mask_index")) return e;
@@ -660,8 +698,10 @@ int b200_mask_index_build(const void *mask, int64_t mask_nb_row, int64_t Nq, int
                                                              (int32_t *) ((char *) index + index_plan_offset(Nq, nw)));
     if (int e = check_launch("fattn_plan")) return e;
     if (Nq >= fattn_tile_min_nq() && fattn_tile_min_nq() > 0) {   // only ubatches the query-tiled kernel may take need the vote
-        fattn_tile_vote_kernel<<<(unsigned) ((Nq + 15) / 16), 256, 0, (cudaStream_t) stream>>>((const unsigned long long *) index, Nq, nw,
-                                                                                                 (int32_t *) ((char *) index + index_plan_offset(Nq, nw)));
+        int32_t *flags = (int32_t *) ((char *) index + index_tiles_offset(Nq, nw));
+        const int64_t stride = index_tiles_stride(Nq);
+        fattn_tile_vote_kernel<<<(unsigned) ((Nq + 31) / 32), 256, 0, (cudaStream_t) stream>>>(
+            (const unsigned long long *) index, (const int32_t *) ((char *) index + index_count_offset(Nq, nw)), Nq, nw, plan, flags, flags + 4 * stride, stride);
         return check_launch("fattn_tile_vote");
     }
     return B200_OK;
@@ -730,6 +770,8 @@ static int flash_attn_impl(bool parity, int64_t D, int64_t H, int64_t Hkv, int64
     const ActDims ad = act_dims(H * D, Nq);
     p.qout = (uint8_t *) act; p.q_d_offset = ad.d_offset; p.q_nb = ad.nb; p.q_nbp = ad.nbp;
     p.q_variant = variant;
+    p.tflags = p.tlist = p.tcount = nullptr;
+    p.spread_rows = 0;
     p.order = index ? (const int32_t *) ((const char *) index + index_order_offset(Nq, p.nw)) : nullptr;
     p.plan = index ? (const int32_t *) ((const char *) index + index_plan_offset(Nq, p.nw)) : nullptr;
     p.slots = FA_MIN_CTAS * fa_sm_count();
@@ -757,7 +799,18 @@ static int flash_attn_impl(bool parity, int64_t D, int64_t H, int64_t Hkv, int64
         const size_t tpart = pt.nsplit > 1 ? (size_t) Nq * H * pt.nsplit * (D + 2) * sizeof(float) : 0;
         if (tpart && (!scratch || scratch_bytes < tpart || !is_aligned(scratch, 16))) pt.nsplit = 1;   // an older scratch size: no splits
         const int tile_tokens = 64 >> gqa_log2;
-        dim3 tgrid((unsigned) Hkv, (unsigned) ((Nq + tile_tokens - 1) / tile_tokens), (unsigned) pt.nsplit);
+        const int64_t tiles = (Nq + tile_tokens - 1) / tile_tokens;
+        if (index) {
+            const int k = 4 - gqa_log2;   // tiles of 4 << k tokens
+            const int64_t stride = index_tiles_stride(Nq);
+            const int32_t *flags = (const int32_t *) ((const char *) index + index_tiles_offset(Nq, p.nw));
+            pt.tflags = flags + k * stride;
+            pt.tlist = flags + (4 + k) * stride;
+            pt.tcount = p.plan + 4 + k;
+            // one round of CTAs, fewer when all tokens together are less
+            pt.spread_rows = (int) std::min<int64_t>(tiles * (tile_tokens / 4), (3 * (int64_t) fa_sm_count() + Hkv * pt.nsplit - 1) / (Hkv * pt.nsplit));
+        }
+        dim3 tgrid((unsigned) Hkv, (unsigned) (tiles + pt.spread_rows), (unsigned) pt.nsplit);
         // the opt-in to more than 48 KB of shared memory is per function and device
         static thread_local int tile_smem_dev = -1;
         int dev_now = 0;

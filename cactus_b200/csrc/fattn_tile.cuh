@@ -35,7 +35,350 @@ __device__ __forceinline__ void ft_ldmatrix_x4_trans(uint32_t (&r)[4], uint32_t 
 }
 
 // dynamic shared memory of the kernel: FT_STAGES stages of K and V rows
-constexpr int fattn_tile_smem_bytes(int D) { return FT_STAGES * 2 * FT_CHUNK * (D * 2 + 16); }
+constexpr int fattn_tile_smem_bytes(int D) { return FT_STAGES * 2 * FT_CHUNK * (D * 2 + 16); }   // as much as ft_spread's 4 x 3 x 16 rows
+
+// ---- the steps of one chunk of 32 cells; rows g and g + 8 of a warp's 16 ----
+// S = Q K^T for n-tiles C0 .. C0 + CN - 1 of 8 cells (independent accumulator chains); Ks: the staged row of the first cell
+template <int D, int C0, int CN>
+__device__ __forceinline__ void ft_s(float (&sacc)[4][4], const uint32_t (&qa)[D / 16][4], const uint8_t *Ks, int g, int t) {
+    constexpr int ROW = D * 2 + 16;
+#pragma unroll
+    for (int c = C0; c < C0 + CN; ++c) sacc[c][0] = sacc[c][1] = sacc[c][2] = sacc[c][3] = 0.0f;
+#pragma unroll
+    for (int ks = 0; ks < D / 16; ++ks)
+#pragma unroll
+        for (int c = C0; c < C0 + CN; ++c) {
+            const uint8_t *krow = Ks + (8 * (c - C0) + g) * ROW + 4 * t + 32 * ks;
+            const uint32_t b0 = *reinterpret_cast<const uint32_t *>(krow), b1 = *reinterpret_cast<const uint32_t *>(krow + 16);
+            mma_f16(sacc[c], qa[ks][0], qa[ks][1], qa[ks][2], qa[ks][3], b0, b1);
+        }
+}
+// Online softmax: element [c][2 i + e] is (row g + 8 i, cell 8 c + 2 t + e of the chunk); rm: which cells row g + 8 i attends
+// to; cells: the chunk's cell list.  P comes back as A fragments of two k-steps of 16 cells, fp16 hi + lo.
+template <int D>
+__device__ __forceinline__ void ft_softmax(const FattnParams &p, float (&sacc)[4][4], const unsigned (&rm)[2], bool binary_mask, const __half *const (&mrow)[2],
+                                           const float (&slope)[2], const int *cells, int t, float (&m_run)[2], float (&l_run)[2], float (&o)[D / 8][4],
+                                           uint32_t (&ph)[2][4], uint32_t (&pl)[2][4]) {
+    float mx[2] = {-CUDART_INF_F, -CUDART_INF_F};
+#pragma unroll
+    for (int c = 0; c < 4; ++c)
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+            const int x = 8 * c + 2 * t + e;
+#pragma unroll
+            for (int i = 0; i < 2; ++i) {
+                float a = sacc[c][2 * i + e] * p.scale;
+                if (p.softcap != 0.0f) a = p.softcap * tanhf(a);
+                if (!((rm[i] >> x) & 1u)) a = -CUDART_INF_F;
+                else if (!binary_mask && mrow[i]) a += slope[i] * __half2float(mrow[i][cells[x]]);
+                sacc[c][2 * i + e] = a;
+                mx[i] = fmaxf(mx[i], a);
+            }
+        }
+    float alpha[2];
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+        mx[i] = fmaxf(mx[i], __shfl_xor_sync(0xffffffffu, mx[i], 1));
+        mx[i] = fmaxf(mx[i], __shfl_xor_sync(0xffffffffu, mx[i], 2));
+        const float m_new = fmaxf(m_run[i], mx[i]);
+        // a row that has seen no participating cell yet keeps a zero state (exp(-inf - -inf) must not be formed)
+        alpha[i] = (m_new == -CUDART_INF_F) ? 1.0f : __expf(m_run[i] - m_new);
+        const float m_use = (m_new == -CUDART_INF_F) ? 0.0f : m_new;
+        float sum = 0.0f;
+#pragma unroll
+        for (int c = 0; c < 4; ++c)
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+                const float pr = __expf(sacc[c][2 * i + e] - m_use);
+                sacc[c][2 * i + e] = pr;
+                sum += pr;
+            }
+        l_run[i] = l_run[i] * alpha[i] + sum;
+        m_run[i] = m_new;
+    }
+    if (__any_sync(0xffffffffu, alpha[0] != 1.0f || alpha[1] != 1.0f)) {
+#pragma unroll
+        for (int nt = 0; nt < D / 8; ++nt) {
+            o[nt][0] *= alpha[0]; o[nt][1] *= alpha[0]; o[nt][2] *= alpha[1]; o[nt][3] *= alpha[1];
+        }
+    }
+#pragma unroll
+    for (int c = 0; c < 4; ++c)
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+            const float x0 = sacc[c][2 * i], x1 = sacc[c][2 * i + 1];
+            const __half2 h = __floats2half2_rn(x0, x1);
+            const float2 f = __half22float2(h);
+            ph[c >> 1][2 * (c & 1) + i] = *reinterpret_cast<const uint32_t *>(&h);
+            pl[c >> 1][2 * (c & 1) + i] = pack_half2(x0 - f.x, x1 - f.y);
+        }
+}
+// O += P V for one k-step of 16 cells, whose V rows start at Vs: V^T fragments of two n-tiles per ldmatrix
+template <int D>
+__device__ __forceinline__ void ft_pv(float (&o)[D / 8][4], const uint32_t (&ph)[4], const uint32_t (&pl)[4], uint32_t Vs, int lane) {
+    constexpr int ROW = D * 2 + 16;
+    const int mi = lane >> 3, mr = lane & 7;
+#pragma unroll
+    for (int nt = 0; nt < D / 8; nt += 2) {
+        uint32_t vb[4];   // {cells 0-7, cells 8-15} of this k-step for n-tile nt, then for n-tile nt + 1
+        ft_ldmatrix_x4_trans(vb, Vs + (uint32_t) ((8 * (mi & 1) + mr) * ROW + (8 * (nt + (mi >> 1))) * 2));
+        mma_f16(o[nt], ph[0], ph[1], ph[2], ph[3], vb[0], vb[1]);
+        mma_f16(o[nt], pl[0], pl[1], pl[2], pl[3], vb[0], vb[1]);
+        mma_f16(o[nt + 1], ph[0], ph[1], ph[2], ph[3], vb[2], vb[3]);
+        mma_f16(o[nt + 1], pl[0], pl[1], pl[2], pl[3], vb[2], vb[3]);
+    }
+}
+// The words any of the tile's tokens attends to, ascending, from the tokens' lists (all of them without a mask).  bits: one per
+// word.  The whole CTA calls it; the result may be read after it.
+__device__ __forceinline__ int ft_union(const FattnParams &p, int64_t tok0, int n_tok, unsigned *bits, unsigned short *uw_index, int *warp_cnt) {
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int n32 = (int) ((p.nw + 31) / 32);
+    for (int i = tid; i < n32; i += FT_THREADS) bits[i] = p.words ? 0u : (p.nw - 32 * i >= 32 ? ~0u : (1u << (p.nw - 32 * i)) - 1u);
+    __syncthreads();
+    if (p.words)
+        for (int j = warp; j < n_tok; j += FT_THREADS / 32) {
+            const int32_t *wl = p.wlist + (tok0 + j) * p.nw;
+            const int n = p.wcount[tok0 + j];
+            for (int e = lane; e < n; e += 32) atomicOr(bits + (wl[e] >> 5), 1u << (wl[e] & 31));
+        }
+    __syncthreads();
+    const unsigned mine = tid < n32 ? bits[tid] : 0u;   // FT_MAX_WORDS / 32 <= FT_THREADS
+    const int cnt = __popc(mine);
+    int pre = cnt;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int x = __shfl_up_sync(0xffffffffu, pre, o);
+        if (lane >= o) pre += x;
+    }
+    if (lane == 31) warp_cnt[warp] = pre;
+    __syncthreads();
+    int at = pre - cnt, all = 0;
+#pragma unroll
+    for (int w = 0; w < FT_THREADS / 32; ++w) {
+        at += w < warp ? warp_cnt[w] : 0;
+        all += warp_cnt[w];
+    }
+    for (unsigned m = mine; m; m &= m - 1) uw_index[at++] = (unsigned short) (32 * tid + __ffs((int) m) - 1);
+    __syncthreads();
+    return all;
+}
+// A finished row pair: O / l, or the split's partial triple
+template <int D>
+__device__ __forceinline__ void ft_write(const FattnParams &p, int64_t tok, int head, int split, int i, const float (&o)[D / 8][4], float m, float l, int t) {
+    if (p.nsplit == 1) {
+        const float inv = 1.0f / l;
+        float *dst = p.dst + (tok * p.H + head) * D;
+#pragma unroll
+        for (int nt = 0; nt < D / 8; ++nt) *reinterpret_cast<float2 *>(dst + 8 * nt + 2 * t) = make_float2(o[nt][2 * i] * inv, o[nt][2 * i + 1] * inv);
+    } else {
+        float *pp = p.partial + ((tok * p.H + head) * p.nsplit + split) * (D + 2);
+#pragma unroll
+        for (int nt = 0; nt < D / 8; ++nt) *reinterpret_cast<float2 *>(pp + 8 * nt + 2 * t) = make_float2(o[nt][2 * i], o[nt][2 * i + 1]);
+        if (t == 0) {
+            pp[D] = m;
+            pp[D + 1] = l;
+        }
+    }
+}
+
+struct FtTileShared {
+    int cell_list[FT_LIST];                    // the cells of this round, ascending
+    unsigned short cell_kb[FT_LIST];           // where each sits among the round's words: 64 * slot + bit
+    unsigned short uw_index[FT_MAX_WORDS];     // the mask words any token of the tile attends to, ascending
+    unsigned long long tile_words[FT_MAX_TILE][FT_RW];   // the round's words, token by token
+    unsigned long long ubits[FT_RW];           // their union
+    int wbase[FT_RW];                          // cells listed before each word
+    unsigned rmask[FT_MAX_TILE][FT_LIST / FT_CHUNK];   // per token and chunk: which of the chunk's 32 cells the token attends to
+    unsigned bits[FT_MAX_WORDS / 32];
+    int list_count, warp_cnt[FT_THREADS / 32];
+};
+struct FtSpreadShared {
+    unsigned short uw_index[FT_MAX_WORDS];
+    unsigned bits[FT_MAX_WORDS / 32];
+    int warp_cnt[FT_THREADS / 32];
+    alignas(16) short list[FT_THREADS / 32][FT_LIST];     // per warp: the round's union positions, 64 * slot + bit of a cell its token attends to or -1
+    int cells[FT_THREADS / 32][2][FT_CHUNK];   // per warp: the cells of the chunk at work and of the next
+};
+
+// Tokens of tiles whose tokens share few cells (decode tokens beside a prompt, in which a shared walk of the union would have
+// every token step over all the others' cells): one warp per token, over the chunks its token attends to.  The chunks are
+// those of the shared walk -- 32 neighbours in the tile's union list, every nsplit-th to each split -- and a chunk without a
+// cell of the token would have changed nothing, so results are the same bits.
+// What bounds it: the K/V rows (each read once) and the latency of a warp's chain of chunks; 12 warps per SM and half chunks in
+// flight (three slots of 16 rows per warp: K rows 0-15 and 16-31, then V rows 0-15; V rows 16-31 take the first slot when its
+// K rows are used, and the next chunk moves on by one slot) cover both.  48 tokens of 16-2048 cells beside a 464-token prompt
+// (32 heads, 8 KV heads): see the comment at fattn_tile_kernel.
+template <int D>
+__device__ __forceinline__ void ft_spread(const FattnParams &p, int gqa_log2, FtSpreadShared &sh, uint8_t *kv_s) {
+    constexpr int KS = D / 16, NT = D / 8, ROW = D * 2 + 16, HALF = 16 * ROW;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
+    const int gqa = 1 << gqa_log2, tile_tok = 64 >> gqa_log2, quads = tile_tok >> 2;
+    const int hk = blockIdx.x, split = blockIdx.z, nsplit = p.nsplit;
+    const bool binary_mask = p.plan[2] == 0;
+    const char *kbase = p.k + (int64_t) hk * p.k_nb_head, *vbase = p.v + (int64_t) hk * p.v_nb_head;
+    uint8_t *slots = kv_s + warp * 3 * HALF;
+    const uint32_t slots_u32 = (uint32_t) __cvta_generic_to_shared(slots);
+    short *list = sh.list[warp];
+    const int n_units = *p.tcount * quads;
+    for (int unit = blockIdx.y; unit < n_units; unit += p.spread_rows) {
+        const int64_t tok0 = (int64_t) p.tlist[unit / quads] * tile_tok, tok = tok0 + (unit % quads) * 4 + warp;
+        __syncthreads();   // the lists of the unit before are no longer read
+        const int n_uw = ft_union(p, tok0, (int) min((int64_t) tile_tok, p.Nq - tok0), sh.bits, sh.uw_index, sh.warp_cnt);
+        if (tok >= p.Nq) continue;
+        const int n_tok = (int) min((int64_t) tile_tok, p.Nq - tok0);
+        uint32_t qa[KS][4];
+        int head[2];
+        bool live[2];
+        float slope[2];
+        const __half *mrow[2];
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {   // row r is head r of the group
+            const int r = g + 8 * i;
+            live[i] = r < gqa;
+            head[i] = hk * gqa + (live[i] ? r : 0);
+            const float *qp = reinterpret_cast<const float *>(reinterpret_cast<const char *>(p.q) + tok * p.q_nb_tok + (int64_t) head[i] * p.q_nb_head);
+#pragma unroll
+            for (int ks = 0; ks < KS; ++ks) {
+                const float2 lo = live[i] ? *reinterpret_cast<const float2 *>(qp + 16 * ks + 2 * t) : make_float2(0.f, 0.f);
+                const float2 hi = live[i] ? *reinterpret_cast<const float2 *>(qp + 16 * ks + 8 + 2 * t) : make_float2(0.f, 0.f);
+                qa[ks][i] = pack_half2(lo.x, lo.y);
+                qa[ks][2 + i] = pack_half2(hi.x, hi.y);
+            }
+            const uint32_t hh = (uint32_t) head[i];
+            slope[i] = (p.max_bias > 0.0f) ? (hh < p.n_head_log2 ? powf(p.m0, (float) (hh + 1)) : powf(p.m1, (float) (2 * (hh - p.n_head_log2) + 1))) : 1.0f;
+            mrow[i] = live[i] && p.mask ? reinterpret_cast<const __half *>(p.mask + tok * p.mask_nb_row) : nullptr;
+        }
+        float o[NT][4];
+#pragma unroll
+        for (int nt = 0; nt < NT; ++nt) o[nt][0] = o[nt][1] = o[nt][2] = o[nt][3] = 0.0f;
+        float m_run[2] = {-CUDART_INF_F, -CUDART_INF_F}, l_run[2] = {0.0f, 0.0f};
+
+        // the chunks of this split with a cell of the token, one after the other: rm and, in sh.cells[warp][b], 32 cells (where the
+        // token does not attend, one that it does attend)
+        int r0 = -FT_RW, chunk = 0, n_chunks = 0;   // r0: the round whose list is built
+        auto next_chunk = [&](int b) -> unsigned {
+            while (true) {
+                if (chunk >= n_chunks) {   // on to the next round in which the token attends to a word
+                    unsigned long long own = 0, all = 0;
+                    int n_own = 0;
+                    do {
+                        r0 += FT_RW;
+                        if (r0 >= n_uw) return 0u;
+                        const int k = lane & 15;
+                        own = 0;
+                        if (r0 + k < n_uw) own = p.words[tok * p.nw + sh.uw_index[r0 + k]];
+                        n_own = __popc(__ballot_sync(0xffffffffu, own != 0ull));
+                    } while (n_own == 0);
+                    const int k = lane & 15;
+                    if (r0 + k < n_uw) {
+                        const unsigned long long *w = p.words + tok0 * p.nw + sh.uw_index[r0 + k];
+#pragma unroll 8
+                        for (int j = lane >> 4; j < n_tok; j += 2) all |= w[j * p.nw];
+                    }
+                    all |= __shfl_xor_sync(0xffffffffu, all, 16);
+                    const int cnt = __popcll(all);
+                    int pre = cnt;
+#pragma unroll
+                    for (int s = 1; s < 16; s <<= 1) {
+                        const int x = __shfl_up_sync(0xffffffffu, pre, s, 16);
+                        if (k >= s) pre += x;
+                    }
+                    const int total = __shfl_sync(0xffffffffu, pre, 15);
+                    n_chunks = (total + FT_CHUNK - 1) / FT_CHUNK;
+                    chunk = split;
+                    for (int i = lane; i < n_chunks * (FT_CHUNK / 8); i += 32) reinterpret_cast<uint4 *>(list)[i] = make_uint4(~0u, ~0u, ~0u, ~0u);
+                    __syncwarp();
+                    for (int w = 0; w < FT_RW; ++w) {
+                        const unsigned long long ow = __shfl_sync(0xffffffffu, own, w);
+                        if (ow == 0ull) continue;
+                        const unsigned long long aw = __shfl_sync(0xffffffffu, all, w);
+                        const int base = __shfl_sync(0xffffffffu, pre - cnt, w);
+#pragma unroll
+                        for (int h = 0; h < 2; ++h) {
+                            const int bit = lane + 32 * h;
+                            if ((ow >> bit) & 1ull) list[base + __popcll(aw & ((1ull << bit) - 1ull))] = (short) (64 * w + bit);
+                        }
+                    }
+                    __syncwarp();
+                }
+                for (; chunk < n_chunks; chunk += nsplit) {
+                    const int v = list[chunk * FT_CHUNK + lane];
+                    const unsigned rm = __ballot_sync(0xffffffffu, v >= 0);
+                    if (!rm) continue;
+                    int cell = v >= 0 ? (int) sh.uw_index[r0 + (v >> 6)] * 64 + (v & 63) : 0;
+                    const int some = __shfl_sync(0xffffffffu, cell, __ffs((int) rm) - 1);
+                    sh.cells[warp][b][lane] = v >= 0 ? cell : some;
+                    __syncwarp();
+                    chunk += nsplit;
+                    return rm;
+                }
+            }
+        };
+        // 16 rows of K or V into a slot; a group of its own
+        constexpr int PIECES = D / 8, PER = 16 * PIECES / 32;
+        auto fetch = [&](const char *base, int64_t nb_cell, const int *cells, int slot) {
+#pragma unroll
+            for (int n = 0; n < PER; ++n) {
+                const int c = lane + 32 * n, r = c / PIECES, piece = c % PIECES;
+                ft_cp16(slots_u32 + (uint32_t) (slot * HALF + r * ROW + piece * 16), base + (int64_t) cells[r] * nb_cell + piece * 16);
+            }
+        };
+        auto commit = [&] { asm volatile("cp.async.commit_group;\n" ::: "memory"); };
+        auto landed = [&] {
+            asm volatile("cp.async.wait_group 2;\n" ::: "memory");
+            __syncwarp();
+        };
+        int b = 0, s0 = 0, s1 = 1, s2 = 2;
+        unsigned rm_now = next_chunk(0);
+        if (rm_now) fetch(kbase, p.k_nb_cell, sh.cells[warp][0], 0);
+        commit();
+        if (rm_now) fetch(kbase, p.k_nb_cell, sh.cells[warp][0] + 16, 1);
+        commit();
+        if (rm_now) fetch(vbase, p.v_nb_cell, sh.cells[warp][0], 2);
+        commit();
+        while (rm_now) {
+            const int *cells = sh.cells[warp][b], *ncells = sh.cells[warp][b ^ 1];
+            const unsigned rm_next = next_chunk(b ^ 1);
+            const unsigned rm[2] = {live[0] ? rm_now : 0u, live[1] ? rm_now : 0u};
+            float sacc[4][4];
+            uint32_t ph[2][4], pl[2][4];
+            landed();
+            ft_s<D, 0, 2>(sacc, qa, slots + s0 * HALF, g, t);
+            __syncwarp();
+            fetch(vbase, p.v_nb_cell, cells + 16, s0);
+            commit();
+            landed();
+            ft_s<D, 2, 2>(sacc, qa, slots + s1 * HALF, g, t);
+            __syncwarp();
+            if (rm_next) fetch(kbase, p.k_nb_cell, ncells, s1);
+            commit();
+            ft_softmax<D>(p, sacc, rm, binary_mask, mrow, slope, cells, t, m_run, l_run, o, ph, pl);
+            landed();
+            ft_pv<D>(o, ph[0], pl[0], slots_u32 + (uint32_t) (s2 * HALF), lane);
+            __syncwarp();
+            if (rm_next) fetch(kbase, p.k_nb_cell, ncells + 16, s2);
+            commit();
+            landed();
+            ft_pv<D>(o, ph[1], pl[1], slots_u32 + (uint32_t) (s0 * HALF), lane);
+            __syncwarp();
+            if (rm_next) fetch(vbase, p.v_nb_cell, ncells, s0);
+            commit();
+            const int x = s0;
+            s0 = s1;
+            s1 = s2;
+            s2 = x;
+            b ^= 1;
+            rm_now = rm_next;
+        }
+        asm volatile("cp.async.wait_all;\n" ::: "memory");
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+            l_run[i] += __shfl_xor_sync(0xffffffffu, l_run[i], 1);
+            l_run[i] += __shfl_xor_sync(0xffffffffu, l_run[i], 2);
+            if (live[i]) ft_write<D>(p, tok, head[i], split, i, o, m_run[i], l_run[i], t);
+        }
+    }
+}
 
 template <int D>
 __global__ void __launch_bounds__(FT_THREADS, 3) fattn_tile_kernel(FattnParams p, int gqa_log2) {
@@ -48,20 +391,28 @@ __global__ void __launch_bounds__(FT_THREADS, 3) fattn_tile_kernel(FattnParams p
     const int g = lane >> 2, t = lane & 3;
     const int gqa = 1 << gqa_log2;
     const int tw = 16 >> gqa_log2;                      // tokens per warp
-    const int64_t tok0 = (int64_t) blockIdx.y * (4 * tw);   // first token of the tile
+    const int64_t tok0 = (int64_t) ((int) blockIdx.y - p.spread_rows) * (4 * tw);   // first token of the tile
     const int hk = blockIdx.x;
     const int split = blockIdx.z, nsplit = p.nsplit;
     const bool binary_mask = p.words && p.plan && p.plan[2] == 0;   // only 0 / -inf in the mask: a row's bit says it all
 
-    __shared__ int cell_list[FT_LIST];                    // the cells of this round, ascending
-    __shared__ unsigned short cell_kb[FT_LIST];           // where each sits among the round's words: 64 * slot + bit
-    __shared__ unsigned short uw_index[FT_MAX_WORDS];     // the mask words any token of the tile attends to, ascending
-    __shared__ unsigned long long tile_words[FT_MAX_TILE][FT_RW];   // the round's words, token by token
-    __shared__ unsigned long long ubits[FT_RW];           // their union
-    __shared__ int wbase[FT_RW];                          // cells listed before each word
-    __shared__ unsigned rmask[FT_MAX_TILE][FT_LIST / FT_CHUNK];   // per token and chunk: which of the chunk's 32 cells the token attends to
-    __shared__ int list_count, uw_count, warp_cnt[4];
+    __shared__ union {
+        FtTileShared tile;
+        FtSpreadShared spread;
+    } sh;
+    int *const cell_list = sh.tile.cell_list;
+    unsigned short *const cell_kb = sh.tile.cell_kb, *const uw_index = sh.tile.uw_index;
+    unsigned long long (*const tile_words)[FT_RW] = sh.tile.tile_words, *const ubits = sh.tile.ubits;
+    int *const wbase = sh.tile.wbase;
+    unsigned (*const rmask)[FT_LIST / FT_CHUNK] = sh.tile.rmask;
+    int &list_count = sh.tile.list_count;
     extern __shared__ __align__(16) uint8_t kv_s[];   // [stage][K, V][FT_CHUNK rows of ROW bytes] (dynamic: fattn_tile_smem_bytes)
+
+    if ((int) blockIdx.y < p.spread_rows) {   // the first rows of the grid: their chains are the longest
+        ft_spread<D>(p, gqa_log2, sh.spread, kv_s);
+        return;
+    }
+    if (p.tflags && p.tflags[(int) blockIdx.y - p.spread_rows]) return;
 
     // rows g and g + 8 of this warp: (token, head)
     int64_t tok[2];
@@ -108,32 +459,7 @@ __global__ void __launch_bounds__(FT_THREADS, 3) fattn_tile_kernel(FattnParams p
     const uint32_t kv_u32 = (uint32_t) __cvta_generic_to_shared(kv_s);
     const int n_tile_tok = (int) min((int64_t) (4 * tw), p.Nq - tok0);
 
-    // ---- the words the tile attends to at all (one pass over the tokens' word rows, 128 words at a time) ----
-    if (tid == 0) uw_count = 0;
-    __syncthreads();
-    for (int64_t b0 = 0; b0 < p.nw; b0 += FT_THREADS) {
-        const int64_t wi = b0 + tid;
-        bool nz = false;
-        if (wi < p.nw) {
-            if (p.words) {
-                unsigned long long bits = 0;
-                for (int j = 0; j < n_tile_tok; ++j) bits |= p.words[(tok0 + j) * p.nw + wi];
-                nz = bits != 0ull;
-            } else {
-                nz = true;
-            }
-        }
-        const unsigned m = __ballot_sync(0xffffffffu, nz);
-        if (lane == 0) warp_cnt[warp] = __popc(m);
-        __syncthreads();
-        int off = uw_count;
-        for (int w = 0; w < warp; ++w) off += warp_cnt[w];
-        if (nz) uw_index[off + __popc(m & ((1u << lane) - 1u))] = (unsigned short) wi;
-        __syncthreads();
-        if (tid == 0) uw_count += warp_cnt[0] + warp_cnt[1] + warp_cnt[2] + warp_cnt[3];
-        __syncthreads();
-    }
-    const int n_uw = uw_count;
+    const int n_uw = ft_union(p, tok0, n_tile_tok, sh.tile.bits, uw_index, sh.tile.warp_cnt);
 
     // one 16-byte piece of a K or V row per copy: D / 8 pieces per row, 32 rows of K then 32 of V.  A thread's copies sit at
     // fixed places of a stage: copy n of thread tid is piece (tid + 128 n) % PIECES of row ((tid + 128 n) / PIECES) % 32.
@@ -199,18 +525,13 @@ __global__ void __launch_bounds__(FT_THREADS, 3) fattn_tile_kernel(FattnParams p
         __syncthreads();
         const int n_chunks = (count + FT_CHUNK - 1) / FT_CHUNK;
         // ---- which cells of each of this split's chunks every token attends to ----
-        for (int e = tid; e < n_tile_tok * n_chunks; e += FT_THREADS) {
-            const int j = e / n_chunks, c = e - j * n_chunks;
-            if (c % nsplit != split) continue;
-            unsigned m = 0;
-            for (int x = 0; x < FT_CHUNK; ++x) {
-                const int idx = c * FT_CHUNK + x;
-                if (idx < count) {
-                    const int kb = cell_kb[idx];
-                    m |= (unsigned) ((tile_words[j][kb >> 6] >> (kb & 63)) & 1ull) << x;
-                }
+        for (int c = split + warp * nsplit; c < n_chunks; c += 4 * nsplit) {   // a warp per chunk, a lane per cell
+            const int idx = c * FT_CHUNK + lane, kb = cell_kb[min(idx, count - 1)];
+#pragma unroll 4
+            for (int j = 0; j < n_tile_tok; ++j) {
+                const unsigned m = __ballot_sync(0xffffffffu, idx < count && ((tile_words[j][kb >> 6] >> (kb & 63)) & 1ull));
+                if (lane == 0) rmask[j][c] = m;
             }
-            rmask[j][c] = m;
         }
         // this split's chunks: split, split + nsplit, ...; FT_STAGES - 1 of them are on their way while one is multiplied
         int issued = 0;
@@ -233,91 +554,16 @@ __global__ void __launch_bounds__(FT_THREADS, 3) fattn_tile_kernel(FattnParams p
             __syncthreads();   // the stage has landed for every thread (and, first time round, the row masks are written)
             const uint8_t *Ks = kv_s + (s * 2) * (FT_CHUNK * ROW);
             const uint32_t Vs = kv_u32 + (uint32_t) ((s * 2 + 1) * (FT_CHUNK * ROW));
-            // ---- S = Q K^T: four n-tiles of 8 cells (four independent accumulator chains) ----
-            float sacc[4][4];
-#pragma unroll
-            for (int c = 0; c < 4; ++c) sacc[c][0] = sacc[c][1] = sacc[c][2] = sacc[c][3] = 0.0f;
-#pragma unroll
-            for (int ks = 0; ks < KS; ++ks)
-#pragma unroll
-                for (int c = 0; c < 4; ++c) {
-                    const uint8_t *krow = Ks + (8 * c + g) * ROW + 4 * t + 32 * ks;
-                    const uint32_t b0 = *reinterpret_cast<const uint32_t *>(krow), b1 = *reinterpret_cast<const uint32_t *>(krow + 16);
-                    mma_f16(sacc[c], qa[ks][0], qa[ks][1], qa[ks][2], qa[ks][3], b0, b1);
-                }
-            // ---- scores: element [c][2 i + e] is (row g + 8 i, cell 8 c + 2 t + e of the chunk) ----
-            const int base = ch * FT_CHUNK;
-            float mx[2] = {-CUDART_INF_F, -CUDART_INF_F};
             unsigned rm[2];
 #pragma unroll
             for (int i = 0; i < 2; ++i) rm[i] = live[i] ? rmask[tl[i]][ch] : 0u;
+            if (__any_sync(0xffffffffu, (rm[0] | rm[1]) != 0u)) {   // a chunk that none of the warp's rows attends to changes nothing
+                float sacc[4][4];
+                uint32_t ph[2][4], pl[2][4];
+                ft_s<D, 0, 4>(sacc, qa, Ks, g, t);
+                ft_softmax<D>(p, sacc, rm, binary_mask, mrow, slope, cell_list + ch * FT_CHUNK, t, m_run, l_run, o, ph, pl);
 #pragma unroll
-            for (int c = 0; c < 4; ++c)
-#pragma unroll
-                for (int e = 0; e < 2; ++e) {
-                    const int x = 8 * c + 2 * t + e;
-#pragma unroll
-                    for (int i = 0; i < 2; ++i) {
-                        float a = sacc[c][2 * i + e] * p.scale;
-                        if (p.softcap != 0.0f) a = p.softcap * tanhf(a);
-                        if (!((rm[i] >> x) & 1u)) a = -CUDART_INF_F;
-                        else if (!binary_mask && mrow[i]) a += slope[i] * __half2float(mrow[i][cell_list[base + x]]);
-                        sacc[c][2 * i + e] = a;
-                        mx[i] = fmaxf(mx[i], a);
-                    }
-                }
-            float alpha[2];
-#pragma unroll
-            for (int i = 0; i < 2; ++i) {
-                mx[i] = fmaxf(mx[i], __shfl_xor_sync(0xffffffffu, mx[i], 1));
-                mx[i] = fmaxf(mx[i], __shfl_xor_sync(0xffffffffu, mx[i], 2));
-                const float m_new = fmaxf(m_run[i], mx[i]);
-                // a row that has seen no participating cell yet keeps a zero state (exp(-inf - -inf) must not be formed)
-                alpha[i] = (m_new == -CUDART_INF_F) ? 1.0f : __expf(m_run[i] - m_new);
-                const float m_use = (m_new == -CUDART_INF_F) ? 0.0f : m_new;
-                float sum = 0.0f;
-#pragma unroll
-                for (int c = 0; c < 4; ++c)
-#pragma unroll
-                    for (int e = 0; e < 2; ++e) {
-                        const float pr = __expf(sacc[c][2 * i + e] - m_use);
-                        sacc[c][2 * i + e] = pr;
-                        sum += pr;
-                    }
-                l_run[i] = l_run[i] * alpha[i] + sum;
-                m_run[i] = m_new;
-            }
-            if (__any_sync(0xffffffffu, alpha[0] != 1.0f || alpha[1] != 1.0f)) {
-#pragma unroll
-                for (int nt = 0; nt < NT; ++nt) {
-                    o[nt][0] *= alpha[0]; o[nt][1] *= alpha[0]; o[nt][2] *= alpha[1]; o[nt][3] *= alpha[1];
-                }
-            }
-            // P as A fragments, two k-steps of 16 cells, fp16 hi + lo
-            uint32_t ph[2][4], pl[2][4];
-#pragma unroll
-            for (int c = 0; c < 4; ++c)
-#pragma unroll
-                for (int i = 0; i < 2; ++i) {
-                    const float x0 = sacc[c][2 * i], x1 = sacc[c][2 * i + 1];
-                    const __half2 h = __floats2half2_rn(x0, x1);
-                    const float2 f = __half22float2(h);
-                    ph[c >> 1][2 * (c & 1) + i] = *reinterpret_cast<const uint32_t *>(&h);
-                    pl[c >> 1][2 * (c & 1) + i] = pack_half2(x0 - f.x, x1 - f.y);
-                }
-            // ---- O += P V: V^T fragments of two n-tiles per ldmatrix ----
-#pragma unroll
-            for (int nt = 0; nt < NT; nt += 2) {
-#pragma unroll
-                for (int kk = 0; kk < 2; ++kk) {
-                    uint32_t vb[4];   // {cells 0-7, cells 8-15} of this k-step for n-tile nt, then for n-tile nt + 1
-                    const int mi = lane >> 3, mr = lane & 7;
-                    ft_ldmatrix_x4_trans(vb, Vs + (uint32_t) ((16 * kk + 8 * (mi & 1) + mr) * ROW + (8 * (nt + (mi >> 1))) * 2));
-                    mma_f16(o[nt], ph[kk][0], ph[kk][1], ph[kk][2], ph[kk][3], vb[0], vb[1]);
-                    mma_f16(o[nt], pl[kk][0], pl[kk][1], pl[kk][2], pl[kk][3], vb[0], vb[1]);
-                    mma_f16(o[nt + 1], ph[kk][0], ph[kk][1], ph[kk][2], ph[kk][3], vb[2], vb[3]);
-                    mma_f16(o[nt + 1], pl[kk][0], pl[kk][1], pl[kk][2], pl[kk][3], vb[2], vb[3]);
-                }
+                for (int kk = 0; kk < 2; ++kk) ft_pv<D>(o, ph[kk], pl[kk], Vs + (uint32_t) (16 * kk * ROW), lane);
             }
             __syncthreads();   // this stage may be refilled by the copy issued in the next step
         }
@@ -329,20 +575,7 @@ __global__ void __launch_bounds__(FT_THREADS, 3) fattn_tile_kernel(FattnParams p
         l_run[i] += __shfl_xor_sync(0xffffffffu, l_run[i], 1);
         l_run[i] += __shfl_xor_sync(0xffffffffu, l_run[i], 2);
         if (!live[i]) continue;
-        if (nsplit == 1) {
-            const float inv = 1.0f / l_run[i];
-            float *dst = p.dst + (tok[i] * p.H + head[i]) * D;
-#pragma unroll
-            for (int nt = 0; nt < NT; ++nt) *reinterpret_cast<float2 *>(dst + 8 * nt + 2 * t) = make_float2(o[nt][2 * i] * inv, o[nt][2 * i + 1] * inv);
-        } else {
-            float *pp = p.partial + ((tok[i] * p.H + head[i]) * nsplit + split) * (D + 2);
-#pragma unroll
-            for (int nt = 0; nt < NT; ++nt) *reinterpret_cast<float2 *>(pp + 8 * nt + 2 * t) = make_float2(o[nt][2 * i], o[nt][2 * i + 1]);
-            if (t == 0) {
-                pp[D] = m_run[i];
-                pp[D + 1] = l_run[i];
-            }
-        }
+        ft_write<D>(p, tok[i], head[i], split, i, o, m_run[i], l_run[i], t);
     }
 }
 

@@ -34,96 +34,178 @@ constexpr int FA_SUPER_WORDS = 32;  // 2048 cells listed per round
 constexpr int FA_MIN_SPLIT_WORDS = 2;   // 64-cell words a KV split walks at least (when the mask index gives a token's word count)
 constexpr int FA_ADAPTIVE_SPLITS = 2;   // most KV splits a long sequence is cut into when the batch is small
 
-// ---- mask scan: one warp per 64 cells of one token row ------------------------------------------
-__global__ void __launch_bounds__(256) mask_index_kernel(const __half *__restrict__ mask, int64_t mask_nb_row, int64_t Nq,
-                                                        int64_t n_kv, int64_t nw, unsigned long long *__restrict__ words, int32_t *soft) {
-    const int lane = threadIdx.x & 31;
-    const int64_t wid = ((int64_t) blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    if (wid >= Nq * nw) return;
-    const int64_t j = wid / nw, wi = wid - j * nw;
+// ---- mask scan: one CTA per token row --------------------------------------------------------------
+// The row as one bit per cell, 64 cells to a word; the indices of the words that have any participating cell, in ascending
+// order, and their count (a token of a 64-sequence batch owns a few dozen of the 1024 words of a 65536-cell cache, and the
+// attention kernels walk only those); whether the row holds more than 0 and -inf in participating cells.
+// Reads the mask once, 16 bytes (8 cells) per thread and load, four loads in flight; one kernel for what was a memset, a scan
+// and a pass over the words that the scan had written.  Whole index build, us before / now on B200 (tokens x cells): 1 x 1024
+// 8.3 / 3.5, 64 x 65536 23.9 / 9.4, 512 x 8192 49.7 / 13.3, 512 x 65536 109 / 27.  A cluster of 2 or 4 CTAs per row was faster at
+// 64 x 65536 only (7.9) and slower from 1 x 1024 (4.6) to 512 x 65536 (32, 43).
+constexpr int MI_THREADS = 512, MI_WORDS = 2048;   // words whose indices are listed per round
+template <bool VEC>
+__global__ void __launch_bounds__(MI_THREADS, 3) mask_index_kernel(const __half *__restrict__ mask, int64_t mask_nb_row, int64_t n_kv, int64_t nw,
+                                                               unsigned long long *__restrict__ words, int32_t *__restrict__ wlist, int32_t *__restrict__ wcount,
+                                                               int32_t *__restrict__ soft) {
+    pdl_prologue();
+    __shared__ unsigned bits[MI_WORDS / 32];
+    __shared__ int warp_cnt[MI_WORDS / 1024], any_soft;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int64_t j = blockIdx.x;
     const __half *row = reinterpret_cast<const __half *>(reinterpret_cast<const char *>(mask) + j * mask_nb_row);
-    const int64_t c0 = wi * 64 + lane, c1 = c0 + 32;
-    const unsigned short ninf = 0xFC00u;
-    const unsigned short m0 = c0 < n_kv ? __half_as_ushort(row[c0]) : ninf, m1 = c1 < n_kv ? __half_as_ushort(row[c1]) : ninf;
-    const bool v0 = m0 != ninf, v1 = m1 != ninf;
-    // a participating cell whose mask value is not +-0 is added to the score: the mask is then more than its bits
-    if (((v0 && (m0 & 0x7fffu)) || (v1 && (m1 & 0x7fffu))) && soft) *soft = 1;
-    const unsigned lo = __ballot_sync(0xffffffffu, v0), hi = __ballot_sync(0xffffffffu, v1);
-    if (lane == 0) words[wid] = (unsigned long long) lo | ((unsigned long long) hi << 32);
-}
-
-// Second pass of the mask scan: per token, the indices of the 64-cell words that have any participating cell,
-// in ascending order, and their count.  A token of a 64-sequence batch owns a few dozen of the 1024 words of a
-// 65536-cell cache, and the attention kernel walks only those.
-__global__ void __launch_bounds__(256) mask_words_compact_kernel(const unsigned long long *__restrict__ words, int64_t Nq, int64_t nw,
-                                                                int32_t *__restrict__ wlist, int32_t *__restrict__ wcount) {
-    const int lane = threadIdx.x & 31;
-    const int64_t j = ((int64_t) blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    if (j >= Nq) return;
-    const unsigned long long *row = words + j * nw;
-    int32_t *out = wlist + j * nw;
-    int base = 0;
-    for (int64_t w0 = 0; w0 < nw; w0 += 32) {
-        const int64_t wi = w0 + lane;
-        const bool nz = wi < nw && row[wi] != 0ull;
-        const unsigned m = __ballot_sync(0xffffffffu, nz);
-        if (nz) out[base + __popc(m & ((1u << lane) - 1u))] = (int32_t) wi;
-        base += __popc(m);
+    unsigned long long *out = words + j * nw;
+    int32_t *list = wlist + j * nw;
+    int base = 0;   // listed so far
+    unsigned soft_bits = 0;
+    if (tid == 0) any_soft = 0;
+    for (int64_t w0 = 0; w0 < nw; w0 += MI_WORDS) {
+        const int n = (int) min((int64_t) MI_WORDS, nw - w0);
+        if (tid < MI_WORDS / 32) bits[tid] = 0u;
+        __syncthreads();
+#pragma unroll 4
+        for (int i = tid; i < (n * 8 + 31) / 32 * 32; i += MI_THREADS) {   // 8 cells; whole warps
+            const int64_t c0 = (w0 * 8 + i) * 8;
+            unsigned h[4] = {0xFC00FC00u, 0xFC00FC00u, 0xFC00FC00u, 0xFC00FC00u};
+            if (VEC ? c0 + 8 <= n_kv : false) {
+                const uint4 v = __ldg(reinterpret_cast<const uint4 *>(row + c0));
+                h[0] = v.x; h[1] = v.y; h[2] = v.z; h[3] = v.w;
+            } else {
+#pragma unroll
+                for (int x = 0; x < 8; ++x)
+                    if (c0 + x < n_kv) h[x >> 1] = (h[x >> 1] & (x & 1 ? 0xffffu : 0xffff0000u)) | ((unsigned) __half_as_ushort(row[c0 + x]) << (16 * (x & 1)));
+            }
+            unsigned m = 0;
+#pragma unroll
+            for (int x = 0; x < 4; ++x) {   // two cells at a time: all ones where the value is not -inf
+                const unsigned in = ~__heq2_mask(*reinterpret_cast<const __half2 *>(&h[x]), __half2half2(__ushort_as_half((unsigned short) 0xFC00u)));
+                m |= in & ((1u << (2 * x)) | (1u << (17 + 2 * x)));
+                soft_bits |= h[x] & in & 0x7fff7fffu;   // not +-0: added to the score
+            }
+            m = (m | (m >> 16)) & 0xffu;
+            if (i < n * 8) reinterpret_cast<uint8_t *>(out + w0)[i] = (uint8_t) m;   // byte by byte in the order of the words' bits
+            unsigned any8 = __ballot_sync(0xffffffffu, m != 0u);
+            if (any8 && lane == 0) {   // the warp's four words
+                any8 |= any8 >> 4;
+                any8 |= any8 >> 2;
+                any8 |= any8 >> 1;
+                atomicOr(bits + (i >> 8), ((any8 & 1u) | ((any8 >> 7) & 2u) | ((any8 >> 14) & 4u) | ((any8 >> 21) & 8u)) << ((i >> 3) & 31));
+            }
+        }
+        __syncthreads();
+        const unsigned mine = tid < MI_WORDS / 32 ? bits[tid] : 0u;
+        const int cnt = __popc(mine);
+        int pre = cnt;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int x = __shfl_up_sync(0xffffffffu, pre, o);
+            if (lane >= o) pre += x;
+        }
+        if (lane == 31 && warp < MI_WORDS / 1024) warp_cnt[warp] = pre;
+        __syncthreads();
+        int at = base + pre - cnt;
+#pragma unroll
+        for (int w = 0; w < MI_WORDS / 1024; ++w) {
+            at += w < warp ? warp_cnt[w] : 0;
+            base += warp_cnt[w];
+        }
+        for (unsigned m = mine; m; m &= m - 1) list[at++] = (int32_t) (w0 + 32 * tid + __ffs((int) m) - 1);
+        __syncthreads();
     }
-    if (lane == 0) wcount[j] = base;
+    if (soft_bits) any_soft = 1;
+    __syncthreads();
+    if (tid == 0) {
+        wcount[j] = base;
+        soft[j] = any_soft;
+    }
 }
 
-// Third pass: the tokens ordered by decreasing word count (longest sequence first, so the scheduler hands the long
+// Second pass: the tokens ordered by decreasing word count (longest sequence first, so the scheduler hands the long
 // walks out first and the short ones fill the gaps), and the total number of words, from which the attention kernel
-// derives how many words one CTA should walk.
-__global__ void __launch_bounds__(1024) fattn_plan_kernel(const int32_t *__restrict__ wcount, int64_t Nq, int32_t *__restrict__ order,
-                                                         int32_t *__restrict__ plan) {
-    __shared__ long long total_s;
-    if (threadIdx.x == 0) total_s = 0;
-    __syncthreads();
-    long long part = 0;
-    for (int64_t j = threadIdx.x; j < Nq; j += blockDim.x) {
+// derives how many words one CTA should walk.  A warp per token counts the tokens that come before it; the first CTA also
+// makes the totals.
+__global__ void __launch_bounds__(256) fattn_plan_kernel(const int32_t *__restrict__ wcount, const int32_t *__restrict__ soft, int64_t Nq, int32_t *__restrict__ order,
+                                                        int32_t *__restrict__ plan) {
+    pdl_prologue();
+    const int lane = threadIdx.x & 31;
+    const int64_t j = (int64_t) blockIdx.x * 8 + (threadIdx.x >> 5);
+    if (j < Nq) {
         const int32_t c = wcount[j];
-        part += c;
-        int64_t rank = 0;   // tokens with more words, or as many and a lower index, come first
-        for (int64_t i = 0; i < Nq; ++i) {
+        int rank = 0;   // tokens with more words, or as many and a lower index, come first
+        for (int64_t i = lane; i < Nq; i += 32) {
             const int32_t ci = wcount[i];
             rank += (ci > c || (ci == c && i < j)) ? 1 : 0;
         }
-        order[rank] = (int32_t) j;
+        rank = __reduce_add_sync(0xffffffffu, rank);
+        if (lane == 0) order[rank] = (int32_t) j;
     }
-    atomicAdd((unsigned long long *) &total_s, (unsigned long long) part);
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        plan[0] = (int32_t) min(total_s, (long long) 0x7fffffff);
+    if (blockIdx.x == 0) {
+        __shared__ unsigned long long part_s[8];
+        __shared__ int any;
+        if (threadIdx.x == 0) any = 0;
+        __syncthreads();
+        unsigned long long part = 0;
+        int s = 0;
+        for (int64_t i = threadIdx.x; i < Nq; i += blockDim.x) {
+            part += (unsigned long long) wcount[i];
+            s |= soft[i];
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) part += __shfl_xor_sync(0xffffffffu, part, o);
+        if (lane == 0) part_s[threadIdx.x >> 5] = part;
+        if (s) any = 1;
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            unsigned long long total = 0;
+            for (int w = 0; w < 8; ++w) total += part_s[w];
+            plan[0] = (int32_t) min(total, 0x7fffffffull);
+            plan[1] = 0;   // this and the last four: fattn_tile_vote_kernel
+            plan[2] = any;
+            plan[4] = plan[5] = plan[6] = plan[7] = 0;
+        }
     }
 }
 
-// Fourth pass: how much the tokens of a ubatch share their cells.  plan[1] = the sum, over groups of 16 consecutive
+// Third pass: how much the tokens of a ubatch share their cells.  plan[1] = the sum, over groups of 16 consecutive
 // tokens, of the number of mask words any token of the group attends to.  Against plan[0] (the same sum token by token)
 // it tells whether walking the cells once per group (fattn_tile_kernel) beats walking them once per token: a prompt's
 // tokens share nearly all their words, the tokens of a decode batch share none.  And the same for every tile the
 // query-tiled kernel may use (4, 8, 16 or 32 tokens): tiles whose tokens share little (decode tokens beside a prompt) are
 // flagged and listed, their tokens are walked one by one (plan[4 + k] = listed tiles of 4 << k tokens).  The line lies at
 // three tokens per word: a shared chunk costs its CTA about as much as two to three chunks of single tokens cost theirs.
-__global__ void __launch_bounds__(256) fattn_tile_vote_kernel(const unsigned long long *__restrict__ words, const int32_t *__restrict__ wcount, int64_t Nq, int64_t nw,
+constexpr int VOTE_WORDS = 4096;
+__global__ void __launch_bounds__(256) fattn_tile_vote_kernel(const int32_t *__restrict__ wlist, const int32_t *__restrict__ wcount, int64_t Nq, int64_t nw,
                                                              int32_t *__restrict__ plan, int32_t *__restrict__ flags, int32_t *__restrict__ lists, int64_t stride) {
+    pdl_prologue();
     const int64_t t0 = (int64_t) blockIdx.x * 32;
     const int n = (int) min((int64_t) 32, Nq - t0);
     int cnt[15];   // words of: 8 groups of 4 tokens, 4 of 8, 2 of 16, 1 of 32
 #pragma unroll
     for (int i = 0; i < 15; ++i) cnt[i] = 0;
-    for (int64_t wi = threadIdx.x; wi < nw; wi += blockDim.x) {
-        unsigned nz = 0;
-#pragma unroll 8
-        for (int j = 0; j < n; ++j) nz |= (words[(t0 + j) * nw + wi] != 0ull ? 1u : 0u) << j;
+    __shared__ unsigned who[VOTE_WORDS];   // per word: the tokens that attend to it
+    for (int64_t w0 = 0; w0 < nw; w0 += VOTE_WORDS) {
+        const int m = (int) min((int64_t) VOTE_WORDS, nw - w0);
+        for (int i = threadIdx.x; i < m; i += blockDim.x) who[i] = 0u;
+        __syncthreads();
+        for (int j = threadIdx.x >> 5; j < n; j += 8) {
+            const int32_t *wl = wlist + (t0 + j) * nw;
+            const int c = wcount[t0 + j];
+            for (int e = threadIdx.x & 31; e < c; e += 32) {
+                const int64_t wi = wl[e] - w0;
+                if (wi >= 0 && wi < m) atomicOr(who + wi, 1u << j);
+            }
+        }
+        __syncthreads();
+        for (int wi = threadIdx.x; wi < m; wi += blockDim.x) {
+            const unsigned nz = who[wi];
 #pragma unroll
-        for (int i = 0; i < 8; ++i) cnt[i] += ((nz >> (4 * i)) & 0xfu) != 0;
+            for (int i = 0; i < 8; ++i) cnt[i] += ((nz >> (4 * i)) & 0xfu) != 0;
 #pragma unroll
-        for (int i = 0; i < 4; ++i) cnt[8 + i] += ((nz >> (8 * i)) & 0xffu) != 0;
+            for (int i = 0; i < 4; ++i) cnt[8 + i] += ((nz >> (8 * i)) & 0xffu) != 0;
 #pragma unroll
-        for (int i = 0; i < 2; ++i) cnt[12 + i] += ((nz >> (16 * i)) & 0xffffu) != 0;
-        cnt[14] += nz != 0;
+            for (int i = 0; i < 2; ++i) cnt[12 + i] += ((nz >> (16 * i)) & 0xffffu) != 0;
+            cnt[14] += nz != 0;
+        }
+        __syncthreads();
     }
     __shared__ int sum[15];
     if (threadIdx.x < 15) sum[threadIdx.x] = 0;
@@ -560,32 +642,61 @@ __global__ void __launch_bounds__(128) fattn_parity_kernel(FattnParams p) {
     for (int i = 0; i < E; ++i) p.dst[row * D + lane + 32 * i] = __fmul_rn(__half2float(acc[i]), S_inv);
 }
 
-template <int D, bool QUANT>
-__global__ void __launch_bounds__(D) fattn_combine_kernel(FattnParams p, int ctas_per_token) {
+// Adds a row's KV splits.  A warp per row (ALL), 8 warps per CTA: with a CTA per row most of the time went into starting 16384
+// CTAs (512 tokens x 32 heads, 3 splits of 128: 24 us, now 9.5).  Few rows are bound by the chain of one warp, which then takes
+// 32 elements of a row.  Lane s has the scale of split s, so the parts themselves are loaded without waiting for it.
+constexpr int FC_THREADS = 256, FC_ALL_ROWS = 2048;   // rows from which a warp takes a whole row
+template <int D, bool QUANT, bool ALL>
+__global__ void __launch_bounds__(FC_THREADS) fattn_combine_kernel(FattnParams p, int ctas_per_token) {
     pdl_prologue(p.early != 0);
     if (p.vote == 1 && fattn_tiled_chosen(p.plan)) return;    // the query-tiled kernel wrote the result
     if (p.vote == 2 && !fattn_tiled_chosen(p.plan)) return;   // this is the query-tiled kernel's combine pass and the per-token kernel worked
-    const float *__restrict__ partial = p.partial;
+    constexpr int E = ALL ? D / 32 : 1, PER_ROW = D / 32 / E;
+    const int lane = threadIdx.x & 31;
+    const unsigned unit = blockIdx.x * (FC_THREADS / 32) + (threadIdx.x >> 5);
+    const int64_t row = unit / PER_ROW;   // token * H + head
+    const int d = (int) (unit % PER_ROW) * 32 + lane;
+    if (row >= p.Nq * p.H) return;
+    const float *pp = p.partial + row * p.nsplit * (D + 2);
     int nsplit = p.nsplit;
-    const int64_t row = blockIdx.x;  // token * H + head
-    const int d = threadIdx.x;
-    const float *pp = partial + row * nsplit * (D + 2);
+    const unsigned H = (unsigned) p.H, tok = (unsigned) row / H, head = (unsigned) row - tok * H;
     if (p.w0 != 0) {   // the splits this token really has; a token with one split was written directly
         const int w0 = fattn_target_words(p, ctas_per_token);
-        const int64_t n_words = p.wcount ? (int64_t) p.wcount[row / p.H] : p.nw;
+        const int64_t n_words = p.wcount ? (int64_t) p.wcount[tok] : p.nw;
         nsplit = (int) min((int64_t) nsplit, max((int64_t) 1, (n_words + w0 - 1) / w0));
         if (nsplit == 1) return;
     }
-    float mn = -CUDART_INF_F;
-    for (int s = 0; s < nsplit; ++s) mn = fmaxf(mn, pp[s * (D + 2) + D]);
-    float a = 0.0f, ls = 0.0f;
-    for (int s = 0; s < nsplit; ++s) {
-        const float ms = pp[s * (D + 2) + D];
-        const float sc = (ms == -CUDART_INF_F) ? 0.0f : expf(ms - mn);
-        a += pp[s * (D + 2) + d] * sc;
-        ls += pp[s * (D + 2) + D + 1] * sc;
+    float ms[2], l[2];   // of splits lane and lane + 32 (at most 64)
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+        const int s = lane + 32 * i;
+        ms[i] = s < nsplit ? pp[s * (D + 2) + D] : -CUDART_INF_F;
+        l[i] = s < nsplit ? pp[s * (D + 2) + D + 1] : 0.0f;
     }
-    fattn_store_out<D, QUANT>(p, row / p.H, row % p.H, d, a * (1.0f / ls));
+    float mn = fmaxf(ms[0], ms[1]);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) mn = fmaxf(mn, __shfl_xor_sync(0xffffffffu, mn, o));
+    float sc[2];
+#pragma unroll
+    for (int i = 0; i < 2; ++i) sc[i] = ms[i] == -CUDART_INF_F ? 0.0f : expf(ms[i] - mn);
+    float a[E], ls = 0.0f;
+#pragma unroll
+    for (int i = 0; i < E; ++i) a[i] = 0.0f;
+#pragma unroll 4
+    for (int s = 0; s < nsplit; ++s) {
+        const float f = __shfl_sync(0xffffffffu, s < 32 ? sc[0] : sc[1], s & 31), ll = __shfl_sync(0xffffffffu, s < 32 ? l[0] : l[1], s & 31);
+#pragma unroll
+        for (int i = 0; i < E; ++i) a[i] = fmaf(pp[s * (D + 2) + d + 32 * i], f, a[i]);
+        ls = fmaf(ll, f, ls);
+    }
+#pragma unroll
+    for (int i = 0; i < E; ++i) fattn_store_out<D, QUANT>(p, tok, head, d + 32 * i, a[i] * (1.0f / ls));
+}
+template <int D, bool QUANT>
+static void launch_combine(const FattnParams &p, int ctas_per_token, cudaStream_t st) {
+    const int64_t rows = p.Nq * p.H;
+    if (rows >= FC_ALL_ROWS) launch_pdl(fattn_combine_kernel<D, QUANT, true>, dim3((unsigned) ((rows + 7) / 8)), dim3(FC_THREADS), 0, st, p, ctas_per_token);
+    else launch_pdl(fattn_combine_kernel<D, QUANT, false>, dim3((unsigned) ((rows * (D / 32) + 7) / 8)), dim3(FC_THREADS), 0, st, p, ctas_per_token);
 }
 
 
@@ -626,7 +737,6 @@ static int fattn_nsplit(int64_t Nq, int64_t Hkv, int hgroups, int64_t n_kv) {
     return (int) std::min<int64_t>(ns, 64);
 }
 
-static bool cuda_memset_ok(void *p, size_t n, cudaStream_t st) { return cudaMemsetAsync(p, 0, n, st) == cudaSuccess; }
 int fattn_tile_min_nq();
 
 // KV splits of the query-tiled kernel: enough CTAs for two per SM twice over, a split walks at least 256 cells
@@ -661,7 +771,7 @@ extern "C" {
 // index layout: words [Nq][nw] u64 | list of non-empty word indices [Nq][nw] i32 | their counts [Nq] i32 |
 // tokens by decreasing count [Nq] i32 | plan: total words i32, words summed over 16-token groups i32, 1 if the mask
 // holds values other than 0 and -inf in participating cells i32, unused, listed tiles of 4, 8, 16, 32 tokens 4 x i32 |
-// flag per tile, 4 x [Nq / 4] i32 | lists of flagged tiles, 4 x [Nq / 4] i32
+// flag per tile, 4 x [Nq / 4] i32 | lists of flagged tiles, 4 x [Nq / 4] i32 | per token: the row is more than its bits [Nq] i32
 static size_t index_list_offset(int64_t Nq, int64_t nw) { return align_up((size_t) Nq * nw * 8, 256); }
 static size_t index_count_offset(int64_t Nq, int64_t nw) { return index_list_offset(Nq, nw) + align_up((size_t) Nq * nw * 4, 256); }
 
@@ -670,11 +780,12 @@ static size_t index_plan_offset(int64_t Nq, int64_t nw) { return index_order_off
 
 static size_t index_tiles_offset(int64_t Nq, int64_t nw) { return index_plan_offset(Nq, nw) + 256; }
 static int64_t index_tiles_stride(int64_t Nq) { return (Nq + 255) / 256 * 64; }   // of one flag array or list, in elements
+static size_t index_soft_offset(int64_t Nq, int64_t nw) { return index_tiles_offset(Nq, nw) + 8 * index_tiles_stride(Nq) * 4; }
 
 size_t b200_mask_index_bytes(int64_t Nq, int64_t n_kv) {
     if (Nq <= 0 || n_kv <= 0) return 0;
     const int64_t nw = (n_kv + 63) / 64;
-    return index_tiles_offset(Nq, nw) + 8 * index_tiles_stride(Nq) * 4;
+    return index_soft_offset(Nq, nw) + align_up((size_t) Nq * 4, 256);
 }
 
 int b200_mask_index_build(const void *mask, int64_t mask_nb_row, int64_t Nq, int64_t n_kv, void *index, size_t index_bytes,
@@ -683,25 +794,22 @@ int b200_mask_index_build(const void *mask, int64_t mask_nb_row, int64_t Nq, int
     B200_REQUIRE(is_aligned(mask, 2) && mask_nb_row % 2 == 0 && is_aligned(index, 8), "misaligned mask or index");
     if (index_bytes < b200_mask_index_bytes(Nq, n_kv)) return set_error(B200_E_SCRATCH, "mask index buffer too small");
     const int64_t nw = (n_kv + 63) / 64;
-    const int64_t threads = Nq * nw * 32;
-    int32_t *plan = (int32_t *) ((char *) index + index_plan_offset(Nq, nw));
-    if (!cuda_memset_ok(plan, 32, (cudaStream_t) stream)) return set_error(B200_E_CUDA, "mask index: cudaMemsetAsync failed");
-    mask_index_kernel<<<(unsigned) ((threads + 255) / 256), 256, 0, (cudaStream_t) stream>>>(
-        (const __half *) mask, mask_nb_row, Nq, n_kv, nw, (unsigned long long *) index, plan + 2);
+    B200_REQUIRE(Nq <= 0x0fffffff, "too many tokens");
+    const cudaStream_t st = (cudaStream_t) stream;
+    char *ix = (char *) index;
+    int32_t *plan = (int32_t *) (ix + index_plan_offset(Nq, nw)), *wlist = (int32_t *) (ix + index_list_offset(Nq, nw)), *wcount = (int32_t *) (ix + index_count_offset(Nq, nw));
+    int32_t *soft = (int32_t *) (ix + index_soft_offset(Nq, nw));
+    const bool vec = is_aligned(mask, 16) && mask_nb_row % 16 == 0;
+    launch_pdl(vec ? mask_index_kernel<true> : mask_index_kernel<false>, dim3((unsigned) Nq), dim3(MI_THREADS), 0, st, (const __half *) mask, mask_nb_row, n_kv, nw,
+               (unsigned long long *) index, wlist, wcount, soft);
     if (int e = check_launch("mask_index")) return e;
-    mask_words_compact_kernel<<<(unsigned) ((Nq * 32 + 255) / 256), 256, 0, (cudaStream_t) stream>>>(
-        (const unsigned long long *) index, Nq, nw, (int32_t *) ((char *) index + index_list_offset(Nq, nw)),
-        (int32_t *) ((char *) index + index_count_offset(Nq, nw)));
-    if (int e = check_launch("mask_words_compact")) return e;
-    fattn_plan_kernel<<<1, 1024, 0, (cudaStream_t) stream>>>((const int32_t *) ((char *) index + index_count_offset(Nq, nw)), Nq,
-                                                             (int32_t *) ((char *) index + index_order_offset(Nq, nw)),
-                                                             (int32_t *) ((char *) index + index_plan_offset(Nq, nw)));
+    launch_pdl(fattn_plan_kernel, dim3((unsigned) ((Nq + 7) / 8)), dim3(256), 0, st, (const int32_t *) wcount, (const int32_t *) soft, Nq, (int32_t *) (ix + index_order_offset(Nq, nw)), plan);
     if (int e = check_launch("fattn_plan")) return e;
     if (Nq >= fattn_tile_min_nq() && fattn_tile_min_nq() > 0) {   // only ubatches the query-tiled kernel may take need the vote
         int32_t *flags = (int32_t *) ((char *) index + index_tiles_offset(Nq, nw));
         const int64_t stride = index_tiles_stride(Nq);
-        fattn_tile_vote_kernel<<<(unsigned) ((Nq + 31) / 32), 256, 0, (cudaStream_t) stream>>>(
-            (const unsigned long long *) index, (const int32_t *) ((char *) index + index_count_offset(Nq, nw)), Nq, nw, plan, flags, flags + 4 * stride, stride);
+        launch_pdl(fattn_tile_vote_kernel, dim3((unsigned) ((Nq + 31) / 32)), dim3(256), 0, st, (const int32_t *) wlist, (const int32_t *) wcount, Nq, nw, plan, flags,
+                   flags + 4 * stride, stride);
         return check_launch("fattn_tile_vote");
     }
     return B200_OK;
@@ -824,8 +932,8 @@ static int flash_attn_impl(bool parity, int64_t D, int64_t H, int64_t Hkv, int64
         else launch_pdl(fattn_tile_kernel<64>, tgrid, dim3(FT_THREADS), (size_t) fattn_tile_smem_bytes(64), st, pt, gqa_log2);
         if (int e = check_launch("fattn_tile")) return e;
         if (pt.nsplit > 1) {
-            if (D == 128) launch_pdl(fattn_combine_kernel<128, false>, dim3((unsigned) (Nq * H)), dim3(128), 0, st, pt, 1);
-            else launch_pdl(fattn_combine_kernel<64, false>, dim3((unsigned) (Nq * H)), dim3(64), 0, st, pt, 1);
+            if (D == 128) launch_combine<128, false>(pt, 1, st);
+            else launch_combine<64, false>(pt, 1, st);
             if (int e = check_launch("fattn_combine")) return e;
         }
         if (!index) return B200_OK;   // no mask: every token attends every cell, nothing to vote on
@@ -842,14 +950,13 @@ static int flash_attn_impl(bool parity, int64_t D, int64_t H, int64_t Hkv, int64
     }
     if (int e = check_launch("fattn_mma")) return e;
     if (ns > 1) {
-        const dim3 cgrid((unsigned) (Nq * H));
         const int cpt = (int) (Hkv * hgroups);
         if (D == 128) {
-            if (qo) launch_pdl(fattn_combine_kernel<128, true>, cgrid, dim3(128), 0, st, p, cpt);
-            else launch_pdl(fattn_combine_kernel<128, false>, cgrid, dim3(128), 0, st, p, cpt);
+            if (qo) launch_combine<128, true>(p, cpt, st);
+            else launch_combine<128, false>(p, cpt, st);
         } else {
-            if (qo) launch_pdl(fattn_combine_kernel<64, true>, cgrid, dim3(64), 0, st, p, cpt);
-            else launch_pdl(fattn_combine_kernel<64, false>, cgrid, dim3(64), 0, st, p, cpt);
+            if (qo) launch_combine<64, true>(p, cpt, st);
+            else launch_combine<64, false>(p, cpt, st);
         }
         return check_launch("fattn_combine");
     }

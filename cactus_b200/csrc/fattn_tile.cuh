@@ -34,23 +34,29 @@ __device__ __forceinline__ void ft_ldmatrix_x4_trans(uint32_t (&r)[4], uint32_t 
     asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];\n" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr));
 }
 
+__device__ __forceinline__ void ft_ldmatrix_x4(uint32_t (&r)[4], uint32_t addr) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];\n" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr));
+}
+
 // dynamic shared memory of the kernel: FT_STAGES stages of K and V rows
 constexpr int fattn_tile_smem_bytes(int D) { return FT_STAGES * 2 * FT_CHUNK * (D * 2 + 16); }   // as much as ft_spread's 4 x 3 x 16 rows
 
 // ---- the steps of one chunk of 32 cells; rows g and g + 8 of a warp's 16 ----
 // S = Q K^T for n-tiles C0 .. C0 + CN - 1 of 8 cells (independent accumulator chains); Ks: the staged row of the first cell
 template <int D, int C0, int CN>
-__device__ __forceinline__ void ft_s(float (&sacc)[4][4], const uint32_t (&qa)[D / 16][4], const uint8_t *Ks, int g, int t) {
+__device__ __forceinline__ void ft_s(float (&sacc)[4][4], const uint32_t (&qa)[D / 16][4], uint32_t Ks, int lane) {
     constexpr int ROW = D * 2 + 16;
+    const uint32_t at = Ks + (uint32_t) ((8 * (lane >> 4) + (lane & 7)) * ROW + ((lane >> 3) & 1) * 16);
 #pragma unroll
     for (int c = C0; c < C0 + CN; ++c) sacc[c][0] = sacc[c][1] = sacc[c][2] = sacc[c][3] = 0.0f;
 #pragma unroll
     for (int ks = 0; ks < D / 16; ++ks)
 #pragma unroll
-        for (int c = C0; c < C0 + CN; ++c) {
-            const uint8_t *krow = Ks + (8 * (c - C0) + g) * ROW + 4 * t + 32 * ks;
-            const uint32_t b0 = *reinterpret_cast<const uint32_t *>(krow), b1 = *reinterpret_cast<const uint32_t *>(krow + 16);
-            mma_f16(sacc[c], qa[ks][0], qa[ks][1], qa[ks][2], qa[ks][3], b0, b1);
+        for (int c = C0; c < C0 + CN; c += 2) {
+            uint32_t b[4];   // both halves of this k-step for n-tile c, then for n-tile c + 1
+            ft_ldmatrix_x4(b, at + (uint32_t) (8 * (c - C0) * ROW + 32 * ks));
+            mma_f16(sacc[c], qa[ks][0], qa[ks][1], qa[ks][2], qa[ks][3], b[0], b[1]);
+            mma_f16(sacc[c + 1], qa[ks][0], qa[ks][1], qa[ks][2], qa[ks][3], b[2], b[3]);
         }
 }
 // Online softmax: element [c][2 i + e] is (row g + 8 i, cell 8 c + 2 t + e of the chunk); rm: which cells row g + 8 i attends
@@ -130,12 +136,19 @@ __device__ __forceinline__ void ft_pv(float (&o)[D / 8][4], const uint32_t (&ph)
 }
 // The words any of the tile's tokens attends to, ascending, from the tokens' lists (all of them without a mask).  bits: one per
 // word.  The whole CTA calls it; the result may be read after it.
-__device__ __forceinline__ int ft_union(const FattnParams &p, int64_t tok0, int n_tok, unsigned *bits, unsigned short *uw_index, int *warp_cnt) {
+__device__ __forceinline__ int ft_union(const FattnParams &p, int64_t tok0, int n_tok, unsigned *bits, unsigned short *uw_index, int *warp_cnt, unsigned short *before = nullptr) {
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int n32 = (int) ((p.nw + 31) / 32);
-    for (int i = tid; i < n32; i += FT_THREADS) bits[i] = p.words ? 0u : (p.nw - 32 * i >= 32 ? ~0u : (1u << (p.nw - 32 * i)) - 1u);
+    if (p.words && p.nw <= FT_THREADS) {   // a thread per word: no dependent loads (list length, list, word)
+        unsigned long long w = 0;
+        if (tid < p.nw)
+#pragma unroll 8
+            for (int j = 0; j < n_tok; ++j) w |= p.words[(tok0 + j) * p.nw + tid];
+        const unsigned m = __ballot_sync(0xffffffffu, w != 0ull);
+        if (lane == 0) bits[warp] = m;
+    } else for (int i = tid; i < n32; i += FT_THREADS) bits[i] = p.words ? 0u : (p.nw - 32 * i >= 32 ? ~0u : (1u << (p.nw - 32 * i)) - 1u);
     __syncthreads();
-    if (p.words)
+    if (p.words && p.nw > FT_THREADS)
         for (int j = warp; j < n_tok; j += FT_THREADS / 32) {
             const int32_t *wl = p.wlist + (tok0 + j) * p.nw;
             const int n = p.wcount[tok0 + j];
@@ -158,6 +171,7 @@ __device__ __forceinline__ int ft_union(const FattnParams &p, int64_t tok0, int 
         at += w < warp ? warp_cnt[w] : 0;
         all += warp_cnt[w];
     }
+    if (before && tid < n32) before[tid] = (unsigned short) at;
     for (unsigned m = mine; m; m &= m - 1) uw_index[at++] = (unsigned short) (32 * tid + __ffs((int) m) - 1);
     __syncthreads();
     return all;
@@ -195,6 +209,7 @@ struct FtTileShared {
 struct FtSpreadShared {
     unsigned short uw_index[FT_MAX_WORDS];
     unsigned bits[FT_MAX_WORDS / 32];
+    unsigned short before[FT_MAX_WORDS / 32];   // union words before each 32
     int warp_cnt[FT_THREADS / 32];
     alignas(16) short list[FT_THREADS / 32][FT_LIST];     // per warp: the round's union positions, 64 * slot + bit of a cell its token attends to or -1
     int cells[FT_THREADS / 32][2][FT_CHUNK];   // per warp: the cells of the chunk at work and of the next
@@ -216,14 +231,13 @@ __device__ __forceinline__ void ft_spread(const FattnParams &p, int gqa_log2, Ft
     const int hk = blockIdx.x, split = blockIdx.z, nsplit = p.nsplit;
     const bool binary_mask = p.plan[2] == 0;
     const char *kbase = p.k + (int64_t) hk * p.k_nb_head, *vbase = p.v + (int64_t) hk * p.v_nb_head;
-    uint8_t *slots = kv_s + warp * 3 * HALF;
-    const uint32_t slots_u32 = (uint32_t) __cvta_generic_to_shared(slots);
+    const uint32_t slots_u32 = (uint32_t) __cvta_generic_to_shared(kv_s + warp * 3 * HALF);
     short *list = sh.list[warp];
     const int n_units = *p.tcount * quads;
     for (int unit = blockIdx.y; unit < n_units; unit += p.spread_rows) {
         const int64_t tok0 = (int64_t) p.tlist[unit / quads] * tile_tok, tok = tok0 + (unit % quads) * 4 + warp;
         __syncthreads();   // the lists of the unit before are no longer read
-        const int n_uw = ft_union(p, tok0, (int) min((int64_t) tile_tok, p.Nq - tok0), sh.bits, sh.uw_index, sh.warp_cnt);
+        const int n_uw = ft_union(p, tok0, (int) min((int64_t) tile_tok, p.Nq - tok0), sh.bits, sh.uw_index, sh.warp_cnt, sh.before);
         if (tok >= p.Nq) continue;
         const int n_tok = (int) min((int64_t) tile_tok, p.Nq - tok0);
         uint32_t qa[KS][4];
@@ -255,26 +269,31 @@ __device__ __forceinline__ void ft_spread(const FattnParams &p, int gqa_log2, Ft
 
         // the chunks of this split with a cell of the token, one after the other: rm and, in sh.cells[warp][b], 32 cells (where the
         // token does not attend, one that it does attend)
-        int r0 = -FT_RW, chunk = 0, n_chunks = 0;   // r0: the round whose list is built
+        int r0 = 0, chunk = 0, n_chunks = 0;   // r0: the round whose list is built
+        const int32_t *wl = p.wlist + tok * p.nw;
+        const int n_wl = p.wcount[tok];
+        int entry = 0, wl_at = 0;              // the token's words up to `entry` are in rounds up to r0; lane i holds the word wl_at + i
+        int wl_mine = lane < n_wl ? wl[lane] : 0;
         auto next_chunk = [&](int b) -> unsigned {
             while (true) {
                 if (chunk >= n_chunks) {   // on to the next round in which the token attends to a word
+                    if (entry >= n_wl) return 0u;
+                    if (entry - wl_at >= 32) {
+                        wl_at = entry;
+                        wl_mine = wl_at + lane < n_wl ? wl[wl_at + lane] : 0;
+                    }
+                    const int first = __shfl_sync(0xffffffffu, wl_mine, entry - wl_at);
+                    r0 = (sh.before[first >> 5] + __popc(sh.bits[first >> 5] & ((1u << (first & 31)) - 1u))) & ~(FT_RW - 1);
                     unsigned long long own = 0, all = 0;
-                    int n_own = 0;
-                    do {
-                        r0 += FT_RW;
-                        if (r0 >= n_uw) return 0u;
-                        const int k = lane & 15;
-                        own = 0;
-                        if (r0 + k < n_uw) own = p.words[tok * p.nw + sh.uw_index[r0 + k]];
-                        n_own = __popc(__ballot_sync(0xffffffffu, own != 0ull));
-                    } while (n_own == 0);
                     const int k = lane & 15;
                     if (r0 + k < n_uw) {
-                        const unsigned long long *w = p.words + tok0 * p.nw + sh.uw_index[r0 + k];
+                        const unsigned long long *w = p.words + sh.uw_index[r0 + k];
+                        own = w[tok * p.nw];
 #pragma unroll 8
-                        for (int j = lane >> 4; j < n_tok; j += 2) all |= w[j * p.nw];
+                        for (int j = lane >> 4; j < n_tok; j += 2) all |= w[(tok0 + j) * p.nw];
                     }
+                    unsigned own_set = __ballot_sync(0xffffffffu, own != 0ull) & 0xffffu;
+                    entry += __popc(own_set);
                     all |= __shfl_xor_sync(0xffffffffu, all, 16);
                     const int cnt = __popcll(all);
                     int pre = cnt;
@@ -288,9 +307,9 @@ __device__ __forceinline__ void ft_spread(const FattnParams &p, int gqa_log2, Ft
                     chunk = split;
                     for (int i = lane; i < n_chunks * (FT_CHUNK / 8); i += 32) reinterpret_cast<uint4 *>(list)[i] = make_uint4(~0u, ~0u, ~0u, ~0u);
                     __syncwarp();
-                    for (int w = 0; w < FT_RW; ++w) {
+                    for (; own_set; own_set &= own_set - 1) {
+                        const int w = __ffs((int) own_set) - 1;
                         const unsigned long long ow = __shfl_sync(0xffffffffu, own, w);
-                        if (ow == 0ull) continue;
                         const unsigned long long aw = __shfl_sync(0xffffffffu, all, w);
                         const int base = __shfl_sync(0xffffffffu, pre - cnt, w);
 #pragma unroll
@@ -343,12 +362,12 @@ __device__ __forceinline__ void ft_spread(const FattnParams &p, int gqa_log2, Ft
             float sacc[4][4];
             uint32_t ph[2][4], pl[2][4];
             landed();
-            ft_s<D, 0, 2>(sacc, qa, slots + s0 * HALF, g, t);
+            ft_s<D, 0, 2>(sacc, qa, slots_u32 + (uint32_t) (s0 * HALF), lane);
             __syncwarp();
             fetch(vbase, p.v_nb_cell, cells + 16, s0);
             commit();
             landed();
-            ft_s<D, 2, 2>(sacc, qa, slots + s1 * HALF, g, t);
+            ft_s<D, 2, 2>(sacc, qa, slots_u32 + (uint32_t) (s1 * HALF), lane);
             __syncwarp();
             if (rm_next) fetch(kbase, p.k_nb_cell, ncells, s1);
             commit();
@@ -535,32 +554,27 @@ __global__ void __launch_bounds__(FT_THREADS, 3) fattn_tile_kernel(FattnParams p
         }
         // this split's chunks: split, split + nsplit, ...; FT_STAGES - 1 of them are on their way while one is multiplied
         int issued = 0;
-        for (int k = 0; k < FT_STAGES - 1; ++k) {
-            const int c = split + k * nsplit;
-            if (c < n_chunks) stage(c, count, k);
+        auto issue = [&] {
+            const int c = split + issued * nsplit;
+            if (c < n_chunks) stage(c, count, issued % FT_STAGES);
             else asm volatile("cp.async.commit_group;\n" ::: "memory");
             ++issued;
-        }
+        };
+        for (int k = 0; k < FT_STAGES - 1; ++k) issue();
         int it = 0;
         for (int ch = split; ch < n_chunks; ch += nsplit, ++it) {
             const int s = it % FT_STAGES;
-            {
-                const int c = split + issued * nsplit;
-                if (c < n_chunks) stage(c, count, issued % FT_STAGES);
-                else asm volatile("cp.async.commit_group;\n" ::: "memory");
-                ++issued;
-            }
+            issue();
             asm volatile("cp.async.wait_group %0;\n" ::"n"(FT_STAGES - 1) : "memory");
             __syncthreads();   // the stage has landed for every thread (and, first time round, the row masks are written)
-            const uint8_t *Ks = kv_s + (s * 2) * (FT_CHUNK * ROW);
-            const uint32_t Vs = kv_u32 + (uint32_t) ((s * 2 + 1) * (FT_CHUNK * ROW));
+            const uint32_t Ks = kv_u32 + (uint32_t) ((s * 2) * (FT_CHUNK * ROW)), Vs = Ks + (uint32_t) (FT_CHUNK * ROW);
             unsigned rm[2];
 #pragma unroll
             for (int i = 0; i < 2; ++i) rm[i] = live[i] ? rmask[tl[i]][ch] : 0u;
             if (__any_sync(0xffffffffu, (rm[0] | rm[1]) != 0u)) {   // a chunk that none of the warp's rows attends to changes nothing
                 float sacc[4][4];
                 uint32_t ph[2][4], pl[2][4];
-                ft_s<D, 0, 4>(sacc, qa, Ks, g, t);
+                ft_s<D, 0, 4>(sacc, qa, Ks, lane);
                 ft_softmax<D>(p, sacc, rm, binary_mask, mrow, slope, cell_list + ch * FT_CHUNK, t, m_run, l_run, o, ph, pl);
 #pragma unroll
                 for (int kk = 0; kk < 2; ++kk) ft_pv<D>(o, ph[kk], pl[kk], Vs + (uint32_t) (16 * kk * ROW), lane);
@@ -574,8 +588,7 @@ __global__ void __launch_bounds__(FT_THREADS, 3) fattn_tile_kernel(FattnParams p
     for (int i = 0; i < 2; ++i) {
         l_run[i] += __shfl_xor_sync(0xffffffffu, l_run[i], 1);
         l_run[i] += __shfl_xor_sync(0xffffffffu, l_run[i], 2);
-        if (!live[i]) continue;
-        ft_write<D>(p, tok[i], head[i], split, i, o, m_run[i], l_run[i], t);
+        if (live[i]) ft_write<D>(p, tok[i], head[i], split, i, o, m_run[i], l_run[i], t);
     }
 }
 

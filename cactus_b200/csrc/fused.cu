@@ -5,6 +5,8 @@
 //   SILU (ops.cpp:2902-2981) * up + quantize_row_q8_0
 //   ROPE of q and k (ops.cpp:5080-5362) + the f32 -> f16 stores of k and v into the cache rows (cpy_k / cpy_v,
 //   cactus/llama-kv-cache.cpp:617-656)
+#include <algorithm>
+
 #include "common.cuh"
 
 namespace b200 {
@@ -13,28 +15,36 @@ namespace b200 {
 // quantised store.  The sum of squares is accumulated in the order rms_norm_kernel uses (rms_block_sum), so the
 // scale -- and with it every quantised value -- is bit-identical to the unfused chain.
 // (x, res and h carry no __restrict__: a graph allocator may hand the same memory to the residual and to the normalised output)
-__global__ void __launch_bounds__(1024) add_rms_norm_quantize_kernel(float *x, int64_t x_nb_row, const float *res,
+// Bound by latency at few rows (load, reduce, 32 dependent double additions, scale), by memory at many.  One group per thread
+// (GMAX 1: rows of up to 4096 elements) fits 32 registers, so two CTAs of 1024 threads share an SM, and the weight is loaded
+// with the row; only the first warp adds up the warps' sums and works the scale out, with the exact reciprocal where d is a
+// power of two (the same quotient), instead of all of them.  Before / now: the table at the head of this file.
+template <int GMAX>   // groups of 4 elements per thread: d <= 4 GMAX blockDim.x
+__global__ void __launch_bounds__(1024, GMAX == 1 ? 2 : 1) add_rms_norm_quantize_kernel(float *x, int64_t x_nb_row, const float *res,
                                                                     int64_t res_nb_row, const float *__restrict__ w, float *h,
-                                                                    int64_t h_nb_row, int64_t d, int64_t N, float eps, int64_t nb, int64_t nbp,
+                                                                    int64_t h_nb_row, int d, int64_t N, float eps, double inv_d, int64_t nb, int64_t nbp,
                                                                     uint8_t *__restrict__ out, size_t d_offset, int variant, int early) {
     pdl_prologue(early != 0);
-    constexpr int GMAX = 4;   // groups of 4 elements per thread: d <= 16 * blockDim.x
     const int64_t n = blockIdx.x;
     const bool row_real = n < N;
-    const int64_t groups = d / 4, groups_padded = nbp * 8;
+    const int groups = d / 4, groups_padded = (int) nbp * 8;
+    const bool w_vec = (reinterpret_cast<uintptr_t>(w) & 15) == 0;
     float v[GMAX][4];
+    float4 wv[GMAX];
     double sum = 0.0;
     float *xr = row_real ? reinterpret_cast<float *>(reinterpret_cast<char *>(x) + n * x_nb_row) : nullptr;
     const float *rr = (row_real && res) ? reinterpret_cast<const float *>(reinterpret_cast<const char *>(res) + n * res_nb_row) : nullptr;
 #pragma unroll
     for (int k = 0; k < GMAX; ++k) {
-        const int64_t gi = threadIdx.x + (int64_t) k * blockDim.x;
+        const int gi = threadIdx.x + k * blockDim.x;
         v[k][0] = v[k][1] = v[k][2] = v[k][3] = 0.0f;
+        wv[k] = make_float4(1.0f, 1.0f, 1.0f, 1.0f);
         if (row_real && gi < groups) {
             const float4 a = *reinterpret_cast<const float4 *>(xr + gi * 4);
+            const float4 b = rr ? *reinterpret_cast<const float4 *>(rr + gi * 4) : make_float4(0.f, 0.f, 0.f, 0.f);
+            if (w) wv[k] = w_vec ? __ldg(reinterpret_cast<const float4 *>(w) + gi) : make_float4(w[gi * 4], w[gi * 4 + 1], w[gi * 4 + 2], w[gi * 4 + 3]);
             v[k][0] = a.x; v[k][1] = a.y; v[k][2] = a.z; v[k][3] = a.w;
             if (rr) {
-                const float4 b = *reinterpret_cast<const float4 *>(rr + gi * 4);
                 v[k][0] = v[k][0] + b.x; v[k][1] = v[k][1] + b.y; v[k][2] = v[k][2] + b.z; v[k][3] = v[k][3] + b.w;
                 *reinterpret_cast<float4 *>(xr + gi * 4) = make_float4(v[k][0], v[k][1], v[k][2], v[k][3]);
             }
@@ -42,54 +52,71 @@ __global__ void __launch_bounds__(1024) add_rms_norm_quantize_kernel(float *x, i
             for (int i = 0; i < 4; ++i) sum += (double) (v[k][i] * v[k][i]);
         }
     }
-    const double tot = rms_block_sum(sum);
-    const float mean = (float) (tot / (double) d);
-    const float sc = 1.0f / sqrtf(mean + eps);
+    __shared__ double red[32];
+    __shared__ float sc_s;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+    if (lane == 0) red[warp] = sum;
+    __syncthreads();
+    if (warp == 0) {
+        double tot = 0.0;
+        if (warps == 32) {
+#pragma unroll
+            for (int i = 0; i < 32; ++i) tot += red[i];
+        } else {
+#pragma unroll 4
+            for (int i = 0; i < warps; ++i) tot += red[i];
+        }
+        const float mean = (float) (inv_d != 0.0 ? tot * inv_d : tot / (double) d);
+        if (lane == 0) sc_s = 1.0f / sqrtf(mean + eps);
+    }
+    __syncthreads();
+    pdl_trigger();
+    const float sc = sc_s;
     float *hr = (h && row_real) ? reinterpret_cast<float *>(reinterpret_cast<char *>(h) + n * h_nb_row) : nullptr;
 #pragma unroll
     for (int k = 0; k < GMAX; ++k) {
-        const int64_t gi = threadIdx.x + (int64_t) k * blockDim.x;
+        const int gi = threadIdx.x + k * blockDim.x;
         if (gi >= groups_padded) continue;   // whole 8-lane block groups leave together
         const bool real = row_real && gi < groups;
         float o[4] = {0.f, 0.f, 0.f, 0.f};
         if (real) {
+            const float wf[4] = {wv[k].x, wv[k].y, wv[k].z, wv[k].w};
 #pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                const float t = v[k][i] * sc;
-                o[i] = w ? t * w[gi * 4 + i] : t;
-            }
+            for (int i = 0; i < 4; ++i) o[i] = (v[k][i] * sc) * wf[i];   // (without a weight: times one)
             if (hr) *reinterpret_cast<float4 *>(hr + gi * 4) = make_float4(o[0], o[1], o[2], o[3]);
         }
-        q8_quantize_store<1>(o, out, d_offset, nb, nbp, n, gi >> 3, (int) (gi & 7), real, variant);
+        q8_quantize_store<1>(o, out, d_offset, nb, nbp, n, gi >> 3, gi & 7, real, variant);
     }
 }
 
-// silu(gate) * up, quantised; the same index space as quantize_q8_0_kernel
+// silu(gate) * up, quantised; the same index space as quantize_q8_0_kernel: a row per x, 256 groups of 4 elements per y (no
+// 64-bit division per thread, which was most of the instructions)
 __global__ void __launch_bounds__(256) silu_mul_quantize_kernel(const float *gate, const float *up, int64_t nb_row,
                                                                float *dst, int64_t dst_nb_row,
-                                                               int64_t N, int64_t n_rows_padded, int64_t nb, int64_t nbp,
+                                                               int64_t N, int64_t nb, int64_t nbp,
                                                                uint8_t *__restrict__ out, size_t d_offset, int variant, int early) {
     pdl_prologue(early != 0);
-    const int64_t gid = (int64_t) blockIdx.x * blockDim.x + threadIdx.x;
-    const int j = (int) (gid & 7);
-    const int64_t blk = gid >> 3;
-    const int64_t n = blk / nbp;
-    const int64_t b = blk - n * nbp;
-    if (n >= n_rows_padded) return;
-    float v[4] = {0.f, 0.f, 0.f, 0.f};
-    const bool real = (n < N) && (b < nb);
-    if (real) {
-        const float4 a = *reinterpret_cast<const float4 *>(reinterpret_cast<const char *>(gate) + n * nb_row + (b * 32 + j * 4) * 4);
-        const float4 u = *reinterpret_cast<const float4 *>(reinterpret_cast<const char *>(up) + n * nb_row + (b * 32 + j * 4) * 4);
-        const float ga[4] = {a.x, a.y, a.z, a.w}, ua[4] = {u.x, u.y, u.z, u.w};
+    const int64_t n = blockIdx.x;
+    for (int64_t at = blockIdx.y * 256 + threadIdx.x; at < nbp * 8; at += gridDim.y * 256) {   // whole groups of 8 lanes leave together
+        const int j = (int) at & 7;
+        const int64_t b = at >> 3;
+        float v[4] = {0.f, 0.f, 0.f, 0.f};
+        const bool real = (n < N) && (b < nb);
+        if (real) {
+            const float4 a = *reinterpret_cast<const float4 *>(reinterpret_cast<const char *>(gate) + n * nb_row + at * 16);
+            const float4 u = *reinterpret_cast<const float4 *>(reinterpret_cast<const char *>(up) + n * nb_row + at * 16);
+            const float ga[4] = {a.x, a.y, a.z, a.w}, ua[4] = {u.x, u.y, u.z, u.w};
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            const float s = ga[i] / (1.0f + expf(-ga[i]));
-            v[i] = s * ua[i];
+            for (int i = 0; i < 4; ++i) {
+                const float s = ga[i] / (1.0f + expf(-ga[i]));
+                v[i] = s * ua[i];
+            }
+            if (dst) *reinterpret_cast<float4 *>(reinterpret_cast<char *>(dst) + n * dst_nb_row + at * 16) = make_float4(v[0], v[1], v[2], v[3]);
         }
-        if (dst) *reinterpret_cast<float4 *>(reinterpret_cast<char *>(dst) + n * dst_nb_row + (b * 32 + j * 4) * 4) = make_float4(v[0], v[1], v[2], v[3]);
+        q8_quantize_store<1>(v, out, d_offset, nb, nbp, n, b, j, real, variant);
     }
-    q8_quantize_store<1>(v, out, d_offset, nb, nbp, n, b, j, real, variant);
 }
 
 // One CTA per token: the angles as rope_norm_kernel builds them, q rotated into qo (which may be q itself, with the same
@@ -101,56 +128,63 @@ __global__ void __launch_bounds__(512) rope_store_kernel(const float *q, float *
                                                         const int32_t *__restrict__ slots, __half *__restrict__ kc, int64_t kc_nb_row,
                                                         __half *__restrict__ vc, int64_t vc_nb_row, int early) {
     pdl_prologue(early != 0);
-    extern __shared__ float cs[];   // [n_dims/2] cos, [n_dims/2] sin, [n_dims/2] theta
+    extern __shared__ float cs[];   // [n_dims/2] cos, [n_dims/2] sin
     const int64_t t = blockIdx.x;
     const int half_dims = n_dims / 2;
-    float *th_s = cs + 2 * half_dims;
-    if (threadIdx.x == 0) {
-        float theta = (float) pos[t];
-        for (int i = 0; i < half_dims; ++i) {
-            th_s[i] = theta;
-            theta *= theta_scale;
-        }
+    const unsigned pairs = (unsigned) (D / 2), n_q = (unsigned) H, n_qk = (unsigned) (H + Hkv), total = (unsigned) (H + (v ? 2 : 1) * Hkv) * pairs;
+    auto load = [&](unsigned i) -> float2 {
+        const unsigned hh = i / pairs, p = i - hh * pairs;
+        if (hh < n_q) return *(reinterpret_cast<const float2 *>(reinterpret_cast<const char *>(q) + t * q_nb_tok + hh * q_nb_head) + p);
+        if (hh < n_qk) return *(reinterpret_cast<const float2 *>(reinterpret_cast<const char *>(k) + t * k_nb_tok + (hh - n_q) * k_nb_head) + p);
+        return *(reinterpret_cast<const float2 *>(reinterpret_cast<const char *>(v) + t * v_nb_tok) + (hh - n_qk) * pairs + p);
+    };
+    // the rows travel while the angles are worked out
+    constexpr int U = 6;   // 6 x 512 pairs: 32 + 2 x 8 heads of 128
+    float2 x[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+        const unsigned i = threadIdx.x + u * blockDim.x;
+        x[u] = i < total ? load(i) : make_float2(0.f, 0.f);
     }
-    __syncthreads();
+    const int64_t slot = slots ? (int64_t) slots[t] : t;   // no slot list: token t goes to row t of the cache pointers given
     for (int i = threadIdx.x; i < 2 * half_dims; i += blockDim.x) {   // first half of the threads: cosines, second half: sines
         const int a = i < half_dims ? i : i - half_dims;
         const float f = ff ? ff[a] : 1.0f;
-        const float th = freq_scale * (th_s[a] / f);
+        // theta_a = pos * theta_scale^a by repeated multiplication, as the reference builds it: every thread walks the chain
+        // to its own angle (a multiplication per step, against a store and a barrier when one thread does it for all)
+        float theta = (float) pos[t], mine = theta;
+#pragma unroll 8
+        for (int s = 0; s <= a; ++s) {
+            mine = theta;
+            theta *= theta_scale;
+        }
+        const float th = freq_scale * (mine / f);
         cs[i] = (i < half_dims ? cosf(th) : sinf(th)) * attn_factor;
     }
     __syncthreads();
-    const int64_t pairs = D / 2;
-    const int64_t slot = slots ? (int64_t) slots[t] : t;   // no slot list: token t goes to row t of the cache pointers given
+    pdl_trigger();
     __half *krow = reinterpret_cast<__half *>(reinterpret_cast<char *>(kc) + slot * kc_nb_row);
     __half *vrow = reinterpret_cast<__half *>(reinterpret_cast<char *>(vc) + slot * vc_nb_row);
-    for (int64_t i = threadIdx.x; i < (H + 2 * Hkv) * pairs; i += blockDim.x) {
-        const int64_t hh = i / pairs, p = i - hh * pairs;
-        if (hh < H) {
-            const int64_t off = t * q_nb_tok + hh * q_nb_head;
-            const float2 x = *(reinterpret_cast<const float2 *>(reinterpret_cast<const char *>(q) + off) + p);
-            float2 *d = reinterpret_cast<float2 *>(reinterpret_cast<char *>(qo) + off) + p;
-            if (p < half_dims) {
-                const float c = cs[p], sn = cs[half_dims + p];
-                *d = make_float2(x.x * c - x.y * sn, x.x * sn + x.y * c);
-            } else if (qo != q) {
-                *d = x;
-            }
-        } else if (hh < H + Hkv) {
-            const int64_t hk = hh - H;
-            const float2 x = *reinterpret_cast<const float2 *>(reinterpret_cast<const float *>(reinterpret_cast<const char *>(k) + t * k_nb_tok + hk * k_nb_head) + 2 * p);
-            float2 r = x;
-            if (p < half_dims) {
-                const float c = cs[p], sn = cs[half_dims + p];
-                r = make_float2(x.x * c - x.y * sn, x.x * sn + x.y * c);
-            }
-            *reinterpret_cast<__half2 *>(krow + hk * D + 2 * p) = __halves2half2(__float2half_rn(r.x), __float2half_rn(r.y));
-        } else if (v) {
-            const int64_t hv = hh - H - Hkv;
-            const float2 x = *reinterpret_cast<const float2 *>(reinterpret_cast<const float *>(reinterpret_cast<const char *>(v) + t * v_nb_tok) + hv * D + 2 * p);
-            *reinterpret_cast<__half2 *>(vrow + hv * D + 2 * p) = __halves2half2(__float2half_rn(x.x), __float2half_rn(x.y));
+    auto finish = [&](unsigned i, float2 x) {
+        const unsigned hh = i / pairs, p = i - hh * pairs;
+        float2 r = x;
+        if (hh < n_qk && p < (unsigned) half_dims) {
+            const float c = cs[p], sn = cs[half_dims + p];
+            r = make_float2(x.x * c - x.y * sn, x.x * sn + x.y * c);
         }
+        if (hh < n_q) {
+            if (p < (unsigned) half_dims || qo != q) *(reinterpret_cast<float2 *>(reinterpret_cast<char *>(qo) + t * q_nb_tok + hh * q_nb_head) + p) = r;
+        } else {
+            __half *to = hh < n_qk ? krow + (hh - n_q) * D : vrow + (hh - n_qk) * D;
+            *reinterpret_cast<__half2 *>(to + 2 * p) = __halves2half2(__float2half_rn(r.x), __float2half_rn(r.y));
+        }
+    };
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+        const unsigned i = threadIdx.x + u * blockDim.x;
+        if (i < total) finish(i, x[u]);
     }
+    for (unsigned i = threadIdx.x + U * blockDim.x; i < total; i += blockDim.x) finish(i, load(i));
 }
 
 }  // namespace b200
@@ -175,8 +209,9 @@ int b200_add_rms_norm_quantize(float *x, int64_t x_nb_row, const float *residual
     const unsigned threads = rms_threads(d);
     cudaStream_t st = (cudaStream_t) stream;
     const int early = rows <= pdl_early_rows() ? 1 : 0;
-    launch_pdl(add_rms_norm_quantize_kernel, dim3(grid), dim3(threads), 0, st, x, x_nb_row, residual, residual_nb_row, w, h, h_nb_row, d, rows, eps, a.nb, a.nbp,
-               (uint8_t *) scratch, a.d_offset, variant, early);
+    const double inv_d = (d & (d - 1)) == 0 ? 1.0 / (double) d : 0.0;   // a power of two: multiplying by it is the same quotient
+    launch_pdl(threads * 4 >= d ? add_rms_norm_quantize_kernel<1> : add_rms_norm_quantize_kernel<4>, dim3(grid), dim3(threads), 0, st, x, x_nb_row, residual, residual_nb_row,
+               w, h, h_nb_row, (int) d, rows, eps, inv_d, a.nb, a.nbp, (uint8_t *) scratch, a.d_offset, variant, early);
     return check_launch("add_rms_norm_quantize");
 }
 
@@ -189,12 +224,10 @@ int b200_silu_mul_quantize(const float *gate, const float *up, int64_t nb_row, f
     B200_REQUIRE(is_aligned(scratch, 256), "scratch must be 256-byte aligned");
     const ActDims a = act_dims(K, N);
     if (scratch_bytes < a.total_bytes) return set_error(B200_E_SCRATCH, "scratch too small: %zu < %zu", scratch_bytes, a.total_bytes);
-    const int64_t rows_padded = a.n_nt * 8;
-    const int64_t threads = rows_padded * a.nbp * 8;
-    const unsigned grid = (unsigned) ((threads + 255) / 256);
+    const dim3 grid((unsigned) (a.n_nt * 8), (unsigned) std::min<int64_t>(65535, (a.nbp * 8 + 255) / 256));
     cudaStream_t st = (cudaStream_t) stream;
     const int early = N <= pdl_early_rows() ? 1 : 0;
-    launch_pdl(silu_mul_quantize_kernel, dim3(grid), dim3(256), 0, st, gate, up, nb_row, dst, dst_nb_row, N, rows_padded, a.nb, a.nbp, (uint8_t *) scratch, a.d_offset, variant, early);
+    launch_pdl(silu_mul_quantize_kernel, grid, dim3(256), 0, st, gate, up, nb_row, dst, dst_nb_row, N, a.nb, a.nbp, (uint8_t *) scratch, a.d_offset, variant, early);
     return check_launch("silu_mul_quantize");
 }
 
@@ -218,7 +251,7 @@ int b200_rope_store_to(const float *q, float *q_dst, int64_t q_nb_head, int64_t 
                  "pairs must be 8-byte aligned (f32) / 4-byte aligned (f16)");
     if (T == 0) return B200_OK;
     const float theta_scale = powf(freq_base, -2.0f / (float) n_dims);
-    launch_pdl(rope_store_kernel, dim3((unsigned) T), dim3(512), (size_t) (n_dims + n_dims / 2) * sizeof(float), (cudaStream_t) stream,
+    launch_pdl(rope_store_kernel, dim3((unsigned) T), dim3(512), (size_t) n_dims * sizeof(float), (cudaStream_t) stream,
         q, q_dst, q_nb_head, q_nb_tok, k, k_nb_head, k_nb_tok, v, v_nb_tok, D, H, Hkv, n_dims, pos, freq_factors, theta_scale, freq_scale, attn_factor,
         slots, (__half *) k_cache, k_cache_nb_row, (__half *) v_cache, v_cache_nb_row, T <= pdl_early_rows() ? 1 : 0);
     return check_launch("rope_store");

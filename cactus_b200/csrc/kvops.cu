@@ -25,6 +25,38 @@ __global__ void __launch_bounds__(256) kq_mask_kernel(const int32_t *__restrict_
     reinterpret_cast<unsigned short *>(reinterpret_cast<char *>(mask) + j * mask_nb_row)[i] = v;
 }
 
+// The same for 8 cells per thread and MASK_ROWS rows per CTA, where 8 cells are 16 aligned bytes: the cells' positions and
+// sequences are loaded once and the stores are 16 bytes wide (512 x 65536: 77.6 us with the kernel above, KQ_NEW with this one).
+constexpr int MASK_ROWS = 16;
+__global__ void __launch_bounds__(256) kq_mask8_kernel(const int32_t *__restrict__ cell_pos, const int32_t *__restrict__ cell_seq,
+                                                      int64_t n_kv, const int32_t *__restrict__ tok_pos,
+                                                      const int32_t *__restrict__ tok_seq, int64_t n_tokens, int64_t n_rows,
+                                                      __half *__restrict__ mask, int64_t mask_nb_row) {
+    pdl_prologue();
+    const int64_t i = ((int64_t) blockIdx.x * blockDim.x + threadIdx.x) * 8;
+    if (i >= n_kv) return;
+    int32_t cs[8], cp[8];
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        const int4 s = *reinterpret_cast<const int4 *>(cell_seq + i + 4 * h), p = *reinterpret_cast<const int4 *>(cell_pos + i + 4 * h);
+        cs[4 * h] = s.x; cs[4 * h + 1] = s.y; cs[4 * h + 2] = s.z; cs[4 * h + 3] = s.w;
+        cp[4 * h] = p.x; cp[4 * h + 1] = p.y; cp[4 * h + 2] = p.z; cp[4 * h + 3] = p.w;
+    }
+    const int64_t j0 = (int64_t) blockIdx.y * MASK_ROWS, j1 = min(n_rows, j0 + MASK_ROWS);
+#pragma unroll 4
+    for (int64_t j = j0; j < j1; ++j) {
+        const bool row = j < n_tokens;
+        const int32_t ts = row ? tok_seq[j] : -1, tp = row ? tok_pos[j] : 0;
+        uint32_t v[4];
+#pragma unroll
+        for (int x = 0; x < 4; ++x) {
+            const bool a = row && cs[2 * x] >= 0 && cs[2 * x] == ts && cp[2 * x] <= tp, b = row && cs[2 * x + 1] >= 0 && cs[2 * x + 1] == ts && cp[2 * x + 1] <= tp;
+            v[x] = (a ? 0u : 0xFC00u) | (b ? 0u : 0xFC000000u);
+        }
+        *reinterpret_cast<uint4 *>(reinterpret_cast<char *>(mask) + j * mask_nb_row + i * 2) = make_uint4(v[0], v[1], v[2], v[3]);
+    }
+}
+
 __global__ void __launch_bounds__(256) scatter_i32_kernel(int32_t *__restrict__ dst, const int32_t *__restrict__ idx,
                                                          const int32_t *__restrict__ src, int64_t n) {
     const int64_t i = (int64_t) blockIdx.x * blockDim.x + threadIdx.x;
@@ -108,6 +140,11 @@ int b200_kq_mask_build(const int32_t *cell_pos, const int32_t *cell_seq, int64_t
     B200_REQUIRE(cell_pos && cell_seq && tok_pos && tok_seq && mask && n_kv > 0 && n_tokens > 0, "bad kq_mask arguments");
     B200_REQUIRE(mask_nb_row % 2 == 0 && mask_nb_row >= n_kv * 2, "bad mask row stride");
     const int64_t n_rows = (n_tokens + 63) / 64 * 64;
+    if (n_kv % 8 == 0 && mask_nb_row % 16 == 0 && is_aligned(mask, 16) && is_aligned(cell_pos, 16) && is_aligned(cell_seq, 16)) {
+        launch_pdl(kq_mask8_kernel, dim3((unsigned) ((n_kv / 8 + 255) / 256), (unsigned) ((n_rows + MASK_ROWS - 1) / MASK_ROWS)), dim3(256), 0, (cudaStream_t) stream,
+                   cell_pos, cell_seq, n_kv, tok_pos, tok_seq, n_tokens, n_rows, (__half *) mask, mask_nb_row);
+        return check_launch("kq_mask");
+    }
     dim3 grid((unsigned) ((n_kv + 255) / 256), (unsigned) n_rows);
     kq_mask_kernel<<<grid, 256, 0, (cudaStream_t) stream>>>(cell_pos, cell_seq, n_kv, tok_pos, tok_seq, n_tokens, n_rows,
                                                             (__half *) mask, mask_nb_row);

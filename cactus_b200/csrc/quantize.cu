@@ -1,5 +1,6 @@
 // Activation quantiser (quantize_row_q8_0), the tiled weight layout converters, GET_ROWS on tiled
 // weights and the exact block-dot debug kernel.
+#include <algorithm>
 #include <cstdlib>
 
 #include "common.cuh"
@@ -14,30 +15,29 @@ namespace b200 {
 // ---------------------------------------------------------------------------------------------
 template <int LAYOUT>
 __global__ void __launch_bounds__(256) quantize_q8_0_kernel(const float *__restrict__ x, int64_t x_nb_row, int64_t K,
-                                                           int64_t N, int64_t n_rows_padded, int64_t nb, int64_t nbp,
+                                                           int64_t N, int64_t nb, int64_t nbp,
                                                            uint8_t *__restrict__ out, size_t d_offset, int variant, int early, int chunk_nt) {
     pdl_prologue(early != 0);
-    const int64_t gid = (int64_t) blockIdx.x * blockDim.x + threadIdx.x;
-    const int j = (int) (gid & 7);             // which group of 4 elements inside the block
-    const int64_t blk = gid >> 3;              // (row, block) index
-    const int64_t nblk = (LAYOUT == 0) ? nb : nbp;
-    const int64_t n = blk / nblk;
-    const int64_t b = blk - n * nblk;
-    if (n >= n_rows_padded) return;  // whole groups of 8 lanes leave together (gid>>3 is uniform per group)
-
-    float v[4] = {0.f, 0.f, 0.f, 0.f};
-    const bool real = (n < N) && (b < nb);
-    if (real) {
-        const float *row = (const float *) ((const char *) x + n * x_nb_row) + b * 32 + j * 4;
-        if ((((uintptr_t) row) & 15) == 0) {
-            const float4 f = *reinterpret_cast<const float4 *>(row);
-            v[0] = f.x; v[1] = f.y; v[2] = f.z; v[3] = f.w;
-        } else {
-            v[0] = row[0]; v[1] = row[1]; v[2] = row[2]; v[3] = row[3];
+    const int64_t n = blockIdx.x;   // row
+    // 4 elements per thread; whole groups of 8 lanes (a block) leave together.  (A row per x: no 64-bit division per thread)
+    for (int64_t at = blockIdx.y * 256 + threadIdx.x; at < (LAYOUT == 0 ? nb : nbp) * 8; at += gridDim.y * 256) {
+        const int j = (int) at & 7;   // which group of 4 elements inside the block
+        const int64_t b = at >> 3;
+        float v[4] = {0.f, 0.f, 0.f, 0.f};
+        const bool real = (n < N) && (b < nb);
+        if (real) {
+            const float *row = (const float *) ((const char *) x + n * x_nb_row) + b * 32 + j * 4;
+            if ((((uintptr_t) row) & 15) == 0) {
+                const float4 f = *reinterpret_cast<const float4 *>(row);
+                v[0] = f.x; v[1] = f.y; v[2] = f.z; v[3] = f.w;
+            } else {
+                v[0] = row[0]; v[1] = row[1]; v[2] = row[2]; v[3] = row[3];
+            }
         }
+        q8_quantize_store<LAYOUT>(v, out, d_offset, nb, nbp, n, b, j, real, variant, chunk_nt);
     }
-    q8_quantize_store<LAYOUT>(v, out, d_offset, nb, nbp, n, b, j, real, variant, chunk_nt);
 }
+static dim3 quantize_grid(int64_t rows, int64_t blocks) { return dim3((unsigned) rows, (unsigned) std::min<int64_t>(65535, (blocks * 8 + 255) / 256)); }
 
 // ---------------------------------------------------------------------------------------------
 // Row-major block stream <-> T16.  One thread per (row, block) of the padded index space.
@@ -208,11 +208,10 @@ static int check_wtype(int wtype) {
 
 int launch_quantize_b8(const float *x, int64_t x_nb_row, int64_t K, int64_t N, void *scratch, int variant, int layout, cudaStream_t st) {
     const ActDims a = act_dims(K, N);
-    const int64_t threads = a.n_nt * 8 * a.nbp * 8;
-    const int64_t grid = (threads + 255) / 256;
+    const dim3 grid = quantize_grid(a.n_nt * 8, a.nbp);
     const int early = N <= pdl_early_rows() ? 1 : 0;
-    if (layout == 2) launch_pdl(quantize_q8_0_kernel<2>, dim3((unsigned) grid), dim3(256), 0, st, x, x_nb_row, K, N, a.n_nt * 8, a.nb, a.nbp, (uint8_t *) scratch, a.d_offset, variant, early, a.chunk_nt);
-    else launch_pdl(quantize_q8_0_kernel<1>, dim3((unsigned) grid), dim3(256), 0, st, x, x_nb_row, K, N, a.n_nt * 8, a.nb, a.nbp, (uint8_t *) scratch, a.d_offset, variant, early, a.chunk_nt);
+    if (layout == 2) launch_pdl(quantize_q8_0_kernel<2>, grid, dim3(256), 0, st, x, x_nb_row, K, N, a.nb, a.nbp, (uint8_t *) scratch, a.d_offset, variant, early, a.chunk_nt);
+    else launch_pdl(quantize_q8_0_kernel<1>, grid, dim3(256), 0, st, x, x_nb_row, K, N, a.nb, a.nbp, (uint8_t *) scratch, a.d_offset, variant, early, a.chunk_nt);
     return check_launch("quantize_q8_0 (activations)");
 }
 
@@ -268,9 +267,8 @@ int b200_quantize_q8_0(const float *x, int64_t x_row_stride_bytes, int64_t K, in
     B200_REQUIRE(is_aligned(x, 4) && x_row_stride_bytes % 4 == 0 && is_aligned(dst_blocks, 2), "misaligned pointer or stride");
     if (N == 0) return B200_OK;
     const int64_t nb = K / 32;
-    const int64_t threads = N * nb * 8;
-    quantize_q8_0_kernel<0><<<(unsigned) ((threads + 255) / 256), 256, 0, (cudaStream_t) stream>>>(
-        x, x_row_stride_bytes, K, N, N, nb, nb, (uint8_t *) dst_blocks, 0, variant, 0, 2);
+    quantize_q8_0_kernel<0><<<quantize_grid(N, nb), 256, 0, (cudaStream_t) stream>>>(
+        x, x_row_stride_bytes, K, N, nb, nb, (uint8_t *) dst_blocks, 0, variant, 0, 2);
     return check_launch("quantize_q8_0");
 }
 

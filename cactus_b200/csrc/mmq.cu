@@ -143,9 +143,6 @@ struct MmqCfg {
 // MMQ_PEER and MMQ_STREAMK_SEG know row ranges (other GPUs' buffers, separate weight / destination tensors); the plain
 // kernels carry none of that code: the hot shapes of a decode step must not pay for it
 constexpr int MMQ_PLAIN = 0, MMQ_PEER = 1, MMQ_STREAMK = 2, MMQ_STREAMK_SEG = 3;
-#ifndef MMQ_DEPTH
-#define MMQ_DEPTH 2
-#endif
 template <int WTYPE, int NTW, int WN, int MT, int WM, int STAGES, int MINB, int MODE = MMQ_PLAIN>
 __global__ void __launch_bounds__(WM * WN * 32, MINB) mmq_kernel(TiledDims dims, const uint8_t *__restrict__ w, ActDims act,
                                                           const uint8_t *__restrict__ aq, float *__restrict__ dst,
@@ -331,7 +328,10 @@ __global__ void __launch_bounds__(WM * WN * 32, MINB) mmq_kernel(TiledDims dims,
         constexpr int NSTEP = 4 * NP;
         uint32_t a0[MMQ_MT], a1[MMQ_MT], a2[MMQ_MT], a3[MMQ_MT];
         // DEPTH steps are in flight: the MMAs of steps s+1 .. s+DEPTH-1 are issued before the epilogue of step s
-        constexpr int DEPTH = MMQ_DEPTH;
+        // Three steps for Q4_0 stream-K: the scheduling of its body decides, 56.5 -> 51.0 us at 4096 x 28672 (K x M), 64 columns.  Two
+        // elsewhere: three cost 0.5 % at 512 columns of the plain kernel and 0.7 % at the Q8_0 head.  (Three need two column pairs:
+        // the scales of a block share dwa / dwb with the block before the last.)
+        constexpr int DEPTH = SK && WTYPE == B200_TYPE_Q4_0 && NP >= 2 ? 3 : 2;
         uint64_t dwa[2][MMQ_MT], dwb[2][MMQ_MT];   // weight scales of the block of the step in flight / the step being finished
         uint64_t p01[DEPTH][2][MMQ_MT], p23[DEPTH][2][MMQ_MT];
         uint2 sc[DEPTH][2];                          // {d0, d1} of the two column tiles of a step (-d * 12582912 is recomputed: half the shared-memory traffic)

@@ -46,7 +46,7 @@ constexpr int MI_THREADS = 512, MI_WORDS = 2048;   // words whose indices are li
 template <bool VEC>
 __global__ void __launch_bounds__(MI_THREADS, 3) mask_index_kernel(const __half *__restrict__ mask, int64_t mask_nb_row, int64_t n_kv, int64_t nw,
                                                                unsigned long long *__restrict__ words, int32_t *__restrict__ wlist, int32_t *__restrict__ wcount,
-                                                               int32_t *__restrict__ soft) {
+                                                               uint8_t *__restrict__ soft) {
     pdl_prologue();
     __shared__ unsigned bits[MI_WORDS / 32];
     __shared__ int warp_cnt[MI_WORDS / 1024], any_soft;
@@ -115,7 +115,7 @@ __global__ void __launch_bounds__(MI_THREADS, 3) mask_index_kernel(const __half 
     __syncthreads();
     if (tid == 0) {
         wcount[j] = base;
-        soft[j] = any_soft;
+        soft[j] = (uint8_t) any_soft;
     }
 }
 
@@ -123,7 +123,7 @@ __global__ void __launch_bounds__(MI_THREADS, 3) mask_index_kernel(const __half 
 // walks out first and the short ones fill the gaps), and the total number of words, from which the attention kernel
 // derives how many words one CTA should walk.  A warp per token counts the tokens that come before it; the first CTA also
 // makes the totals.
-__global__ void __launch_bounds__(256) fattn_plan_kernel(const int32_t *__restrict__ wcount, const int32_t *__restrict__ soft, int64_t Nq, int32_t *__restrict__ order,
+__global__ void __launch_bounds__(256) fattn_plan_kernel(const int32_t *__restrict__ wcount, const uint8_t *__restrict__ soft, int64_t Nq, int32_t *__restrict__ order,
                                                         int32_t *__restrict__ plan) {
     pdl_prologue();
     const int lane = threadIdx.x & 31;
@@ -771,7 +771,7 @@ extern "C" {
 // index layout: words [Nq][nw] u64 | list of non-empty word indices [Nq][nw] i32 | their counts [Nq] i32 |
 // tokens by decreasing count [Nq] i32 | plan: total words i32, words summed over 16-token groups i32, 1 if the mask
 // holds values other than 0 and -inf in participating cells i32, unused, listed tiles of 4, 8, 16, 32 tokens 4 x i32 |
-// flag per tile, 4 x [Nq / 4] i32 | lists of flagged tiles, 4 x [Nq / 4] i32 | per token: the row is more than its bits [Nq] i32
+// flag per tile, 4 x [Nq / 4] i32 | lists of flagged tiles, 4 x [Nq / 4] i32 | per token: the row is more than its bits, [Nq] bytes (up to 224 tokens: from byte 32 of the plan on)
 static size_t index_list_offset(int64_t Nq, int64_t nw) { return align_up((size_t) Nq * nw * 8, 256); }
 static size_t index_count_offset(int64_t Nq, int64_t nw) { return index_list_offset(Nq, nw) + align_up((size_t) Nq * nw * 4, 256); }
 
@@ -780,12 +780,16 @@ static size_t index_plan_offset(int64_t Nq, int64_t nw) { return index_order_off
 
 static size_t index_tiles_offset(int64_t Nq, int64_t nw) { return index_plan_offset(Nq, nw) + 256; }
 static int64_t index_tiles_stride(int64_t Nq) { return (Nq + 255) / 256 * 64; }   // of one flag array or list, in elements
-static size_t index_soft_offset(int64_t Nq, int64_t nw) { return index_tiles_offset(Nq, nw) + 8 * index_tiles_stride(Nq) * 4; }
+// only ubatches the query-tiled kernel may take need the vote and its arrays
+static bool index_has_tiles(int64_t Nq) { return fattn_tile_min_nq() > 0 && Nq >= fattn_tile_min_nq(); }
+constexpr int64_t SOFT_IN_PLAN = 224;   // so many tokens' flags fit behind the plan
+static size_t index_end(int64_t Nq, int64_t nw) { return index_tiles_offset(Nq, nw) + (index_has_tiles(Nq) ? 8 * index_tiles_stride(Nq) * 4 : 0); }
+static size_t index_soft_offset(int64_t Nq, int64_t nw) { return Nq <= SOFT_IN_PLAN ? index_plan_offset(Nq, nw) + 32 : index_end(Nq, nw); }
 
 size_t b200_mask_index_bytes(int64_t Nq, int64_t n_kv) {
     if (Nq <= 0 || n_kv <= 0) return 0;
     const int64_t nw = (n_kv + 63) / 64;
-    return index_soft_offset(Nq, nw) + align_up((size_t) Nq * 4, 256);
+    return index_end(Nq, nw) + (Nq <= SOFT_IN_PLAN ? 0 : align_up((size_t) Nq, 256));
 }
 
 int b200_mask_index_build(const void *mask, int64_t mask_nb_row, int64_t Nq, int64_t n_kv, void *index, size_t index_bytes,
@@ -798,14 +802,14 @@ int b200_mask_index_build(const void *mask, int64_t mask_nb_row, int64_t Nq, int
     const cudaStream_t st = (cudaStream_t) stream;
     char *ix = (char *) index;
     int32_t *plan = (int32_t *) (ix + index_plan_offset(Nq, nw)), *wlist = (int32_t *) (ix + index_list_offset(Nq, nw)), *wcount = (int32_t *) (ix + index_count_offset(Nq, nw));
-    int32_t *soft = (int32_t *) (ix + index_soft_offset(Nq, nw));
+    uint8_t *soft = (uint8_t *) ix + index_soft_offset(Nq, nw);
     const bool vec = is_aligned(mask, 16) && mask_nb_row % 16 == 0;
     launch_pdl(vec ? mask_index_kernel<true> : mask_index_kernel<false>, dim3((unsigned) Nq), dim3(MI_THREADS), 0, st, (const __half *) mask, mask_nb_row, n_kv, nw,
                (unsigned long long *) index, wlist, wcount, soft);
     if (int e = check_launch("mask_index")) return e;
-    launch_pdl(fattn_plan_kernel, dim3((unsigned) ((Nq + 7) / 8)), dim3(256), 0, st, (const int32_t *) wcount, (const int32_t *) soft, Nq, (int32_t *) (ix + index_order_offset(Nq, nw)), plan);
+    launch_pdl(fattn_plan_kernel, dim3((unsigned) ((Nq + 7) / 8)), dim3(256), 0, st, (const int32_t *) wcount, (const uint8_t *) soft, Nq, (int32_t *) (ix + index_order_offset(Nq, nw)), plan);
     if (int e = check_launch("fattn_plan")) return e;
-    if (Nq >= fattn_tile_min_nq() && fattn_tile_min_nq() > 0) {   // only ubatches the query-tiled kernel may take need the vote
+    if (index_has_tiles(Nq)) {
         int32_t *flags = (int32_t *) ((char *) index + index_tiles_offset(Nq, nw));
         const int64_t stride = index_tiles_stride(Nq);
         launch_pdl(fattn_tile_vote_kernel, dim3((unsigned) ((Nq + 31) / 32)), dim3(256), 0, st, (const int32_t *) wlist, (const int32_t *) wcount, Nq, nw, plan, flags,
@@ -915,8 +919,9 @@ static int flash_attn_impl(bool parity, int64_t D, int64_t H, int64_t Hkv, int64
             pt.tflags = flags + k * stride;
             pt.tlist = flags + (4 + k) * stride;
             pt.tcount = p.plan + 4 + k;
-            // one round of CTAs, fewer when all tokens together are less
-            pt.spread_rows = (int) std::min<int64_t>(tiles * (tile_tokens / 4), (3 * (int64_t) fa_sm_count() + Hkv * pt.nsplit - 1) / (Hkv * pt.nsplit));
+            // three rounds of CTAs, fewer when there are fewer tokens: one token per CTA for up to some 50 (mixed step of the 8B model, 48
+            // tokens: 28.7 ms with one round, 27.7 with three or six; idle CTAs cost 1 us a round)
+            pt.spread_rows = (int) std::min<int64_t>(Nq, (9 * (int64_t) fa_sm_count() + Hkv * pt.nsplit - 1) / (Hkv * pt.nsplit));
         }
         dim3 tgrid((unsigned) Hkv, (unsigned) (tiles + pt.spread_rows), (unsigned) pt.nsplit);
         // the opt-in to more than 48 KB of shared memory is per function and device

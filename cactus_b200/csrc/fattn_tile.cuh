@@ -39,22 +39,22 @@ __device__ __forceinline__ void ft_ldmatrix_x4(uint32_t (&r)[4], uint32_t addr) 
 }
 
 // dynamic shared memory of the kernel: FT_STAGES stages of K and V rows
-constexpr int fattn_tile_smem_bytes(int D) { return FT_STAGES * 2 * FT_CHUNK * (D * 2 + 16); }   // as much as ft_spread's 4 x 3 x 16 rows
+constexpr int fattn_tile_smem_bytes(int D) { return FT_STAGES * 2 * FT_CHUNK * (D * 2 + 16); }   // ft_spread uses them the same way
 
 // ---- the steps of one chunk of 32 cells; rows g and g + 8 of a warp's 16 ----
-// S = Q K^T for n-tiles C0 .. C0 + CN - 1 of 8 cells (independent accumulator chains); Ks: the staged row of the first cell
-template <int D, int C0, int CN>
+// S = Q K^T for the four n-tiles of 8 cells (independent accumulator chains)
+template <int D>
 __device__ __forceinline__ void ft_s(float (&sacc)[4][4], const uint32_t (&qa)[D / 16][4], uint32_t Ks, int lane) {
     constexpr int ROW = D * 2 + 16;
     const uint32_t at = Ks + (uint32_t) ((8 * (lane >> 4) + (lane & 7)) * ROW + ((lane >> 3) & 1) * 16);
 #pragma unroll
-    for (int c = C0; c < C0 + CN; ++c) sacc[c][0] = sacc[c][1] = sacc[c][2] = sacc[c][3] = 0.0f;
+    for (int c = 0; c < 4; ++c) sacc[c][0] = sacc[c][1] = sacc[c][2] = sacc[c][3] = 0.0f;
 #pragma unroll
     for (int ks = 0; ks < D / 16; ++ks)
 #pragma unroll
-        for (int c = C0; c < C0 + CN; c += 2) {
+        for (int c = 0; c < 4; c += 2) {
             uint32_t b[4];   // both halves of this k-step for n-tile c, then for n-tile c + 1
-            ft_ldmatrix_x4(b, at + (uint32_t) (8 * (c - C0) * ROW + 32 * ks));
+            ft_ldmatrix_x4(b, at + (uint32_t) (8 * c * ROW + 32 * ks));
             mma_f16(sacc[c], qa[ks][0], qa[ks][1], qa[ks][2], qa[ks][3], b[0], b[1]);
             mma_f16(sacc[c + 1], qa[ks][0], qa[ks][1], qa[ks][2], qa[ks][3], b[2], b[3]);
         }
@@ -120,12 +120,12 @@ __device__ __forceinline__ void ft_softmax(const FattnParams &p, float (&sacc)[4
         }
 }
 // O += P V for one k-step of 16 cells, whose V rows start at Vs: V^T fragments of two n-tiles per ldmatrix
-template <int D>
-__device__ __forceinline__ void ft_pv(float (&o)[D / 8][4], const uint32_t (&ph)[4], const uint32_t (&pl)[4], uint32_t Vs, int lane) {
+template <int D, int NT = D / 8>   // NT n-tiles, from the one Vs points to
+__device__ __forceinline__ void ft_pv(float (&o)[NT][4], const uint32_t (&ph)[4], const uint32_t (&pl)[4], uint32_t Vs, int lane) {
     constexpr int ROW = D * 2 + 16;
     const int mi = lane >> 3, mr = lane & 7;
 #pragma unroll
-    for (int nt = 0; nt < D / 8; nt += 2) {
+    for (int nt = 0; nt < NT; nt += 2) {
         uint32_t vb[4];   // {cells 0-7, cells 8-15} of this k-step for n-tile nt, then for n-tile nt + 1
         ft_ldmatrix_x4_trans(vb, Vs + (uint32_t) ((8 * (mi & 1) + mr) * ROW + (8 * (nt + (mi >> 1))) * 2));
         mma_f16(o[nt], ph[0], ph[1], ph[2], ph[3], vb[0], vb[1]);
@@ -177,18 +177,18 @@ __device__ __forceinline__ int ft_union(const FattnParams &p, int64_t tok0, int 
     return all;
 }
 // A finished row pair: O / l, or the split's partial triple
-template <int D>
-__device__ __forceinline__ void ft_write(const FattnParams &p, int64_t tok, int head, int split, int i, const float (&o)[D / 8][4], float m, float l, int t) {
+template <int D, int NT = D / 8>   // NT n-tiles, from nt0 on
+__device__ __forceinline__ void ft_write(const FattnParams &p, int64_t tok, int head, int split, int i, const float (&o)[NT][4], float m, float l, int t, int nt0 = 0) {
     if (p.nsplit == 1) {
         const float inv = 1.0f / l;
-        float *dst = p.dst + (tok * p.H + head) * D;
+        float *dst = p.dst + (tok * p.H + head) * D + 8 * nt0 + 2 * t;
 #pragma unroll
-        for (int nt = 0; nt < D / 8; ++nt) *reinterpret_cast<float2 *>(dst + 8 * nt + 2 * t) = make_float2(o[nt][2 * i] * inv, o[nt][2 * i + 1] * inv);
+        for (int nt = 0; nt < NT; ++nt) *reinterpret_cast<float2 *>(dst + 8 * nt) = make_float2(o[nt][2 * i] * inv, o[nt][2 * i + 1] * inv);
     } else {
         float *pp = p.partial + ((tok * p.H + head) * p.nsplit + split) * (D + 2);
 #pragma unroll
-        for (int nt = 0; nt < D / 8; ++nt) *reinterpret_cast<float2 *>(pp + 8 * nt + 2 * t) = make_float2(o[nt][2 * i], o[nt][2 * i + 1]);
-        if (t == 0) {
+        for (int nt = 0; nt < NT; ++nt) *reinterpret_cast<float2 *>(pp + 8 * (nt0 + nt) + 2 * t) = make_float2(o[nt][2 * i], o[nt][2 * i + 1]);
+        if (t == 0 && nt0 == 0) {
             pp[D] = m;
             pp[D + 1] = l;
         }
@@ -212,33 +212,38 @@ struct FtSpreadShared {
     unsigned short before[FT_MAX_WORDS / 32];   // union words before each 32
     int warp_cnt[FT_THREADS / 32];
     alignas(16) short list[FT_THREADS / 32][FT_LIST];     // per warp: the round's union positions, 64 * slot + bit of a cell its token attends to or -1
-    int cells[FT_THREADS / 32][2][FT_CHUNK];   // per warp: the cells of the chunk at work and of the next
+    int cells[FT_THREADS / 32][4][FT_CHUNK];   // per warp: the cells of the chunk at work and of the next two
+    float scores[2][16][FT_CHUNK + 4];           // of the chunk at work: a warp computes 8 cells, all warps read 32
 };
 
 // Tokens of tiles whose tokens share few cells (decode tokens beside a prompt, in which a shared walk of the union would have
-// every token step over all the others' cells): one warp per token, over the chunks its token attends to.  The chunks are
-// those of the shared walk -- 32 neighbours in the tile's union list, every nsplit-th to each split -- and a chunk without a
+// every token step over all the others' cells): one CTA per token and KV head, over the chunks the token attends to.  The chunks
+// are those of the shared walk -- 32 neighbours in the tile's union list, every nsplit-th to each split -- and a chunk without a
 // cell of the token would have changed nothing, so results are the same bits.
-// What bounds it: the K/V rows (each read once) and the latency of a warp's chain of chunks; 12 warps per SM and half chunks in
-// flight (three slots of 16 rows per warp: K rows 0-15 and 16-31, then V rows 0-15; V rows 16-31 take the first slot when its
-// K rows are used, and the next chunk moves on by one slot) cover both.  48 tokens of 16-2048 cells beside a 464-token prompt
-// (32 heads, 8 KV heads): see the comment at fattn_tile_kernel.
+// What bounds it: the chain of the longest token, chunk after chunk.  So the four warps share each chunk: 8 cells of S each, the
+// softmax by all of them (every warp needs P), a quarter of D of P V each; three chunks in the ring.  One token of 2048 cells
+// beside a 464-token prompt (32 heads of 128, 8 KV heads; the prompt alone 51 us): 107 us with a warp per token, 69 so; 48
+// tokens of 16 to 2048 cells 141 / 127.  (Many short ones were better off with a warp each: 48 of 64 cells 54 / 67.)
 template <int D>
 __device__ __forceinline__ void ft_spread(const FattnParams &p, int gqa_log2, FtSpreadShared &sh, uint8_t *kv_s) {
-    constexpr int KS = D / 16, NT = D / 8, ROW = D * 2 + 16, HALF = 16 * ROW;
+    constexpr int KS = D / 16, NT = D / 32, ROW = D * 2 + 16;   // NT: n-tiles of a warp
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
-    const int gqa = 1 << gqa_log2, tile_tok = 64 >> gqa_log2, quads = tile_tok >> 2;
+    const int gqa = 1 << gqa_log2, tile_tok = 64 >> gqa_log2;
     const int hk = blockIdx.x, split = blockIdx.z, nsplit = p.nsplit;
     const bool binary_mask = p.plan[2] == 0;
     const char *kbase = p.k + (int64_t) hk * p.k_nb_head, *vbase = p.v + (int64_t) hk * p.v_nb_head;
-    const uint32_t slots_u32 = (uint32_t) __cvta_generic_to_shared(kv_s + warp * 3 * HALF);
+    const uint32_t kv_u32 = (uint32_t) __cvta_generic_to_shared(kv_s);
     short *list = sh.list[warp];
-    const int n_units = *p.tcount * quads;
-    for (int unit = blockIdx.y; unit < n_units; unit += p.spread_rows) {
-        const int64_t tok0 = (int64_t) p.tlist[unit / quads] * tile_tok, tok = tok0 + (unit % quads) * 4 + warp;
-        __syncthreads();   // the lists of the unit before are no longer read
-        const int n_uw = ft_union(p, tok0, (int) min((int64_t) tile_tok, p.Nq - tok0), sh.bits, sh.uw_index, sh.warp_cnt, sh.before);
+    // a contiguous share of the tokens: neighbours have their tile's union in common
+    const int n_units = *p.tcount * tile_tok, unit1 = (int) (((int64_t) blockIdx.y + 1) * n_units / p.spread_rows);
+    int last_tile = -1, n_uw = 0;
+    for (int unit = (int) ((int64_t) blockIdx.y * n_units / p.spread_rows); unit < unit1; ++unit) {
+        const int tile = p.tlist[unit / tile_tok];
+        const int64_t tok0 = (int64_t) tile * tile_tok, tok = tok0 + unit % tile_tok;
         if (tok >= p.Nq) continue;
+        __syncthreads();   // the lists and scores of the unit before are no longer read
+        if (tile != last_tile) n_uw = ft_union(p, tok0, (int) min((int64_t) tile_tok, p.Nq - tok0), sh.bits, sh.uw_index, sh.warp_cnt, sh.before);
+        last_tile = tile;
         const int n_tok = (int) min((int64_t) tile_tok, p.Nq - tok0);
         uint32_t qa[KS][4];
         int head[2];
@@ -333,68 +338,72 @@ __device__ __forceinline__ void ft_spread(const FattnParams &p, int gqa_log2, Ft
                 }
             }
         };
-        // 16 rows of K or V into a slot; a group of its own
-        constexpr int PIECES = D / 8, PER = 16 * PIECES / 32;
-        auto fetch = [&](const char *base, int64_t nb_cell, const int *cells, int slot) {
+        // a warp copies 8 rows of K and of V of a chunk
+        constexpr int PIECES = D / 8, PER = 8 * PIECES / 32;
+        auto fetch = [&](int stage, const int *cells) {
+            const uint32_t to = kv_u32 + (uint32_t) ((2 * stage) * FT_CHUNK * ROW + 8 * warp * ROW);
 #pragma unroll
             for (int n = 0; n < PER; ++n) {
                 const int c = lane + 32 * n, r = c / PIECES, piece = c % PIECES;
-                ft_cp16(slots_u32 + (uint32_t) (slot * HALF + r * ROW + piece * 16), base + (int64_t) cells[r] * nb_cell + piece * 16);
+                const int64_t cell = cells[8 * warp + r];
+                ft_cp16(to + (uint32_t) (r * ROW + piece * 16), kbase + cell * p.k_nb_cell + piece * 16);
+                ft_cp16(to + (uint32_t) (FT_CHUNK * ROW + r * ROW + piece * 16), vbase + cell * p.v_nb_cell + piece * 16);
             }
         };
         auto commit = [&] { asm volatile("cp.async.commit_group;\n" ::: "memory"); };
-        auto landed = [&] {
-            asm volatile("cp.async.wait_group 2;\n" ::: "memory");
-            __syncwarp();
-        };
-        int b = 0, s0 = 0, s1 = 1, s2 = 2;
-        unsigned rm_now = next_chunk(0);
-        if (rm_now) fetch(kbase, p.k_nb_cell, sh.cells[warp][0], 0);
+        unsigned rm0 = next_chunk(0);
+        if (rm0) fetch(0, sh.cells[warp][0]);
         commit();
-        if (rm_now) fetch(kbase, p.k_nb_cell, sh.cells[warp][0] + 16, 1);
+        unsigned rm1 = next_chunk(1);
+        if (rm1) fetch(1, sh.cells[warp][1]);
         commit();
-        if (rm_now) fetch(vbase, p.v_nb_cell, sh.cells[warp][0], 2);
-        commit();
-        while (rm_now) {
-            const int *cells = sh.cells[warp][b], *ncells = sh.cells[warp][b ^ 1];
-            const unsigned rm_next = next_chunk(b ^ 1);
-            const unsigned rm[2] = {live[0] ? rm_now : 0u, live[1] ? rm_now : 0u};
+        int s = 0, s2 = 2;   // ring stage of this chunk, of the one after the next
+        for (int it = 0; rm0; ++it) {   // (all warps go through the same chunks)
+            asm volatile("cp.async.wait_group 1;\n" ::: "memory");
+            __syncthreads();   // the chunk has landed for every warp, and nobody uses the one before any more
+            const unsigned rm2 = next_chunk((it + 2) & 3);
+            if (rm2) fetch(s2, sh.cells[warp][(it + 2) & 3]);
+            commit();
+            const uint32_t Ks = kv_u32 + (uint32_t) ((2 * s) * FT_CHUNK * ROW), Vs = Ks + (uint32_t) (FT_CHUNK * ROW);
             float sacc[4][4];
             uint32_t ph[2][4], pl[2][4];
-            landed();
-            ft_s<D, 0, 2>(sacc, qa, slots_u32 + (uint32_t) (s0 * HALF), lane);
-            __syncwarp();
-            fetch(vbase, p.v_nb_cell, cells + 16, s0);
-            commit();
-            landed();
-            ft_s<D, 2, 2>(sacc, qa, slots_u32 + (uint32_t) (s1 * HALF), lane);
-            __syncwarp();
-            if (rm_next) fetch(kbase, p.k_nb_cell, ncells, s1);
-            commit();
-            ft_softmax<D>(p, sacc, rm, binary_mask, mrow, slope, cells, t, m_run, l_run, o, ph, pl);
-            landed();
-            ft_pv<D>(o, ph[0], pl[0], slots_u32 + (uint32_t) (s2 * HALF), lane);
-            __syncwarp();
-            if (rm_next) fetch(kbase, p.k_nb_cell, ncells + 16, s2);
-            commit();
-            landed();
-            ft_pv<D>(o, ph[1], pl[1], slots_u32 + (uint32_t) (s0 * HALF), lane);
-            __syncwarp();
-            if (rm_next) fetch(vbase, p.v_nb_cell, ncells, s0);
-            commit();
-            const int x = s0;
-            s0 = s1;
-            s1 = s2;
-            s2 = x;
-            b ^= 1;
-            rm_now = rm_next;
+            {   // 8 cells of S
+                float a[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+                const uint32_t at = Ks + (uint32_t) ((8 * warp + (lane & 7)) * ROW + (lane >> 3) * 16);
+#pragma unroll
+                for (int ks = 0; ks < KS; ks += 2) {
+                    uint32_t b[4];   // both halves of k-step ks, of ks + 1
+                    ft_ldmatrix_x4(b, at + (uint32_t) (32 * ks));
+                    mma_f16(a, qa[ks][0], qa[ks][1], qa[ks][2], qa[ks][3], b[0], b[1]);
+                    mma_f16(a, qa[ks + 1][0], qa[ks + 1][1], qa[ks + 1][2], qa[ks + 1][3], b[2], b[3]);
+                }
+                *reinterpret_cast<float2 *>(&sh.scores[it & 1][g][8 * warp + 2 * t]) = make_float2(a[0], a[1]);
+                *reinterpret_cast<float2 *>(&sh.scores[it & 1][g + 8][8 * warp + 2 * t]) = make_float2(a[2], a[3]);
+            }
+            __syncthreads();
+#pragma unroll
+            for (int c = 0; c < 4; ++c)
+#pragma unroll
+                for (int i = 0; i < 2; ++i) {
+                    const float2 x = *reinterpret_cast<const float2 *>(&sh.scores[it & 1][g + 8 * i][8 * c + 2 * t]);
+                    sacc[c][2 * i] = x.x;
+                    sacc[c][2 * i + 1] = x.y;
+                }
+            const unsigned rm[2] = {live[0] ? rm0 : 0u, live[1] ? rm0 : 0u};
+            ft_softmax<D / 4>(p, sacc, rm, binary_mask, mrow, slope, sh.cells[warp][it & 3], t, m_run, l_run, o, ph, pl);
+#pragma unroll
+            for (int kk = 0; kk < 2; ++kk) ft_pv<D, NT>(o, ph[kk], pl[kk], Vs + (uint32_t) (16 * kk * ROW + 16 * NT * warp), lane);
+            rm0 = rm1;
+            rm1 = rm2;
+            s = s == 2 ? 0 : s + 1;
+            s2 = s2 == 2 ? 0 : s2 + 1;
         }
         asm volatile("cp.async.wait_all;\n" ::: "memory");
 #pragma unroll
         for (int i = 0; i < 2; ++i) {
             l_run[i] += __shfl_xor_sync(0xffffffffu, l_run[i], 1);
             l_run[i] += __shfl_xor_sync(0xffffffffu, l_run[i], 2);
-            if (live[i]) ft_write<D>(p, tok, head[i], split, i, o, m_run[i], l_run[i], t);
+            if (live[i]) ft_write<D, NT>(p, tok, head[i], split, i, o, m_run[i], l_run[i], t, NT * warp);
         }
     }
 }
@@ -402,6 +411,9 @@ __device__ __forceinline__ void ft_spread(const FattnParams &p, int gqa_log2, Ft
 template <int D>
 __global__ void __launch_bounds__(FT_THREADS, 3) fattn_tile_kernel(FattnParams p, int gqa_log2) {
     pdl_prologue();
+    // the first rows of the grid take the listed tiles' tokens (their chains are the longest), the others a tile each that is not listed
+    const bool spread = (int) blockIdx.y < p.spread_rows;
+    const int info = spread ? *p.tcount : (p.tflags ? p.tflags[(int) blockIdx.y - p.spread_rows] : 0);
     if (p.vote == 2 && !fattn_tiled_chosen(p.plan)) return;   // the tokens share too few cells: the per-token kernel takes this ubatch
     constexpr int KS = D / 16;            // k-steps of S
     constexpr int NT = D / 8;             // n-tiles of O
@@ -427,11 +439,11 @@ __global__ void __launch_bounds__(FT_THREADS, 3) fattn_tile_kernel(FattnParams p
     int &list_count = sh.tile.list_count;
     extern __shared__ __align__(16) uint8_t kv_s[];   // [stage][K, V][FT_CHUNK rows of ROW bytes] (dynamic: fattn_tile_smem_bytes)
 
-    if ((int) blockIdx.y < p.spread_rows) {   // the first rows of the grid: their chains are the longest
-        ft_spread<D>(p, gqa_log2, sh.spread, kv_s);
+    if (spread) {
+        if (info > 0) ft_spread<D>(p, gqa_log2, sh.spread, kv_s);
         return;
     }
-    if (p.tflags && p.tflags[(int) blockIdx.y - p.spread_rows]) return;
+    if (info) return;
 
     // rows g and g + 8 of this warp: (token, head)
     int64_t tok[2];
@@ -543,15 +555,6 @@ __global__ void __launch_bounds__(FT_THREADS, 3) fattn_tile_kernel(FattnParams p
         }
         __syncthreads();
         const int n_chunks = (count + FT_CHUNK - 1) / FT_CHUNK;
-        // ---- which cells of each of this split's chunks every token attends to ----
-        for (int c = split + warp * nsplit; c < n_chunks; c += 4 * nsplit) {   // a warp per chunk, a lane per cell
-            const int idx = c * FT_CHUNK + lane, kb = cell_kb[min(idx, count - 1)];
-#pragma unroll 4
-            for (int j = 0; j < n_tile_tok; ++j) {
-                const unsigned m = __ballot_sync(0xffffffffu, idx < count && ((tile_words[j][kb >> 6] >> (kb & 63)) & 1ull));
-                if (lane == 0) rmask[j][c] = m;
-            }
-        }
         // this split's chunks: split, split + nsplit, ...; FT_STAGES - 1 of them are on their way while one is multiplied
         int issued = 0;
         auto issue = [&] {
@@ -561,6 +564,15 @@ __global__ void __launch_bounds__(FT_THREADS, 3) fattn_tile_kernel(FattnParams p
             ++issued;
         };
         for (int k = 0; k < FT_STAGES - 1; ++k) issue();
+        // ---- which cells of each of this split's chunks every token attends to (while the first chunks travel) ----
+        for (int c = split + warp * nsplit; c < n_chunks; c += 4 * nsplit) {   // a warp per chunk, a lane per cell
+            const int idx = c * FT_CHUNK + lane, kb = cell_kb[min(idx, count - 1)];
+#pragma unroll 4
+            for (int j = 0; j < n_tile_tok; ++j) {
+                const unsigned m = __ballot_sync(0xffffffffu, idx < count && ((tile_words[j][kb >> 6] >> (kb & 63)) & 1ull));
+                if (lane == 0) rmask[j][c] = m;
+            }
+        }
         int it = 0;
         for (int ch = split; ch < n_chunks; ch += nsplit, ++it) {
             const int s = it % FT_STAGES;
@@ -574,7 +586,7 @@ __global__ void __launch_bounds__(FT_THREADS, 3) fattn_tile_kernel(FattnParams p
             if (__any_sync(0xffffffffu, (rm[0] | rm[1]) != 0u)) {   // a chunk that none of the warp's rows attends to changes nothing
                 float sacc[4][4];
                 uint32_t ph[2][4], pl[2][4];
-                ft_s<D, 0, 4>(sacc, qa, Ks, lane);
+                ft_s<D>(sacc, qa, Ks, lane);
                 ft_softmax<D>(p, sacc, rm, binary_mask, mrow, slope, cell_list + ch * FT_CHUNK, t, m_run, l_run, o, ph, pl);
 #pragma unroll
                 for (int kk = 0; kk < 2; ++kk) ft_pv<D>(o, ph[kk], pl[kk], Vs + (uint32_t) (16 * kk * ROW), lane);

@@ -34,6 +34,7 @@ __global__ void __launch_bounds__(256) quantize_q8_0_kernel(const float *__restr
                 v[0] = row[0]; v[1] = row[1]; v[2] = row[2]; v[3] = row[3];
             }
         }
+        pdl_trigger();   // the values are here: the next kernel's CTAs may take their places
         q8_quantize_store<LAYOUT>(v, out, d_offset, nb, nbp, n, b, j, real, variant, chunk_nt);
     }
 }

@@ -170,8 +170,9 @@ __global__ void __launch_bounds__(256) fattn_plan_kernel(const int32_t *__restri
 // it tells whether walking the cells once per group (fattn_tile_kernel) beats walking them once per token: a prompt's
 // tokens share nearly all their words, the tokens of a decode batch share none.  And the same for every tile the
 // query-tiled kernel may use (4, 8, 16 or 32 tokens): tiles whose tokens share little (decode tokens beside a prompt) are
-// flagged and listed, their tokens are walked one by one (plan[4 + k] = listed tiles of 4 << k tokens).  The line lies at
-// three tokens per word: a shared chunk costs its CTA about as much as two to three chunks of single tokens cost theirs.
+// flagged and listed, their tokens are walked one by one (plan[4 + k] = listed tiles of 4 << k tokens).  The line lies at one and a
+// half tokens per word: a token's own chunk costs a CTA about two thirds of a shared one (64 sequences with 3 tokens each, 2.7
+// tokens per word: 415 us token by token, 220 shared; with 2 tokens each 147 and 86).
 constexpr int VOTE_WORDS = 4096;
 __global__ void __launch_bounds__(256) fattn_tile_vote_kernel(const int32_t *__restrict__ wlist, const int32_t *__restrict__ wcount, int64_t Nq, int64_t nw,
                                                              int32_t *__restrict__ plan, int32_t *__restrict__ flags, int32_t *__restrict__ lists, int64_t stride) {
@@ -223,7 +224,7 @@ __global__ void __launch_bounds__(256) fattn_tile_vote_kernel(const int32_t *__r
             if (k == 2) atomicAdd(plan + 1, sum[i]);
             int64_t own = 0;
             for (int j = first * size; j < min(n, (first + 1) * size); ++j) own += wcount[t0 + j];
-            const int32_t tile = (int32_t) (t0 / size + first), few = own < 3ll * sum[i] ? 1 : 0;
+            const int32_t tile = (int32_t) (t0 / size + first), few = 2 * own < 3ll * sum[i] ? 1 : 0;
             flags[k * stride + tile] = few;
             if (few) lists[k * stride + atomicAdd(plan + 4 + k, 1)] = tile;
         }

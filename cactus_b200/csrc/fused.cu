@@ -18,7 +18,7 @@ namespace b200 {
 // Bound by latency at few rows (load, reduce, 32 dependent double additions, scale), by memory at many.  One group per thread
 // (GMAX 1: rows of up to 4096 elements) fits 32 registers, so two CTAs of 1024 threads share an SM, and the weight is loaded
 // with the row; only the first warp adds up the warps' sums and works the scale out, with the exact reciprocal where d is a
-// power of two (the same quotient), instead of all of them.  Before / now: the table at the head of this file.
+// power of two (the same quotient), instead of all of them.  us per launch on B200, before / now: 512 x 4096 17.2 / 11.5, 512 x 2048 10.9 / 9.3.
 template <int GMAX>   // groups of 4 elements per thread: d <= 4 GMAX blockDim.x
 __global__ void __launch_bounds__(1024, GMAX == 1 ? 2 : 1) add_rms_norm_quantize_kernel(float *x, int64_t x_nb_row, const float *res,
                                                                     int64_t res_nb_row, const float *__restrict__ w, float *h,
@@ -92,7 +92,7 @@ __global__ void __launch_bounds__(1024, GMAX == 1 ? 2 : 1) add_rms_norm_quantize
 }
 
 // silu(gate) * up, quantised; the same index space as quantize_q8_0_kernel: a row per x, 256 groups of 4 elements per y (no
-// 64-bit division per thread, which was most of the instructions)
+// 64-bit division per thread, which was most of the instructions: 64 x 14336 10.3 / 6.6 us before / now, 512 x 14336 23.6 / 20.3)
 __global__ void __launch_bounds__(256) silu_mul_quantize_kernel(const float *gate, const float *up, int64_t nb_row,
                                                                float *dst, int64_t dst_nb_row,
                                                                int64_t N, int64_t nb, int64_t nbp,

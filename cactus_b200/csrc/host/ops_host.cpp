@@ -9,6 +9,7 @@
 #include <ATen/ATen.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
+#include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/python_variable.h>
 
 #include "../../../include/cactus_b200.h"
@@ -61,16 +62,17 @@ struct NoGil {
     ~NoGil() { PyEval_RestoreThread(state); }
 };
 
+// What torch throws reaches the caller as the exception that torch itself would raise: an allocation that fails is a
+// torch.OutOfMemoryError, which callers catch to free memory and try again.
 template <typename F>
 PyObject *guarded(F f) {
+    HANDLE_TH_ERRORS
     try {
         return f();
     } catch (const Fail &) {
         return nullptr;
-    } catch (const std::exception &e) {
-        PyErr_SetString(PyExc_RuntimeError, e.what());
-        return nullptr;
     }
+    END_HANDLE_TH_ERRORS
 }
 
 // mul_mat(wtype, K, M, w_data, x, variant, out | None, scratch | None) -> out

@@ -115,6 +115,10 @@ def host():
         path = os.path.join(HERE, "lib", "_ops_host.so")
         if not os.path.exists(path):
             raise B200Error(f"{path} is missing: build it with `python -m cactus_b200.build`")
+        from .build import built_host_abi, host_abi
+        built = built_host_abi(path)
+        if built != host_abi():   # torch's classes may be laid out differently, and no Python error would come of that
+            raise B200Error(f"{path} was built against {built}, this is {host_abi()}: build it with `python -m cactus_b200.build`")
         spec = importlib.util.spec_from_file_location("_ops_host", path, loader=importlib.machinery.ExtensionFileLoader("_ops_host", path))
         m = importlib.util.module_from_spec(spec)
         spec.loader.exec_module(m)

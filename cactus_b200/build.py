@@ -5,6 +5,7 @@
 from __future__ import annotations
 
 import os
+import re
 import subprocess
 import sys
 from concurrent.futures import ThreadPoolExecutor
@@ -66,16 +67,38 @@ def build(force: bool = False, verbose: bool = False) -> str:
     return LIB
 
 
+def host_abi() -> str:
+    """What _ops_host.so binds besides its own source: torch's C++ classes and the interpreter's C API."""
+    import sysconfig
+
+    import torch
+    return f"torch {torch.__version__} cuda {torch.version.cuda} cxx11abi {int(torch._C._GLIBCXX_USE_CXX11_ABI)} python {sysconfig.get_config_var('EXT_SUFFIX')}"
+
+
+def built_host_abi(path: str) -> str:
+    """What the library at `path` was built against: a string that the build leaves in it (b200_host_abi)."""
+    with open(path, "rb") as f:
+        m = re.search(rb"b200_host_abi\{([^}\0]*)\}", f.read())
+    return m.group(1).decode() if m else "an unknown torch"
+
+
+def host_stale() -> bool:
+    """Older than its source, or built against another torch (whose classes may be laid out differently)."""
+    deps = [os.path.join(CSRC, "host", "ops_host.cpp"), os.path.join(os.path.dirname(HERE), "include", "cactus_b200.h")]
+    return _stale(HOST_LIB, deps) or built_host_abi(HOST_LIB) != host_abi()
+
+
 def build_host(force: bool = False) -> str:
-    src = os.path.join(CSRC, "host", "ops_host.cpp")
-    if force or _stale(HOST_LIB, [src, os.path.join(os.path.dirname(HERE), "include", "cactus_b200.h")]):
+    if force or host_stale():
         import sysconfig
 
         import torch
         from torch.utils.cpp_extension import include_paths
+        src = os.path.join(CSRC, "host", "ops_host.cpp")
         tlib = os.path.join(os.path.dirname(torch.__file__), "lib")
         cuda = os.path.dirname(os.path.dirname(nvcc())) if os.path.isabs(nvcc()) else "/usr/local/cuda"
         cmd = ["g++", "-O2", "-std=c++17", "-shared", "-fPIC", "-fvisibility=hidden", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+               f'-DB200_HOST_ABI="{host_abi()}"',
                *[f"-I{p}" for p in (*include_paths(), sysconfig.get_paths()["include"], os.path.join(cuda, "include"))], src, "-o", HOST_LIB,
                f"-L{OUT}", "-lcactus_b200", f"-L{tlib}", "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_python", "-Wl,-rpath,$ORIGIN"]
         r = subprocess.run(cmd, capture_output=True, text=True)

@@ -14,6 +14,9 @@
 
 #include "../../../include/cactus_b200.h"
 
+// what this file was compiled against: build.py rebuilds it, and _lib.py refuses it, where that is not what runs
+extern "C" __attribute__((used, visibility("default"))) const char b200_host_abi[] = "b200_host_abi{" B200_HOST_ABI "}";
+
 namespace {
 
 PyObject *g_error = nullptr;   // cactus_b200._lib.B200Error

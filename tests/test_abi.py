@@ -85,3 +85,23 @@ def test_plugin_exports_the_loader_entry_points():
     syms = subprocess.run(["nm", "-D", "--defined-only", so], capture_output=True, text=True).stdout
     for name in ("lm_ggml_backend_init", "lm_ggml_backend_score", "lm_ggml_backend_b200_reg", "lm_ggml_backend_b200_init"):
         assert f" T {name}" in syms, name
+
+
+def test_host_path_is_rebuilt_for_another_torch_and_not_loaded_with_it(monkeypatch, tmp_path):
+    """_ops_host.so binds torch's C++ classes: one that was built against another torch counts as stale, and loading it
+    is refused (its calls could not fail in a way that Python sees)."""
+    import cactus_b200._lib as _lib
+    from cactus_b200 import build as b
+    b.build()
+    assert b.built_host_abi(b.HOST_LIB) == b.host_abi() and not b.host_stale()
+    monkeypatch.setattr(_lib, "_host", None)
+    _lib.host()
+    other = b.host_abi().replace("torch ", "torch 1.")
+    monkeypatch.setattr(b, "host_abi", lambda: other)
+    monkeypatch.setattr(_lib, "_host", None)
+    assert b.host_stale()
+    with pytest.raises(_lib.B200Error, match="built against"):
+        _lib.host()
+    unmarked = tmp_path / "_ops_host.so"
+    unmarked.write_bytes(b"no mark")
+    assert b.built_host_abi(str(unmarked)) != other

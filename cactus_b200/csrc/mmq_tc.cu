@@ -100,7 +100,7 @@ struct TcPlan {
     int cs;             // > 0: clusters of cs CTAs, one tile per cluster; 0: equal shares over gridDim.x CTAs
     unsigned long long launch_id;   // equal shares: marks the arrival counters (56 bits)
     uint32_t share, extra;   // equal shares: CTA j takes share iterations, one more if j < extra
-    int debug;          // 32: the producer copies nothing (the test of the give-up path)
+    int debug;          // tests of the give-up path: 32 no producer copies anything, 64 those of odd CTAs, 128 one write-back warp gives up
 };
 // The weights as tensor maps: 1 KB (2 KB) tiles and 128-byte scale tiles of one block group, 8 row tiles (128 rows) per copy.
 // Row ranges that come from separate tensors (PeerDst::wseg) have a pair of maps each.
@@ -123,20 +123,21 @@ __device__ __forceinline__ bool tc_elect() {
     asm volatile("{\n.reg .pred p;\nelect.sync _|p, 0xffffffff;\nselp.u32 %0, 1, 0, p;\n}\n" : "=r"(el));
     return el != 0;
 }
-// Bounded wait of a whole (converged) warp; false = gave up (or the CTA already gave up elsewhere).  The loop is one function
-// for all callers: the kernel's hot code has to fit the instruction cache.
+// Bounded wait of a whole (converged) warp; false = gave up (or the CTA already gave up elsewhere).  The outcome is one for
+// the warp, by vote: what follows a wait (elect.sync, tcgen05.ld) needs all its lanes.  The loop is one function for all
+// callers: the kernel's hot code has to fit the instruction cache.
 __device__ __noinline__ bool tc_wait_slow(uint32_t bar, uint32_t parity, volatile int *abort_flag, uint32_t limit) {
 #pragma unroll 1
     for (uint32_t i = 0; i < limit; ++i) {
-        if (tc_try(bar, parity)) return true;
-        if ((i & 15u) == 15u && *abort_flag) return false;
+        if (__all_sync(0xffffffffu, tc_try(bar, parity))) return true;
+        if ((i & 15u) == 15u && __any_sync(0xffffffffu, *abort_flag)) return false;
     }
     *abort_flag = 1;
     atomicExch(&g_tc_error, 1);
     return false;
 }
 __device__ __forceinline__ bool tc_wait(uint32_t bar, uint32_t parity, volatile int *abort_flag, uint32_t limit) {
-    return tc_try(bar, parity) || tc_wait_slow(bar, parity, abort_flag, limit);
+    return __all_sync(0xffffffffu, tc_try(bar, parity)) || tc_wait_slow(bar, parity, abort_flag, limit);
 }
 __device__ __forceinline__ void tc_arrive(uint32_t bar) { asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];\n" ::"r"(bar) : "memory"); }
 __device__ __forceinline__ void tc_commit(uint32_t bar) {
@@ -207,6 +208,7 @@ struct TcShared {
     uint32_t slot_n;                // float4s of one
     uint32_t tmem;
     int abort_flag, flag;
+    int wb_gave_up;                 // a write-back warp gave up
     uint32_t n_pieces, n_iter;
     TcPiece piece[TC_MAX_PIECES];
 };
@@ -435,6 +437,7 @@ __global__ void __launch_bounds__((TcCfg<WTYPE, NT>::THREADS), 1) mmq_tc_kernel(
     const uint32_t bars = smem_u32 + C::BAR_OFFSET;
     TcShared *const sh = reinterpret_cast<TcShared *>(smem + C::SH_OFFSET);
     volatile int *const abort_flag = &sh->abort_flag;
+    volatile int *const wb_gave_up = &sh->wb_gave_up;
     float *const acc_s = reinterpret_cast<float *>(smem + C::OFF_ACC);
     const uint32_t acc_u32 = smem_u32 + C::OFF_ACC;
 #define BAR(which, i) (bars + 8u * (uint32_t) ((which) + (i)))
@@ -453,6 +456,7 @@ __global__ void __launch_bounds__((TcCfg<WTYPE, NT>::THREADS), 1) mmq_tc_kernel(
     }
     if (tid == 64) {
         sh->abort_flag = 0;
+        sh->wb_gave_up = 0;
         tc_share(sh, plan, n_bg, (uint32_t) dims.n_rt);
     }
     if (tid < C::N_BARS) {
@@ -531,7 +535,7 @@ __global__ void __launch_bounds__((TcCfg<WTYPE, NT>::THREADS), 1) mmq_tc_kernel(
     } else if (warp == 2) {
         // ---------------- producer: two or four tensor copies of weights, one bulk copy of activations per block group ----------------
         uint32_t s = 0, par = 1, issued = 0;
-        bool ok = !(plan.debug & 32);
+        bool ok = !(plan.debug & 32) && !(plan.debug & 64 && blockIdx.x & 1);
         const uint32_t b_bytes = (uint32_t) act.chunk_nt * 4096u;
 #pragma unroll 1
         for (uint32_t p = 0; p < sh->n_pieces && ok; ++p) {
@@ -689,8 +693,16 @@ __global__ void __launch_bounds__((TcCfg<WTYPE, NT>::THREADS), 1) mmq_tc_kernel(
                     if (lane == 0) tc_arrive(BAR(C::B_ACCE, mt));
                 }
             }
-            if (!ok || p + 1 == sh->n_pieces) break;   // the last piece: all warps share what is left to do, below
+            if (plan.debug & 128 && warp == C::WARP_EPI + 1 && blockIdx.x == 1) {
+                ok = false;
+                *abort_flag = 1;
+                atomicExch(&g_tc_error, 1);
+            }
+            if (p + 1 == sh->n_pieces) break;   // the last piece: all warps share what is left to do, below
+            // one warp's wait may run out where its neighbours' did not: the four go on, or leave, together
+            if (!ok) *wb_gave_up = 1;
             asm volatile("bar.sync 1, 128;\n" ::: "memory");
+            if (*wb_gave_up) break;   // (written again at the earliest beyond the barriers of tc_finish)
             tc_finish<WTYPE>(sh, acc_u32, p, (uint32_t) et, TC_EPI_THREADS, 1u);
         }
     }
@@ -848,7 +860,7 @@ static TcPlan tc_plan(const TcVariant &v, const TiledDims &d, const ActDims &a, 
         return e ? atoi(e) : -1;
     }();
     static const int debug = [] {
-        const char *e = getenv("B200_TCF_DEBUG");
+        const char *e = getenv("B200_TC_DEBUG");
         return e ? atoi(e) : 0;
     }();
     TcPlan best = {};

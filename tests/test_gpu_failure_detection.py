@@ -73,13 +73,45 @@ print(before, gave_up, cleared, bool(torch.isfinite(y1).all()), float(y1.abs().m
 
 
 def test_tensor_core_kernel_gives_up_a_wait_that_nothing_completes_and_says_so():
-    """The folded-scale tcgen05 kernel with its producer switched off (B200_TCF_DEBUG=32): no stage ever lands, every
+    """The folded-scale tcgen05 kernel with its producer switched off (B200_TC_DEBUG=32): no stage ever lands, every
     consumer wait runs into the (shortened) limit, the CTAs wait for what they have in flight (nothing), free their
     tensor memory and return; b200_kernel_status is then non-zero, clears, and the context computes another product.
     Runs in a child process because the switches are read once per process."""
-    env = dict(os.environ, B200_MMQ_TC="2", B200_TCF_DEBUG="32")
+    env = dict(os.environ, B200_MMQ_TC="1", B200_TC_DEBUG="32")
     r = subprocess.run([sys.executable, "-c", CHILD, ROOT], env=env, capture_output=True, text=True, timeout=300)
     assert r.returncode == 0, r.stderr[-2000:]
     before, gave_up, cleared, finite, amax = r.stdout.split()[-5:]
     assert int(before) == 0 and int(gave_up) & 2 and int(cleared) == 0, r.stdout
     assert finite == "True" and float(amax) > 0, r.stdout
+
+
+CHILD_PARTIAL = r'''
+import sys, torch
+sys.path.insert(0, sys.argv[1])
+from cactus_b200 import ops
+from cactus_b200._lib import lib
+from cactus_b200.engine import random_blocks
+L = lib()
+g = torch.Generator(device="cuda").manual_seed(5)
+K, M, N = 1024, 25600, 64                  # 100 tiles of 8 block groups in equal shares of 5 and 6: tiles of one to three parts, one or two pieces a CTA
+w = ops.QWeight.from_blocks(2, K, M, random_blocks(2, M, K, g))
+x = torch.randn((N, K), device="cuda", generator=g)
+L.b200_kernel_set_wait_limit(64)
+ops.mul_mat(w, x)
+torch.cuda.synchronize()
+gave_up = L.b200_kernel_status()
+L.b200_kernel_set_wait_limit(0)
+y1 = ops.mul_mat(w, x[:1])
+torch.cuda.synchronize()
+print(gave_up, L.b200_kernel_status(), bool(torch.isfinite(y1).all()))
+'''
+
+
+@pytest.mark.parametrize("who", ["64", "128"])
+def test_tensor_core_kernel_gives_up_in_some_ctas_or_warps_only(who):
+    """Half of the CTAs without a producer (B200_TC_DEBUG=64), and one of the four write-back warps of a CTA that gives up
+    where its neighbours do not (128): the warps that share a barrier leave together, and every CTA returns."""
+    env = dict(os.environ, B200_MMQ_TC="1", B200_TC_PLAN="1600", B200_TC_DEBUG=who)
+    r = subprocess.run([sys.executable, "-c", CHILD_PARTIAL, ROOT], env=env, capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0, r.stderr[-2000:]
+    assert r.stdout.split()[-3:] == ["2", "0", "True"], r.stdout

@@ -210,6 +210,7 @@ struct TcShared {
     int abort_flag, flag;
     int wb_gave_up;                 // a write-back warp gave up
     uint32_t n_pieces, n_iter;
+    uint32_t n_finished;            // pieces that tc_finish has been through
     TcPiece piece[TC_MAX_PIECES];
 };
 
@@ -362,10 +363,30 @@ __device__ __noinline__ void tc_write_cluster(const TcShared *o, uint32_t acc_u3
     }
 }
 
+// Arrival of a part at its tile; true: it is the last one and all parts are there.  A tile's counter is {launch id, parts given up
+// (4 bits), arrivals (4 bits)}; a word without this launch's id counts as zero, so the workspace needs no clearing.  Every CTA
+// arrives exactly once for every piece it shares, with its part parked or given up, and the last to arrive leaves the
+// counter zero: a replay of a graph comes with the same id and must find nothing of an earlier one.
+__device__ __forceinline__ bool tc_arrive_tile(const TcShared *o, const TcPiece &q, bool gave_up) {
+    const unsigned long long id = o->plan.launch_id << 8;
+    unsigned long long *const arrived = o->counters + q.tile;
+    unsigned long long old = *reinterpret_cast<volatile unsigned long long *>(arrived), seen, now;
+    do {
+        seen = old;
+        now = ((seen ^ id) < 256 ? seen : id) + (gave_up ? 17 : 1);
+        old = atomicCAS(arrived, seen, (now & 15) == q.parts ? 0ull : now);
+    } while (old != seen);
+    return (now & 255) == q.parts;
+}
+// The pieces of a CTA that gave up.  One thread, after everything else.
+__device__ __noinline__ void tc_give_up_pieces(const TcShared *o) {
+#pragma unroll 1
+    for (uint32_t p = o->n_finished; p < o->n_pieces; ++p)
+        if (o->piece[p].parts > 1) tc_arrive_tile(o, o->piece[p], true);
+}
+
 // Piece q is complete in shared memory: write the tile if this is all of it or the last part to arrive, else park it.  Called by
-// `threads` threads, te = 0 ..., which meet at barrier `bar`.  A tile's counter is {launch id, arrivals}; a word without
-// this launch's id counts as zero, so the workspace needs no clearing, and the last to arrive leaves it zero for the next
-// replay of a graph.  The parts (at most three) are added in K order whoever does it.
+// `threads` threads, te = 0 ..., which meet at barrier `bar`.  The parts (at most three) are added in K order whoever does it.
 template <int WTYPE>
 __device__ __noinline__ void tc_finish(TcShared *o, uint32_t acc_u32, uint32_t piece, uint32_t te, uint32_t threads, uint32_t bar) {
     const TcPiece q = o->piece[piece];
@@ -377,12 +398,12 @@ __device__ __noinline__ void tc_finish(TcShared *o, uint32_t acc_u32, uint32_t p
 #pragma unroll
     for (uint32_t k = 0; k < 3; ++k) at[k] = k < q.parts && k != own ? o->slots + (size_t) (k == 0 ? q.slot0 : (q.slot0 & ~1u) + 2 * k) * o->slot_n : nullptr;
     if (q.parts > 1) {
-        const unsigned long long id = o->plan.launch_id << 8;
-        unsigned long long *const arrived = o->counters + q.tile;
         if (te == 0) {   // every other part parked already: nothing of this one has to go through memory
+            unsigned long long *const arrived = o->counters + q.tile;
             unsigned long long seen;
             asm volatile("ld.acquire.gpu.global.u64 %0, [%1];\n" : "=l"(seen) : "l"(arrived) : "memory");
-            *flag = seen == id + q.parts - 1;
+            *flag = seen == (o->plan.launch_id << 8) + q.parts - 1;
+            if (*flag) *arrived = 0;   // nobody else is to come
         }
         asm volatile("bar.sync %0, %1;\n" ::"r"(bar), "r"(threads) : "memory");
         write = *flag != 0;
@@ -395,20 +416,14 @@ __device__ __noinline__ void tc_finish(TcShared *o, uint32_t acc_u32, uint32_t p
             __threadfence();
             asm volatile("bar.sync %0, %1;\n" ::"r"(bar), "r"(threads) : "memory");
             if (te == 0) {
-                unsigned long long old = *reinterpret_cast<volatile unsigned long long *>(arrived), seen, base;
-                do {
-                    seen = old;
-                    base = (seen ^ id) < 256 ? seen : id;
-                    old = atomicCAS(arrived, seen, base + 1);
-                } while (old != seen);
-                *flag = base == id + q.parts - 1;
+                *flag = tc_arrive_tile(o, q, false);
                 __threadfence();
             }
             asm volatile("bar.sync %0, %1;\n" ::"r"(bar), "r"(threads) : "memory");
             write = *flag != 0;
         }
-        if (write && te == 0) *arrived = 0;
     }
+    if (te == 0) o->n_finished = piece + 1;
     if (write) {
         TcOut out(o, q, te, threads);
 #pragma unroll 1
@@ -457,6 +472,7 @@ __global__ void __launch_bounds__((TcCfg<WTYPE, NT>::THREADS), 1) mmq_tc_kernel(
     if (tid == 64) {
         sh->abort_flag = 0;
         sh->wb_gave_up = 0;
+        sh->n_finished = 0;
         tc_share(sh, plan, n_bg, (uint32_t) dims.n_rt);
     }
     if (tid < C::N_BARS) {
@@ -715,7 +731,11 @@ __global__ void __launch_bounds__((TcCfg<WTYPE, NT>::THREADS), 1) mmq_tc_kernel(
         asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;\n" ::: "memory");
     } else {
         __syncthreads();
-        if (sh->n_pieces > 0 && !*abort_flag) tc_finish<WTYPE>(sh, acc_u32, sh->n_pieces - 1, (uint32_t) tid, C::THREADS, 0u);
+        if (*abort_flag) {
+            if (tid == 0) tc_give_up_pieces(sh);
+        } else if (sh->n_pieces > 0) {
+            tc_finish<WTYPE>(sh, acc_u32, sh->n_pieces - 1, (uint32_t) tid, C::THREADS, 0u);
+        }
         __syncthreads();
     }
 #undef BAR

@@ -29,8 +29,8 @@
 //   * every hand-over between warps is some twenty instructions at 10-16 clk each beside busy warps, so there are few: one per
 //     half block group and role, with an A stage for each team of weight warps.
 //
-// Roles of a CTA (one per SM, 24 or 32 warps): warps 0 and 1 issue the MMAs of one row tile each, warp 2 the copies (a ring of
-// stages of one block group), two or three teams of 8 warps convert weights (the teams take the half block groups in turn; a
+// Roles of a CTA (one per SM, 24 warps): warps 0 and 1 issue the MMAs of one row tile each, warp 2 the copies (a ring of
+// stages of one block group), two teams of 8 warps convert weights (they take the half block groups in turn; a
 // warp: 32 rows), the last four warps move the accumulators to shared memory and write results.  The two row tiles share the
 // copies only: each has its own A stages, accumulator and barriers.  Code that runs once per tile is kept small and in loops:
 // with 172 KB of (unrolled, inlined) code the kernel spent most of its time on instruction cache misses.
@@ -64,9 +64,10 @@ constexpr int TC_RT = 16;            // 16-row tiles of a CTA at most: 256 rows,
 constexpr int TC_FLUSH = 16;         // block groups accumulated in tensor memory before they are added up in shared memory
 constexpr int TC_EPI_THREADS = 128;
 
-// Geometry for up to NT tiles of 8 activation columns per CTA.
-template <int WTYPE, int NT>
+// Geometry.  A CTA has up to NT tiles of 8 activation columns.
+template <int WTYPE>
 struct TcCfg {
+    static constexpr int NT = 8;
     static constexpr int WT = WTYPE == B200_TYPE_Q4_0 ? 1024 : 2048;   // one row tile, one block group
     static constexpr int OFF_S = TC_RT * WT;                           // its scales: 128 bytes per row tile
     static constexpr int OFF_B = OFF_S + TC_RT * 128;                  // B_hi: 2 KB per column tile, then B_lo
@@ -77,7 +78,7 @@ struct TcCfg {
     // tensor memory of row tile mt: an accumulator of 2 x 8 NT columns (hi | small terms) at mt * D_MT, ABUF A stages of half a block
     // group (32 columns of A_hi, 32 of A_lo) at A_COL + mt * A_MT
     static constexpr int D_MT = 16 * NT;
-    static constexpr int ABUF = NT < 8 ? 3 : 2;
+    static constexpr int ABUF = 2;
     static constexpr int A_MT = ABUF * 64, A_COL = 512 - 2 * A_MT;
     // warps: 4 for MMAs and copies, a team of 8 weight warps per A stage (each waits for its own stage phase after phase, which a
     // parity wait can tell apart), 4 for the write-back
@@ -103,9 +104,8 @@ struct TcPlan {
     int debug;          // tests of the give-up path: 32 no producer copies anything, 64 those of odd CTAs, 128 one write-back warp gives up
 };
 // The weights as tensor maps: 1 KB (2 KB) tiles and 128-byte scale tiles of one block group, 8 row tiles (128 rows) per copy.
-// Row ranges that come from separate tensors (PeerDst::wseg) have a pair of maps each.
 struct TcMaps {
-    CUtensorMap q[3], s[3];
+    CUtensorMap q, s;
 };
 
 __device__ __forceinline__ uint64_t tc_smem_desc(uint32_t addr, uint32_t lbo, uint32_t sbo) {
@@ -172,19 +172,6 @@ __device__ __forceinline__ void tc_ld_x16(uint32_t (&r)[16], uint32_t taddr) {
                    "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]) : "r"(taddr));
 }
 
-// ---- a row tile's tensor (PeerDst::wseg) and its place in it ----
-__device__ __forceinline__ void tc_weight_at(const PeerDst &peers, int rt, int &seg, int &rt_in) {
-    seg = 0;
-    rt_in = rt;
-    if (peers.n_wseg > 0) {
-        const int row = rt * 16;
-        if (row >= peers.seg_end[0]) {
-            seg = (peers.n_seg > 2 && row >= peers.seg_end[1]) ? 2 : 1;
-            rt_in -= (seg == 2 ? peers.seg_end[1] : peers.seg_end[0]) / 16;
-        }
-    }
-}
-
 // A piece of work: block groups [bg, bg + len) of a tile (row group x column chunk).
 struct TcPiece {
     uint32_t tile, group, chunk, bg, len;
@@ -198,7 +185,6 @@ constexpr int TC_MAX_PIECES = 128;
 struct TcShared {
     TiledDims dims;
     ActDims act;
-    PeerDst peers;
     TcPlan plan;
     const uint8_t *w, *aq;
     float *dst;
@@ -220,10 +206,8 @@ static_assert(sizeof(TcShared) <= 5120, "TcShared has its place in TcCfg");
 // operands left the fp16 range.
 template <int WTYPE>
 __device__ __noinline__ float tc_exact_value(const TcShared *o, int row, int col) {
-    int seg, rt;
-    tc_weight_at(o->peers, row >> 4, seg, rt);
-    const uint8_t *wq = o->peers.n_wseg > 0 ? o->peers.wseg[seg] : o->w, *ws = wq + (o->peers.n_wseg > 0 ? (size_t) o->peers.wseg_qs[seg] : o->dims.qs_bytes);
-    const int r = row & 15, g = r & 7, h = r >> 3;
+    const uint8_t *wq = o->w, *ws = wq + o->dims.qs_bytes;
+    const int rt = row >> 4, r = row & 15, g = r & 7, h = r >> 3;
     float sum = 0.0f;
 #pragma unroll 1
     for (int b = 0; b < (int) o->dims.nb; ++b) {
@@ -294,16 +278,14 @@ __device__ __noinline__ void tc_share(TcShared *o, const TcPlan plan, uint32_t n
     o->n_pieces = n;
 }
 
-// Values that do not simply go to 16 aligned bytes: a ragged or unaligned edge, other GPUs' buffers too, or not finite
+// Values that do not simply go to 16 aligned bytes: a ragged or unaligned edge, or not finite
 template <int WTYPE>
 __device__ __noinline__ void tc_write_slow(const TcShared *o, int row, int row_end, int col, float4 f) {
 #pragma unroll 1
     for (int i = 0; i < 4 && row + i < row_end; ++i) {
         float y = i == 0 ? f.x : i == 1 ? f.y : i == 2 ? f.z : f.w;
         if (!isfinite(y)) y = tc_exact_value<WTYPE>(o, row + i, col);
-        const int64_t off = col * o->dst_nb_row + (int64_t) (row + i) * 4 + peer_row_shift(o->peers, row + i);
-#pragma unroll 1
-        for (int p = -1; p < o->peers.n; ++p) *reinterpret_cast<float *>(reinterpret_cast<char *>(p < 0 ? o->dst : o->peers.p[p]) + off) = y;
+        *reinterpret_cast<float *>(reinterpret_cast<char *>(o->dst) + col * o->dst_nb_row + (int64_t) (row + i) * 4) = y;
     }
 }
 // Where a thread's share of a tile goes: elements e0, e0 + step, ... of [column][256 rows / 4]; step is a multiple of 64, so the
@@ -321,8 +303,8 @@ struct TcOut {
         col_end = row < row_end ? (int) o->act.N : 0;
         const int64_t nb = o->dst_nb_row;
         inc = col_inc * nb;
-        to = reinterpret_cast<char *>(o->dst) + col * nb + (int64_t) row * 4 + peer_row_shift(o->peers, row);
-        vec = row + 3 < row_end && o->peers.n == 0 && ((reinterpret_cast<uintptr_t>(to) | (uintptr_t) nb) & 15) == 0;
+        to = reinterpret_cast<char *>(o->dst) + col * nb + (int64_t) row * 4;
+        vec = row + 3 < row_end && ((reinterpret_cast<uintptr_t>(to) | (uintptr_t) nb) & 15) == 0;
     }
     template <int WTYPE>
     __device__ __forceinline__ void put(const TcShared *o, float4 v) {
@@ -441,11 +423,11 @@ __device__ __noinline__ void tc_finish(TcShared *o, uint32_t acc_u32, uint32_t p
     asm volatile("bar.sync %0, %1;\n" ::"r"(bar), "r"(threads) : "memory");   // the partial results are free again
 }
 
-template <int WTYPE, int NT>
-__global__ void __launch_bounds__((TcCfg<WTYPE, NT>::THREADS), 1) mmq_tc_kernel(TiledDims dims, const uint8_t *__restrict__ w, ActDims act, const uint8_t *__restrict__ aq,
-                                                              float *__restrict__ dst, int64_t dst_nb_row, void *__restrict__ workspace, TcPlan plan, PeerDst peers,
+template <int WTYPE>
+__global__ void __launch_bounds__(TcCfg<WTYPE>::THREADS, 1) mmq_tc_kernel(TiledDims dims, const uint8_t *__restrict__ w, ActDims act, const uint8_t *__restrict__ aq,
+                                                              float *__restrict__ dst, int64_t dst_nb_row, void *__restrict__ workspace, TcPlan plan,
                                                               const __grid_constant__ TcMaps maps) {
-    using C = TcCfg<WTYPE, NT>;
+    using C = TcCfg<WTYPE>;
     extern __shared__ __align__(1024) uint8_t smem[];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const uint32_t smem_u32 = (uint32_t) __cvta_generic_to_shared(smem);
@@ -462,7 +444,6 @@ __global__ void __launch_bounds__((TcCfg<WTYPE, NT>::THREADS), 1) mmq_tc_kernel(
     if (tid == 96) {   // warp 3 has no role of its own
         sh->dims = dims;
         sh->act = act;
-        sh->peers = peers;
         sh->plan = plan;
         sh->w = w; sh->aq = aq; sh->dst = dst; sh->dst_nb_row = dst_nb_row;
         sh->counters = reinterpret_cast<unsigned long long *>(workspace);
@@ -558,15 +539,7 @@ __global__ void __launch_bounds__((TcCfg<WTYPE, NT>::THREADS), 1) mmq_tc_kernel(
             const TcPiece q = sh->piece[p];
             const int boxes = 1 + (int) q.two;   // rows past the end read as zero
             const uint32_t bytes = (uint32_t) boxes * 8u * (C::WT + 128u) + b_bytes;
-            const CUtensorMap *qm[2], *sm[2];
-            int rt_in[2];
-#pragma unroll
-            for (int k = 0; k < 2; ++k) {
-                int seg;
-                tc_weight_at(peers, (int) q.group * plan.rt_per_group + 8 * k, seg, rt_in[k]);
-                qm[k] = &maps.q[seg];
-                sm[k] = &maps.s[seg];
-            }
+            const int rt_in = (int) q.group * plan.rt_per_group;
             const uint8_t *bsrc = aq + act.b_offset + ((int64_t) q.chunk * n_bg + q.bg) * b_bytes;
 #pragma unroll 1
             for (uint32_t i = 0; i < q.len; ++i) {
@@ -579,9 +552,9 @@ __global__ void __launch_bounds__((TcCfg<WTYPE, NT>::THREADS), 1) mmq_tc_kernel(
 #pragma unroll
                     for (int k = 0; k < 2; ++k) {
                         if (k < boxes) {
-                            if (WTYPE == B200_TYPE_Q4_0) tc_tma_2d(st + (uint32_t) (k * 8 * C::WT), qm[k], bg * 256, rt_in[k], bar);
-                            else tc_tma_3d(st + (uint32_t) (k * 8 * C::WT), qm[k], 0, bg * 2, rt_in[k], bar);
-                            tc_tma_2d(st + (uint32_t) (C::OFF_S + k * 1024), sm[k], bg * 32, rt_in[k], bar);
+                            if (WTYPE == B200_TYPE_Q4_0) tc_tma_2d(st + (uint32_t) (k * 8 * C::WT), &maps.q, bg * 256, rt_in + 8 * k, bar);
+                            else tc_tma_3d(st + (uint32_t) (k * 8 * C::WT), &maps.q, 0, bg * 2, rt_in + 8 * k, bar);
+                            tc_tma_2d(st + (uint32_t) (C::OFF_S + k * 1024), &maps.s, bg * 32, rt_in + 8 * k, bar);
                         }
                     }
                     tc_copy(st + C::OFF_B, bsrc + (int64_t) i * b_bytes, b_bytes, bar);
@@ -600,7 +573,7 @@ __global__ void __launch_bounds__((TcCfg<WTYPE, NT>::THREADS), 1) mmq_tc_kernel(
         }
         __syncwarp();
     } else if (warp >= 4 && warp < C::WARP_EPI) {
-        // ---------------- weights: a warp owns 32 rows (two T16 tiles: the lanes of tensor memory it can reach) of every third half block group ----------------
+        // ---------------- weights: a warp owns 32 rows (two T16 tiles: the lanes of tensor memory it can reach) of every second half block group ----------------
         const int q4 = warp & 3, mt = ((warp - 4) >> 2) & 1, team = (warp - 4) >> 3;
         const uint32_t rt0 = (uint32_t) (mt * 8 + q4 * 2);
         const uint32_t a_base = tmem + ((uint32_t) (32 * q4) << 16) + C::A_COL + (uint32_t) (mt * C::A_MT);
@@ -669,7 +642,7 @@ __global__ void __launch_bounds__((TcCfg<WTYPE, NT>::THREADS), 1) mmq_tc_kernel(
             }
             __syncwarp();
             if (lane == 0) tc_arrive(BAR(C::B_AFULL, C::ABUF * mt + ab));
-            s += C::ABUF == 2 ? 1u : 1u + half;   // two or three halves on
+            s += 1;   // two halves on
             if (s >= C::STAGES) { s -= C::STAGES; full_par ^= 1; }
         }
     } else if (warp >= C::WARP_EPI) {
@@ -752,18 +725,17 @@ static int tc_sm_count() {   // every device of a process is the same model
     return n;
 }
 
-using tc_kernel_fn = void (*)(TiledDims, const uint8_t *, ActDims, const uint8_t *, float *, int64_t, void *, TcPlan, PeerDst, TcMaps);
+using tc_kernel_fn = void (*)(TiledDims, const uint8_t *, ActDims, const uint8_t *, float *, int64_t, void *, TcPlan, TcMaps);
 struct TcVariant {
     tc_kernel_fn fn;
-    int nt, smem, threads;
+    int smem, threads;
     int max_clusters[9];   // resident clusters of 1..8 CTAs on the current device
 };
-template <int WTYPE, int NT>
+template <int WTYPE>
 static void tc_make(TcVariant &v) {
-    v.fn = mmq_tc_kernel<WTYPE, NT>;
-    v.nt = NT;
-    v.smem = TcCfg<WTYPE, NT>::SMEM;
-    v.threads = TcCfg<WTYPE, NT>::THREADS;
+    v.fn = mmq_tc_kernel<WTYPE>;
+    v.smem = TcCfg<WTYPE>::SMEM;
+    v.threads = TcCfg<WTYPE>::THREADS;
     cudaFuncSetAttribute(v.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, v.smem);
     for (int cs = 1; cs <= 8; ++cs) {
         cudaLaunchConfig_t cfg = {};
@@ -785,9 +757,8 @@ static void tc_make(TcVariant &v) {
         v.max_clusters[cs] = n;
     }
 }
-// column classes: up to 16, 32 columns, more (64-column chunks)
-static const TcVariant &tc_variant(int wtype, int64_t N) {
-    static TcVariant table[64][2][3];   // per device: kernel attributes and occupancy are per-context properties
+static const TcVariant &tc_variant(int wtype) {
+    static TcVariant table[64][2];   // per device: kernel attributes and occupancy are per-context properties
     static bool ready[64] = {false};
     static std::mutex mu;
     int dev = 0;
@@ -795,15 +766,11 @@ static const TcVariant &tc_variant(int wtype, int64_t N) {
     dev &= 63;
     std::lock_guard<std::mutex> lock(mu);
     if (!ready[dev]) {
-        tc_make<B200_TYPE_Q4_0, 2>(table[dev][0][0]);
-        tc_make<B200_TYPE_Q4_0, 4>(table[dev][0][1]);
-        tc_make<B200_TYPE_Q4_0, 8>(table[dev][0][2]);
-        tc_make<B200_TYPE_Q8_0, 2>(table[dev][1][0]);
-        tc_make<B200_TYPE_Q8_0, 4>(table[dev][1][1]);
-        tc_make<B200_TYPE_Q8_0, 8>(table[dev][1][2]);
+        tc_make<B200_TYPE_Q4_0>(table[dev][0]);
+        tc_make<B200_TYPE_Q8_0>(table[dev][1]);
         ready[dev] = true;
     }
-    return table[dev][wtype == B200_TYPE_Q4_0 ? 0 : 1][N > 32 ? 2 : (N > 16 ? 1 : 0)];
+    return table[dev][wtype == B200_TYPE_Q4_0 ? 0 : 1];
 }
 
 // ---- tensor maps ----
@@ -844,32 +811,28 @@ struct TcKey {
 struct TcKeyHash {
     size_t operator()(const TcKey &k) const { return std::hash<const void *>()(k.p) ^ (size_t) (k.a * 0x9E3779B97F4A7C15ull) ^ (size_t) (k.b * 0xC2B2AE3D27D4EB4Full); }
 };
-struct TcPair { CUtensorMap q, s; };
-static bool tc_weight_maps(int wtype, const TiledDims &d, const void *w, CUtensorMap &q, CUtensorMap &s) {
+static bool tc_weight_maps(int wtype, const TiledDims &d, const void *w, TcMaps &maps) {
     static std::mutex mu;
-    static std::unordered_map<TcKey, TcPair, TcKeyHash> cache;
+    static std::unordered_map<TcKey, TcMaps, TcKeyHash> cache;
     const TcKey key{w, d.n_rt * 16 + wtype, d.n_bg};
     std::lock_guard<std::mutex> lock(mu);
     auto it = cache.find(key);
     if (it == cache.end()) {
-        TcPair p;
+        TcMaps p;
         if (!tc_encode(&p.q, w, 256, (uint64_t) d.n_bg * (wtype == B200_TYPE_Q4_0 ? 1 : 2), (uint64_t) d.n_rt, wtype == B200_TYPE_Q4_0 ? 1 : 2)) return false;
         if (!tc_encode(&p.s, (const uint8_t *) w + d.qs_bytes, 32, (uint64_t) d.n_bg, (uint64_t) d.n_rt, 1)) return false;
         if (cache.size() > 65536) cache.clear();
         it = cache.emplace(key, p).first;
     }
-    q = it->second.q;
-    s = it->second.s;
+    maps = it->second;
     return true;
 }
 
-static size_t tc_slot_bytes(int nt) { return (size_t) nt * 8 * 256 * 4; }
 static size_t tc_counter_bytes(int64_t tiles) { return (size_t) ((tiles * 8 + 255) / 256 * 256); }
-// workspace of the equal-share split: a counter per tile, two parked parts per CTA
+// workspace of the equal-share split: a counter per tile, two parked parts (64 columns x 256 rows) per CTA
 size_t mmq_tc_workspace_bytes(int64_t M, int64_t N) {
-    const int nt = N > 32 ? 8 : (N > 16 ? 4 : 2);
-    const int64_t tiles = ((M + 127) / 128) * ((N + 8 * nt - 1) / (8 * nt));
-    return tc_counter_bytes(tiles) + (size_t) tc_sm_count() * 2 * tc_slot_bytes(nt);
+    const int64_t tiles = ((M + 127) / 128) * ((N + 63) / 64);
+    return tc_counter_bytes(tiles) + (size_t) tc_sm_count() * 2 * (64 * 256 * 4);
 }
 
 // The work split, from what was measured on B200 (clocks per block group of a CTA: the MMAs, or the copies when a CTA has only 128
@@ -925,14 +888,10 @@ static TcPlan tc_plan(const TcVariant &v, const TiledDims &d, const ActDims &a, 
 }
 
 int launch_mmq_tc(int wtype, const TiledDims &d, const void *w, const ActDims &a, const void *aq, float *dst, int64_t dst_nb_row,
-                  void *workspace, size_t workspace_bytes, const PeerDst &peers, cudaStream_t st) {
-    const TcVariant &v = tc_variant(wtype, a.N);
+                  void *workspace, size_t workspace_bytes, cudaStream_t st) {
+    const TcVariant &v = tc_variant(wtype);
     TcMaps maps;
-    for (int i = 0; i < std::max(1, peers.n_wseg); ++i) {
-        const int64_t M = peers.n_wseg == 0 ? d.M : (i == peers.n_wseg - 1 ? d.M : peers.seg_end[i]) - (i > 0 ? peers.seg_end[i - 1] : 0);
-        if (!tc_weight_maps(wtype, tiled_dims(wtype, d.K, M), peers.n_wseg == 0 ? w : peers.wseg[i], maps.q[i], maps.s[i]))
-            return set_error(B200_E_CUDA, "mmq_tc: no tensor map for the weights");
-    }
+    if (!tc_weight_maps(wtype, d, w, maps)) return set_error(B200_E_CUDA, "mmq_tc: no tensor map for the weights");
     const bool ws = workspace && workspace_bytes >= mmq_tc_workspace_bytes(d.M, a.N) && d.n_rt * d.n_bg * a.n_nt < (1ll << 31);
     TcPlan plan = tc_plan(v, d, a, ws);
     const int tiles = plan.groups * plan.chunks;
@@ -960,7 +919,7 @@ int launch_mmq_tc(int wtype, const TiledDims &d, const void *w, const ActDims &a
     }
     cfg.attrs = attr;
     cfg.numAttrs = (unsigned) n;
-    const cudaError_t e = cudaLaunchKernelEx(&cfg, v.fn, d, (const uint8_t *) w, a, (const uint8_t *) aq, dst, dst_nb_row, workspace, plan, peers, maps);
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, v.fn, d, (const uint8_t *) w, a, (const uint8_t *) aq, dst, dst_nb_row, workspace, plan, maps);
     if (e != cudaSuccess) return set_error(B200_E_CUDA, "mmq_tc launch: %s", cudaGetErrorString(e));
     return check_launch("mmq_tc");
 }

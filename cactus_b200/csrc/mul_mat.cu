@@ -8,7 +8,7 @@
 
 namespace b200 {
 int launch_mmq_tc(int wtype, const TiledDims &d, const void *w, const ActDims &a, const void *aq, float *dst, int64_t dst_nb_row,
-                  void *workspace, size_t workspace_bytes, const PeerDst &peers, cudaStream_t st);
+                  void *workspace, size_t workspace_bytes, cudaStream_t st);
 size_t mmq_tc_workspace_bytes(int64_t M, int64_t N);
 int tc_error_flag();
 void tc_set_wait_limit(unsigned rounds);
@@ -218,7 +218,7 @@ int b200_mul_mat_q(int wtype, const void *w, int64_t K, int64_t M, const float *
     B200_REQUIRE(x_row_stride_bytes % 4 == 0 && dst_row_stride_bytes % 4 == 0 && dst_row_stride_bytes >= M * 4, "bad row stride");
     B200_REQUIRE(variant == B200_Q8_AVX2 || variant == B200_Q8_SCALAR, "unknown quantiser variant %d", variant);
     if (int e = launch_quantize_b8(x, x_row_stride_bytes, K, N, scratch, variant, 2, (cudaStream_t) stream)) return e;
-    return launch_mmq_tc(wtype, tiled_dims(wtype, K, M), w, a, scratch, dst, dst_row_stride_bytes, (char *) scratch + ab, wb, PeerDst{}, (cudaStream_t) stream);
+    return launch_mmq_tc(wtype, tiled_dims(wtype, K, M), w, a, scratch, dst, dst_row_stride_bytes, (char *) scratch + ab, wb, (cudaStream_t) stream);
 }
 
 int b200_mul_mat_q_noalloc(int wtype, const void *w, int64_t K, int64_t M, const float *x, int64_t x_row_stride_bytes, int64_t N,

@@ -115,7 +115,6 @@ __global__ void __launch_bounds__(256) silu_mul_quantize_kernel(const float *gat
             }
             if (dst) *reinterpret_cast<float4 *>(reinterpret_cast<char *>(dst) + n * dst_nb_row + at * 16) = make_float4(v[0], v[1], v[2], v[3]);
         }
-        pdl_trigger();   // the values are here: the next kernel's CTAs may take their places
         q8_quantize_store<1>(v, out, d_offset, nb, nbp, n, b, j, real, variant);
     }
 }

@@ -17,6 +17,8 @@ template <int LAYOUT>
 __global__ void __launch_bounds__(256) quantize_q8_0_kernel(const float *__restrict__ x, int64_t x_nb_row, int64_t K,
                                                            int64_t N, int64_t nb, int64_t nbp,
                                                            uint8_t *__restrict__ out, size_t d_offset, int variant, int early, int chunk_nt) {
+    // (No trigger between the loads and the stores: with one here and in silu_mul_quantize_kernel the 8B decode step of 64
+    // sequences, back to back, takes 6.91 ms instead of 6.41; with the one here only 6.48, with the other only 6.85.)
     pdl_prologue(early != 0);
     const int64_t n = blockIdx.x;   // row
     // 4 elements per thread; whole groups of 8 lanes (a block) leave together.  (A row per x: no 64-bit division per thread)
@@ -34,7 +36,6 @@ __global__ void __launch_bounds__(256) quantize_q8_0_kernel(const float *__restr
                 v[0] = row[0]; v[1] = row[1]; v[2] = row[2]; v[3] = row[3];
             }
         }
-        pdl_trigger();   // the values are here: the next kernel's CTAs may take their places
         q8_quantize_store<LAYOUT>(v, out, d_offset, nb, nbp, n, b, j, real, variant, chunk_nt);
     }
 }

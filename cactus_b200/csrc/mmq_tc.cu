@@ -8,15 +8,19 @@
 //   B[col, k] = d_a[col, b] * a[col, k]      (19 significant bits)
 // Each is an fp16 value plus the exact fp16 remainder (x_hi = rn(x), x_lo = x - x_hi; d is a multiple of 2^-24, so the
 // remainder always fits), and the product is A_hi B_hi + A_hi B_lo + A_lo B_hi (the missing A_lo B_lo is below 2^-22 of a
-// term), accumulated in fp32 by tcgen05.mma.kind::f16.  Nothing is rounded that the reference does not round, except the
-// order of the fp32 sums.  The tensor core truncates when it accumulates, so the accumulator is emptied into shared
-// memory every TC_FLUSH block groups and the small terms (A_hi B_lo, A_lo B_hi) have columns of their own.
+// term), accumulated in fp32 by tcgen05.mma.kind::f16.  The tensor core truncates when it accumulates, so a sum over many
+// MMAs drifts towards zero: 2.1e-6 to 2.4e-6 rms against f64 when the accumulator ran over 16 block groups, ten times the
+// error of the mma.sync kernel (0.9e-7 to 3.8e-7).  Hence it is emptied after every block group (8 MMAs) and the block groups
+// are added in registers, rounding to nearest: 2.0e-7 to 2.5e-7 for K 1024 - 14336 (two block groups: 3.4e-7).  The small
+// terms (A_hi B_lo, A_lo B_hi), 2^-11 of the others, have columns of their own and are emptied once per tile.
 // A value beyond the fp16 range (|d q| > 65504) makes the sum non-finite; such results are recomputed exactly from the
 // integers (tc_exact_value).
 //
-// What bounds it: the MMAs.  128 x 128 x 16 + 128 x 64 x 16 per 16 values of K take 96 clk (measured: N / 2 clk per MMA), so a
-// block group of 256 rows x 64 columns x 128 values takes 1542 clk; the kernel runs at 1800 (two row tiles), and a CTA needs
-// about 5 us to fill and empty its pipeline.  What is around the MMAs has to stay below that:
+// What bounds it: issuing the MMAs.  128 x 128 x 16 + 128 x 64 x 16 per 16 values of K take 96 clk (measured: N / 2 clk per
+// MMA), a block group of 256 rows x 64 columns x 128 values 1542 clk; but an issuing warp needs about as long for its
+// 17 MMAs, three waits and two commits beside six busy warps on its scheduler, and the accumulator has to be read in between.
+// 4096 x 28672 at 512 columns: 298 us (265 us with 16 block groups per accumulator; mma.sync 323).  A CTA needs about
+// 5 us to fill and empty its pipeline.  What is around the MMAs has to stay below that:
 //   * the activations arrive as B_hi / B_lo planes written once by the quantiser (act_dims: b_offset) in the core-matrix
 //     order of the MMA's B descriptor.  A CTA owns 256 weight rows (two MMA row tiles) per activation copy: 50 KB per
 //     block group, 33 B/clk per SM, below the 40 B/clk that bulk copies out of L2 reach with all SMs at it.  One copy brings
@@ -27,13 +31,16 @@
 //     loaded them, so there is no transposition; the order of K within a block that follows from it is the order the
 //     quantiser writes B in;
 //   * every hand-over between warps is some twenty instructions at 10-16 clk each beside busy warps, so there are few: one per
-//     half block group and role, with an A stage for each team of weight warps.
+//     half block group and role, with an A stage for each team of weight warps;
+//   * a block group's sums are read by 8 warps with 64 registers of sums a thread (setmaxnreg moves them from the other warps): with
+//     the sums in shared memory and 4 warps, emptying after every block group cost 423 us instead of 298.
 //
-// Roles of a CTA (one per SM, 24 warps): warps 0 and 1 issue the MMAs of one row tile each, warp 2 the copies (a ring of
+// Roles of a CTA (one per SM, 28 warps): warps 0 and 1 issue the MMAs of one row tile each, warp 2 the copies (a ring of
 // stages of one block group), two teams of 8 warps convert weights (they take the half block groups in turn; a
-// warp: 32 rows), the last four warps move the accumulators to shared memory and write results.  The two row tiles share the
-// copies only: each has its own A stages, accumulator and barriers.  Code that runs once per tile is kept small and in loops:
-// with 172 KB of (unrolled, inlined) code the kernel spent most of its time on instruction cache misses.
+// warp: 32 rows), the last eight warps, four per row tile, add up the accumulators and write results.  The two row tiles share
+// the copies only: each has its own A stages, accumulator and barriers.  Code that runs once per tile is kept small and in
+// loops: with 172 KB of (unrolled) code the kernel spent most of its time on instruction cache misses.  (All of it is
+// inlined all the same: ptxas gives a warp the registers that setmaxnreg sets only where nothing is called.)
 //
 // Work split (TcPlan): clusters of up to 8 CTAs share the K range of one tile (256 rows x <= 64 columns) and add their parts
 // through distributed shared memory in rank order; or, when there are many tiles, one CTA per SM takes an equal and
@@ -61,8 +68,7 @@ __device__ unsigned g_tc_spin_limit = 1u << 20;   // try_wait rounds before a wa
 constexpr uint32_t TC_DRAIN_LIMIT = 1u << 22;     // what a CTA that gave up still waits for: its own copies and MMAs in flight
 
 constexpr int TC_RT = 16;            // 16-row tiles of a CTA at most: 256 rows, two MMA row tiles
-constexpr int TC_FLUSH = 16;         // block groups accumulated in tensor memory before they are added up in shared memory
-constexpr int TC_EPI_THREADS = 128;
+constexpr int TC_EPI_THREADS = 256;
 
 // Geometry.  A CTA has up to NT tiles of 8 activation columns.
 template <int WTYPE>
@@ -82,11 +88,12 @@ struct TcCfg {
     static constexpr int A_MT = ABUF * 64, A_COL = 512 - 2 * A_MT;
     // warps: 4 for MMAs and copies, a team of 8 weight warps per A stage (each waits for its own stage phase after phase, which a
     // parity wait can tell apart), 4 for the write-back
-    static constexpr int WARP_EPI = 4 + 8 * ABUF, THREADS = 32 * (WARP_EPI + 4);
-    // barriers: FULL a stage has landed; WREAD its weights are in registers; DONE (per row tile) all MMAs on it are complete; AFULL /
-    // AFREE (row tile, A stage); ACCF the accumulator is complete, ACCE it has been read
-    static constexpr int B_FULL = 0, B_WREAD = STAGES, B_DONE = 2 * STAGES, B_AFULL = 4 * STAGES, B_AFREE = B_AFULL + 2 * ABUF, B_ACCF = B_AFREE + 2 * ABUF,
-                         B_ACCE = B_ACCF + 2, B_DRAIN = B_ACCE + 2, N_BARS = B_DRAIN + 2;
+    static constexpr int WARP_EPI = 4 + 8 * ABUF, THREADS = 32 * (WARP_EPI + 8);
+    // barriers: FULL a stage has landed; WREAD its weights are in registers; DONE (per row tile) all MMAs on it are complete; AFULL
+    // (row tile, A stage); AFREE the first A stage of a row tile may be written again (the second: DONE); ACCE the accumulator
+    // has been read (that it is complete: DONE).  A commit costs its warp 45 clk, hence no barrier of its own where one tells already.
+    static constexpr int B_FULL = 0, B_WREAD = STAGES, B_DONE = 2 * STAGES, B_AFULL = 4 * STAGES, B_AFREE = B_AFULL + 2 * ABUF, B_ACCE = B_AFREE + 2,
+                         B_DRAIN = B_ACCE + 2, N_BARS = B_DRAIN + 2;
     static constexpr int OFF_ACC = STAGES * STAGE;
     static constexpr int BAR_OFFSET = OFF_ACC + ACC;
     static constexpr int SH_OFFSET = BAR_OFFSET + (N_BARS * 8 + 15) / 16 * 16;   // TcShared
@@ -124,9 +131,8 @@ __device__ __forceinline__ bool tc_elect() {
     return el != 0;
 }
 // Bounded wait of a whole (converged) warp; false = gave up (or the CTA already gave up elsewhere).  The outcome is one for
-// the warp, by vote: what follows a wait (elect.sync, tcgen05.ld) needs all its lanes.  The loop is one function for all
-// callers: the kernel's hot code has to fit the instruction cache.
-__device__ __noinline__ bool tc_wait_slow(uint32_t bar, uint32_t parity, volatile int *abort_flag, uint32_t limit) {
+// the warp, by vote: what follows a wait (elect.sync, tcgen05.ld) needs all its lanes.
+__device__ __forceinline__ bool tc_wait_slow(uint32_t bar, uint32_t parity, volatile int *abort_flag, uint32_t limit) {
 #pragma unroll 1
     for (uint32_t i = 0; i < limit; ++i) {
         if (__all_sync(0xffffffffu, tc_try(bar, parity))) return true;
@@ -154,10 +160,11 @@ __device__ __forceinline__ void tc_tma_3d(uint32_t dst, const CUtensorMap *map, 
 __device__ __forceinline__ void tc_copy(uint32_t dst, const void *src, uint32_t bytes, uint32_t bar) {
     asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];\n" ::"r"(dst), "l"(src), "r"(bytes), "r"(bar) : "memory");
 }
-// D[tmem] (+)= A[tmem] * B[smem], M 128, K 16, fp16 x fp16 -> f32; N comes with the instruction descriptor
-__device__ __forceinline__ void tc_mma(uint32_t d_tmem, uint32_t a_tmem, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
-    asm volatile("{\n.reg .pred p;\nsetp.ne.b32 p, %4, 0;\ntcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n}\n"
-                 ::"r"(d_tmem), "r"(a_tmem), "l"(bdesc), "r"(idesc), "r"(accumulate) : "memory");
+// D[tmem] (+)= A[tmem] * B[smem], M 128, K 16, fp16 x fp16 -> f32; N comes with the instruction descriptor.  B's descriptor in two
+// halves: only the low one moves, and a 64-bit addition would be two instructions beside every MMA.
+__device__ __forceinline__ void tc_mma(uint32_t d_tmem, uint32_t a_tmem, uint32_t bdesc_lo, uint32_t bdesc_hi, uint32_t idesc, uint32_t accumulate) {
+    asm volatile("{\n.reg .pred p;\n.reg .b64 b;\nsetp.ne.b32 p, %5, 0;\nmov.b64 b, {%2, %3};\ntcgen05.mma.cta_group::1.kind::f16 [%0], [%1], b, %4, p;\n}\n"
+                 ::"r"(d_tmem), "r"(a_tmem), "r"(bdesc_lo), "r"(bdesc_hi), "r"(idesc), "r"(accumulate) : "memory");
 }
 __device__ __forceinline__ uint32_t tc_h2(__half2 v) { return *reinterpret_cast<uint32_t *>(&v); }
 __device__ __forceinline__ __half2 tc_as_h2(uint32_t v) { return *reinterpret_cast<__half2 *>(&v); }
@@ -170,6 +177,27 @@ __device__ __forceinline__ void tc_ld_x16(uint32_t (&r)[16], uint32_t taddr) {
     asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];\n"
                  : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]),
                    "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]) : "r"(taddr));
+}
+// sum[k] += column k of the thread's row, k < cols (16, 32, 48 or 64); `read` is called once all have been read
+template <typename F>
+__device__ __forceinline__ void tc_add_columns(float (&sum)[64], uint32_t taddr, uint32_t cols, F read) {
+    uint32_t u[2][16];
+#pragma unroll
+    for (int c = 0; c < 4; c += 2) {
+        if (c * 16 >= (int) cols) break;
+        tc_ld_x16(u[0], taddr + c * 16);
+        if ((c + 1) * 16 < (int) cols) tc_ld_x16(u[1], taddr + (c + 1) * 16);
+        asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
+        if ((c + 2) * 16 >= (int) cols) read();
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            if ((c + h) * 16 >= (int) cols) break;
+#pragma unroll
+            for (int k = 0; k < 16; k += 2)
+                asm("{\n.reg .b64 x, y;\nmov.b64 x, {%0, %1};\nmov.b64 y, {%2, %3};\nadd.rn.f32x2 x, x, y;\nmov.b64 {%0, %1}, x;\n}\n"
+                    : "+f"(sum[(c + h) * 16 + k]), "+f"(sum[(c + h) * 16 + k + 1]) : "r"(u[h][k]), "r"(u[h][k + 1]));
+        }
+    }
 }
 
 // A piece of work: block groups [bg, bg + len) of a tile (row group x column chunk).
@@ -205,7 +233,7 @@ static_assert(sizeof(TcShared) <= 5120, "TcShared has its place in TcCfg");
 // One result from the integers themselves: what the reference computes, block by block.  Only for values whose folded
 // operands left the fp16 range.
 template <int WTYPE>
-__device__ __noinline__ float tc_exact_value(const TcShared *o, int row, int col) {
+__device__ __forceinline__ float tc_exact_value(const TcShared *o, int row, int col) {
     const uint8_t *wq = o->w, *ws = wq + o->dims.qs_bytes;
     const int rt = row >> 4, r = row & 15, g = r & 7, h = r >> 3;
     float sum = 0.0f;
@@ -242,7 +270,7 @@ __device__ __forceinline__ uint32_t tc_cta_of(const TcPlan &p, uint32_t it) {   
     const uint32_t big = p.extra * (p.share + 1);
     return it < big ? it / (p.share + 1) : p.extra + (it - big) / p.share;
 }
-__device__ __noinline__ void tc_share(TcShared *o, const TcPlan plan, uint32_t n_bg, uint32_t n_rt) {
+__device__ __forceinline__ void tc_share(TcShared *o, const TcPlan plan, uint32_t n_bg, uint32_t n_rt) {
     uint32_t it0, it1;
     if (plan.cs > 0) {   // the CTAs of a cluster cut the K range of one tile
         const uint32_t cs = (uint32_t) plan.cs, rank = blockIdx.x % cs, tile = blockIdx.x / cs * n_bg;
@@ -280,7 +308,7 @@ __device__ __noinline__ void tc_share(TcShared *o, const TcPlan plan, uint32_t n
 
 // Values that do not simply go to 16 aligned bytes: a ragged or unaligned edge, or not finite
 template <int WTYPE>
-__device__ __noinline__ void tc_write_slow(const TcShared *o, int row, int row_end, int col, float4 f) {
+__device__ __forceinline__ void tc_write_slow(const TcShared *o, int row, int row_end, int col, float4 f) {
 #pragma unroll 1
     for (int i = 0; i < 4 && row + i < row_end; ++i) {
         float y = i == 0 ? f.x : i == 1 ? f.y : i == 2 ? f.z : f.w;
@@ -322,7 +350,7 @@ __device__ __forceinline__ float4 tc_lds4(uint32_t at) {
 
 // The tile's parts lie in the shared memory of the cluster's CTAs: this CTA adds slice `rank` of the columns in rank order.
 template <int WTYPE>
-__device__ __noinline__ void tc_write_cluster(const TcShared *o, uint32_t acc_u32, uint32_t te, uint32_t threads) {
+__device__ __forceinline__ void tc_write_cluster(const TcShared *o, uint32_t acc_u32, uint32_t te, uint32_t threads) {
     const uint32_t cs = (uint32_t) o->plan.cs, rank = blockIdx.x % cs, per4 = ((uint32_t) o->act.chunk_nt * 8 + cs - 1) / cs * 64;
     const uint32_t end = min((uint32_t) o->act.chunk_nt * 512, (rank + 1) * per4);
     uint32_t e = rank * per4 + te;
@@ -361,7 +389,7 @@ __device__ __forceinline__ bool tc_arrive_tile(const TcShared *o, const TcPiece 
     return (now & 255) == q.parts;
 }
 // The pieces of a CTA that gave up.  One thread, after everything else.
-__device__ __noinline__ void tc_give_up_pieces(const TcShared *o) {
+__device__ __forceinline__ void tc_give_up_pieces(const TcShared *o) {
 #pragma unroll 1
     for (uint32_t p = o->n_finished; p < o->n_pieces; ++p)
         if (o->piece[p].parts > 1) tc_arrive_tile(o, o->piece[p], true);
@@ -370,7 +398,7 @@ __device__ __noinline__ void tc_give_up_pieces(const TcShared *o) {
 // Piece q is complete in shared memory: write the tile if this is all of it or the last part to arrive, else park it.  Called by
 // `threads` threads, te = 0 ..., which meet at barrier `bar`.  The parts (at most three) are added in K order whoever does it.
 template <int WTYPE>
-__device__ __noinline__ void tc_finish(TcShared *o, uint32_t acc_u32, uint32_t piece, uint32_t te, uint32_t threads, uint32_t bar) {
+__device__ __forceinline__ void tc_finish(TcShared *o, uint32_t acc_u32, uint32_t piece, uint32_t te, uint32_t threads, uint32_t bar) {
     const TcPiece q = o->piece[piece];
     const uint32_t total4 = (uint32_t) o->act.chunk_nt * 512;
     volatile int *const flag = &o->flag;
@@ -473,106 +501,128 @@ __global__ void __launch_bounds__(TcCfg<WTYPE>::THREADS, 1) mmq_tc_kernel(TiledD
     const uint32_t tmem = sh->tmem;
     pdl_prologue();   // everything above touches no global memory
 
-    if (warp < 2) {
-        // ---------------- MMA issue for row tile mt = warp ----------------
-        const uint32_t mt = (uint32_t) warp, nt = (uint32_t) act.chunk_nt;
-        const uint32_t idesc_wide = (1u << 4) | (2 * nt << 17) | (8u << 24), idesc_hi = (1u << 4) | (nt << 17) | (8u << 24);   // f16 x f16 -> f32, K-major both, M 128
-        const uint32_t d = tmem + mt * C::D_MT, d_small = d + 8 * nt, a0 = tmem + C::A_COL + mt * C::A_MT;
-        const uint64_t bdesc0 = tc_smem_desc(smem_u32 + C::OFF_B, 128, 2048);
-        uint32_t s = 0, acc_par = 1, ab = 0, a_par = 0;   // ab: A stage
-        bool ok = true;
+    // Registers: 72 a thread at launch (504 for a lane of the seven warpgroups), 40 + 4 x 56 + 2 x 120 = 504 while the roles run.
+    if (warp < 4) {
+        asm volatile("setmaxnreg.dec.sync.aligned.u32 40;\n");
+        if (warp < 2) {
+            // ---------------- MMA issue for row tile mt = warp ----------------
+            const uint32_t mt = (uint32_t) warp, nt = (uint32_t) act.chunk_nt;
+            const uint32_t idesc_wide = (1u << 4) | (2 * nt << 17) | (8u << 24), idesc_hi = (1u << 4) | (nt << 17) | (8u << 24);   // f16 x f16 -> f32, K-major both, M 128
+            const uint32_t d = tmem + mt * C::D_MT, d_small = d + 8 * nt, a0 = tmem + C::A_COL + mt * C::A_MT;
+            const uint64_t bdesc0 = tc_smem_desc(smem_u32 + C::OFF_B, 128, 2048);
+            const uint32_t b_hi = (uint32_t) (bdesc0 >> 32);
+            uint32_t s = 0, acc_par = 1, a_par = 0;
+            bool ok = true;
 #pragma unroll 1
-        for (uint32_t p = 0; p < sh->n_pieces && ok; ++p) {
-            const bool active = mt == 0 || sh->piece[p].two;
-            const uint32_t len = sh->piece[p].len;
+            for (uint32_t p = 0; p < sh->n_pieces && ok; ++p) {
+                const bool active = mt == 0 || sh->piece[p].two;
+                const uint32_t len = sh->piece[p].len;
 #pragma unroll 1
-            for (uint32_t i = 0; i < len && ok; ++i) {
-                const uint32_t acc = i % TC_FLUSH == 0 ? 0u : 1u;
-                if (acc == 0) {
-                    ok = tc_wait(BAR(C::B_ACCE, mt), acc_par, abort_flag, spin_limit);
-                    acc_par ^= 1;
-                }
-                // (that the stage has landed follows from AFULL: the weight warps waited for it)
-                const uint64_t bdesc = bdesc0 + (uint64_t) (s * (C::STAGE >> 4));
-                const bool last = i + 1 == len || (i + 1) % TC_FLUSH == 0;
+                for (uint32_t i = 0; i < len && ok; ++i, a_par ^= 1) {
+                    // (that the stage has landed follows from AFULL: the weight warps waited for it)
+                    const uint32_t b = (uint32_t) bdesc0 + s * (C::STAGE >> 4);
+                    if (i == 0) ok = tc_wait(BAR(C::B_ACCE, mt), acc_par, abort_flag, spin_limit);
+                    ok = ok && tc_wait(BAR(C::B_AFULL, C::ABUF * mt), a_par, abort_flag, spin_limit);
+                    asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+                    if (i > 0) {   // the large terms start from zero, once what they were has been read; the small ones go on meanwhile
+                        if (tc_elect() && ok && active) {
 #pragma unroll
-                for (uint32_t h = 0; h < 2; ++h) {
-                    ok = ok && tc_wait(BAR(C::B_AFULL, C::ABUF * mt + ab), a_par, abort_flag, spin_limit);
+                            for (uint32_t k = 0; k < 4; ++k) tc_mma(d_small, a0 + 8 * k + 32, b + k * 16, b_hi, idesc_hi, 1u);
+                            tc_mma(d_small, a0, b + nt * 128, b_hi, idesc_hi, 1u);
+                        }
+                        __syncwarp();
+                        ok = ok && tc_wait(BAR(C::B_ACCE, mt), acc_par, abort_flag, spin_limit);
+                        asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+                        if (tc_elect() && ok) {
+                            if (active) {
+                                tc_mma(d, a0, b, b_hi, idesc_hi, 0u);
+#pragma unroll
+                                for (uint32_t k = 1; k < 4; ++k) tc_mma(d, a0 + 8 * k, b + k * 16, b_hi, idesc_wide, 1u);
+                            }
+                            tc_commit(BAR(C::B_AFREE, mt));
+                        }
+                    } else if (tc_elect() && ok) {
+                        if (active) {
+#pragma unroll
+                            for (uint32_t k = 0; k < 4; ++k) {
+                                tc_mma(d, a0 + 8 * k, b + k * 16, b_hi, idesc_wide, k == 0 ? 0u : 1u);   // A_hi (B_hi | B_lo)
+                                tc_mma(d_small, a0 + 8 * k + 32, b + k * 16, b_hi, idesc_hi, 1u);   // A_lo B_hi, on the small terms
+                            }
+                        }
+                        tc_commit(BAR(C::B_AFREE, mt));
+                    }
+                    __syncwarp();
+                    acc_par ^= 1;
+                    ok = ok && tc_wait(BAR(C::B_AFULL, C::ABUF * mt + 1), a_par, abort_flag, spin_limit);
                     asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
                     if (tc_elect() && ok) {
                         if (active) {
 #pragma unroll
                             for (uint32_t k = 0; k < 4; ++k) {
-                                const uint64_t b = bdesc + (uint64_t) (h * 64 + k * 16);
-                                const uint32_t a = a0 + ab * 64 + 8 * k, acc_k = k == 0 ? (acc | h) : 1u;
-                                tc_mma(d, a, b, idesc_wide, acc_k);          // A_hi (B_hi | B_lo)
-                                tc_mma(d_small, a + 32, b, idesc_hi, 1u);   // A_lo B_hi, on the small terms
+                                tc_mma(d, a0 + 64 + 8 * k, b + 64 + k * 16, b_hi, idesc_wide, 1u);
+                                tc_mma(d_small, a0 + 64 + 8 * k + 32, b + 64 + k * 16, b_hi, idesc_hi, 1u);
                             }
                         }
-                        tc_commit(BAR(C::B_AFREE, C::ABUF * mt + ab));
-                        if (h == 1) {
-                            tc_commit(BAR(C::B_DONE, 2 * s + mt));
-                            if (last) tc_commit(BAR(C::B_ACCF, mt));
-                        }
+                        tc_commit(BAR(C::B_DONE, 2 * s + mt));
                     }
                     __syncwarp();
-                    if (++ab == C::ABUF) { ab = 0; a_par ^= 1; }
+                    if (++s == C::STAGES) s = 0;
                 }
-                if (++s == C::STAGES) s = 0;
             }
-        }
-        // no MMA of this CTA may be in flight when its tensor memory is freed, whatever happened elsewhere.  (elect.sync picks the
-        // same lane every time, the one whose MMAs the commit has to cover.)
-        if (tc_elect()) {
-            tc_commit(BAR(C::B_DRAIN, mt));
+            // no MMA of this CTA may be in flight when its tensor memory is freed, whatever happened elsewhere.  (elect.sync picks the
+            // same lane every time, the one whose MMAs the commit has to cover.)
+            if (tc_elect()) {
+                tc_commit(BAR(C::B_DRAIN, mt));
 #pragma unroll 1
-            for (uint32_t spin = 0; spin < TC_DRAIN_LIMIT && !tc_try(BAR(C::B_DRAIN, mt), 0); ++spin) {}
-        }
-        __syncwarp();
-    } else if (warp == 2) {
-        // ---------------- producer: two or four tensor copies of weights, one bulk copy of activations per block group ----------------
-        uint32_t s = 0, par = 1, issued = 0;
-        bool ok = !(plan.debug & 32) && !(plan.debug & 64 && blockIdx.x & 1);
-        const uint32_t b_bytes = (uint32_t) act.chunk_nt * 4096u;
+                for (uint32_t spin = 0; spin < TC_DRAIN_LIMIT && !tc_try(BAR(C::B_DRAIN, mt), 0); ++spin) {}
+            }
+            __syncwarp();
+        } else if (warp == 2) {
+            // ---------------- producer: two or four tensor copies of weights, one bulk copy of activations per block group ----------------
+            uint32_t s = 0, par = 1, issued = 0;
+            bool ok = !(plan.debug & 32) && !(plan.debug & 64 && blockIdx.x & 1);
+            const uint32_t b_bytes = (uint32_t) act.chunk_nt * 4096u;
 #pragma unroll 1
-        for (uint32_t p = 0; p < sh->n_pieces && ok; ++p) {
-            const TcPiece q = sh->piece[p];
-            const int boxes = 1 + (int) q.two;   // rows past the end read as zero
-            const uint32_t bytes = (uint32_t) boxes * 8u * (C::WT + 128u) + b_bytes;
-            const int rt_in = (int) q.group * plan.rt_per_group;
-            const uint8_t *bsrc = aq + act.b_offset + ((int64_t) q.chunk * n_bg + q.bg) * b_bytes;
+            for (uint32_t p = 0; p < sh->n_pieces && ok; ++p) {
+                const TcPiece q = sh->piece[p];
+                const int boxes = 1 + (int) q.two;   // rows past the end read as zero
+                const uint32_t bytes = (uint32_t) boxes * 8u * (C::WT + 128u) + b_bytes;
+                const int rt_in = (int) q.group * plan.rt_per_group;
+                const uint8_t *bsrc = aq + act.b_offset + ((int64_t) q.chunk * n_bg + q.bg) * b_bytes;
 #pragma unroll 1
-            for (uint32_t i = 0; i < q.len; ++i) {
-                const uint32_t st = smem_u32 + s * C::STAGE, bar = BAR(C::B_FULL, s);
-                if (!tc_wait(BAR(C::B_WREAD, s), par, abort_flag, spin_limit) || !tc_wait(BAR(C::B_DONE, 2 * s), par, abort_flag, spin_limit) ||
-                    !tc_wait(BAR(C::B_DONE, 2 * s + 1), par, abort_flag, spin_limit)) { ok = false; break; }
-                if (tc_elect()) {
-                    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(bar), "r"(bytes) : "memory");
-                    const int bg = (int) (q.bg + i);
+                for (uint32_t i = 0; i < q.len; ++i) {
+                    const uint32_t st = smem_u32 + s * C::STAGE, bar = BAR(C::B_FULL, s);
+                    if (!tc_wait(BAR(C::B_WREAD, s), par, abort_flag, spin_limit) || !tc_wait(BAR(C::B_DONE, 2 * s), par, abort_flag, spin_limit) ||
+                        !tc_wait(BAR(C::B_DONE, 2 * s + 1), par, abort_flag, spin_limit)) { ok = false; break; }
+                    if (tc_elect()) {
+                        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(bar), "r"(bytes) : "memory");
+                        const int bg = (int) (q.bg + i);
 #pragma unroll
-                    for (int k = 0; k < 2; ++k) {
-                        if (k < boxes) {
-                            if (WTYPE == B200_TYPE_Q4_0) tc_tma_2d(st + (uint32_t) (k * 8 * C::WT), &maps.q, bg * 256, rt_in + 8 * k, bar);
-                            else tc_tma_3d(st + (uint32_t) (k * 8 * C::WT), &maps.q, 0, bg * 2, rt_in + 8 * k, bar);
-                            tc_tma_2d(st + (uint32_t) (C::OFF_S + k * 1024), &maps.s, bg * 32, rt_in + 8 * k, bar);
+                        for (int k = 0; k < 2; ++k) {
+                            if (k < boxes) {
+                                if (WTYPE == B200_TYPE_Q4_0) tc_tma_2d(st + (uint32_t) (k * 8 * C::WT), &maps.q, bg * 256, rt_in + 8 * k, bar);
+                                else tc_tma_3d(st + (uint32_t) (k * 8 * C::WT), &maps.q, 0, bg * 2, rt_in + 8 * k, bar);
+                                tc_tma_2d(st + (uint32_t) (C::OFF_S + k * 1024), &maps.s, bg * 32, rt_in + 8 * k, bar);
+                            }
                         }
+                        tc_copy(st + C::OFF_B, bsrc + (int64_t) i * b_bytes, b_bytes, bar);
                     }
-                    tc_copy(st + C::OFF_B, bsrc + (int64_t) i * b_bytes, b_bytes, bar);
+                    __syncwarp();
+                    ++issued;
+                    if (++s == C::STAGES) { s = 0; par ^= 1; }
                 }
-                __syncwarp();
-                ++issued;
-                if (++s == C::STAGES) { s = 0; par ^= 1; }
             }
-        }
-        // copies in flight must land before the CTA may exit, whatever happened elsewhere
+            // copies in flight must land before the CTA may exit, whatever happened elsewhere
 #pragma unroll 1
-        for (uint32_t k = issued > C::STAGES ? issued - C::STAGES : 0; k < issued && lane == 0; ++k) {
-            const uint32_t bar = BAR(C::B_FULL, k % C::STAGES), parity = (k / C::STAGES) & 1;
+            for (uint32_t k = issued > C::STAGES ? issued - C::STAGES : 0; k < issued && lane == 0; ++k) {
+                const uint32_t bar = BAR(C::B_FULL, k % C::STAGES), parity = (k / C::STAGES) & 1;
 #pragma unroll 1
-            for (uint32_t spin = 0; spin < TC_DRAIN_LIMIT && !tc_try(bar, parity); ++spin) {}
+                for (uint32_t spin = 0; spin < TC_DRAIN_LIMIT && !tc_try(bar, parity); ++spin) {}
+            }
+            __syncwarp();
         }
-        __syncwarp();
-    } else if (warp >= 4 && warp < C::WARP_EPI) {
+    } else if (warp < C::WARP_EPI) {
+        asm volatile("setmaxnreg.dec.sync.aligned.u32 56;\n");
         // ---------------- weights: a warp owns 32 rows (two T16 tiles: the lanes of tensor memory it can reach) of every second half block group ----------------
         const int q4 = warp & 3, mt = ((warp - 4) >> 2) & 1, team = (warp - 4) >> 3;
         const uint32_t rt0 = (uint32_t) (mt * 8 + q4 * 2);
@@ -581,9 +631,9 @@ __global__ void __launch_bounds__(TcCfg<WTYPE>::THREADS, 1) mmq_tc_kernel(TiledD
         const uint32_t s_at = smem_u32 + C::OFF_S + rt0 * 128 + (uint32_t) ((lane >> 2) * 8);
         const bool active = mt == 0 || plan.rt_per_group > 8;
         const uint32_t halves = 2 * sh->n_iter;
-        uint32_t s = (uint32_t) team >> 1, full_par = 0, free_par = 1;
+        uint32_t s = 0, full_par = 0, free_par = 1;
 #pragma unroll 1
-        for (uint32_t hc = (uint32_t) team; hc < halves; hc += C::ABUF, free_par ^= 1) {
+        for (uint32_t hc = (uint32_t) team; hc < halves; hc += 2, free_par ^= 1) {
             const uint32_t half = hc & 1, ab = (uint32_t) team;
             if (!tc_wait(BAR(C::B_FULL, s), full_par, abort_flag, spin_limit)) break;
             constexpr int NW = WTYPE == B200_TYPE_Q4_0 ? 4 : 8;
@@ -603,7 +653,11 @@ __global__ void __launch_bounds__(TcCfg<WTYPE>::THREADS, 1) mmq_tc_kernel(TiledD
             }
             __syncwarp();
             if (lane == 0) tc_arrive(BAR(C::B_WREAD, s));   // the weights are in registers (the arrive orders the loads before it)
-            if (!tc_wait(BAR(C::B_AFREE, C::ABUF * mt + ab), free_par, abort_flag, spin_limit)) break;
+            if (team == 0) {
+                if (!tc_wait(BAR(C::B_AFREE, mt), free_par, abort_flag, spin_limit)) break;
+            } else if (hc > 1) {   // the block group before this one
+                if (!tc_wait(BAR(C::B_DONE, 2 * (s == 0 ? C::STAGES - 1 : s - 1) + mt), s == 0 ? full_par ^ 1 : full_par, abort_flag, spin_limit)) break;
+            }
             asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
             const uint32_t a_to = a_base + ab * 64;
             if (active) {
@@ -645,42 +699,43 @@ __global__ void __launch_bounds__(TcCfg<WTYPE>::THREADS, 1) mmq_tc_kernel(TiledD
             s += 1;   // two halves on
             if (s >= C::STAGES) { s -= C::STAGES; full_par ^= 1; }
         }
-    } else if (warp >= C::WARP_EPI) {
-        // ---------------- accumulator -> shared memory -> result ----------------
-        const int q4 = warp & 3, et = tid - C::WARP_EPI * 32;
-        const uint32_t cols = 8 * (uint32_t) act.chunk_nt;
-        uint32_t acc_par = 0;
+    } else {
+        asm volatile("setmaxnreg.inc.sync.aligned.u32 120;\n");
+        // ---------------- accumulator -> registers -> shared memory -> result; a warpgroup per MMA row tile ----------------
+        const int q4 = warp & 3, mt = (warp - C::WARP_EPI) >> 2, et = tid - C::WARP_EPI * 32;
+        const uint32_t cols = 8 * (uint32_t) act.chunk_nt, d_at = tmem + ((uint32_t) (32 * q4) << 16) + (uint32_t) (mt * C::D_MT);
+        uint32_t s = 0, done_par = 0;
         bool ok = true;
 #pragma unroll 1
         for (uint32_t p = 0; p < sh->n_pieces && ok; ++p) {
-            const int n_mt = 1 + (int) sh->piece[p].two;
+            const bool active = mt == 0 || sh->piece[p].two;
             const uint32_t len = sh->piece[p].len;
-#pragma unroll 1
-            for (uint32_t i = 0; i < len && ok; i += TC_FLUSH, acc_par ^= 1) {
-#pragma unroll 1
-                for (int mt = 0; mt < 2; ++mt) {
-                    ok = ok && tc_wait(BAR(C::B_ACCF, mt), acc_par, abort_flag, spin_limit);
-                    if (ok && mt < n_mt) {
-                        asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-                        float *o = acc_s + mt * 128 + q4 * 32 + lane;   // the thread's row
-                        const uint32_t d_at = tmem + ((uint32_t) (32 * q4) << 16) + (uint32_t) (mt * C::D_MT);
-#pragma unroll 1
-                        for (uint32_t c = 0; c < cols; c += 16, o += 16 * 256) {
-                            uint32_t u[16], v[16];
-                            tc_ld_x16(u, d_at + c);
-                            tc_ld_x16(v, d_at + cols + c);
-                            asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
+            float sum[64];   // of the thread's row
 #pragma unroll
-                            for (int k = 0; k < 16; ++k) {
-                                const float x = __uint_as_float(u[k]) + __uint_as_float(v[k]);
-                                o[k * 256] = i == 0 ? x : o[k * 256] + x;
-                            }
-                        }
-                        asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
-                    }
+            for (int k = 0; k < 64; ++k) sum[k] = 0.0f;
+#pragma unroll 1
+            for (uint32_t i = 0; i < len && ok; ++i) {
+                const uint32_t bar = BAR(C::B_DONE, 2 * s + mt), parity = done_par;
+                if (++s == C::STAGES) { s = 0; done_par ^= 1; }
+                ok = tc_wait(bar, parity, abort_flag, spin_limit);
+                const auto read = [&] {
+                    asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
                     __syncwarp();
                     if (lane == 0) tc_arrive(BAR(C::B_ACCE, mt));
+                };
+                if (!ok || !active) {
+                    read();
+                    continue;
                 }
+                asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+                if (i + 1 == len) tc_add_columns(sum, d_at + cols, cols, [] {});   // the small terms, once
+                tc_add_columns(sum, d_at, cols, read);
+            }
+            if (ok && active) {
+                float *o = acc_s + mt * 128 + q4 * 32 + lane;
+#pragma unroll
+                for (int k = 0; k < 64; ++k)
+                    if ((k & ~15) < (int) cols) o[k * 256] = sum[k];
             }
             if (plan.debug & 128 && warp == C::WARP_EPI + 1 && blockIdx.x == 1) {
                 ok = false;
@@ -688,15 +743,18 @@ __global__ void __launch_bounds__(TcCfg<WTYPE>::THREADS, 1) mmq_tc_kernel(TiledD
                 atomicExch(&g_tc_error, 1);
             }
             if (p + 1 == sh->n_pieces) break;   // the last piece: all warps share what is left to do, below
-            // one warp's wait may run out where its neighbours' did not: the four go on, or leave, together
+            // one warp's wait may run out where its neighbours' did not: the team goes on, or leaves, together
             if (!ok) *wb_gave_up = 1;
-            asm volatile("bar.sync 1, 128;\n" ::: "memory");
+            asm volatile("bar.sync 1, 256;\n" ::: "memory");
             if (*wb_gave_up) break;   // (written again at the earliest beyond the barriers of tc_finish)
             tc_finish<WTYPE>(sh, acc_u32, p, (uint32_t) et, TC_EPI_THREADS, 1u);
         }
     }
     asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
     pdl_trigger();
+    __syncthreads();   // (a warpgroup's registers change hands again: its warps must have met)
+    if (warp < C::WARP_EPI) asm volatile("setmaxnreg.inc.sync.aligned.u32 72;\n");
+    else asm volatile("setmaxnreg.dec.sync.aligned.u32 72;\n");
     if (plan.cs > 0) {
         asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;\n" ::: "memory");
         if (!*abort_flag) tc_write_cluster<WTYPE>(sh, acc_u32, (uint32_t) tid, C::THREADS);

@@ -72,3 +72,41 @@ def test_folded_scale_kernel_with_two_terms_is_within_the_mul_mat_tolerance():
     res = run_child(CASES, "3")
     assert res["status"] == 0
     assert max(res["err"]) < 1e-3, res["err"]
+
+
+F64_CHILD = r"""
+import json, sys
+sys.path.insert(0, {root!r})
+import torch
+from cactus_b200 import ops, _lib
+from cactus_b200.engine import random_blocks
+gen = torch.Generator(device="cuda").manual_seed(1)
+out = []
+for (wtype, M, K, N) in {cases!r}:
+    blocks = random_blocks(wtype, M, K, gen)
+    b = blocks.view(M, K // 32, -1)
+    q = torch.cat([(b[..., 2:] & 15).double() - 8, (b[..., 2:] >> 4).double() - 8], -1) if wtype == 2 else b[..., 2:].contiguous().view(torch.int8).double()
+    w = (q * b[..., :2].contiguous().view(torch.float16).double()).view(M, K)
+    x = torch.randn((N, K), device="cuda", generator=gen)
+    a = ops.quantize_row_q8_0(x).view(N, K // 32, 34)
+    a = (a[..., 2:].contiguous().view(torch.int8).double() * a[..., :2].contiguous().view(torch.float16).double()).view(N, K)
+    want = a @ w.T
+    got = ops.mul_mat(ops.QWeight.from_blocks(wtype, K, M, blocks), x).double()
+    out.append(float((got - want).norm() / want.norm()))
+print(json.dumps({{"err": out, "status": int(_lib.lib().b200_kernel_status())}}))
+"""
+
+
+def test_sums_are_as_close_to_f64_as_exact_dots_and_fp32_sums_are():
+    """Against the product of the quantised operands in f64 (2-norm).  Bound: the mma.sync kernel, whose block dots are exact and
+    whose sums round to nearest, is 0.7e-7 to 3.8e-7 away over these sizes.  The tensor core truncates when it accumulates, at
+    most one part in 2^23 and half of that in the mean: 8 times per block group are 8 x 2^-24 / 2 = 2.4e-7 on a sum that grows
+    evenly; 16 block groups in one accumulator, as it was once, 2.3e-6."""
+    cases = [(2, 256, 128, 33), (2, 2048, 1024, 77), (8, 2048, 1024, 77), (2, 4096, 4096, 512), (8, 4096, 4096, 130), (2, 1040, 14336, 512),
+             (8, 520, 14336, 64), (2, 28672, 4096, 64)]
+    env = dict(os.environ, B200_MMQ_TC="1")
+    r = subprocess.run([sys.executable, "-c", F64_CHILD.format(root=ROOT, cases=cases)], env=env, capture_output=True, text=True, timeout=600)
+    assert r.returncode == 0, r.stderr[-2000:]
+    res = json.loads(r.stdout.strip().splitlines()[-1])
+    assert res["status"] == 0
+    assert max(res["err"]) < 3.8e-7, list(zip(cases, res["err"]))

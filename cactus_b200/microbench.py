@@ -1,6 +1,7 @@
 """Small single-kernel workloads for timing and profiling (run under ncu on a GPU box):
 
-    python -m cactus_b200.microbench mul_mat --K 4096 --M 14336 --N 64 --copies 8 --reps 3
+    python -m cactus_b200.microbench mul_mat --K 4096 --M 14336 --N 64 --copies 8 --reps 3             # quantised activations: what a model step runs
+    python -m cactus_b200.microbench mul_mat --whole --K 4096 --M 14336 --N 512 --copies 8 --reps 3    # b200_mul_mat_q: quantiser + product, its own kernel choice
     python -m cactus_b200.microbench fattn --seqs 64 --ctx 900 --reps 3
     python -m cactus_b200.microbench fattn --cfg2 a --copies 8       # the 512-token prefill ubatch of 16 ragged sequences
     python -m cactus_b200.microbench quantize --K 4096 --N 64
@@ -47,9 +48,16 @@ def bench_mul_mat(a):
     st = torch.cuda.current_stream().cuda_stream
     check(L.b200_quantize_activations(x.data_ptr(), a.K * 4, a.K, a.N, act.data_ptr(), act.numel(), 0, st))
 
+    whole = getattr(a, "whole", False)
+    scratch = torch.empty(max(256, L.b200_mul_mat_scratch_bytes(a.wtype, a.K, a.M, a.N)), dtype=torch.uint8, device="cuda") if whole else None
+
     def run():
         st = torch.cuda.current_stream().cuda_stream   # the capture stream while a graph is being recorded
         for w in ws:
+            if whole:
+                check(L.b200_mul_mat_q(w.wtype, w.data.data_ptr(), w.K, w.M, x.data_ptr(), a.K * 4, a.N, out.data_ptr(), a.M * 4,
+                                       scratch.data_ptr(), scratch.numel(), 0, st))
+                continue
             check(L.b200_mul_mat_q_prequant(w.wtype, w.data.data_ptr(), w.K, w.M, act.data_ptr(), a.N, out.data_ptr(), a.M * 4,
                                             wsp.data_ptr(), wsp.numel(), st))
         return len(ws)
@@ -61,7 +69,7 @@ def bench_mul_mat(a):
     ms = time_launches(lambda: (g.replay(), len(ws))[1], a.reps)
     bb = 18 if a.wtype == 2 else 34
     alg = a.M * (a.K // 32) * bb + a.N * a.K * 4 + a.N * a.M * 4
-    return {"kernel": "mul_mat", "K": a.K, "M": a.M, "N": a.N, "wtype": a.wtype, "ms_per_launch": ms, "GBps": alg / ms / 1e6,
+    return {"kernel": "mul_mat_q" if whole else "mul_mat", "K": a.K, "M": a.M, "N": a.N, "wtype": a.wtype, "ms_per_launch": ms, "GBps": alg / ms / 1e6,
             "TOPS": 2 * a.M * a.N * a.K / ms / 1e9}
 
 
@@ -271,6 +279,7 @@ def main():
     ap.add_argument("--head-major", action="store_true", help="fattn: address the cache as [Hkv][cells][D] instead of the reference's [cells][Hkv][D]")
     ap.add_argument("--quant", action="store_true", help="fattn: b200_flash_attn_ext_quant (quantised output only)")
     ap.add_argument("--cfg2", choices=["a", "b"], default=None, help="fattn: the 16-sequence prefill ubatch (a: fits 8192 slots, b: cache enlarged)")
+    ap.add_argument("--whole", action="store_true", help="mul_mat: the whole op from f32 activations (b200_mul_mat_q) instead of the product alone")
     ap.add_argument("--K", type=int, default=4096)
     ap.add_argument("--M", type=int, default=14336)
     ap.add_argument("--N", type=int, default=64)

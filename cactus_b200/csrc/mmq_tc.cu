@@ -1,10 +1,10 @@
-// MUL_MAT for a batch of activation columns on the 5th-generation tensor cores, with the block scales folded into the
+// Q4_0 MUL_MAT for a batch of activation columns on the 5th-generation tensor cores, with the block scales folded into the
 // operands so that one accumulator in tensor memory runs over K.
 //
 // lm_ggml_compute_forward_mul_mat (cactus/ggml-cpu/ggml-cpu.c:1257-1449) computes, per output value,
 // sum over blocks b of d_w[row, b] * d_a[col, b] * dot_b with dot_b an integer.  Scaling after every block (mmq.cu) costs a
 // pass over the accumulator tile per 32 values of K; here the scales go into the operands instead:
-//   A[row, k] = d_w[row, b] * q[row, k]      (15 significant bits for Q4_0, 19 for Q8_0: 11 of the fp16 scale and the quant)
+//   A[row, k] = d_w[row, b] * q[row, k]      (15 significant bits: 11 of the fp16 scale and the quant)
 //   B[col, k] = d_a[col, b] * a[col, k]      (19 significant bits)
 // Each is an fp16 value plus the exact fp16 remainder (x_hi = rn(x), x_lo = x - x_hi; d is a multiple of 2^-24, so the
 // remainder always fits), and the product is A_hi B_hi + A_hi B_lo + A_lo B_hi (the missing A_lo B_lo is below 2^-22 of a
@@ -71,10 +71,9 @@ constexpr int TC_RT = 16;            // 16-row tiles of a CTA at most: 256 rows,
 constexpr int TC_EPI_THREADS = 256;
 
 // Geometry.  A CTA has up to NT tiles of 8 activation columns.
-template <int WTYPE>
 struct TcCfg {
     static constexpr int NT = 8;
-    static constexpr int WT = WTYPE == B200_TYPE_Q4_0 ? 1024 : 2048;   // one row tile, one block group
+    static constexpr int WT = 1024;                                    // one row tile, one block group
     static constexpr int OFF_S = TC_RT * WT;                           // its scales: 128 bytes per row tile
     static constexpr int OFF_B = OFF_S + TC_RT * 128;                  // B_hi: 2 KB per column tile, then B_lo
     static constexpr int STAGE = OFF_B + NT * 4096;
@@ -110,7 +109,7 @@ struct TcPlan {
     uint32_t share, extra;   // equal shares: CTA j takes share iterations, one more if j < extra
     int debug;          // tests of the give-up path: 32 no producer copies anything, 64 those of odd CTAs, 128 one write-back warp gives up
 };
-// The weights as tensor maps: 1 KB (2 KB) tiles and 128-byte scale tiles of one block group, 8 row tiles (128 rows) per copy.
+// The weights as tensor maps: 1 KB tiles and 128-byte scale tiles of one block group, 8 row tiles (128 rows) per copy.
 struct TcMaps {
     CUtensorMap q, s;
 };
@@ -152,10 +151,6 @@ __device__ __forceinline__ void tc_commit(uint32_t bar) {
 __device__ __forceinline__ void tc_tma_2d(uint32_t dst, const CUtensorMap *map, int x, int y, uint32_t bar) {
     asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];\n"
                  ::"r"(dst), "l"(map), "r"(x), "r"(y), "r"(bar) : "memory");
-}
-__device__ __forceinline__ void tc_tma_3d(uint32_t dst, const CUtensorMap *map, int x, int y, int z, uint32_t bar) {
-    asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];\n"
-                 ::"r"(dst), "l"(map), "r"(x), "r"(y), "r"(z), "r"(bar) : "memory");
 }
 __device__ __forceinline__ void tc_copy(uint32_t dst, const void *src, uint32_t bytes, uint32_t bar) {
     asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];\n" ::"r"(dst), "l"(src), "r"(bytes), "r"(bar) : "memory");
@@ -232,7 +227,6 @@ static_assert(sizeof(TcShared) <= 5120, "TcShared has its place in TcCfg");
 
 // One result from the integers themselves: what the reference computes, block by block.  Only for values whose folded
 // operands left the fp16 range.
-template <int WTYPE>
 __device__ __forceinline__ float tc_exact_value(const TcShared *o, int row, int col) {
     const uint8_t *wq = o->w, *ws = wq + o->dims.qs_bytes;
     const int rt = row >> 4, r = row & 15, g = r & 7, h = r >> 3;
@@ -245,17 +239,11 @@ __device__ __forceinline__ float tc_exact_value(const TcShared *o, int row, int 
         int dot = 0;
 #pragma unroll 1
         for (int t = 0; t < 4; ++t) {
-            if (WTYPE == B200_TYPE_Q4_0) {
-                const uint32_t word = reinterpret_cast<const uint32_t *>(wq + at * 1024 + (g * 4 + t) * 32)[h * 4 + j];
-                dot = __dp4a((int) ((word << 4) & 0xF0F0F0F0u), (int) a[t].x, dot);
-                dot = __dp4a((int) (word & 0xF0F0F0F0u), (int) a[t].y, dot);
-            } else {
-                const uint32_t *word = reinterpret_cast<const uint32_t *>(wq + at * 2048 + j * 512 + (g * 4 + t) * 16);
-                dot = __dp4a((int) word[h], (int) a[t].x, dot);
-                dot = __dp4a((int) word[2 + h], (int) a[t].y, dot);
-            }
+            const uint32_t word = reinterpret_cast<const uint32_t *>(wq + at * 1024 + (g * 4 + t) * 32)[h * 4 + j];
+            dot = __dp4a((int) ((word << 4) & 0xF0F0F0F0u), (int) a[t].x, dot);
+            dot = __dp4a((int) (word & 0xF0F0F0F0u), (int) a[t].y, dot);
         }
-        const float dw = __half2float(reinterpret_cast<const __half *>(ws)[at * 64 + r * 4 + j]) * (WTYPE == B200_TYPE_Q4_0 ? 0.0625f : 1.0f);
+        const float dw = __half2float(reinterpret_cast<const __half *>(ws)[at * 64 + r * 4 + j]) * 0.0625f;
         const float da = reinterpret_cast<const float *>(o->aq + o->act.d_offset)[((col >> 3) * o->act.n_bg + (b >> 2)) * 64 + act_scale_index(j, col & 7)];
         sum = fmaf(dw * da, (float) dot, sum);
     }
@@ -307,12 +295,11 @@ __device__ __forceinline__ void tc_share(TcShared *o, const TcPlan plan, uint32_
 }
 
 // Values that do not simply go to 16 aligned bytes: a ragged or unaligned edge, or not finite
-template <int WTYPE>
 __device__ __forceinline__ void tc_write_slow(const TcShared *o, int row, int row_end, int col, float4 f) {
 #pragma unroll 1
     for (int i = 0; i < 4 && row + i < row_end; ++i) {
         float y = i == 0 ? f.x : i == 1 ? f.y : i == 2 ? f.z : f.w;
-        if (!isfinite(y)) y = tc_exact_value<WTYPE>(o, row + i, col);
+        if (!isfinite(y)) y = tc_exact_value(o, row + i, col);
         *reinterpret_cast<float *>(reinterpret_cast<char *>(o->dst) + col * o->dst_nb_row + (int64_t) (row + i) * 4) = y;
     }
 }
@@ -334,10 +321,9 @@ struct TcOut {
         to = reinterpret_cast<char *>(o->dst) + col * nb + (int64_t) row * 4;
         vec = row + 3 < row_end && ((reinterpret_cast<uintptr_t>(to) | (uintptr_t) nb) & 15) == 0;
     }
-    template <int WTYPE>
-    __device__ __forceinline__ void put(const TcShared *o, float4 v) {
+        __device__ __forceinline__ void put(const TcShared *o, float4 v) {
         if (vec && isfinite((v.x + v.y) + (v.z + v.w))) *reinterpret_cast<float4 *>(to) = v;
-        else tc_write_slow<WTYPE>(o, row, row_end, col, v);
+        else tc_write_slow(o, row, row_end, col, v);
         to += inc;
         col += col_inc;
     }
@@ -349,7 +335,6 @@ __device__ __forceinline__ float4 tc_lds4(uint32_t at) {
 }
 
 // The tile's parts lie in the shared memory of the cluster's CTAs: this CTA adds slice `rank` of the columns in rank order.
-template <int WTYPE>
 __device__ __forceinline__ void tc_write_cluster(const TcShared *o, uint32_t acc_u32, uint32_t te, uint32_t threads) {
     const uint32_t cs = (uint32_t) o->plan.cs, rank = blockIdx.x % cs, per4 = ((uint32_t) o->act.chunk_nt * 8 + cs - 1) / cs * 64;
     const uint32_t end = min((uint32_t) o->act.chunk_nt * 512, (rank + 1) * per4);
@@ -369,7 +354,7 @@ __device__ __forceinline__ void tc_write_cluster(const TcShared *o, uint32_t acc
         }
 #pragma unroll
         for (uint32_t k = 1; k < 8; ++k) { x[0].x += x[k].x; x[0].y += x[k].y; x[0].z += x[k].z; x[0].w += x[k].w; }
-        out.template put<WTYPE>(o, x[0]);
+        out.put(o, x[0]);
     }
 }
 
@@ -397,7 +382,6 @@ __device__ __forceinline__ void tc_give_up_pieces(const TcShared *o) {
 
 // Piece q is complete in shared memory: write the tile if this is all of it or the last part to arrive, else park it.  Called by
 // `threads` threads, te = 0 ..., which meet at barrier `bar`.  The parts (at most three) are added in K order whoever does it.
-template <int WTYPE>
 __device__ __forceinline__ void tc_finish(TcShared *o, uint32_t acc_u32, uint32_t piece, uint32_t te, uint32_t threads, uint32_t bar) {
     const TcPiece q = o->piece[piece];
     const uint32_t total4 = (uint32_t) o->act.chunk_nt * 512;
@@ -445,17 +429,16 @@ __device__ __forceinline__ void tc_finish(TcShared *o, uint32_t acc_u32, uint32_
                 if (at[k]) x[k] = __ldcg(at[k] + e);
                 else if (k == own) x[k] = tc_lds4(acc_u32 + e * 16u);
             }
-            out.template put<WTYPE>(o, make_float4(x[0].x + x[1].x + x[2].x, x[0].y + x[1].y + x[2].y, x[0].z + x[1].z + x[2].z, x[0].w + x[1].w + x[2].w));
+            out.put(o, make_float4(x[0].x + x[1].x + x[2].x, x[0].y + x[1].y + x[2].y, x[0].z + x[1].z + x[2].z, x[0].w + x[1].w + x[2].w));
         }
     }
     asm volatile("bar.sync %0, %1;\n" ::"r"(bar), "r"(threads) : "memory");   // the partial results are free again
 }
 
-template <int WTYPE>
-__global__ void __launch_bounds__(TcCfg<WTYPE>::THREADS, 1) mmq_tc_kernel(TiledDims dims, const uint8_t *__restrict__ w, ActDims act, const uint8_t *__restrict__ aq,
+__global__ void __launch_bounds__(TcCfg::THREADS, 1) mmq_tc_kernel(TiledDims dims, const uint8_t *__restrict__ w, ActDims act, const uint8_t *__restrict__ aq,
                                                               float *__restrict__ dst, int64_t dst_nb_row, void *__restrict__ workspace, TcPlan plan,
                                                               const __grid_constant__ TcMaps maps) {
-    using C = TcCfg<WTYPE>;
+    using C = TcCfg;
     extern __shared__ __align__(1024) uint8_t smem[];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const uint32_t smem_u32 = (uint32_t) __cvta_generic_to_shared(smem);
@@ -600,8 +583,7 @@ __global__ void __launch_bounds__(TcCfg<WTYPE>::THREADS, 1) mmq_tc_kernel(TiledD
 #pragma unroll
                         for (int k = 0; k < 2; ++k) {
                             if (k < boxes) {
-                                if (WTYPE == B200_TYPE_Q4_0) tc_tma_2d(st + (uint32_t) (k * 8 * C::WT), &maps.q, bg * 256, rt_in + 8 * k, bar);
-                                else tc_tma_3d(st + (uint32_t) (k * 8 * C::WT), &maps.q, 0, bg * 2, rt_in + 8 * k, bar);
+                                tc_tma_2d(st + (uint32_t) (k * 8 * C::WT), &maps.q, bg * 256, rt_in + 8 * k, bar);
                                 tc_tma_2d(st + (uint32_t) (C::OFF_S + k * 1024), &maps.s, bg * 32, rt_in + 8 * k, bar);
                             }
                         }
@@ -627,7 +609,7 @@ __global__ void __launch_bounds__(TcCfg<WTYPE>::THREADS, 1) mmq_tc_kernel(TiledD
         const int q4 = warp & 3, mt = ((warp - 4) >> 2) & 1, team = (warp - 4) >> 3;
         const uint32_t rt0 = (uint32_t) (mt * 8 + q4 * 2);
         const uint32_t a_base = tmem + ((uint32_t) (32 * q4) << 16) + C::A_COL + (uint32_t) (mt * C::A_MT);
-        const uint32_t w_at = smem_u32 + rt0 * C::WT + (uint32_t) (lane * (WTYPE == B200_TYPE_Q4_0 ? 32 : 16));
+        const uint32_t w_at = smem_u32 + rt0 * C::WT + (uint32_t) (lane * 32);
         const uint32_t s_at = smem_u32 + C::OFF_S + rt0 * 128 + (uint32_t) ((lane >> 2) * 8);
         const bool active = mt == 0 || plan.rt_per_group > 8;
         const uint32_t halves = 2 * sh->n_iter;
@@ -636,16 +618,14 @@ __global__ void __launch_bounds__(TcCfg<WTYPE>::THREADS, 1) mmq_tc_kernel(TiledD
         for (uint32_t hc = (uint32_t) team; hc < halves; hc += 2, free_par ^= 1) {
             const uint32_t half = hc & 1, ab = (uint32_t) team;
             if (!tc_wait(BAR(C::B_FULL, s), full_par, abort_flag, spin_limit)) break;
-            constexpr int NW = WTYPE == B200_TYPE_Q4_0 ? 4 : 8;
-            uint32_t r[2][NW];      // Q4_0: rows g, g + 8 x word t of the two blocks; Q8_0: block j: (g, t), (g + 8, t), (g, 4 + t), (g + 8, 4 + t)
+            uint32_t r[2][4];       // rows g, g + 8 x word t of the two blocks
             uint32_t sc[2][2];      // the two block scales of rows g, g + 8
 #pragma unroll
             for (int u = 0; u < 2; ++u) {
 #pragma unroll
                 for (int v = 0; v < 2; ++v) {
-                    const uint32_t at = w_at + s * C::STAGE + half * (WTYPE == B200_TYPE_Q4_0 ? 8 : 1024) + (uint32_t) (u * C::WT + v * (WTYPE == B200_TYPE_Q4_0 ? 16 : 512));
-                    if (WTYPE == B200_TYPE_Q4_0) asm volatile("ld.shared.v2.u32 {%0,%1}, [%2];\n" : "=r"(r[u][2 * v]), "=r"(r[u][2 * v + 1]) : "r"(at));
-                    else asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];\n" : "=r"(r[u][(4 * v) % NW]), "=r"(r[u][(4 * v + 1) % NW]), "=r"(r[u][(4 * v + 2) % NW]), "=r"(r[u][(4 * v + 3) % NW]) : "r"(at));
+                    const uint32_t at = w_at + s * C::STAGE + half * 8 + (uint32_t) (u * C::WT + v * 16);
+                    asm volatile("ld.shared.v2.u32 {%0,%1}, [%2];\n" : "=r"(r[u][2 * v]), "=r"(r[u][2 * v + 1]) : "r"(at));
                 }
                 const uint32_t sa = s_at + s * C::STAGE + half * 4 + (uint32_t) (u * 128);
                 asm volatile("ld.shared.u32 %0, [%1];\n" : "=r"(sc[u][0]) : "r"(sa));
@@ -672,16 +652,11 @@ __global__ void __launch_bounds__(TcCfg<WTYPE>::THREADS, 1) mmq_tc_kernel(TiledD
 #pragma unroll
                             for (int si = 0; si < 4; ++si) {
                                 __half2 q2;
-                                if (WTYPE == B200_TYPE_Q4_0) {
-                                    // nibbles at bits 4 si and 16 + 4 si, two's complement; v = q + 8.  0x6400 | v is the fp16
-                                    // 1024 + v, 0x6400 | 16 v is 1024 + 16 v; both steps to q are exact
-                                    const uint32_t word = r[u][row * 2 + j], w8 = si < 2 ? word : word >> 8;
-                                    if ((si & 1) == 0) q2 = __hadd2(tc_as_h2((w8 & 0x000F000Fu) ^ 0x64086408u), __float2half2_rn(-1032.0f));
-                                    else q2 = __hfma2(tc_as_h2((w8 & 0x00F000F0u) ^ 0x64806480u), __float2half2_rn(0.0625f), __float2half2_rn(-72.0f));
-                                } else {
-                                    const uint32_t word = r[u][(4 * j + row + 2 * (si & 1)) % NW] ^ 0x80808080u;   // q + 128
-                                    q2 = __hadd2(tc_as_h2(__byte_perm(word, 0x64646464u, si < 2 ? 0x4240 : 0x4341)), __float2half2_rn(-1152.0f));
-                                }
+                                // nibbles at bits 4 si and 16 + 4 si, two's complement; v = q + 8.  0x6400 | v is the fp16
+                                // 1024 + v, 0x6400 | 16 v is 1024 + 16 v; both steps to q are exact
+                                const uint32_t word = r[u][row * 2 + j], w8 = si < 2 ? word : word >> 8;
+                                if ((si & 1) == 0) q2 = __hadd2(tc_as_h2((w8 & 0x000F000Fu) ^ 0x64086408u), __float2half2_rn(-1032.0f));
+                                else q2 = __hfma2(tc_as_h2((w8 & 0x00F000F0u) ^ 0x64806480u), __float2half2_rn(0.0625f), __float2half2_rn(-72.0f));
                                 const __half2 x = __hmul2(q2, d2);
                                 hi[si * 2 + row] = tc_h2(x);
                                 lo[si * 2 + row] = tc_h2(__hfma2(q2, d2, __hneg2(x)));
@@ -747,7 +722,7 @@ __global__ void __launch_bounds__(TcCfg<WTYPE>::THREADS, 1) mmq_tc_kernel(TiledD
             if (!ok) *wb_gave_up = 1;
             asm volatile("bar.sync 1, 256;\n" ::: "memory");
             if (*wb_gave_up) break;   // (written again at the earliest beyond the barriers of tc_finish)
-            tc_finish<WTYPE>(sh, acc_u32, p, (uint32_t) et, TC_EPI_THREADS, 1u);
+            tc_finish(sh, acc_u32, p, (uint32_t) et, TC_EPI_THREADS, 1u);
         }
     }
     asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
@@ -757,7 +732,7 @@ __global__ void __launch_bounds__(TcCfg<WTYPE>::THREADS, 1) mmq_tc_kernel(TiledD
     else asm volatile("setmaxnreg.dec.sync.aligned.u32 72;\n");
     if (plan.cs > 0) {
         asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;\n" ::: "memory");
-        if (!*abort_flag) tc_write_cluster<WTYPE>(sh, acc_u32, (uint32_t) tid, C::THREADS);
+        if (!*abort_flag) tc_write_cluster(sh, acc_u32, (uint32_t) tid, C::THREADS);
         // nobody leaves while a neighbour may still read its part
         asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;\n" ::: "memory");
     } else {
@@ -765,7 +740,7 @@ __global__ void __launch_bounds__(TcCfg<WTYPE>::THREADS, 1) mmq_tc_kernel(TiledD
         if (*abort_flag) {
             if (tid == 0) tc_give_up_pieces(sh);
         } else if (sh->n_pieces > 0) {
-            tc_finish<WTYPE>(sh, acc_u32, sh->n_pieces - 1, (uint32_t) tid, C::THREADS, 0u);
+            tc_finish(sh, acc_u32, sh->n_pieces - 1, (uint32_t) tid, C::THREADS, 0u);
         }
         __syncthreads();
     }
@@ -789,11 +764,10 @@ struct TcVariant {
     int smem, threads;
     int max_clusters[9];   // resident clusters of 1..8 CTAs on the current device
 };
-template <int WTYPE>
 static void tc_make(TcVariant &v) {
-    v.fn = mmq_tc_kernel<WTYPE>;
-    v.smem = TcCfg<WTYPE>::SMEM;
-    v.threads = TcCfg<WTYPE>::THREADS;
+    v.fn = mmq_tc_kernel;
+    v.smem = TcCfg::SMEM;
+    v.threads = TcCfg::THREADS;
     cudaFuncSetAttribute(v.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, v.smem);
     for (int cs = 1; cs <= 8; ++cs) {
         cudaLaunchConfig_t cfg = {};
@@ -815,8 +789,8 @@ static void tc_make(TcVariant &v) {
         v.max_clusters[cs] = n;
     }
 }
-static const TcVariant &tc_variant(int wtype) {
-    static TcVariant table[64][2];   // per device: kernel attributes and occupancy are per-context properties
+static const TcVariant &tc_variant() {
+    static TcVariant table[64];   // per device: kernel attributes and occupancy are per-context properties
     static bool ready[64] = {false};
     static std::mutex mu;
     int dev = 0;
@@ -824,11 +798,10 @@ static const TcVariant &tc_variant(int wtype) {
     dev &= 63;
     std::lock_guard<std::mutex> lock(mu);
     if (!ready[dev]) {
-        tc_make<B200_TYPE_Q4_0>(table[dev][0]);
-        tc_make<B200_TYPE_Q8_0>(table[dev][1]);
+        tc_make(table[dev]);
         ready[dev] = true;
     }
-    return table[dev][wtype == B200_TYPE_Q4_0 ? 0 : 1];
+    return table[dev];
 }
 
 // ---- tensor maps ----
@@ -844,23 +817,16 @@ static tc_encode_fn tc_encoder() {
     }();
     return fn;
 }
-// rows of `line_words` 32-bit words x `lines` lines x `rows`, a box of one line (2-D: `box_lines` 1) or box_lines lines, 8 rows
-static bool tc_encode(CUtensorMap *m, const void *base, uint32_t line_words, uint64_t lines, uint64_t rows, uint32_t box_lines) {
+// `rows` rows of `words` 32-bit words, a box of box_words x 8 rows
+static bool tc_encode(CUtensorMap *m, const void *base, uint64_t words, uint64_t rows, uint32_t box_words) {
     tc_encode_fn enc = tc_encoder();
     if (!enc) return false;
-    const cuuint32_t elem[3] = {1, 1, 1};
-    if (box_lines == 1) {
-        const cuuint64_t dims[2] = {line_words * lines, rows}, strides[1] = {line_words * lines * 4};
-        const cuuint32_t box[2] = {line_words, 8};
-        return enc(m, CU_TENSOR_MAP_DATA_TYPE_UINT32, 2, const_cast<void *>(base), dims, strides, box, elem, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                   CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
-    }
-    const cuuint64_t dims[3] = {line_words, lines, rows}, strides[2] = {line_words * 4ull, line_words * lines * 4};
-    const cuuint32_t box[3] = {line_words, box_lines, 8};
-    return enc(m, CU_TENSOR_MAP_DATA_TYPE_UINT32, 3, const_cast<void *>(base), dims, strides, box, elem, CU_TENSOR_MAP_INTERLEAVE_NONE,
+    const cuuint32_t elem[2] = {1, 1}, box[2] = {box_words, 8};
+    const cuuint64_t dims[2] = {words, rows}, strides[1] = {words * 4};
+    return enc(m, CU_TENSOR_MAP_DATA_TYPE_UINT32, 2, const_cast<void *>(base), dims, strides, box, elem, CU_TENSOR_MAP_INTERLEAVE_NONE,
                CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
-// encoded maps are pure functions of (pointer, type, extents): kept, a model has a few hundred weights
+// encoded maps are pure functions of (pointer, extents): kept, a model has a few hundred weights
 struct TcKey {
     const void *p;
     int64_t a, b;
@@ -869,16 +835,16 @@ struct TcKey {
 struct TcKeyHash {
     size_t operator()(const TcKey &k) const { return std::hash<const void *>()(k.p) ^ (size_t) (k.a * 0x9E3779B97F4A7C15ull) ^ (size_t) (k.b * 0xC2B2AE3D27D4EB4Full); }
 };
-static bool tc_weight_maps(int wtype, const TiledDims &d, const void *w, TcMaps &maps) {
+static bool tc_weight_maps(const TiledDims &d, const void *w, TcMaps &maps) {
     static std::mutex mu;
     static std::unordered_map<TcKey, TcMaps, TcKeyHash> cache;
-    const TcKey key{w, d.n_rt * 16 + wtype, d.n_bg};
+    const TcKey key{w, d.n_rt, d.n_bg};
     std::lock_guard<std::mutex> lock(mu);
     auto it = cache.find(key);
     if (it == cache.end()) {
         TcMaps p;
-        if (!tc_encode(&p.q, w, 256, (uint64_t) d.n_bg * (wtype == B200_TYPE_Q4_0 ? 1 : 2), (uint64_t) d.n_rt, wtype == B200_TYPE_Q4_0 ? 1 : 2)) return false;
-        if (!tc_encode(&p.s, (const uint8_t *) w + d.qs_bytes, 32, (uint64_t) d.n_bg, (uint64_t) d.n_rt, 1)) return false;
+        if (!tc_encode(&p.q, w, (uint64_t) d.n_bg * 256, (uint64_t) d.n_rt, 256)) return false;
+        if (!tc_encode(&p.s, (const uint8_t *) w + d.qs_bytes, (uint64_t) d.n_bg * 32, (uint64_t) d.n_rt, 32)) return false;
         if (cache.size() > 65536) cache.clear();
         it = cache.emplace(key, p).first;
     }
@@ -945,11 +911,11 @@ static TcPlan tc_plan(const TcVariant &v, const TiledDims &d, const ActDims &a, 
     return best;
 }
 
-int launch_mmq_tc(int wtype, const TiledDims &d, const void *w, const ActDims &a, const void *aq, float *dst, int64_t dst_nb_row,
+int launch_mmq_tc(const TiledDims &d, const void *w, const ActDims &a, const void *aq, float *dst, int64_t dst_nb_row,
                   void *workspace, size_t workspace_bytes, cudaStream_t st) {
-    const TcVariant &v = tc_variant(wtype);
+    const TcVariant &v = tc_variant();
     TcMaps maps;
-    if (!tc_weight_maps(wtype, d, w, maps)) return set_error(B200_E_CUDA, "mmq_tc: no tensor map for the weights");
+    if (!tc_weight_maps(d, w, maps)) return set_error(B200_E_CUDA, "mmq_tc: no tensor map for the weights");
     const bool ws = workspace && workspace_bytes >= mmq_tc_workspace_bytes(d.M, a.N) && d.n_rt * d.n_bg * a.n_nt < (1ll << 31);
     TcPlan plan = tc_plan(v, d, a, ws);
     const int tiles = plan.groups * plan.chunks;

@@ -7,7 +7,7 @@
 #include "common.cuh"
 
 namespace b200 {
-int launch_mmq_tc(int wtype, const TiledDims &d, const void *w, const ActDims &a, const void *aq, float *dst, int64_t dst_nb_row,
+int launch_mmq_tc(const TiledDims &d, const void *w, const ActDims &a, const void *aq, float *dst, int64_t dst_nb_row,
                   void *workspace, size_t workspace_bytes, cudaStream_t st);
 size_t mmq_tc_workspace_bytes(int64_t M, int64_t N);
 int tc_error_flag();
@@ -59,27 +59,38 @@ static bool shape_ok(int wtype, int64_t K, int64_t M, int64_t N) {
 
 // b200_mul_mat_q alone chooses between the two tensor-core kernels: it knows the weights' shape when it quantises, and the
 // tcgen05 kernel wants its operands laid out by the quantiser.  (Products of activations that are quantised on their own feed
-// whole models, whose results stay bit for bit what they were: every product re-quantises its input, so a last-bit
-// difference in one sum is a different rounding somewhere in the next.)
-// Measured on B200 (us, tcgen05 / mma.sync kernel): up to 32 columns the latter is as fast or faster at every size
-// (4096 x 28672: 37.7 / 38.2 at 32, 34.0 / 22.6 at 16).  From there on the tensor core wins where there is enough work to
-// fill its pipeline, which takes about 5 us to start and to finish:
-//   K x M            N = 40        64           80            256
-//   4096 x 28672     39.7 / 56.6   44.3 / 57.8   62.9 / 103.4   131 / 177
-//   14336 x 4096     27.4 / 28.6   30.1 / 28.7   35.8 / 49.0    71.1 / 91.3
-//   4096 x 6144      15.1 / 17.2   16.8 / 17.2   22.4 / 24.9    37.6 / 47.6
-//   4096 x 4096      13.5 / 12.8   13.9 / 13.0   15.8 / 17.9    24.7 / 30.8
-//   2048 x 2048       9.2 / 8.0     9.1 / 8.0    10.5 / 9.1     13.1 / 11.8
-// so: one column chunk needs 24 row groups (a K split over at most five CTAs), more chunks 8 M weights.
-// B200_MMQ_TC decides by hand (0: never, else from 9 columns on).
-static bool use_tc(int64_t K, int64_t M, int64_t N) {
+// whole models and keep the mma.sync kernel.)
+// Measured on B200, quantiser and product, weights larger than L2 in turn (us, tcgen05 / mma.sync, Q4_0):
+//   K x M            N = 33       64           65           128          192          256          384          512
+//   4096 x 28672     48.8 / 53.5  53.3 / 54.3  81.6 / 103   89.9 / 104   122 / 138    156 / 178    231 / 248    316 / 321
+//   4096 x 20480     1.14         1.07         1.27         1.18         1.13         1.10         1.09         1.05   (ratios)
+//   8192 x 16384     1.10         1.01         1.22         1.12         1.19         1.16         1.14         0.97
+//   4096 x 14336     31.5 / 32.8  34.6 / 33.1  47.3 / 54.6  51.0 / 55.3  68.5 / 78.7  88.4 / 103   121 / 138    156 / 178
+//   4096 x 10240     0.96         0.89         1.18         1.11         1.04         1.18         1.14         1.10
+//   8192 x 8192      33.6 / 32.6  36.3 / 32.9  52.1 / 56.8  57.0 / 57.7  74.0 / 82.5  93.7 / 105   134 / 158    184 / 201
+//   4096 x 8192      0.85         0.79         0.99         0.94         1.06         1.01         1.15         1.07
+//   14336 x 4096     36.5 / 30.1  39.0 / 30.5  48.2 / 50.2  52.9 / 51.7  86.8 / 71.5  91.8 / 96.3  124 / 134    167 / 183
+//   4096 x 6144      20.8 / 18.4  23.2 / 18.8  31.1 / 25.7  34.2 / 28.0  34.8 / 33.1  46.5 / 49.4  55.8 / 56.1  76.6 / 86.8
+//   4096 x 4096      18.8 / 14.7  20.9 / 14.9  23.1 / 19.1  24.5 / 19.7  34.0 / 28.3  34.8 / 33.1  46.7 / 50.3  56.4 / 56.6
+//   2048 x 16384     21.6 / 20.8  24.0 / 21.2  31.4 / 30.4  34.3 / 30.9  48.7 / 50.8  60.5 / 56.6  83.8 / 81.6  105 / 95.5
+// The tcgen05 kernel needs about 5 us to fill and empty a CTA's pipeline and pays per 256 rows x 64 columns x K, so it wants
+// a long K and enough row groups that no SM waits: hence the lines below.  Beyond 100 G multiply-adds it falls behind again
+// (8192 x 32768 at 320 / 384 / 448 / 512 columns: 434 / 453, 535 / 531, 670 / 624, 762 / 675).
+// Q8_0 never: a stage of its ring holds twice the weights, so that two fit instead of three and copies and MMAs hardly overlap
+// (4096 x 28672 at 65 / 256 / 512 columns 95.8 / 101, 193 / 175, 371 / 310; 4096 x 14336 54.2 / 53.8, 100 / 101, 182 / 176;
+// 14336 x 4096 55.4 / 49.9, 109 / 94.0, 179 / 177; 8192 x 32768 191 / 193, 419 / 347, 869 / 651).
+// B200_MMQ_TC decides by hand for Q4_0 (0: never, else from 9 columns on).
+static bool use_tc(int wtype, int64_t K, int64_t M, int64_t N) {
     static const int forced = [] {
         const char *e = getenv("B200_MMQ_TC");
         return e ? atoi(e) : -1;
     }();
-    if (forced == 0 || N < 9 || mmq_sync_forced()) return false;
+    if (wtype != B200_TYPE_Q4_0 || forced == 0 || N < 9 || mmq_sync_forced()) return false;
     if (forced > 0) return true;
-    return N > 64 ? M * K >= (8 << 20) : N > 32 && M >= 6144 && K >= 1024;
+    if (N <= 32 || K < 4096 || (double) M * K * N > 1e11) return false;
+    if (N <= 64) return M >= 20480;
+    if (N <= 192) return M >= 10240;
+    return M >= 4096 && M * K >= (24 << 20);
 }
 
 extern "C" {
@@ -95,7 +106,7 @@ size_t b200_mul_mat_workspace_bytes(int wtype, int64_t K, int64_t M, int64_t N) 
 size_t b200_mul_mat_scratch_bytes(int wtype, int64_t K, int64_t M, int64_t N) {
     if (!shape_ok(wtype, K, M, N)) return 0;
     const ActDims a = act_dims(K, N);
-    return a.total_bytes + (use_tc(K, M, N) ? a.b_bytes + mmq_tc_workspace_bytes(M, N) : mmq_workspace_bytes(wtype, K, M, N));
+    return a.total_bytes + (use_tc(wtype, K, M, N) ? a.b_bytes + mmq_tc_workspace_bytes(M, N) : mmq_workspace_bytes(wtype, K, M, N));
 }
 
 static int mul_mat_prequant(int wtype, const void *w, int64_t K, int64_t M, const void *act, int64_t N, float *dst, int64_t dst_row_stride_bytes,
@@ -207,7 +218,7 @@ int b200_mul_mat_q(int wtype, const void *w, int64_t K, int64_t M, const float *
                    float *dst, int64_t dst_row_stride_bytes, void *scratch, size_t scratch_bytes, int variant, b200_stream_t stream) {
     B200_REQUIRE(shape_ok(wtype, K, M, N), "bad mul_mat shape/type: type %d K %lld M %lld N %lld", wtype, (long long) K, (long long) M, (long long) N);
     const ActDims a = act_dims(K, N);
-    const bool tc = use_tc(K, M, N);
+    const bool tc = use_tc(wtype, K, M, N);
     const size_t ab = a.total_bytes + (tc ? a.b_bytes : 0), wb = tc ? mmq_tc_workspace_bytes(M, N) : mmq_workspace_bytes(wtype, K, M, N);
     if (!scratch || scratch_bytes < ab + wb) return set_error(B200_E_SCRATCH, "scratch too small: %zu < %zu", scratch_bytes, ab + wb);
     if (!tc) {
@@ -218,7 +229,7 @@ int b200_mul_mat_q(int wtype, const void *w, int64_t K, int64_t M, const float *
     B200_REQUIRE(x_row_stride_bytes % 4 == 0 && dst_row_stride_bytes % 4 == 0 && dst_row_stride_bytes >= M * 4, "bad row stride");
     B200_REQUIRE(variant == B200_Q8_AVX2 || variant == B200_Q8_SCALAR, "unknown quantiser variant %d", variant);
     if (int e = launch_quantize_b8(x, x_row_stride_bytes, K, N, scratch, variant, 2, (cudaStream_t) stream)) return e;
-    return launch_mmq_tc(wtype, tiled_dims(wtype, K, M), w, a, scratch, dst, dst_row_stride_bytes, (char *) scratch + ab, wb, (cudaStream_t) stream);
+    return launch_mmq_tc(tiled_dims(wtype, K, M), w, a, scratch, dst, dst_row_stride_bytes, (char *) scratch + ab, wb, (cudaStream_t) stream);
 }
 
 int b200_mul_mat_q_noalloc(int wtype, const void *w, int64_t K, int64_t M, const float *x, int64_t x_row_stride_bytes, int64_t N,

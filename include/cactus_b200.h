@@ -105,7 +105,7 @@ B200_API int b200_quantize_q8_0(const float *x, int64_t x_row_stride_bytes, int6
  *            by the kernel workspace (b200_mul_mat_workspace_bytes: split-K partial sums or the parked tiles and
  *            arrival counters of the stream-K work split)
  * N <= 2 uses the HBM-bound dp4a kernel (B200_MMVQ_MAX_N moves the border up to 8), larger N the int8 tensor-core kernel,
- * b200_mul_mat_q with more than 32 columns and enough weights the tcgen05 kernel (B200_MMQ_TC=0: never).
+ * b200_mul_mat_q with Q4_0 weights, more than 32 columns and enough work the tcgen05 kernel (B200_MMQ_TC=0: never).
  * ---------------------------------------------------------------------------------------------- */
 B200_API size_t b200_act_bytes(int64_t K, int64_t N);
 B200_API size_t b200_mul_mat_workspace_bytes(int wtype, int64_t K, int64_t M, int64_t N);

@@ -105,3 +105,20 @@ def test_host_path_is_rebuilt_for_another_torch_and_not_loaded_with_it(monkeypat
     unmarked = tmp_path / "_ops_host.so"
     unmarked.write_bytes(b"no mark")
     assert b.built_host_abi(str(unmarked)) != other
+
+
+def test_kernel_choice_of_the_single_product_goes_by_type_and_size():
+    """b200_mul_mat_q takes the tcgen05 kernel only where it was measured to be faster: the scratch size tells, since that kernel
+    wants its operands and parked parts behind the activations.  Q8_0 never; Q4_0 at the lines of the rule."""
+    from cactus_b200._lib import lib
+    L = lib()
+
+    def tcgen05(wtype, K, M, N):
+        return L.b200_mul_mat_scratch_bytes(wtype, K, M, N) != L.b200_act_bytes(K, N) + L.b200_mul_mat_workspace_bytes(wtype, K, M, N)
+    for K, M, N in [(4096, 28672, 512), (8192, 32768, 256), (14336, 4096, 512), (4096, 14336, 65), (2048, 128256, 100)]:
+        assert not tcgen05(8, K, M, N), (K, M, N)
+    for K, M, N in [(4096, 20480, 33), (4096, 20480, 64), (4096, 10240, 65), (4096, 10240, 192), (4096, 6144, 193), (14336, 4096, 512), (8192, 32768, 320)]:
+        assert tcgen05(2, K, M, N), (K, M, N)
+    for K, M, N in [(4096, 28672, 32), (4096, 20464, 64), (4096, 10224, 65), (4096, 4096, 512), (4064, 28672, 512), (14336, 4080, 512), (4096, 6128, 193),
+                    (8192, 32768, 400)]:
+        assert not tcgen05(2, K, M, N), (K, M, N)

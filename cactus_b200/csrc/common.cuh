@@ -33,6 +33,10 @@ bool pdl_enabled();
 // let the next kernel's CTAs take their places at once (pdl_prologue(true)), and the few-column product asks for its
 // weights -- which no kernel of a step writes -- to be brought into L2 before it waits for the kernel ahead of it.
 int pdl_early_rows();
+// When the quantisers (plain, and of silu * up) let the next kernel's CTAs take their places: 1 at once (pdl_early_rows),
+// 2 when the values are loaded, 0 at their end.  Measured on the 8B decode step, back to back (ms, 2 / 0): 4 sequences
+// 2.79 / 2.83, 7 2.90 / 2.91, 12 3.04 / 3.05, 16 3.15 / 3.15, 32 4.45 / 4.45, 48 6.02 / 5.62, 64 6.93 / 6.49.
+static inline int pdl_quantiser(int64_t rows) { return rows <= pdl_early_rows() ? 1 : rows <= 16 ? 2 : 0; }
 #ifdef __CUDACC__
 __device__ __forceinline__ void pdl_prologue() {
 #ifdef B200_PDL_EARLY_TRIGGER   // lets the next kernel's CTAs take their places for the whole run of this one: measured slower

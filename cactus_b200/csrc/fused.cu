@@ -97,7 +97,7 @@ __global__ void __launch_bounds__(256) silu_mul_quantize_kernel(const float *gat
                                                                float *dst, int64_t dst_nb_row,
                                                                int64_t N, int64_t nb, int64_t nbp,
                                                                uint8_t *__restrict__ out, size_t d_offset, int variant, int early) {
-    pdl_prologue(early != 0);
+    pdl_prologue(early == 1);
     const int64_t n = blockIdx.x;
     for (int64_t at = blockIdx.y * 256 + threadIdx.x; at < nbp * 8; at += gridDim.y * 256) {   // whole groups of 8 lanes leave together
         const int j = (int) at & 7;
@@ -115,6 +115,7 @@ __global__ void __launch_bounds__(256) silu_mul_quantize_kernel(const float *gat
             }
             if (dst) *reinterpret_cast<float4 *>(reinterpret_cast<char *>(dst) + n * dst_nb_row + at * 16) = make_float4(v[0], v[1], v[2], v[3]);
         }
+        if (early == 2) pdl_trigger();
         q8_quantize_store<1>(v, out, d_offset, nb, nbp, n, b, j, real, variant);
     }
 }
@@ -226,7 +227,7 @@ int b200_silu_mul_quantize(const float *gate, const float *up, int64_t nb_row, f
     if (scratch_bytes < a.total_bytes) return set_error(B200_E_SCRATCH, "scratch too small: %zu < %zu", scratch_bytes, a.total_bytes);
     const dim3 grid((unsigned) (a.n_nt * 8), (unsigned) std::min<int64_t>(65535, (a.nbp * 8 + 255) / 256));
     cudaStream_t st = (cudaStream_t) stream;
-    const int early = N <= pdl_early_rows() ? 1 : 0;
+    const int early = pdl_quantiser(N);
     launch_pdl(silu_mul_quantize_kernel, grid, dim3(256), 0, st, gate, up, nb_row, dst, dst_nb_row, N, a.nb, a.nbp, (uint8_t *) scratch, a.d_offset, variant, early);
     return check_launch("silu_mul_quantize");
 }

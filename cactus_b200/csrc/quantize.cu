@@ -17,9 +17,7 @@ template <int LAYOUT>
 __global__ void __launch_bounds__(256) quantize_q8_0_kernel(const float *__restrict__ x, int64_t x_nb_row, int64_t K,
                                                            int64_t N, int64_t nb, int64_t nbp,
                                                            uint8_t *__restrict__ out, size_t d_offset, int variant, int early, int chunk_nt) {
-    // (No trigger between the loads and the stores: with one here and in silu_mul_quantize_kernel the 8B decode step of 64
-    // sequences, back to back, takes 6.91 ms instead of 6.41; with the one here only 6.48, with the other only 6.85.)
-    pdl_prologue(early != 0);
+    pdl_prologue(early == 1);
     const int64_t n = blockIdx.x;   // row
     // 4 elements per thread; whole groups of 8 lanes (a block) leave together.  (A row per x: no 64-bit division per thread)
     for (int64_t at = blockIdx.y * 256 + threadIdx.x; at < (LAYOUT == 0 ? nb : nbp) * 8; at += gridDim.y * 256) {
@@ -36,6 +34,7 @@ __global__ void __launch_bounds__(256) quantize_q8_0_kernel(const float *__restr
                 v[0] = row[0]; v[1] = row[1]; v[2] = row[2]; v[3] = row[3];
             }
         }
+        if (early == 2) pdl_trigger();
         q8_quantize_store<LAYOUT>(v, out, d_offset, nb, nbp, n, b, j, real, variant, chunk_nt);
     }
 }
@@ -211,7 +210,7 @@ static int check_wtype(int wtype) {
 int launch_quantize_b8(const float *x, int64_t x_nb_row, int64_t K, int64_t N, void *scratch, int variant, int layout, cudaStream_t st) {
     const ActDims a = act_dims(K, N);
     const dim3 grid = quantize_grid(a.n_nt * 8, a.nbp);
-    const int early = N <= pdl_early_rows() ? 1 : 0;
+    const int early = pdl_quantiser(N);
     if (layout == 2) launch_pdl(quantize_q8_0_kernel<2>, grid, dim3(256), 0, st, x, x_nb_row, K, N, a.nb, a.nbp, (uint8_t *) scratch, a.d_offset, variant, early, a.chunk_nt);
     else launch_pdl(quantize_q8_0_kernel<1>, grid, dim3(256), 0, st, x, x_nb_row, K, N, a.nb, a.nbp, (uint8_t *) scratch, a.d_offset, variant, early, a.chunk_nt);
     return check_launch("quantize_q8_0 (activations)");

@@ -1,6 +1,7 @@
 """The folded-scale tcgen05 mul_mat kernel at the edges of its tiles, and where a folded operand leaves the fp16 range.
 
-B200_MMQ_TC=1 takes it wherever it is possible, which is read once per process: the cases run in a child interpreter."""
+B200_MMQ_TC=1 takes it for every Q4_0 product of at least 9 columns, which is read once per process: the cases run in a child
+interpreter.  (The Q8_0 cases run the mma.sync kernel: the same edges, the same bounds.)"""
 import json
 import os
 import subprocess

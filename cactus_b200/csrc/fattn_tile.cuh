@@ -11,7 +11,7 @@
 // mask value comes from its mask-word bits (turned, once per round of 1024 cells, into 32 bits per token and chunk in
 // shared memory) instead of from the f16 mask in global memory.  Long tiles are cut into KV splits (grid z): split z takes every nsplit-th
 // chunk of the union list, the partial (max, sum, accumulator) triples go to scratch and fattn_combine_kernel finishes.
-//   S = Q K^T   m16n8k16, Q rounded to fp16 as the reference rounds it, K fragments straight from the staged rows
+//   S = Q K^T   m16n8k16, Q rounded to fp16 as the reference rounds it, K fragments from the staged rows through ldmatrix
 //   online softmax per row (the four lanes of a row share max and sum through two shuffles)
 //   O += P V    P goes in as fp16 hi + lo parts (two MMAs), which keeps the probabilities at fp32 accuracy; V fragments
 //               come from the staged rows through ldmatrix.trans

@@ -19,7 +19,7 @@
 // What bounds it: issuing the MMAs.  128 x 128 x 16 + 128 x 64 x 16 per 16 values of K take 96 clk (measured: N / 2 clk per
 // MMA), a block group of 256 rows x 64 columns x 128 values 1542 clk; but an issuing warp needs about as long for its
 // 17 MMAs, three waits and two commits beside six busy warps on its scheduler, and the accumulator has to be read in between.
-// 4096 x 28672 at 512 columns: 298 us (265 us with 16 block groups per accumulator; mma.sync 323).  A CTA needs about
+// 4096 x 28672 at 512 columns: 298 us (296 to 316 by run; 265 with 16 block groups per accumulator; mma.sync 321 to 324).  A CTA needs about
 // 5 us to fill and empty its pipeline.  What is around the MMAs has to stay below that:
 //   * the activations arrive as B_hi / B_lo planes written once by the quantiser (act_dims: b_offset) in the core-matrix
 //     order of the MMA's B descriptor.  A CTA owns 256 weight rows (two MMA row tiles) per activation copy: 50 KB per

@@ -15,7 +15,7 @@ CSRC = os.path.join(HERE, "csrc")
 OUT = os.path.join(HERE, "lib")
 LIB = os.path.join(OUT, "libcactus_b200.so")
 HOST_LIB = os.path.join(OUT, "_ops_host.so")   # the Python-facing host path (needs torch's headers)
-SOURCES = ["abi.cu", "quantize.cu", "mmvq.cu", "mmq.cu", "mmq_tc.cu", "mul_mat.cu", "fattn.cu", "rowops.cu", "kvops.cu", "fused.cu", "peer.cu"]
+SOURCES = ["abi.cu", "quantize.cu", "mmvq.cu", "mmq.cu", "mmq_stream.cu", "mmq_tc.cu", "mul_mat.cu", "fattn.cu", "rowops.cu", "kvops.cu", "fused.cu", "peer.cu"]
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
     "-Xcompiler", "-fPIC,-fvisibility=hidden", "--fmad=true",

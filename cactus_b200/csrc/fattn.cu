@@ -16,6 +16,7 @@
 #include <cstdlib>
 
 #include "common.cuh"
+#include "mma_s8.cuh"
 
 namespace b200 {
 
@@ -260,16 +261,6 @@ struct FattnParams {
                      // 1 = these are the per-token kernel's launches, 2 = the query-tiled kernel's
     int early;       // one or two tokens: the combine pass lets the next kernel's CTAs in at once (pdl_early_rows)
 };
-
-__device__ __forceinline__ void mma_f16(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
-    asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"
-        : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
-        : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
-}
-__device__ __forceinline__ uint32_t pack_half2(float lo, float hi) {
-    const __half2 h = __floats2half2_rn(lo, hi);
-    return *reinterpret_cast<const uint32_t *>(&h);
-}
 
 }  // namespace b200
 #include "fattn_tile.cuh"   // the query-tiled kernel for ubatches with many tokens

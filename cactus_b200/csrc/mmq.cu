@@ -22,6 +22,7 @@
 #include <mutex>
 
 #include "common.cuh"
+#include "mma_s8.cuh"
 
 namespace b200 {
 
@@ -33,59 +34,6 @@ __device__ __forceinline__ void cp_async16(void *smem, const void *gmem) {
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
 template <int N>
 __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory"); }
-
-__device__ __forceinline__ void mma_s8_magic(uint32_t (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
-    const uint32_t magic = 0x4B400000u;
-    asm volatile(
-        "mma.sync.aligned.m16n8k32.row.col.s32.s8.s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};\n"
-        : "=r"(c[0]), "=r"(c[1]), "=r"(c[2]), "=r"(c[3])
-        : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "r"(magic));
-}
-// One k=32 step of a 16x8 tile and its epilogue in a single block, so the accumulator pairs stay in aligned
-// register pairs: c = A.B + 0x4B400000 (bits of 12582912 + dot); t = d_a * c - d_a * 12582912; y += d_w * t.
-__device__ __forceinline__ void mma_scale_acc(uint64_t &y01, uint64_t &y23, uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0,
-                                              uint32_t b1, uint64_t da, uint64_t nda, uint64_t dw01, uint64_t dw23) {
-    asm("{\n"
-        ".reg .b32 c0, c1, c2, c3;\n"
-        ".reg .b64 p01, p23;\n"
-        "mma.sync.aligned.m16n8k32.row.col.s32.s8.s8.s32 {c0,c1,c2,c3}, {%2,%3,%4,%5}, {%6,%7}, {%12,%12,%12,%12};\n"
-        "mov.b64 p01, {c0,c1};\n"
-        "mov.b64 p23, {c2,c3};\n"
-        "fma.rn.f32x2 p01, p01, %8, %9;\n"
-        "fma.rn.f32x2 p23, p23, %8, %9;\n"
-        "fma.rn.f32x2 %0, p01, %10, %0;\n"
-        "fma.rn.f32x2 %1, p23, %11, %1;\n"
-        "}\n"
-        : "+l"(y01), "+l"(y23)
-        : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "l"(da), "l"(nda), "l"(dw01), "l"(dw23), "r"(0x4B400000u));
-}
-// k=32 MMA step alone, accumulator pairs returned packed (aligned register pairs for the f32x2 epilogue)
-__device__ __forceinline__ void mma_s8_magic2(uint64_t &p01, uint64_t &p23, uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
-    asm("{\n"
-        ".reg .b32 c0, c1, c2, c3;\n"
-        "mma.sync.aligned.m16n8k32.row.col.s32.s8.s8.s32 {c0,c1,c2,c3}, {%2,%3,%4,%5}, {%6,%7}, {%8,%8,%8,%8};\n"
-        "mov.b64 %0, {c0,c1};\n"
-        "mov.b64 %1, {c2,c3};\n"
-        "}\n"
-        : "=l"(p01), "=l"(p23)
-        : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "r"(0x4B400000u));
-}
-__device__ __forceinline__ uint64_t pack2(uint32_t lo, uint32_t hi) {
-    uint64_t r;
-    asm("mov.b64 %0, {%1,%2};" : "=l"(r) : "r"(lo), "r"(hi));
-    return r;
-}
-__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
-    uint64_t r;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-    return r;
-}
-__device__ __forceinline__ void unpack2(uint64_t v, float &lo, float &hi) {
-    uint32_t a, b;
-    asm("mov.b64 {%0,%1}, %2;" : "=r"(a), "=r"(b) : "l"(v));
-    lo = __uint_as_float(a);
-    hi = __uint_as_float(b);
-}
 
 template <int WTYPE>
 struct WFrag {  // one block group of one 16-row tile: quants of rows g / g+8 and their four block scales

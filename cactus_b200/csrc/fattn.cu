@@ -259,6 +259,7 @@ struct FattnParams {
     int slots;       // CTAs of this kernel the device holds at once
     int vote;        // both attention kernels were launched and the plan decides which one works (the other returns at once):
                      // 1 = these are the per-token kernel's launches, 2 = the query-tiled kernel's
+    int parts;       // every token's result goes through `partial`, also that of a single split: the combine pass quantises them all
     int early;       // one or two tokens: the combine pass lets the next kernel's CTAs in at once (pdl_early_rows)
 };
 
@@ -294,6 +295,17 @@ __device__ __noinline__ void fattn_quant_block(uint8_t *qout, size_t d_offset, i
     q8_quantize_store_warp<1>(val, qout, d_offset, nb, nbp, n, b, real, variant);
 }
 
+// Block b of the padding columns n .. (the rest of their 8-column tile) as the quantiser leaves it: zeros
+__device__ __noinline__ void fattn_quant_pad(uint8_t *qout, size_t d_offset, int64_t nbp, int64_t n, int64_t b) {
+    const int lane = threadIdx.x & 31, g = (int) (n & 7);
+    if (lane >= 4 * g) *reinterpret_cast<uint2 *>(qout + ((n >> 3) * nbp + b) * 256 + lane * 8) = make_uint2(0u, 0u);
+    if (lane >= g && lane < 8) {
+        float *dp = reinterpret_cast<float *>(qout + d_offset) + ((n >> 3) * (nbp >> 2) + (b >> 2)) * 64 + act_scale_index((int) (b & 3), lane);
+        dp[0] = 0.0f;
+        dp[2] = -0.0f;
+    }
+}
+
 // One output element; a warp calls this for 32 consecutive d of one (token, head).  With QUANT the row is also (or only)
 // stored as Q8_0 blocks -- quantize_row_q8_0 applied to the f32 value, bit for bit what the separate quantiser makes of
 // dst -- and the last token's warps zero the padding columns of its 8-column tile.
@@ -306,9 +318,7 @@ __device__ __forceinline__ void fattn_store_out(const FattnParams &p, int64_t j,
     if (p.dst) p.dst[(j * p.H + head) * D + d] = val;
     const int64_t b = (head * D + d) >> 5;
     fattn_quant_block(p.qout, p.q_d_offset, p.q_nb, p.q_nbp, p.q_variant, j, b, val, true);
-    if (j == p.Nq - 1) {
-        for (int64_t n = p.Nq; n < ((p.Nq + 7) & ~(int64_t) 7); ++n) fattn_quant_block(p.qout, p.q_d_offset, p.q_nb, p.q_nbp, p.q_variant, n, b, 0.0f, false);
-    }
+    if (j == p.Nq - 1 && (p.Nq & 7)) fattn_quant_pad(p.qout, p.q_d_offset, p.q_nbp, p.Nq, b);
 }
 
 // QUANT: the instantiation behind b200_flash_attn_ext_quant; kept apart because this kernel sits at its register limit
@@ -542,7 +552,7 @@ __global__ void __launch_bounds__(FA_THREADS, FA_MIN_CTAS) fattn_mma_kernel(Fatt
             ls += merge_l[wv][h] * scl;
         }
         const int64_t head = h0 + h;
-        if (ns_j == 1) {
+        if (ns_j == 1 && !p.parts) {
             fattn_store_out<D, QUANT>(p, j, head, d, a * (1.0f / ls));
         } else {
             float *pp = p.partial + ((j * p.H + head) * p.nsplit + split) * (D + 2);
@@ -656,7 +666,7 @@ __global__ void __launch_bounds__(FC_THREADS) fattn_combine_kernel(FattnParams p
         const int w0 = fattn_target_words(p, ctas_per_token);
         const int64_t n_words = p.wcount ? (int64_t) p.wcount[tok] : p.nw;
         nsplit = (int) min((int64_t) nsplit, max((int64_t) 1, (n_words + w0 - 1) / w0));
-        if (nsplit == 1) return;
+        if (nsplit == 1 && !p.parts) return;
     }
     float ms[2], l[2];   // of splits lane and lane + 32 (at most 64)
 #pragma unroll
@@ -725,7 +735,9 @@ static int fattn_nsplit(int64_t Nq, int64_t Hkv, int hgroups, int64_t n_kv) {
     const int64_t want = 2 * fa_sm_count();
     if (ctas >= want) return 1;
     int64_t ns = (want + ctas - 1) / ctas;
-    ns = std::min<int64_t>(ns, std::max<int64_t>(1, n_kv / 512));
+    // At least 512 cells of the cache to a split, from 1024 cells on 128 (a token's own words are dealt out evenly, two at least): one
+    // sequence of 640 cells in 1024, 1B architecture, 825 us a step with two splits, 778 with four or more.
+    ns = std::min<int64_t>(ns, n_kv >= 1024 ? n_kv / 128 : 1);
     return (int) std::min<int64_t>(ns, 64);
 }
 
@@ -894,6 +906,7 @@ static int flash_attn_impl(bool parity, int64_t D, int64_t H, int64_t Hkv, int64
     int gqa_log2 = 0;
     while ((1 << gqa_log2) < gqa) ++gqa_log2;
     p.vote = 0;
+    p.parts = 0;
     p.early = Nq <= pdl_early_rows() ? 1 : 0;
     if (!act && dst && fattn_tile_possible(Nq, gqa) && p.nw <= 2048) {
         FattnParams pt = p;
@@ -937,7 +950,9 @@ static int flash_attn_impl(bool parity, int64_t D, int64_t H, int64_t Hkv, int64
         p.vote = 1;
     }
     dim3 grid((unsigned) (Hkv * hgroups), (unsigned) Nq, (unsigned) ns);
-    const bool qo = act != nullptr;
+    // With KV splits the combine pass is what quantises: it has the registers for that, the main kernel has not.
+    const bool qo = act != nullptr && ns == 1, qc = act != nullptr;
+    p.parts = qc && ns > 1 ? 1 : 0;
     if (D == 128) {
         if (qo) launch_pdl(fattn_mma_kernel<128, true>, grid, dim3(FA_THREADS), 0, st, p);
         else launch_pdl(fattn_mma_kernel<128, false>, grid, dim3(FA_THREADS), 0, st, p);
@@ -949,10 +964,10 @@ static int flash_attn_impl(bool parity, int64_t D, int64_t H, int64_t Hkv, int64
     if (ns > 1) {
         const int cpt = (int) (Hkv * hgroups);
         if (D == 128) {
-            if (qo) launch_combine<128, true>(p, cpt, st);
+            if (qc) launch_combine<128, true>(p, cpt, st);
             else launch_combine<128, false>(p, cpt, st);
         } else {
-            if (qo) launch_combine<64, true>(p, cpt, st);
+            if (qc) launch_combine<64, true>(p, cpt, st);
             else launch_combine<64, false>(p, cpt, st);
         }
         return check_launch("fattn_combine");

@@ -163,11 +163,6 @@ class LlamaEngine:
         assert n_cells % 256 == 0, "the cache is padded to 256 cells for flash attention (cactus/llama-kv-cache.cpp:20-23)"
         self.w, self.cfg, self.n_cells, self.max_tokens, self.variant = weights, weights.cfg, n_cells, max_tokens, variant
         self.use_graphs = use_graphs
-        # up to this many tokens the attention leaves its output quantised itself (b200_flash_attn_ext_quant: one launch
-        # less per layer, bit-identical).  Off: measured on B200 it is slower at every token count -- one sequence of the
-        # 8B architecture 2.52-2.58 ms per token against 2.40 with the separate quantiser, the 64-token batch 70.5 us per
-        # attention against 57.5 + 2.5 (the attention kernel sits at its register limit).  B200_FA_QUANT_MAX_T sets it.
-        self.fa_quant_max_tokens = int(os.environ.get("B200_FA_QUANT_MAX_T", "0"))
         # row split (cactus_b200.rowsplit.RowSplit): ``weights`` then holds this rank's rows of every mul_mat weight,
         # each product is joined into buffers the peers can write, everything else is replicated
         self.split = split
@@ -240,6 +235,12 @@ class LlamaEngine:
         ws = [L.b200_mul_mat_workspace_bytes(cfg.layer_type, K, M, t) for K, M in shapes for t in range(1, T + 1)]
         ws += [L.b200_mul_mat_workspace_bytes(cfg.head_type, cfg.d_model, cfg.vocab // g, t) for t in range(1, T + 1)]
         self.ws = u8(max(ws))
+        # Where the attention cuts its KV range, the pass that adds the splits leaves the result quantised (b200_flash_attn_ext_quant: one
+        # launch less per layer, bit-identical).  Without splits the attention kernel itself would have to, at its register limit:
+        # 70.5 us for the 64-token batch against 57.5 + 2.5.  B200_FA_QUANT_MAX_T lowers the token count.
+        fa_args = (cfg.head_dim, self.n_head_local, self.n_kv_head_local)
+        split_kv = [L.b200_flash_attn_scratch_bytes(*fa_args, t, n_cells) > L.b200_mask_index_bytes(t, n_cells) for t in range(1, min(T, 128) + 1)]
+        self.fa_quant_max_tokens = min(split_kv.index(False) if False in split_kv else len(split_kv), int(os.environ.get("B200_FA_QUANT_MAX_T", "128")))
         self.fa_scratch = u8(max(L.b200_flash_attn_scratch_bytes(cfg.head_dim, self.n_head_local, self.n_kv_head_local, t, n_cells) for t in range(1, T + 1)))
         self.graphs: dict[int, torch.cuda.CUDAGraph] = {}
         self.launches_per_step: dict[int, int] = {}

@@ -188,6 +188,70 @@ __global__ void __launch_bounds__(512) rope_store_kernel(const float *q, float *
     for (unsigned i = threadIdx.x + U * blockDim.x; i < total; i += blockDim.x) finish(i, load(i));
 }
 
+// The angles of a ubatch's tokens, [token][n_dims/2 cosines, n_dims/2 sines], for rope_store_angles_kernel: every layer rotates by the
+// same ones.  theta_a = pos * theta_scale^a by repeated multiplication, as the reference builds it.
+__global__ void __launch_bounds__(128) rope_angles_kernel(float *__restrict__ angles, int n_dims, const int32_t *__restrict__ pos, const float *__restrict__ ff,
+                                                          float theta_scale, float freq_scale, float attn_factor) {
+    pdl_prologue();
+    const int64_t t = blockIdx.x;
+    const int half_dims = n_dims / 2;
+    for (int i = threadIdx.x; i < n_dims; i += blockDim.x) {
+        const int a = i < half_dims ? i : i - half_dims;
+        const float f = ff ? ff[a] : 1.0f;
+        float theta = (float) pos[t], mine = theta;
+#pragma unroll 8
+        for (int s = 0; s <= a; ++s) {
+            mine = theta;
+            theta *= theta_scale;
+        }
+        const float th = freq_scale * (mine / f);
+        angles[t * n_dims + i] = (i < half_dims ? cosf(th) : sinf(th)) * attn_factor;
+    }
+}
+
+// rounded as the compiler rounds it in rope_store_kernel, whichever of the two products it would fuse here
+__device__ __forceinline__ float2 rotate_pair(float2 x, float c, float sn) { return make_float2(fmaf(x.x, c, -__fmul_rn(x.y, sn)), fmaf(x.y, c, __fmul_rn(x.x, sn))); }
+
+// rope_store_kernel with the angles at hand: nothing to wait for but the rows.  Bound by latency: three CTAs per token for 48 heads of
+// 128, and as many threads as a head has pairs (or a multiple), so that a thread needs one angle for all its pairs.  us per launch on
+// B200, with the angles worked out in each launch / at hand: 64 tokens 6.4 / 4.1, 1 token 4.9 / 3.7.
+constexpr int RA_UNROLL = 4;
+__global__ void __launch_bounds__(256) rope_store_angles_kernel(float *q, int64_t q_nb_head, int64_t q_nb_tok, const float *__restrict__ k, int64_t k_nb_head, int64_t k_nb_tok,
+                                                               const float *__restrict__ v, int64_t v_nb_tok, int pairs, int H, int Hkv, int n_dims,
+                                                               const float *__restrict__ angles, const int32_t *__restrict__ slots, __half *__restrict__ kc, int64_t kc_nb_row,
+                                                               __half *__restrict__ vc, int64_t vc_nb_row, int early) {
+    if (early) pdl_trigger();
+    const int64_t t = blockIdx.x;
+    const int half_dims = n_dims / 2, p = threadIdx.x % pairs, per = blockDim.x / pairs;   // heads of one pass
+    const int h0 = blockIdx.y * per * RA_UNROLL + threadIdx.x / pairs;
+    pdl_prologue();
+    const bool turns = p < half_dims;
+    const float c = turns ? __ldg(angles + t * n_dims + p) : 1.0f, sn = turns ? __ldg(angles + t * n_dims + half_dims + p) : 0.0f;
+    const int64_t slot = slots[t];
+    float2 x[RA_UNROLL];
+#pragma unroll
+    for (int u = 0; u < RA_UNROLL; ++u) {
+        const int h = min(h0 + u * per, H + 2 * Hkv - 1);   // (never conditional: a load behind a branch is waited for where it ends)
+        const char *row = h < H ? reinterpret_cast<const char *>(q) + t * q_nb_tok + h * q_nb_head
+                                : h < H + Hkv ? reinterpret_cast<const char *>(k) + t * k_nb_tok + (h - H) * k_nb_head
+                                              : reinterpret_cast<const char *>(v) + t * v_nb_tok + (int64_t) (h - H - Hkv) * pairs * 8;
+        x[u] = *(reinterpret_cast<const float2 *>(row) + p);
+    }
+    pdl_trigger();
+#pragma unroll
+    for (int u = 0; u < RA_UNROLL; ++u) {
+        const int h = h0 + u * per;
+        if (h >= H + 2 * Hkv) break;
+        const float2 r = h < H + Hkv && turns ? rotate_pair(x[u], c, sn) : x[u];
+        if (h < H) {
+            if (turns) *(reinterpret_cast<float2 *>(reinterpret_cast<char *>(q) + t * q_nb_tok + h * q_nb_head) + p) = r;
+        } else {
+            char *row = h < H + Hkv ? reinterpret_cast<char *>(kc) + slot * kc_nb_row + (int64_t) (h - H) * pairs * 4 : reinterpret_cast<char *>(vc) + slot * vc_nb_row + (int64_t) (h - H - Hkv) * pairs * 4;
+            *(reinterpret_cast<__half2 *>(row) + p) = __halves2half2(__float2half_rn(r.x), __float2half_rn(r.y));
+        }
+    }
+}
+
 }  // namespace b200
 
 using namespace b200;
@@ -256,6 +320,29 @@ int b200_rope_store_to(const float *q, float *q_dst, int64_t q_nb_head, int64_t 
         q, q_dst, q_nb_head, q_nb_tok, k, k_nb_head, k_nb_tok, v, v_nb_tok, D, H, Hkv, n_dims, pos, freq_factors, theta_scale, freq_scale, attn_factor,
         slots, (__half *) k_cache, k_cache_nb_row, (__half *) v_cache, v_cache_nb_row, T <= pdl_early_rows() ? 1 : 0);
     return check_launch("rope_store");
+}
+
+int b200_rope_angles(float *angles, int64_t T, int n_dims, const int32_t *pos, const float *freq_factors, float freq_base, float freq_scale,
+                     float attn_factor, b200_stream_t stream) {
+    B200_REQUIRE(angles && pos && T > 0 && n_dims > 0 && n_dims % 2 == 0 && n_dims <= 8192 && is_aligned(angles, 4), "bad rope arguments");
+    const float theta_scale = powf(freq_base, -2.0f / (float) n_dims);
+    launch_pdl(rope_angles_kernel, dim3((unsigned) T), dim3(128), 0, (cudaStream_t) stream, angles, n_dims, pos, freq_factors, theta_scale, freq_scale, attn_factor);
+    return check_launch("rope_angles");
+}
+
+int b200_rope_store_angles(float *q, int64_t q_nb_head, int64_t q_nb_tok, const float *k, int64_t k_nb_head, int64_t k_nb_tok, const float *v,
+                           int64_t v_nb_tok, int64_t D, int64_t H, int64_t Hkv, int64_t T, int n_dims, const float *angles, const int32_t *slots,
+                           void *k_cache, int64_t k_cache_nb_row, void *v_cache, int64_t v_cache_nb_row, b200_stream_t stream) {
+    B200_REQUIRE(q && k && v && angles && slots && k_cache && v_cache && T > 0 && H > 0 && Hkv > 0 && H + 2 * Hkv <= 4096, "bad rope_store arguments");
+    B200_REQUIRE((D == 64 || D == 128 || D == 256) && n_dims > 0 && n_dims % 2 == 0 && n_dims <= D, "head size %lld not supported (64, 128 or 256)", (long long) D);
+    B200_REQUIRE(is_aligned(q, 8) && is_aligned(k, 8) && is_aligned(v, 8) && q_nb_head % 8 == 0 && q_nb_tok % 8 == 0 && k_nb_head % 8 == 0 && k_nb_tok % 8 == 0 && v_nb_tok % 8 == 0,
+                 "rope rows must be 8-byte aligned");
+    B200_REQUIRE(is_aligned(k_cache, 4) && is_aligned(v_cache, 4) && k_cache_nb_row % 4 == 0 && v_cache_nb_row % 4 == 0, "cache rows must be 4-byte aligned");
+    const int pairs = (int) D / 2, per = 256 / pairs;
+    const dim3 grid((unsigned) T, (unsigned) ((H + 2 * Hkv + per * RA_UNROLL - 1) / (per * RA_UNROLL)));
+    launch_pdl(rope_store_angles_kernel, grid, dim3(256), 0, (cudaStream_t) stream, q, q_nb_head, q_nb_tok, k, k_nb_head, k_nb_tok, v, v_nb_tok, pairs, (int) H, (int) Hkv, n_dims,
+               angles, slots, (__half *) k_cache, k_cache_nb_row, (__half *) v_cache, v_cache_nb_row, T <= pdl_early_rows() ? 1 : 0);
+    return check_launch("rope_store_angles");
 }
 
 }  // extern "C"

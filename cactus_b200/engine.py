@@ -212,6 +212,7 @@ class LlamaEngine:
         self.inp_host = torch.zeros((4, T), dtype=torch.int32).pin_memory()
         self.mask = torch.empty(((T + 63) // 64 * 64, n_cells), dtype=torch.float16, device=dev)
         self.index = u8(L.b200_mask_index_bytes(T, n_cells))
+        self.angles = f32(T, cfg.head_dim)   # of ROPE: the same for every layer
         self.x, self.h, self.attn = f32(T, cfg.d_model), f32(T, cfg.d_model), f32(T, cfg.d_model)
         out = split.carve if split is not None else f32   # mul_mat outputs: where the peers' slices land
         if self.fused:   # the stacked products, and the reference's q/k/v and gate/up as column ranges of them
@@ -271,6 +272,7 @@ class LlamaEngine:
         check(L.b200_scatter_i32(self.cell_pos.data_ptr(), slots, pos, T, st))
         check(L.b200_scatter_i32(self.cell_seq.data_ptr(), slots, seq, T, st))
         check(L.b200_kq_mask_build(self.cell_pos.data_ptr(), self.cell_seq.data_ptr(), nkv, pos, seq, T, self.mask.data_ptr(), nkv * 2, st))
+        check(L.b200_rope_angles(self.angles.data_ptr(), T, D, pos, None, cfg.rope_theta, 1.0, 1.0, st))
         check(L.b200_mask_index_build(self.mask.data_ptr(), nkv * 2, T, nkv, self.index.data_ptr(), self.index.numel(), st))
         emb: QWeight = self.w.tensors["token_embd.weight"]
         check(L.b200_get_rows_q(emb.wtype, emb.data.data_ptr(), emb.K, emb.M, tokens, self.x.data_ptr(), d * 4, T, st))
@@ -294,8 +296,8 @@ class LlamaEngine:
                 self._mm(p + "attn_v.weight", self.act_d, T, self.v)
             kc, vc = self.k_cache[il], self.v_cache[il]
             qs, kst, vst = self.q.stride(0) * 4, self.k.stride(0) * 4, self.v.stride(0) * 4
-            check(L.b200_rope_store(self.q.data_ptr(), D * 4, qs, self.k.data_ptr(), D * 4, kst, self.v.data_ptr(), vst, D, H, Hkv, T, D,
-                                    pos, None, cfg.rope_theta, 1.0, 1.0, slots, kc.data_ptr(), kvd * 2, vc.data_ptr(), kvd * 2, st))
+            check(L.b200_rope_store_angles(self.q.data_ptr(), D * 4, qs, self.k.data_ptr(), D * 4, kst, self.v.data_ptr(), vst, D, H, Hkv, T, D,
+                                           self.angles.data_ptr(), slots, kc.data_ptr(), kvd * 2, vc.data_ptr(), kvd * 2, st))
             attn_args = (D, H, Hkv, T, nkv, self.q.data_ptr(), qs, D * 4, kc.data_ptr(), kvd * 2, D * 2, vc.data_ptr(), kvd * 2, D * 2,
                          self.mask.data_ptr(), nkv * 2, self.index.data_ptr(), D ** -0.5, 0.0, 0.0)
             if T <= self.fa_quant_max_tokens and not self.hp:

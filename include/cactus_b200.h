@@ -298,6 +298,15 @@ B200_API int b200_rope_store_to(const float *q, float *q_dst, int64_t q_nb_head,
                                 const int32_t *slots, void *k_cache, int64_t k_cache_nb_row, void *v_cache, int64_t v_cache_nb_row,
                                 b200_stream_t stream);
 
+/* b200_rope_store in two calls, for a caller whose layers all rotate by the same angles: b200_rope_angles works them out once
+ * ([T][n_dims]: n_dims/2 cosines, n_dims/2 sines), b200_rope_store_angles applies them.  Bit-identical to b200_rope_store. */
+B200_API int b200_rope_angles(float *angles, int64_t T, int n_dims, const int32_t *pos, const float *freq_factors, float freq_base, float freq_scale,
+                              float attn_factor, b200_stream_t stream);
+B200_API int b200_rope_store_angles(float *q, int64_t q_nb_head, int64_t q_nb_tok, const float *k, int64_t k_nb_head, int64_t k_nb_tok, const float *v,
+                                    int64_t v_nb_tok, int64_t D, int64_t H, int64_t Hkv, int64_t T, int n_dims, const float *angles,
+                                    const int32_t *slots, void *k_cache, int64_t k_cache_nb_row, void *v_cache, int64_t v_cache_nb_row,
+                                    b200_stream_t stream);
+
 /* ------------------------------------------------------------------------------------------------
  * Row-split mul_mat over the GPUs of one node (one process per GPU).
  *

@@ -2,7 +2,10 @@
 // the attention mask (llama_kv_cache_unified::set_input_kq_mask, cactus/llama-kv-cache.cpp:696-761),
 // the K/V store into cache rows (cpy_k / cpy_v, :617-656) addressed by slot index, and greedy argmax over
 // logits (the sampler step after llama_get_logits, cactus/cactus_completion.cpp:210).
+#include <cooperative_groups.h>
 #include <math_constants.h>
+
+#include <algorithm>
 
 #include "common.cuh"
 
@@ -73,13 +76,19 @@ __global__ void __launch_bounds__(256) set_rows_f16_kernel(const float *__restri
     reinterpret_cast<__half *>(reinterpret_cast<char *>(dst) + (int64_t) slots[r] * dst_nb_row)[c] = __float2half_rn(v);
 }
 
-// first index of the maximum of each row (ties: lowest index, as a linear scan finds it).  One CTA of 1024 threads per row,
-// 16-byte loads where the row allows them: a vocabulary-sized row is a chain of dependent compares per thread, so the time
-// is the number of elements a thread walks
-constexpr int ARGMAX_THREADS = 1024;
-__global__ void __launch_bounds__(ARGMAX_THREADS) argmax_rows_kernel(const float *__restrict__ x, int64_t x_nb_row, int64_t d,
-                                                                    int32_t *__restrict__ out) {
-    const int64_t r = blockIdx.x;
+// first index of the maximum of each row (ties: lowest index, as a linear scan finds it).  A cluster of 8 CTAs per row, each with an
+// eighth of it: bound by latency, the load of a thread's elements (8 x 16 bytes for a vocabulary of 128256, all on their way at
+// once) and the reduction.  16-byte loads where the row allows them.  us per launch on B200, one CTA of 1024 threads per row / this:
+// 1 x 128256 11.7 / 6.8, 64 x 128256 13.1 / 10.0.
+constexpr int ARGMAX_THREADS = 512, ARGMAX_CTAS = 8;
+__global__ void __cluster_dims__(ARGMAX_CTAS, 1, 1) __launch_bounds__(ARGMAX_THREADS) argmax_rows_kernel(const float *__restrict__ x, int64_t x_nb_row, int64_t d,
+                                                                                                        int32_t *__restrict__ out) {
+    const cooperative_groups::cluster_group cluster = cooperative_groups::this_cluster();
+    cluster.barrier_arrive();   // (the first CTA's shared memory may be written once it has started: the wait is below)
+    pdl_prologue();
+    constexpr int WARPS = ARGMAX_THREADS / 32, ALL = ARGMAX_THREADS * ARGMAX_CTAS;
+    const int64_t r = blockIdx.y;
+    const int part = blockIdx.x, tid = threadIdx.x, me = part * ARGMAX_THREADS + tid;
     const float *row = reinterpret_cast<const float *>(reinterpret_cast<const char *>(x) + r * x_nb_row);
     float best = -CUDART_INF_F;
     int bi = 0x7fffffff;
@@ -87,8 +96,8 @@ __global__ void __launch_bounds__(ARGMAX_THREADS) argmax_rows_kernel(const float
     if ((reinterpret_cast<uintptr_t>(row) & 15) == 0) {
         const int64_t n4 = d >> 2;
         const float4 *row4 = reinterpret_cast<const float4 *>(row);
-#pragma unroll 4
-        for (int64_t i = threadIdx.x; i < n4; i += ARGMAX_THREADS) {
+#pragma unroll 8
+        for (int64_t i = me; i < n4; i += ALL) {
             const float4 v = __ldg(row4 + i);
             const int b = (int) (i << 2);
             if (v.x > best) { best = v.x; bi = b; }
@@ -98,34 +107,45 @@ __global__ void __launch_bounds__(ARGMAX_THREADS) argmax_rows_kernel(const float
         }
         done = n4 << 2;
     }
-    for (int64_t i = done + threadIdx.x; i < d; i += ARGMAX_THREADS) {
+    for (int64_t i = done + me; i < d; i += ALL) {
         const float v = row[i];
         if (v > best) { best = v; bi = (int) i; }
     }
     // a thread's candidate is the first maximum among its own elements; between threads the lower index wins a tie
+    auto fold = [&](int from) {
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        const float ov = __shfl_xor_sync(0xffffffffu, best, o);
-        const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
-        if (ov > best || (ov == best && oi < bi)) { best = ov; bi = oi; }
-    }
-    __shared__ float sv[ARGMAX_THREADS / 32];
-    __shared__ int si[ARGMAX_THREADS / 32];
-    if ((threadIdx.x & 31) == 0) {
-        sv[threadIdx.x >> 5] = best;
-        si[threadIdx.x >> 5] = bi;
-    }
-    __syncthreads();
-    if (threadIdx.x < 32) {
-        best = sv[threadIdx.x];
-        bi = si[threadIdx.x];
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
+        for (int o = from; o > 0; o >>= 1) {
             const float ov = __shfl_xor_sync(0xffffffffu, best, o);
             const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
             if (ov > best || (ov == best && oi < bi)) { best = ov; bi = oi; }
         }
-        if (threadIdx.x == 0) out[r] = bi == 0x7fffffff ? 0 : bi;   // nothing above -inf: a linear scan stays at index 0
+    };
+    __shared__ float sv[WARPS];
+    __shared__ int si[WARPS];
+    __shared__ float cv[ARGMAX_CTAS];   // of the cluster's first CTA: every CTA's candidate
+    __shared__ int ci[ARGMAX_CTAS];
+    fold(16);
+    if ((tid & 31) == 0) {
+        sv[tid >> 5] = best;
+        si[tid >> 5] = bi;
+    }
+    __syncthreads();
+    cluster.barrier_wait();
+    if (tid < 32) {
+        best = sv[tid & (WARPS - 1)];
+        bi = si[tid & (WARPS - 1)];
+        fold(WARPS / 2);
+        if (tid == 0) {
+            cluster.map_shared_rank(cv, 0)[part] = best;
+            cluster.map_shared_rank(ci, 0)[part] = bi;
+        }
+    }
+    cluster.sync();
+    if (part == 0 && tid < 32) {
+        best = cv[tid & (ARGMAX_CTAS - 1)];
+        bi = ci[tid & (ARGMAX_CTAS - 1)];
+        fold(ARGMAX_CTAS / 2);
+        if (tid == 0) out[r] = bi == 0x7fffffff ? 0 : bi;   // nothing above -inf: a linear scan stays at index 0
     }
 }
 
@@ -170,7 +190,10 @@ int b200_set_rows_f16(const float *x, int64_t x_nb_row, const int32_t *slots, vo
 int b200_argmax_rows(const float *x, int64_t x_nb_row, int64_t d, int64_t rows, int32_t *out, b200_stream_t stream) {
     B200_REQUIRE(x && out && d > 0 && rows >= 0 && x_nb_row % 4 == 0, "bad argmax arguments");
     if (rows == 0) return B200_OK;
-    argmax_rows_kernel<<<(unsigned) rows, ARGMAX_THREADS, 0, (cudaStream_t) stream>>>(x, x_nb_row, d, out);
+    for (int64_t r0 = 0; r0 < rows; r0 += 65535) {   // (a grid has at most 65535 rows)
+        const dim3 grid(ARGMAX_CTAS, (unsigned) std::min<int64_t>(65535, rows - r0));
+        launch_pdl(argmax_rows_kernel, grid, dim3(ARGMAX_THREADS), 0, (cudaStream_t) stream, reinterpret_cast<const float *>(reinterpret_cast<const char *>(x) + r0 * x_nb_row), x_nb_row, d, out + r0);
+    }
     return check_launch("argmax_rows");
 }
 

@@ -72,6 +72,40 @@ static inline cudaError_t launch_pdl(void (*kernel)(P...), dim3 grid, dim3 block
 #endif
 static inline bool is_aligned(const void *p, size_t a) { return ((uintptr_t) p % a) == 0; }
 
+// ---- ROPE and the K/V store as the end of the product that makes q, k and v ----------------------------
+// Rows 0 .. q_rows - 1 of the product are q (rotated, into dst as they lie), up to k_end k (rotated, f16 into the token's cache row),
+// then v (f16).  `angles` is what b200_rope_angles makes.  The products of up to 8 columns take it as their end: a launch less per layer and
+// no round trip of k and v through memory.  us per decode step on B200, launch of its own / this: 1B architecture, one sequence 733 / 722,
+// 8B, seven sequences 2568 / 2521.
+struct RopeStore {
+    const float *angles;
+    const int32_t *slots;
+    __half *kc, *vc;
+    int64_t kc_nb_row, vc_nb_row;
+    int q_rows, k_end, pair_mask, half_dims;   // pair_mask: pairs of a head less one (heads of 64, 128 or 256)
+};
+#ifdef __CUDACC__
+// rounded as the compiler rounds it in rope_store_kernel, whichever of the two products it would fuse here
+__device__ __forceinline__ float2 rotate_pair(float2 x, float c, float sn) { return make_float2(fmaf(x.x, c, -__fmul_rn(x.y, sn)), fmaf(x.y, c, __fmul_rn(x.x, sn))); }
+// the angle of pair row / 2 of token n; (1, 0) where nothing turns
+__device__ __forceinline__ float2 rope_angle(const RopeStore &r, int n, int row) {
+    const int p = (row >> 1) & r.pair_mask;
+    if (row >= r.k_end || p >= r.half_dims) return make_float2(1.0f, 0.0f);
+    const float *a = r.angles + (int64_t) n * 2 * r.half_dims + p;
+    return make_float2(__ldg(a), __ldg(a + r.half_dims));
+}
+// rows `row` (even) and row + 1 of column n
+__device__ __forceinline__ void rope_store_pair(const RopeStore &r, float *dst, int64_t dst_nb_row, int n, int row, float2 x, float2 angle, int64_t slot) {
+    if (row < r.k_end && ((row >> 1) & r.pair_mask) < r.half_dims) x = rotate_pair(x, angle.x, angle.y);
+    if (row < r.q_rows) {
+        *reinterpret_cast<float2 *>(reinterpret_cast<char *>(dst) + n * dst_nb_row + (int64_t) row * 4) = x;
+    } else {
+        char *to = row < r.k_end ? reinterpret_cast<char *>(r.kc) + slot * r.kc_nb_row + (row - r.q_rows) * 2 : reinterpret_cast<char *>(r.vc) + slot * r.vc_nb_row + (row - r.k_end) * 2;
+        *reinterpret_cast<__half2 *>(to) = __halves2half2(__float2half_rn(x.x), __float2half_rn(x.y));
+    }
+}
+#endif
+
 // ---- row split: the other GPUs' copies of a product ------------------------------------------------
 // A mul_mat kernel stores every result value into its own dst and, when the weight is one row slice of a split, into
 // the same place of the other GPUs' output buffers (peer memory mapped through CUDA IPC): p[i] is the address in peer

@@ -209,9 +209,6 @@ __global__ void __launch_bounds__(128) rope_angles_kernel(float *__restrict__ an
     }
 }
 
-// rounded as the compiler rounds it in rope_store_kernel, whichever of the two products it would fuse here
-__device__ __forceinline__ float2 rotate_pair(float2 x, float c, float sn) { return make_float2(fmaf(x.x, c, -__fmul_rn(x.y, sn)), fmaf(x.y, c, __fmul_rn(x.x, sn))); }
-
 // rope_store_kernel with the angles at hand: nothing to wait for but the rows.  Bound by latency: three CTAs per token for 48 heads of
 // 128, and as many threads as a head has pairs (or a multiple), so that a thread needs one angle for all its pairs.  us per launch on
 // B200, with the angles worked out in each launch / at hand: 64 tokens 6.4 / 4.1, 1 token 4.9 / 3.7.

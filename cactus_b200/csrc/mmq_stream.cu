@@ -40,9 +40,9 @@ struct MsTile {   // a T16 tile as a lane holds it
     uint2 sa, sb;
 };
 
-template <int WTYPE>
+template <int WTYPE, bool ROPE>   // ROPE: the rows are those of q, k and v (RopeStore)
 __global__ void __launch_bounds__(MS_THREADS, 1) mmq_stream_kernel(TiledDims dims, const uint8_t *__restrict__ w, ActDims act, const uint8_t *__restrict__ aq,
-                                                                float *__restrict__ dst, int64_t dst_nb_row, MsPlan plan) {
+                                                                float *__restrict__ dst, int64_t dst_nb_row, MsPlan plan, RopeStore rope) {
     constexpr int RING = WTYPE == B200_TYPE_Q4_0 ? 4 : 2, TB = WTYPE == B200_TYPE_Q4_0 ? 1024 : 2048;
     constexpr float WS = WTYPE == B200_TYPE_Q4_0 ? 0.0625f : 1.0f;   // Q4_0 quants are used as 16 * value
     extern __shared__ __align__(128) uint8_t smem[];
@@ -142,19 +142,37 @@ __global__ void __launch_bounds__(MS_THREADS, 1) mmq_stream_kernel(TiledDims dim
             }
         }
     }
+    // The chunks of a row tile, in K order.  Threads go over [column][rows], the rows padded to a power of two.
+    const int chunks = min(1 << cl, (n_bg + plan.chunk_bg - 1) / plan.chunk_bg), rows = n_r * 16, lg = 32 - __clz(rows - 1), n_e = (int) act.N << lg;
+    auto angle_of = [&](int e) { return rope_angle(rope, min(e >> lg, (int) act.N - 1), r0 * 16 + (e & ((1 << lg) - 1))); };
+    float2 angle = make_float2(1.0f, 0.0f);
+    int64_t slot = 0;
+    if (ROPE) {   // of the first round; the loads travel while the last warps finish
+        angle = angle_of(tid);
+        slot = rope.slots[min(tid >> lg, (int) act.N - 1)];
+    }
     pdl_trigger();
     __syncthreads();
-    // The chunks of a row tile, in K order.  Threads go over [column][rows], the rows padded to a power of two.
-    const int chunks = min(1 << cl, (n_bg + plan.chunk_bg - 1) / plan.chunk_bg), rows = n_r * 16, lg = 32 - __clz(rows - 1);
-    for (int e = tid; e < (int) act.N << lg; e += MS_THREADS) {
+    for (int e = tid; e < (n_e + 31 & ~31); e += MS_THREADS) {   // whole warps
         const int col = e >> lg, rr = e & ((1 << lg) - 1);
         const int64_t row = (int64_t) r0 * 16 + rr;
-        if (rr >= rows || row >= dims.M) continue;
-        const float *s = slots + ((rr >> 4) << cl) * MS_SLOT + col * 20 + (rr & 15);
+        const bool real = e < n_e && rr < rows && row < dims.M;
         float v = 0.0f;
+        if (real) {
+            const float *s = slots + ((rr >> 4) << cl) * MS_SLOT + col * 20 + (rr & 15);
 #pragma unroll 4
-        for (int c = 0; c < chunks; ++c) v += s[c * MS_SLOT];
-        *reinterpret_cast<float *>(reinterpret_cast<char *>(dst) + col * dst_nb_row + row * 4) = v;
+            for (int c = 0; c < chunks; ++c) v += s[c * MS_SLOT];
+        }
+        if (ROPE) {
+            const float other = __shfl_down_sync(0xffffffffu, v, 1);   // (an even number of rows)
+            if (e >= MS_THREADS) {
+                angle = angle_of(e);
+                slot = rope.slots[min(col, (int) act.N - 1)];
+            }
+            if (real && !(e & 1)) rope_store_pair(rope, dst, dst_nb_row, col, (int) row, make_float2(v, other), angle, slot);
+        } else if (real) {
+            *reinterpret_cast<float *>(reinterpret_cast<char *>(dst) + col * dst_nb_row + row * 4) = v;
+        }
     }
 }
 
@@ -168,14 +186,18 @@ static int ms_sm_count() {   // every device of a process is the same model; the
     if (!n[dev]) {
         cudaDeviceGetAttribute(&n[dev], cudaDevAttrMultiProcessorCount, dev);
         if (n[dev] <= 0) n[dev] = 148;
-        cudaFuncSetAttribute(mmq_stream_kernel<B200_TYPE_Q4_0>, cudaFuncAttributeMaxDynamicSharedMemorySize, MS_SMEM);
-        cudaFuncSetAttribute(mmq_stream_kernel<B200_TYPE_Q8_0>, cudaFuncAttributeMaxDynamicSharedMemorySize, MS_SMEM);
+        cudaFuncSetAttribute(mmq_stream_kernel<B200_TYPE_Q4_0, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, MS_SMEM);
+        cudaFuncSetAttribute(mmq_stream_kernel<B200_TYPE_Q4_0, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, MS_SMEM);
+        cudaFuncSetAttribute(mmq_stream_kernel<B200_TYPE_Q8_0, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, MS_SMEM);
+        cudaFuncSetAttribute(mmq_stream_kernel<B200_TYPE_Q8_0, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, MS_SMEM);
     }
     return n[dev];
 }
 
-// false: the activations and partial tiles do not fit into shared memory (K above some 21000), or nothing does; *rc: how the launch went
-bool launch_mmq_stream(int wtype, const TiledDims &d, const void *w, const ActDims &a, const void *aq, float *dst, int64_t dst_nb_row, cudaStream_t st, int *rc) {
+// false: the activations and partial tiles do not fit into shared memory (K above some 21000), or nothing does; *rc: how the launch went.
+// rope: the rows are those of q, k and v, see there
+bool launch_mmq_stream(int wtype, const TiledDims &d, const void *w, const ActDims &a, const void *aq, float *dst, int64_t dst_nb_row, const RopeStore *rope, cudaStream_t st,
+                       int *rc) {
     if (a.n_nt != 1 || d.n_rt * d.n_bg >= (1ll << 31)) return false;
     const int64_t ctas = std::min<int64_t>(ms_sm_count(), d.n_rt), rt = (d.n_rt + ctas - 1) / ctas, act = d.n_bg * 1280;
     // The most warps a row tile (all work to the end) whose partial tiles fit: tiles of the busiest warp, and what a row tile's end costs
@@ -193,8 +215,9 @@ bool launch_mmq_stream(int wtype, const TiledDims &d, const void *w, const ActDi
         smem = (size_t) bytes;
     }
     if (best < 0) return false;
-    if (wtype == B200_TYPE_Q4_0) launch_pdl(mmq_stream_kernel<B200_TYPE_Q4_0>, dim3((unsigned) ctas), dim3(MS_THREADS), smem, st, d, (const uint8_t *) w, a, (const uint8_t *) aq, dst, dst_nb_row, p);
-    else launch_pdl(mmq_stream_kernel<B200_TYPE_Q8_0>, dim3((unsigned) ctas), dim3(MS_THREADS), smem, st, d, (const uint8_t *) w, a, (const uint8_t *) aq, dst, dst_nb_row, p);
+    const bool q4 = wtype == B200_TYPE_Q4_0;
+    const auto kernel = rope ? (q4 ? mmq_stream_kernel<B200_TYPE_Q4_0, true> : mmq_stream_kernel<B200_TYPE_Q8_0, true>) : (q4 ? mmq_stream_kernel<B200_TYPE_Q4_0, false> : mmq_stream_kernel<B200_TYPE_Q8_0, false>);
+    launch_pdl(kernel, dim3((unsigned) ctas), dim3(MS_THREADS), smem, st, d, (const uint8_t *) w, a, (const uint8_t *) aq, dst, dst_nb_row, p, rope ? *rope : RopeStore{});
     *rc = check_launch("mmq_stream");
     return true;
 }

@@ -11,6 +11,7 @@
 // over the four t lanes with shuffles and over the warps through shared memory in a fixed order, so
 // the result does not depend on scheduling.
 #include <cstdlib>
+#include <type_traits>
 
 #include "common.cuh"
 
@@ -20,10 +21,11 @@ namespace b200 {
 // MMVQ_WARPS warps split the block groups of a row tile: many when there are few row tiles (a 4096-row weight has only 256
 // CTAs, and more warps per CTA are what keeps enough loads in flight), fewer for tall matrices
 // DEPTH: tiles a warp has requested beyond the one it works on (1 or 2)
-template <int WTYPE, int NC, int MMVQ_WARPS, int DEPTH = 1>
+// ROPE: the rows are those of q, k and v (RopeStore)
+template <int WTYPE, int NC, int MMVQ_WARPS, int DEPTH = 1, bool ROPE = false>
 __global__ void __launch_bounds__(MMVQ_WARPS * 32) mmvq_kernel(TiledDims dims, const uint8_t *__restrict__ w, ActDims act,
                                                               const uint8_t *__restrict__ aq, float *__restrict__ dst,
-                                                              int64_t dst_nb_row, PeerDst peers, int early) {
+                                                              int64_t dst_nb_row, PeerDst peers, int early, RopeStore rope) {
     const int64_t rt = blockIdx.x;
     if (early) {
         // the weights of this row tile (one contiguous run of tiles, one of scales) do not depend on the kernel ahead:
@@ -139,7 +141,25 @@ __global__ void __launch_bounds__(MMVQ_WARPS * 32) mmvq_kernel(TiledDims dims, c
             red[warp][g + 8][n] = y[1][n];
         }
     }
+    float2 angle = make_float2(1.0f, 0.0f);
+    int64_t slot = 0;
+    if (ROPE && threadIdx.x < 16 * NC) {   // (they travel while the last warps finish)
+        angle = rope_angle(rope, threadIdx.x >> 4, (int) rt * 16 + (threadIdx.x & 15));
+        slot = rope.slots[threadIdx.x >> 4];
+    }
     __syncthreads();
+    if (ROPE) {
+        static_assert(!ROPE || 16 * NC <= 32, "one warp finishes the rows");
+        const int n = threadIdx.x >> 4, r = threadIdx.x & 15;
+        if (threadIdx.x < 16 * NC) {
+            float s = 0.0f;
+#pragma unroll
+            for (int wv = 0; wv < MMVQ_WARPS; ++wv) s += red[wv][r][n];
+            const float other = __shfl_down_sync(NC == 1 ? 0xffffu : 0xffffffffu, s, 1);
+            if (!(r & 1) && rt * 16 + r < dims.M) rope_store_pair(rope, dst, dst_nb_row, n, (int) rt * 16 + r, make_float2(s, other), angle, slot);
+        }
+        return;
+    }
     for (int i = threadIdx.x; i < 16 * NC; i += MMVQ_WARPS * 32) {
         const int n = i >> 4, r = i & 15;
         const int64_t row = rt * 16 + r;
@@ -183,7 +203,7 @@ static int mmvq_sm_count() {
 // 88.9 / 67.8 / 65.0.  B200_MMVQ_CFG=<warps><depth> (42, 81, 162, ...) forces a variant (tuning aid).
 template <int WTYPE, int NC>
 static int launch_mmvq_n(const TiledDims &d, const uint8_t *w, const ActDims &a, const uint8_t *aq, float *dst, int64_t dst_nb_row, const PeerDst &peers,
-                         cudaStream_t st) {
+                         const RopeStore *rope, cudaStream_t st) {
     static const int forced = [] {
         const char *e = getenv("B200_MMVQ_CFG");
         return e ? atoi(e) : 0;
@@ -198,37 +218,49 @@ static int launch_mmvq_n(const TiledDims &d, const uint8_t *w, const ActDims &a,
         else if (d.n_rt <= sms * mmvq_ctas_per_sm<WTYPE, NC, 4, 1>()) cfg = 41;
         else cfg = 42;
     }
+    auto launch = [&](auto warps, auto depth) {
+        constexpr int W = decltype(warps)::value, DP = decltype(depth)::value;
+        if constexpr (NC <= 2) {
+            if (rope) {
+                launch_pdl(mmvq_kernel<WTYPE, NC, W, DP, true>, grid, dim3(W * 32), 0, st, d, w, a, aq, dst, dst_nb_row, peers, early, *rope);
+                return;
+            }
+        }
+        launch_pdl(mmvq_kernel<WTYPE, NC, W, DP>, grid, dim3(W * 32), 0, st, d, w, a, aq, dst, dst_nb_row, peers, early, RopeStore{});
+    };
+    using std::integral_constant;
     switch (cfg) {
-        case 41: launch_pdl(mmvq_kernel<WTYPE, NC, 4, 1>, grid, dim3(128), 0, st, d, w, a, aq, dst, dst_nb_row, peers, early); break;
-        case 42: launch_pdl(mmvq_kernel<WTYPE, NC, 4, 2>, grid, dim3(128), 0, st, d, w, a, aq, dst, dst_nb_row, peers, early); break;
-        case 81: launch_pdl(mmvq_kernel<WTYPE, NC, 8, 1>, grid, dim3(256), 0, st, d, w, a, aq, dst, dst_nb_row, peers, early); break;
-        case 82: launch_pdl(mmvq_kernel<WTYPE, NC, 8, 2>, grid, dim3(256), 0, st, d, w, a, aq, dst, dst_nb_row, peers, early); break;
-        case 161: launch_pdl(mmvq_kernel<WTYPE, NC, 16, 1>, grid, dim3(512), 0, st, d, w, a, aq, dst, dst_nb_row, peers, early); break;
-        default: launch_pdl(mmvq_kernel<WTYPE, NC, 16, 2>, grid, dim3(512), 0, st, d, w, a, aq, dst, dst_nb_row, peers, early); break;
+        case 41: launch(integral_constant<int, 4>{}, integral_constant<int, 1>{}); break;
+        case 42: launch(integral_constant<int, 4>{}, integral_constant<int, 2>{}); break;
+        case 81: launch(integral_constant<int, 8>{}, integral_constant<int, 1>{}); break;
+        case 82: launch(integral_constant<int, 8>{}, integral_constant<int, 2>{}); break;
+        case 161: launch(integral_constant<int, 16>{}, integral_constant<int, 1>{}); break;
+        default: launch(integral_constant<int, 16>{}, integral_constant<int, 2>{}); break;
     }
     return check_launch("mmvq");
 }
 
 template <int WTYPE>
 static int launch_mmvq_t(const TiledDims &d, const uint8_t *w, const ActDims &a, const uint8_t *aq, float *dst,
-                         int64_t dst_nb_row, const PeerDst &peers, cudaStream_t st) {
+                         int64_t dst_nb_row, const PeerDst &peers, const RopeStore *rope, cudaStream_t st) {
     switch (a.N) {
-        case 1: return launch_mmvq_n<WTYPE, 1>(d, w, a, aq, dst, dst_nb_row, peers, st);
-        case 2: return launch_mmvq_n<WTYPE, 2>(d, w, a, aq, dst, dst_nb_row, peers, st);
-        case 3: return launch_mmvq_n<WTYPE, 3>(d, w, a, aq, dst, dst_nb_row, peers, st);
-        case 4: return launch_mmvq_n<WTYPE, 4>(d, w, a, aq, dst, dst_nb_row, peers, st);
-        case 5: return launch_mmvq_n<WTYPE, 5>(d, w, a, aq, dst, dst_nb_row, peers, st);
-        case 6: return launch_mmvq_n<WTYPE, 6>(d, w, a, aq, dst, dst_nb_row, peers, st);
-        case 7: return launch_mmvq_n<WTYPE, 7>(d, w, a, aq, dst, dst_nb_row, peers, st);
-        case 8: return launch_mmvq_n<WTYPE, 8>(d, w, a, aq, dst, dst_nb_row, peers, st);
+        case 1: return launch_mmvq_n<WTYPE, 1>(d, w, a, aq, dst, dst_nb_row, peers, rope, st);
+        case 2: return launch_mmvq_n<WTYPE, 2>(d, w, a, aq, dst, dst_nb_row, peers, rope, st);
+        case 3: return launch_mmvq_n<WTYPE, 3>(d, w, a, aq, dst, dst_nb_row, peers, rope, st);
+        case 4: return launch_mmvq_n<WTYPE, 4>(d, w, a, aq, dst, dst_nb_row, peers, rope, st);
+        case 5: return launch_mmvq_n<WTYPE, 5>(d, w, a, aq, dst, dst_nb_row, peers, rope, st);
+        case 6: return launch_mmvq_n<WTYPE, 6>(d, w, a, aq, dst, dst_nb_row, peers, rope, st);
+        case 7: return launch_mmvq_n<WTYPE, 7>(d, w, a, aq, dst, dst_nb_row, peers, rope, st);
+        case 8: return launch_mmvq_n<WTYPE, 8>(d, w, a, aq, dst, dst_nb_row, peers, rope, st);
         default: return set_error(B200_E_INVALID, "mmvq handles 1..8 columns, got %lld", (long long) a.N);
     }
 }
 
+// rope (one or two columns only): the rows are those of q, k and v
 int launch_mmvq(int wtype, const TiledDims &d, const void *w, const ActDims &a, const void *aq, float *dst, int64_t dst_nb_row,
-                const PeerDst &peers, cudaStream_t st) {
-    if (wtype == B200_TYPE_Q4_0) return launch_mmvq_t<B200_TYPE_Q4_0>(d, (const uint8_t *) w, a, (const uint8_t *) aq, dst, dst_nb_row, peers, st);
-    return launch_mmvq_t<B200_TYPE_Q8_0>(d, (const uint8_t *) w, a, (const uint8_t *) aq, dst, dst_nb_row, peers, st);
+                const PeerDst &peers, const RopeStore *rope, cudaStream_t st) {
+    if (wtype == B200_TYPE_Q4_0) return launch_mmvq_t<B200_TYPE_Q4_0>(d, (const uint8_t *) w, a, (const uint8_t *) aq, dst, dst_nb_row, peers, rope, st);
+    return launch_mmvq_t<B200_TYPE_Q8_0>(d, (const uint8_t *) w, a, (const uint8_t *) aq, dst, dst_nb_row, peers, rope, st);
 }
 
 }  // namespace b200

@@ -16,10 +16,11 @@ bool mmq_sync_forced();
 int launch_quantize_b8(const float *x, int64_t x_nb_row, int64_t K, int64_t N, void *scratch, int variant, int layout, cudaStream_t st);
 int mmvq_max_n();
 int launch_mmvq(int wtype, const TiledDims &d, const void *w, const ActDims &a, const void *aq, float *dst, int64_t dst_nb_row, const PeerDst &peers,
-                cudaStream_t st);
+                const RopeStore *rope, cudaStream_t st);
 int launch_mmq(int wtype, const TiledDims &d, const void *w, const ActDims &a, const void *aq, float *dst, int64_t dst_nb_row,
                void *workspace, size_t workspace_bytes, cudaStream_t st, const PeerDst &peers);
-bool launch_mmq_stream(int wtype, const TiledDims &d, const void *w, const ActDims &a, const void *aq, float *dst, int64_t dst_nb_row, cudaStream_t st, int *rc);
+bool launch_mmq_stream(int wtype, const TiledDims &d, const void *w, const ActDims &a, const void *aq, float *dst, int64_t dst_nb_row, const RopeStore *rope, cudaStream_t st,
+                       int *rc);
 int launch_peer_signal_wait(void *const *flags_of_rank, int rank, int g, cudaStream_t st);
 size_t mmq_workspace_bytes(int wtype, int64_t K, int64_t M, int64_t N);
 }  // namespace b200
@@ -185,10 +186,33 @@ static int mul_mat_prequant(int wtype, const void *w, int64_t K, int64_t M, cons
     const ActDims a = act_dims(K, N);
     if (peers.n == 0 && peers.n_seg <= 1 && use_stream(d, N)) {
         int rc = 0;
-        if (launch_mmq_stream(wtype, d, w, a, act, dst, dst_row_stride_bytes, (cudaStream_t) stream, &rc)) return rc;
+        if (launch_mmq_stream(wtype, d, w, a, act, dst, dst_row_stride_bytes, nullptr, (cudaStream_t) stream, &rc)) return rc;
     }
-    if (N <= mmvq_max_n()) return launch_mmvq(wtype, d, w, a, act, dst, dst_row_stride_bytes, peers, (cudaStream_t) stream);
+    if (N <= mmvq_max_n()) return launch_mmvq(wtype, d, w, a, act, dst, dst_row_stride_bytes, peers, nullptr, (cudaStream_t) stream);
     return launch_mmq(wtype, d, w, a, act, dst, dst_row_stride_bytes, workspace, workspace_bytes, (cudaStream_t) stream, peers);
+}
+
+int b200_mul_mat_qkv_rope(int wtype, const void *w, int64_t K, const void *act, int64_t N, float *qkv, int64_t qkv_row_stride_bytes, int64_t D, int64_t H, int64_t Hkv,
+                          int n_dims, const float *angles, const int32_t *slots, void *k_cache, int64_t k_cache_nb_row, void *v_cache, int64_t v_cache_nb_row,
+                          void *workspace, size_t workspace_bytes, b200_stream_t stream) {
+    B200_REQUIRE((D == 64 || D == 128 || D == 256) && H > 0 && Hkv > 0 && H + 2 * Hkv <= 4096, "bad heads: %lld and 2 x %lld of %lld", (long long) H, (long long) Hkv, (long long) D);
+    const int64_t M = (H + 2 * Hkv) * D;
+    B200_REQUIRE(shape_ok(wtype, K, M, N), "bad mul_mat shape/type: type %d K %lld M %lld N %lld", wtype, (long long) K, (long long) M, (long long) N);
+    B200_REQUIRE(w && act && qkv && angles && slots && k_cache && v_cache && n_dims > 0 && n_dims % 2 == 0 && n_dims <= D, "null pointer or bad rope arguments");
+    B200_REQUIRE(is_aligned(w, 16) && is_aligned(act, 256) && is_aligned(qkv, 8) && is_aligned(k_cache, 4) && is_aligned(v_cache, 4), "misaligned pointer");
+    B200_REQUIRE(qkv_row_stride_bytes % 8 == 0 && qkv_row_stride_bytes >= M * 4 && k_cache_nb_row % 4 == 0 && v_cache_nb_row % 4 == 0, "bad row stride");
+    const TiledDims d = tiled_dims(wtype, K, M);
+    const ActDims a = act_dims(K, N);
+    const RopeStore rope = {angles, slots, (__half *) k_cache, (__half *) v_cache, k_cache_nb_row, v_cache_nb_row, (int) (H * D), (int) ((H + Hkv) * D), (int) D / 2 - 1, n_dims / 2};
+    if (use_stream(d, N)) {
+        int rc = 0;
+        if (launch_mmq_stream(wtype, d, w, a, act, qkv, qkv_row_stride_bytes, &rope, (cudaStream_t) stream, &rc)) return rc;
+    } else if (N <= std::min(2, mmvq_max_n())) {
+        return launch_mmvq(wtype, d, w, a, act, qkv, qkv_row_stride_bytes, PeerDst{}, &rope, (cudaStream_t) stream);
+    }
+    if (int e = b200_mul_mat_q_prequant(wtype, w, K, M, act, N, qkv, qkv_row_stride_bytes, workspace, workspace_bytes, stream)) return e;
+    return b200_rope_store_angles(qkv, D * 4, qkv_row_stride_bytes, qkv + H * D, D * 4, qkv_row_stride_bytes, qkv + (H + Hkv) * D, qkv_row_stride_bytes, D, H, Hkv, N, n_dims, angles, slots,
+                                  k_cache, k_cache_nb_row, v_cache, v_cache_nb_row, stream);
 }
 
 int b200_mul_mat_q_prequant_multi(int wtype, int n_weights, const void *const *w, const int64_t *M, int64_t K, const void *act, int64_t N,

@@ -253,10 +253,6 @@ class LlamaEngine:
             check(lib().b200_mul_mat_q_prequant(w.wtype, w.data.data_ptr(), w.K, w.M, act.data_ptr(), T, out.data_ptr(), out.stride(0) * 4,
                                                 self.ws.data_ptr(), self.ws.numel(), self._st))
             return
-        if self.hp and name.endswith("attn_qkv.weight"):   # q, k, v of this rank's heads: nobody else needs them
-            check(lib().b200_mul_mat_q_prequant(w.wtype, w.data.data_ptr(), w.K, w.M, act.data_ptr(), T, out.data_ptr(), out.stride(0) * 4,
-                                                self.ws.data_ptr(), self.ws.numel(), self._st))
-            return
         self.split.mul_mat(w, act, T, out, self.ws, self._st)   # this rank's rows, written into every rank's `out`, then the flag exchange
 
     def _quant(self, x: torch.Tensor, K: int, T: int, act: torch.Tensor):
@@ -288,16 +284,21 @@ class LlamaEngine:
         for il in range(cfg.n_layer):
             p = f"blk.{il}."
             norm_quant(p + "attn_norm.weight", pending)
-            if self.fused:
-                self._mm(p + "attn_qkv.weight", self.act_d, T, self.qkv)
-            else:
-                self._mm(p + "attn_q.weight", self.act_d, T, self.q)
-                self._mm(p + "attn_k.weight", self.act_d, T, self.k)
-                self._mm(p + "attn_v.weight", self.act_d, T, self.v)
             kc, vc = self.k_cache[il], self.v_cache[il]
-            qs, kst, vst = self.q.stride(0) * 4, self.k.stride(0) * 4, self.v.stride(0) * 4
-            check(L.b200_rope_store_angles(self.q.data_ptr(), D * 4, qs, self.k.data_ptr(), D * 4, kst, self.v.data_ptr(), vst, D, H, Hkv, T, D,
-                                           self.angles.data_ptr(), slots, kc.data_ptr(), kvd * 2, vc.data_ptr(), kvd * 2, st))
+            if self.fused and (self.split is None or self.hp):   # q, k, v of this rank's heads: nobody else needs them
+                w: QWeight = self.w.tensors[p + "attn_qkv.weight"]
+                check(L.b200_mul_mat_qkv_rope(w.wtype, w.data.data_ptr(), w.K, self.act_d.data_ptr(), T, self.qkv.data_ptr(), self.qkv.stride(0) * 4, D, H, Hkv, D,
+                                              self.angles.data_ptr(), slots, kc.data_ptr(), kvd * 2, vc.data_ptr(), kvd * 2, self.ws.data_ptr(), self.ws.numel(), st))
+            else:
+                if self.fused:
+                    self._mm(p + "attn_qkv.weight", self.act_d, T, self.qkv)
+                else:
+                    self._mm(p + "attn_q.weight", self.act_d, T, self.q)
+                    self._mm(p + "attn_k.weight", self.act_d, T, self.k)
+                    self._mm(p + "attn_v.weight", self.act_d, T, self.v)
+                check(L.b200_rope_store_angles(self.q.data_ptr(), D * 4, self.q.stride(0) * 4, self.k.data_ptr(), D * 4, self.k.stride(0) * 4, self.v.data_ptr(), self.v.stride(0) * 4,
+                                               D, H, Hkv, T, D, self.angles.data_ptr(), slots, kc.data_ptr(), kvd * 2, vc.data_ptr(), kvd * 2, st))
+            qs = self.q.stride(0) * 4
             attn_args = (D, H, Hkv, T, nkv, self.q.data_ptr(), qs, D * 4, kc.data_ptr(), kvd * 2, D * 2, vc.data_ptr(), kvd * 2, D * 2,
                          self.mask.data_ptr(), nkv * 2, self.index.data_ptr(), D ** -0.5, 0.0, 0.0)
             if T <= self.fa_quant_max_tokens and not self.hp:

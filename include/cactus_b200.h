@@ -307,6 +307,13 @@ B200_API int b200_rope_store_angles(float *q, int64_t q_nb_head, int64_t q_nb_to
                                     const int32_t *slots, void *k_cache, int64_t k_cache_nb_row, void *v_cache, int64_t v_cache_nb_row,
                                     b200_stream_t stream);
 
+/* The product with the stacked rows of wq, wk and wv (b200_mul_mat_q_prequant with M = (H + 2 Hkv) D) and b200_rope_store_angles on
+ * its result, bit-identical to the two calls.  q is left, rotated, in the first H D columns of `qkv`; the other columns may or may not be
+ * written (a few tokens: the product itself rotates and stores, and its k and v go to the cache only). */
+B200_API int b200_mul_mat_qkv_rope(int wtype, const void *w, int64_t K, const void *act, int64_t N, float *qkv, int64_t qkv_row_stride_bytes, int64_t D,
+                                   int64_t H, int64_t Hkv, int n_dims, const float *angles, const int32_t *slots, void *k_cache, int64_t k_cache_nb_row,
+                                   void *v_cache, int64_t v_cache_nb_row, void *workspace, size_t workspace_bytes, b200_stream_t stream);
+
 /* ------------------------------------------------------------------------------------------------
  * Row-split mul_mat over the GPUs of one node (one process per GPU).
  *

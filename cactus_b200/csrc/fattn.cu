@@ -11,6 +11,7 @@
 // Q K^T and P V (see fattn_mma_kernel).  With KV splits the partial (max, sum, accumulator) triples go to
 // scratch and a combine kernel finishes.  A second, slow kernel reproduces the reference's own rounding
 // sequence for validation (fattn_parity_kernel).
+#include <cooperative_groups.h>
 #include <math_constants.h>
 
 #include <cstdlib>
@@ -33,6 +34,7 @@ constexpr int FA_THREADS = 128;
 #endif
 constexpr int FA_SUPER_WORDS = 32;  // 2048 cells listed per round
 constexpr int FA_MIN_SPLIT_WORDS = 2;   // 64-cell words a KV split walks at least (when the mask index gives a token's word count)
+constexpr int FA_CLUSTER_MAX = 8;   // CTAs of a cluster
 constexpr int FA_ADAPTIVE_SPLITS = 2;   // most KV splits a long sequence is cut into when the batch is small
 
 // ---- mask scan: one CTA per token row --------------------------------------------------------------
@@ -323,17 +325,20 @@ __device__ __forceinline__ void fattn_store_out(const FattnParams &p, int64_t j,
 
 // QUANT: the instantiation behind b200_flash_attn_ext_quant; kept apart because this kernel sits at its register limit
 // and the plain one must not change with it
-template <int D, bool QUANT>
+// CLUSTER: the KV splits of a token and head group are a cluster of CTAs, which add their parts through each other's shared memory; see
+// launch_mma_cluster
+template <int D, bool QUANT, bool CLUSTER = false>
 __global__ void __launch_bounds__(FA_THREADS, FA_MIN_CTAS) fattn_mma_kernel(FattnParams p) {
     pdl_prologue();
     if (p.vote == 1 && fattn_tiled_chosen(p.plan)) return;   // the query-tiled kernel takes this ubatch
+    constexpr bool PREFETCH_V = FA_PREFETCH_V || (CLUSTER && D == 64);   // (where there are registers for it)
     constexpr int KS = D / 16;   // k-steps of the S MMA
     constexpr int NU = D / 32;   // 16-byte K pieces per lane and cell
     constexpr int NR = D / 64;   // 64-wide d ranges of V
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int g = lane >> 2, t = lane & 3;
     // blocks are handed out heads first, then tokens in the order of the plan: the longest sequences start first
-    const int64_t j = p.order ? p.order[blockIdx.y] : blockIdx.y;
+    const int64_t j = !CLUSTER && p.order ? p.order[blockIdx.y] : blockIdx.y;   // (a cluster grid is resident as a whole)
     const int hk = blockIdx.x / p.hgroups, hg = blockIdx.x % p.hgroups;
     const int split = blockIdx.z;
     const int gqa = (int) (p.H / p.Hkv);
@@ -344,6 +349,7 @@ __global__ void __launch_bounds__(FA_THREADS, FA_MIN_CTAS) fattn_mma_kernel(Fatt
     __shared__ int list_count;
     __shared__ float merge_m[4][8], merge_l[4][8];
     __shared__ float merge_acc[4][8][D];
+    __shared__ float part_m[8], part_l[8];   // with CLUSTER: of this split; its part is in merge_acc[0]
 
     // Q fragments: row g = head h0 + g (zero rows beyond G)
     uint32_t qa0[KS], qa2[KS];
@@ -377,15 +383,17 @@ __global__ void __launch_bounds__(FA_THREADS, FA_MIN_CTAS) fattn_mma_kernel(Fatt
     if (p.w0 != 0) {
         const int w0 = fattn_target_words(p, (int) gridDim.x);
         ns_j = (int) min((int64_t) p.nsplit, max((int64_t) 1, (n_words + w0 - 1) / w0));
-        if (split >= ns_j) return;   // the whole CTA: nothing has been synchronised yet
+        if (!CLUSTER && split >= ns_j) return;   // the whole CTA: nothing has been synchronised yet
     }
     const int64_t per_split = (n_words + ns_j - 1) / ns_j;
-    const int64_t w_begin = (int64_t) split * per_split;
+    const int64_t w_begin = CLUSTER ? min(n_words, (int64_t) split * per_split) : (int64_t) split * per_split;
     const int64_t w_end = min(n_words, w_begin + per_split);
-    const __half *mrow = p.mask ? reinterpret_cast<const __half *>(p.mask + j * p.mask_nb_row) : nullptr;
+    // (a mask of nothing but 0 and -inf adds nothing in the cells that take part)
+    const __half *mrow = p.mask && p.plan[2] != 0 ? reinterpret_cast<const __half *>(p.mask + j * p.mask_nb_row) : nullptr;
     const char *kbase = p.k + (int64_t) hk * p.k_nb_head;
     const char *vbase = p.v + (int64_t) hk * p.v_nb_head;
 
+    auto walk = [&](auto soft) {
     for (int64_t w0 = w_begin; w0 < w_end; w0 += FA_SUPER_WORDS) {
         if (warp == 0) {   // list the participating cells of this round
             const int64_t e = w0 + lane;
@@ -441,7 +449,7 @@ __global__ void __launch_bounds__(FA_THREADS, FA_MIN_CTAS) fattn_mma_kernel(Fatt
             }
         };
         if (FA_PREFETCH_K && warp < n_chunks) load_k(warp);
-        if (FA_PREFETCH_V && warp < n_chunks) load_v(warp);
+        if (PREFETCH_V && warp < n_chunks) load_v(warp);
         for (int ch = warp; ch < n_chunks; ch += 4) {
             const int base = ch << 4;
             if (!FA_PREFETCH_K) load_k(ch);
@@ -456,8 +464,8 @@ __global__ void __launch_bounds__(FA_THREADS, FA_MIN_CTAS) fattn_mma_kernel(Fatt
                     mma_f16(sacc[c], qa0[2 * u + 1], 0u, qa2[2 * u + 1], 0u, kr[c][u].z, kr[c][u].w);
                 }
             }
-            // V rows of cells 2t, 2t+1, 2t+8, 2t+9 (already on their way with FA_PREFETCH_V)
-            if (!FA_PREFETCH_V) load_v(ch);
+            // V rows of cells 2t, 2t+1, 2t+8, 2t+9 (already on their way with PREFETCH_V)
+            if (!PREFETCH_V) load_v(ch);
             // the next chunk's K rows travel during the softmax and the P V MMAs of this one
             if (FA_PREFETCH_K && ch + 4 < n_chunks) load_k(ch + 4);
             // ---- scores of head g for cells base + {2t, 2t+1, 8+2t, 9+2t} ----
@@ -468,7 +476,7 @@ __global__ void __launch_bounds__(FA_THREADS, FA_MIN_CTAS) fattn_mma_kernel(Fatt
                 float a = sacc[i >> 1][i & 1] * p.scale;
                 if (p.softcap != 0.0f) a = p.softcap * tanhf(a);
                 if (idx < count) {
-                    if (mrow) a += slope * __half2float(mrow[cell_list[idx]]);
+                    if (decltype(soft)::value) a += slope * __half2float(mrow[cell_list[idx]]);
                 } else {
                     a = -CUDART_INF_F;
                 }
@@ -516,10 +524,13 @@ __global__ void __launch_bounds__(FA_THREADS, FA_MIN_CTAS) fattn_mma_kernel(Fatt
                 mma_f16(oacc[q], a0, a1, a2, a3, b0h, b1h);
                 mma_f16(oacc[q], a0, a1, a2, a3, b0l, b1l);
             }
-            if (FA_PREFETCH_V && ch + 4 < n_chunks) load_v(ch + 4);
+            if (PREFETCH_V && ch + 4 < n_chunks) load_v(ch + 4);
         }
         __syncthreads();
     }
+    };
+    if (mrow) walk(std::true_type{});
+    else walk(std::false_type{});
 
     pdl_trigger();
     // ---- merge the four warps ----
@@ -552,7 +563,13 @@ __global__ void __launch_bounds__(FA_THREADS, FA_MIN_CTAS) fattn_mma_kernel(Fatt
             ls += merge_l[wv][h] * scl;
         }
         const int64_t head = h0 + h;
-        if (ns_j == 1 && !p.parts) {
+        if (CLUSTER) {
+            merge_acc[0][h][d] = a;   // (this thread was the one to read it)
+            if (d == 0) {
+                part_m[h] = mn;
+                part_l[h] = ls;
+            }
+        } else if (ns_j == 1 && !p.parts) {
             fattn_store_out<D, QUANT>(p, j, head, d, a * (1.0f / ls));
         } else {
             float *pp = p.partial + ((j * p.H + head) * p.nsplit + split) * (D + 2);
@@ -563,6 +580,55 @@ __global__ void __launch_bounds__(FA_THREADS, FA_MIN_CTAS) fattn_mma_kernel(Fatt
             }
         }
     }
+    if (CLUSTER) {   // a warp per 32 elements of a head, dealt out over the cluster; the order of fattn_combine_kernel
+        const cooperative_groups::cluster_group cluster = cooperative_groups::this_cluster();
+        cluster.sync();
+        for (int b = split * (FA_THREADS / 32) + warp; b < G * (D / 32); b += p.nsplit * (FA_THREADS / 32)) {
+            const int h = b / (D / 32), d = (b % (D / 32)) * 32 + lane;
+            float m[FA_CLUSTER_MAX], l[FA_CLUSTER_MAX], v[FA_CLUSTER_MAX], mn = -CUDART_INF_F;
+#pragma unroll
+            for (int s = 0; s < FA_CLUSTER_MAX; ++s) {
+                const int from = min(s, p.nsplit - 1);
+                m[s] = *cluster.map_shared_rank(&part_m[h], from);
+                l[s] = *cluster.map_shared_rank(&part_l[h], from);
+                v[s] = *cluster.map_shared_rank(&merge_acc[0][h][d], from);
+            }
+#pragma unroll
+            for (int s = 0; s < FA_CLUSTER_MAX; ++s) mn = fmaxf(mn, m[s]);
+            float a = 0.0f, ls = 0.0f;
+#pragma unroll
+            for (int s = 0; s < FA_CLUSTER_MAX; ++s) {
+                const float f = s >= p.nsplit || m[s] == -CUDART_INF_F ? 0.0f : expf(m[s] - mn);
+                a = fmaf(v[s], f, a);
+                ls = fmaf(l[s], f, ls);
+            }
+            fattn_store_out<D, QUANT>(p, j, h0 + h, d, a * (1.0f / ls));
+        }
+        cluster.sync();   // its shared memory is read until here
+    }
+}
+
+// The splits of a token as a cluster, where there are at most FA_CLUSTER_MAX of them and the whole grid is resident (a second wave of
+// clusters costs more than the combine pass: 30 sequences of the 1B architecture, 480 CTAs, 1631 us a step against 1528): no partial
+// results in memory, no second launch.  The CTAs meet twice, after their parts are in shared memory and before they leave.  Bound by
+// latency; D = 64 has the registers to ask for the next chunk's V rows early.  us per decode step on B200, combine pass / cluster: 1B, one
+// sequence 722 / 687; 1B, 16 sequences 1323 / 1222; 8B, seven sequences 2521 / 2424.  With two CTAs an SM and V rows asked for early at
+// D = 128 as well, the seven sequences took 2642.
+template <int D, bool QUANT>
+static void launch_mma_cluster(dim3 grid, cudaStream_t st, FattnParams p) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(FA_THREADS);
+    cfg.stream = st;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = grid.z;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = pdl_enabled() ? 2 : 1;
+    cudaLaunchKernelEx(&cfg, fattn_mma_kernel<D, QUANT, true>, p);
 }
 
 // ---- validation variant: the reference's own order of operations ------------------------------------
@@ -738,6 +804,10 @@ static int fattn_nsplit(int64_t Nq, int64_t Hkv, int hgroups, int64_t n_kv) {
     // At least 512 cells of the cache to a split, from 1024 cells on 128 (a token's own words are dealt out evenly, two at least): one
     // sequence of 640 cells in 1024, 1B architecture, 825 us a step with two splits, 778 with four or more.
     ns = std::min<int64_t>(ns, n_kv >= 1024 ? n_kv / 128 : 1);
+    // No more than a cluster has CTAs where those fill the SMs, or where a split has 256 cells then: us per decode step, uncapped / capped,
+    // 1B, three sequences of up to 2048 cells 885 / 860, 8B, four of 16000 3725 / 3671, 8B, one of 2000 in a cache of 2048 2143 / 2090; but
+    // 8B, one of 4000 in 4096 2235 / 2290, two of 8000 2614 / 2727.
+    if (ns > FA_CLUSTER_MAX && (FA_CLUSTER_MAX * ctas >= fa_sm_count() || n_kv <= 256 * FA_CLUSTER_MAX)) ns = FA_CLUSTER_MAX;
     return (int) std::min<int64_t>(ns, 64);
 }
 
@@ -953,6 +1023,16 @@ static int flash_attn_impl(bool parity, int64_t D, int64_t H, int64_t Hkv, int64
     // With KV splits the combine pass is what quantises: it has the registers for that, the main kernel has not.
     const bool qo = act != nullptr && ns == 1, qc = act != nullptr;
     p.parts = qc && ns > 1 ? 1 : 0;
+    if (ns > 1 && ns <= FA_CLUSTER_MAX && (int64_t) grid.x * grid.y * grid.z <= p.slots) {
+        if (D == 128) {
+            if (act) launch_mma_cluster<128, true>(grid, st, p);
+            else launch_mma_cluster<128, false>(grid, st, p);
+        } else {
+            if (act) launch_mma_cluster<64, true>(grid, st, p);
+            else launch_mma_cluster<64, false>(grid, st, p);
+        }
+        return check_launch("fattn_mma");
+    }
     if (D == 128) {
         if (qo) launch_pdl(fattn_mma_kernel<128, true>, grid, dim3(FA_THREADS), 0, st, p);
         else launch_pdl(fattn_mma_kernel<128, false>, grid, dim3(FA_THREADS), 0, st, p);

@@ -64,6 +64,7 @@ SIGNATURES = {
     "b200_rope_store_to": (_i32, [_vp, _vp, _i64, _i64, _vp, _i64, _i64, _vp, _i64, _i64, _i64, _i64, _i64, _i32, _vp, _vp, _f32, _f32, _f32, _vp,
                                   _vp, _i64, _vp, _i64, _vp]),
     "b200_rope_angles": (_i32, [_vp, _i64, _i32, _vp, _vp, _f32, _f32, _f32, _vp]),
+    "b200_ubatch_begin": (_i32, [_vp, _vp, _vp, _vp, _vp, _i64, _vp, _i32, _vp, _f32, _f32, _f32, _vp]),
     "b200_rope_store_angles": (_i32, [_vp, _i64, _i64, _vp, _i64, _i64, _vp, _i64, _i64, _i64, _i64, _i64, _i32, _vp, _vp, _vp, _i64, _vp, _i64, _vp]),
     "b200_mul_mat_qkv_rope": (_i32, [_i32, _vp, _i64, _vp, _i64, _vp, _i64, _i64, _i64, _i64, _i32, _vp, _vp, _vp, _i64, _vp, _i64, _vp, _sz, _vp]),
     "b200_peer_alloc": (_i32, [_sz, C.POINTER(_vp), C.c_char_p]),

@@ -49,7 +49,7 @@ constexpr int MI_THREADS = 512, MI_WORDS = 2048;   // words whose indices are li
 template <bool VEC>
 __global__ void __launch_bounds__(MI_THREADS, 3) mask_index_kernel(const __half *__restrict__ mask, int64_t mask_nb_row, int64_t n_kv, int64_t nw,
                                                                unsigned long long *__restrict__ words, int32_t *__restrict__ wlist, int32_t *__restrict__ wcount,
-                                                               uint8_t *__restrict__ soft) {
+                                                               uint8_t *__restrict__ soft, int32_t *__restrict__ order, int32_t *__restrict__ plan) {
     pdl_prologue();
     __shared__ unsigned bits[MI_WORDS / 32];
     __shared__ int warp_cnt[MI_WORDS / 1024], any_soft;
@@ -119,6 +119,12 @@ __global__ void __launch_bounds__(MI_THREADS, 3) mask_index_kernel(const __half 
     if (tid == 0) {
         wcount[j] = base;
         soft[j] = (uint8_t) any_soft;
+        if (plan) {   // of a single token: what fattn_plan_kernel would make
+            order[0] = 0;
+            plan[0] = base;
+            plan[2] = any_soft;
+            plan[1] = plan[4] = plan[5] = plan[6] = plan[7] = 0;
+        }
     }
 }
 
@@ -878,11 +884,14 @@ int b200_mask_index_build(const void *mask, int64_t mask_nb_row, int64_t Nq, int
     int32_t *plan = (int32_t *) (ix + index_plan_offset(Nq, nw)), *wlist = (int32_t *) (ix + index_list_offset(Nq, nw)), *wcount = (int32_t *) (ix + index_count_offset(Nq, nw));
     uint8_t *soft = (uint8_t *) ix + index_soft_offset(Nq, nw);
     const bool vec = is_aligned(mask, 16) && mask_nb_row % 16 == 0;
+    int32_t *order = (int32_t *) (ix + index_order_offset(Nq, nw)), *const none = nullptr;
     launch_pdl(vec ? mask_index_kernel<true> : mask_index_kernel<false>, dim3((unsigned) Nq), dim3(MI_THREADS), 0, st, (const __half *) mask, mask_nb_row, n_kv, nw,
-               (unsigned long long *) index, wlist, wcount, soft);
+               (unsigned long long *) index, wlist, wcount, soft, Nq == 1 ? order : none, Nq == 1 ? plan : none);
     if (int e = check_launch("mask_index")) return e;
-    launch_pdl(fattn_plan_kernel, dim3((unsigned) ((Nq + 7) / 8)), dim3(256), 0, st, (const int32_t *) wcount, (const uint8_t *) soft, Nq, (int32_t *) (ix + index_order_offset(Nq, nw)), plan);
-    if (int e = check_launch("fattn_plan")) return e;
+    if (Nq > 1) {
+        launch_pdl(fattn_plan_kernel, dim3((unsigned) ((Nq + 7) / 8)), dim3(256), 0, st, (const int32_t *) wcount, (const uint8_t *) soft, Nq, order, plan);
+        if (int e = check_launch("fattn_plan")) return e;
+    }
     if (index_has_tiles(Nq)) {
         int32_t *flags = (int32_t *) ((char *) index + index_tiles_offset(Nq, nw));
         const int64_t stride = index_tiles_stride(Nq);

@@ -189,10 +189,18 @@ __global__ void __launch_bounds__(512) rope_store_kernel(const float *q, float *
 }
 
 // The angles of a ubatch's tokens, [token][n_dims/2 cosines, n_dims/2 sines], for rope_store_angles_kernel: every layer rotates by the
-// same ones.  theta_a = pos * theta_scale^a by repeated multiplication, as the reference builds it.
+// same ones.  theta_a = pos * theta_scale^a by repeated multiplication, as the reference builds it.  With `cell_pos` the tokens' cells are
+// entered as well (b200_ubatch_begin): two launches less at the start of a step (with the mask index's plan, one less for a single token: 1B
+// architecture, one sequence 694 / 689 us a step).
 __global__ void __launch_bounds__(128) rope_angles_kernel(float *__restrict__ angles, int n_dims, const int32_t *__restrict__ pos, const float *__restrict__ ff,
-                                                          float theta_scale, float freq_scale, float attn_factor) {
+                                                          float theta_scale, float freq_scale, float attn_factor, int32_t *__restrict__ cell_pos, int32_t *__restrict__ cell_seq,
+                                                          const int32_t *__restrict__ slots, const int32_t *__restrict__ seq) {
     pdl_prologue();
+    if (cell_pos && threadIdx.x == 0) {
+        const int32_t slot = slots[blockIdx.x];
+        cell_pos[slot] = pos[blockIdx.x];
+        cell_seq[slot] = seq[blockIdx.x];
+    }
     const int64_t t = blockIdx.x;
     const int half_dims = n_dims / 2;
     for (int i = threadIdx.x; i < n_dims; i += blockDim.x) {
@@ -319,12 +327,24 @@ int b200_rope_store_to(const float *q, float *q_dst, int64_t q_nb_head, int64_t 
     return check_launch("rope_store");
 }
 
-int b200_rope_angles(float *angles, int64_t T, int n_dims, const int32_t *pos, const float *freq_factors, float freq_base, float freq_scale,
-                     float attn_factor, b200_stream_t stream) {
+static int launch_rope_angles(float *angles, int64_t T, int n_dims, const int32_t *pos, const float *freq_factors, float freq_base, float freq_scale, float attn_factor,
+                              int32_t *cell_pos, int32_t *cell_seq, const int32_t *slots, const int32_t *seq, b200_stream_t stream) {
     B200_REQUIRE(angles && pos && T > 0 && n_dims > 0 && n_dims % 2 == 0 && n_dims <= 8192 && is_aligned(angles, 4), "bad rope arguments");
     const float theta_scale = powf(freq_base, -2.0f / (float) n_dims);
-    launch_pdl(rope_angles_kernel, dim3((unsigned) T), dim3(128), 0, (cudaStream_t) stream, angles, n_dims, pos, freq_factors, theta_scale, freq_scale, attn_factor);
+    launch_pdl(rope_angles_kernel, dim3((unsigned) T), dim3(128), 0, (cudaStream_t) stream, angles, n_dims, pos, freq_factors, theta_scale, freq_scale, attn_factor,
+               cell_pos, cell_seq, slots, seq);
     return check_launch("rope_angles");
+}
+
+int b200_rope_angles(float *angles, int64_t T, int n_dims, const int32_t *pos, const float *freq_factors, float freq_base, float freq_scale,
+                     float attn_factor, b200_stream_t stream) {
+    return launch_rope_angles(angles, T, n_dims, pos, freq_factors, freq_base, freq_scale, attn_factor, nullptr, nullptr, nullptr, nullptr, stream);
+}
+
+int b200_ubatch_begin(int32_t *cell_pos, int32_t *cell_seq, const int32_t *slots, const int32_t *pos, const int32_t *seq, int64_t T, float *angles, int n_dims,
+                      const float *freq_factors, float freq_base, float freq_scale, float attn_factor, b200_stream_t stream) {
+    B200_REQUIRE(cell_pos && cell_seq && slots && seq, "null pointer");
+    return launch_rope_angles(angles, T, n_dims, pos, freq_factors, freq_base, freq_scale, attn_factor, cell_pos, cell_seq, slots, seq, stream);
 }
 
 int b200_rope_store_angles(float *q, int64_t q_nb_head, int64_t q_nb_tok, const float *k, int64_t k_nb_head, int64_t k_nb_tok, const float *v,

@@ -236,8 +236,8 @@ class LlamaEngine:
         ws = [L.b200_mul_mat_workspace_bytes(cfg.layer_type, K, M, t) for K, M in shapes for t in range(1, T + 1)]
         ws += [L.b200_mul_mat_workspace_bytes(cfg.head_type, cfg.d_model, cfg.vocab // g, t) for t in range(1, T + 1)]
         self.ws = u8(max(ws))
-        # Where the attention cuts its KV range, the pass that adds the splits leaves the result quantised (b200_flash_attn_ext_quant: one
-        # launch less per layer, bit-identical).  Without splits the attention kernel itself would have to, at its register limit:
+        # Where the attention cuts its KV range, what adds the splits leaves the result quantised (b200_flash_attn_ext_quant: one launch
+        # less per layer, bit-identical).  Without splits the attention kernel itself would have to, at its register limit:
         # 70.5 us for the 64-token batch against 57.5 + 2.5.  B200_FA_QUANT_MAX_T lowers the token count.
         fa_args = (cfg.head_dim, self.n_head_local, self.n_kv_head_local)
         split_kv = [L.b200_flash_attn_scratch_bytes(*fa_args, t, n_cells) > L.b200_mask_index_bytes(t, n_cells) for t in range(1, min(T, 128) + 1)]
@@ -264,11 +264,9 @@ class LlamaEngine:
         D, H, Hkv, d, nkv = cfg.head_dim, self.n_head_local, self.n_kv_head_local, cfg.d_model, self.n_cells
         kvd = Hkv * D
         tokens, pos, seq, slots = (self.inp[i].data_ptr() for i in range(4))
-        # cell bookkeeping, mask and its index (shared by all layers)
-        check(L.b200_scatter_i32(self.cell_pos.data_ptr(), slots, pos, T, st))
-        check(L.b200_scatter_i32(self.cell_seq.data_ptr(), slots, seq, T, st))
+        # cell bookkeeping, ROPE angles, mask and its index (shared by all layers)
+        check(L.b200_ubatch_begin(self.cell_pos.data_ptr(), self.cell_seq.data_ptr(), slots, pos, seq, T, self.angles.data_ptr(), D, None, cfg.rope_theta, 1.0, 1.0, st))
         check(L.b200_kq_mask_build(self.cell_pos.data_ptr(), self.cell_seq.data_ptr(), nkv, pos, seq, T, self.mask.data_ptr(), nkv * 2, st))
-        check(L.b200_rope_angles(self.angles.data_ptr(), T, D, pos, None, cfg.rope_theta, 1.0, 1.0, st))
         check(L.b200_mask_index_build(self.mask.data_ptr(), nkv * 2, T, nkv, self.index.data_ptr(), self.index.numel(), st))
         emb: QWeight = self.w.tensors["token_embd.weight"]
         check(L.b200_get_rows_q(emb.wtype, emb.data.data_ptr(), emb.K, emb.M, tokens, self.x.data_ptr(), d * 4, T, st))

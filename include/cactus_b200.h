@@ -302,6 +302,10 @@ B200_API int b200_rope_store_to(const float *q, float *q_dst, int64_t q_nb_head,
  * ([T][n_dims]: n_dims/2 cosines, n_dims/2 sines), b200_rope_store_angles applies them.  Bit-identical to b200_rope_store. */
 B200_API int b200_rope_angles(float *angles, int64_t T, int n_dims, const int32_t *pos, const float *freq_factors, float freq_base, float freq_scale,
                               float attn_factor, b200_stream_t stream);
+/* What a ubatch begins with, in one launch: cell_pos[slots[t]] = pos[t] and cell_seq[slots[t]] = seq[t] (two b200_scatter_i32), and
+ * b200_rope_angles. */
+B200_API int b200_ubatch_begin(int32_t *cell_pos, int32_t *cell_seq, const int32_t *slots, const int32_t *pos, const int32_t *seq, int64_t T, float *angles,
+                               int n_dims, const float *freq_factors, float freq_base, float freq_scale, float attn_factor, b200_stream_t stream);
 B200_API int b200_rope_store_angles(float *q, int64_t q_nb_head, int64_t q_nb_tok, const float *k, int64_t k_nb_head, int64_t k_nb_tok, const float *v,
                                     int64_t v_nb_tok, int64_t D, int64_t H, int64_t Hkv, int64_t T, int n_dims, const float *angles,
                                     const int32_t *slots, void *k_cache, int64_t k_cache_nb_row, void *v_cache, int64_t v_cache_nb_row,

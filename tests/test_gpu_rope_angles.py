@@ -32,3 +32,21 @@ def test_rope_store_angles(T, D, H, Hkv, n_dims, stacked):
     torch.cuda.synchronize()
     for x, y in zip((*a, *caches[:2]), (*b, *caches[2:])):
         assert torch.equal(x, y)
+
+
+@pytest.mark.parametrize("T", [1, 300])
+def test_ubatch_begin(T):
+    from cactus_b200._lib import check, lib
+    L, cells, n_dims = lib(), 512, 128
+    st = torch.cuda.current_stream().cuda_stream
+    slots = torch.randperm(cells, device="cuda")[:T].to(torch.int32)
+    pos, seq = (torch.randint(0, 5000, (T,), device="cuda", dtype=torch.int32) for _ in range(2))
+    cell = [torch.full((cells,), -1, dtype=torch.int32, device="cuda") for _ in range(4)]
+    angles = [torch.empty((T, n_dims), device="cuda") for _ in range(2)]
+    check(L.b200_scatter_i32(cell[0].data_ptr(), slots.data_ptr(), pos.data_ptr(), T, st))
+    check(L.b200_scatter_i32(cell[1].data_ptr(), slots.data_ptr(), seq.data_ptr(), T, st))
+    check(L.b200_rope_angles(angles[0].data_ptr(), T, n_dims, pos.data_ptr(), None, 500000.0, 1.0, 1.0, st))
+    check(L.b200_ubatch_begin(cell[2].data_ptr(), cell[3].data_ptr(), slots.data_ptr(), pos.data_ptr(), seq.data_ptr(), T, angles[1].data_ptr(), n_dims, None,
+                              500000.0, 1.0, 1.0, st))
+    torch.cuda.synchronize()
+    assert torch.equal(cell[0], cell[2]) and torch.equal(cell[1], cell[3]) and torch.equal(*angles)

@@ -46,7 +46,8 @@ constexpr int FA_ADAPTIVE_SPLITS = 2;   // most KV splits a long sequence is cut
 // 8.3 / 3.5, 64 x 65536 23.9 / 9.4, 512 x 8192 49.7 / 13.3, 512 x 65536 109 / 27.  A cluster of 2 or 4 CTAs per row was faster at
 // 64 x 65536 only (7.9) and slower from 1 x 1024 (4.6) to 512 x 65536 (32, 43).
 constexpr int MI_THREADS = 512, MI_WORDS = 2048;   // words whose indices are listed per round
-template <bool VEC>
+// SINGLE: one token, whose plan (below) this kernel makes as well
+template <bool VEC, bool SINGLE>
 __global__ void __launch_bounds__(MI_THREADS, 3) mask_index_kernel(const __half *__restrict__ mask, int64_t mask_nb_row, int64_t n_kv, int64_t nw,
                                                                unsigned long long *__restrict__ words, int32_t *__restrict__ wlist, int32_t *__restrict__ wcount,
                                                                uint8_t *__restrict__ soft, int32_t *__restrict__ order, int32_t *__restrict__ plan) {
@@ -119,7 +120,7 @@ __global__ void __launch_bounds__(MI_THREADS, 3) mask_index_kernel(const __half 
     if (tid == 0) {
         wcount[j] = base;
         soft[j] = (uint8_t) any_soft;
-        if (plan) {   // of a single token: what fattn_plan_kernel would make
+        if (SINGLE) {   // what fattn_plan_kernel would make
             order[0] = 0;
             plan[0] = base;
             plan[2] = any_soft;
@@ -884,9 +885,9 @@ int b200_mask_index_build(const void *mask, int64_t mask_nb_row, int64_t Nq, int
     int32_t *plan = (int32_t *) (ix + index_plan_offset(Nq, nw)), *wlist = (int32_t *) (ix + index_list_offset(Nq, nw)), *wcount = (int32_t *) (ix + index_count_offset(Nq, nw));
     uint8_t *soft = (uint8_t *) ix + index_soft_offset(Nq, nw);
     const bool vec = is_aligned(mask, 16) && mask_nb_row % 16 == 0;
-    int32_t *order = (int32_t *) (ix + index_order_offset(Nq, nw)), *const none = nullptr;
-    launch_pdl(vec ? mask_index_kernel<true> : mask_index_kernel<false>, dim3((unsigned) Nq), dim3(MI_THREADS), 0, st, (const __half *) mask, mask_nb_row, n_kv, nw,
-               (unsigned long long *) index, wlist, wcount, soft, Nq == 1 ? order : none, Nq == 1 ? plan : none);
+    int32_t *order = (int32_t *) (ix + index_order_offset(Nq, nw));
+    const auto kernel = Nq == 1 ? (vec ? mask_index_kernel<true, true> : mask_index_kernel<false, true>) : (vec ? mask_index_kernel<true, false> : mask_index_kernel<false, false>);
+    launch_pdl(kernel, dim3((unsigned) Nq), dim3(MI_THREADS), 0, st, (const __half *) mask, mask_nb_row, n_kv, nw, (unsigned long long *) index, wlist, wcount, soft, order, plan);
     if (int e = check_launch("mask_index")) return e;
     if (Nq > 1) {
         launch_pdl(fattn_plan_kernel, dim3((unsigned) ((Nq + 7) / 8)), dim3(256), 0, st, (const int32_t *) wcount, (const uint8_t *) soft, Nq, order, plan);

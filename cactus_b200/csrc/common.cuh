@@ -25,13 +25,14 @@ static inline size_t align_up(size_t v, size_t a) { return (v + a - 1) / a * a; 
 // ---- programmatic dependent launch ---------------------------------------------------------------
 // The kernels of a decode step run back to back on one stream, each a few to a few dozen microseconds long.  A kernel
 // launched with launch_pdl may have its CTAs placed on the SMs while the previous kernel's last CTAs are still running;
-// its first statement (pdl_prologue) waits until the previous kernel has completed and its writes are visible, so only
-// the launch itself and the CTA start-up overlap.  B200_PDL=0 turns the launch attribute off.
+// before it reads or writes global memory it waits (pdl_prologue) until the previous kernel has completed and its writes are visible, so
+// only the launch itself and the CTA start-up overlap.  That goes for weights as well: an upload or a copy that stacks them may be the
+// kernel ahead.  All that may come before the wait are hints (prefetch_l2_bulk).  B200_PDL=0 turns the launch attribute off.
 bool pdl_enabled();
 // With a single token row every kernel of a step is a few microseconds of latency and the weight stream of a product
 // waits behind each of them.  Up to this many rows (B200_PDL_EARLY_ROWS, default 1; 0 switches it off) the row kernels
 // let the next kernel's CTAs take their places at once (pdl_prologue(true)), and the few-column product asks for its
-// weights -- which no kernel of a step writes -- to be brought into L2 before it waits for the kernel ahead of it.
+// weights to be brought into L2 before it waits for the kernel ahead of it.
 int pdl_early_rows();
 // When the quantisers (plain, and of silu * up) let the next kernel's CTAs take their places: 1 at once (pdl_early_rows),
 // 2 when the values are loaded, 0 at their end.  Measured on the 8B decode step, back to back (ms, 2 / 0): 4 sequences

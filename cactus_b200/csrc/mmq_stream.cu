@@ -6,9 +6,9 @@
 //
 // What bounds it: the weight stream, and at these widths the latency in front of and behind it.  A T16 tile is in the order
 // of an MMA A fragment, so a warp needs no shared memory for weights: it keeps RING tiles on their way in registers (16 warps
-// an SM: 74 KB).  Weights may be what the kernel ahead writes (an upload, a copy that stacks them), so none is read before the
-// wait for it; the first MS_AHEAD tiles of a warp are asked for in L2 before, a hint that no result depends on (7 sequences of the 8B
-// architecture 2485 us a step; with the first tiles loaded before the wait, which read what an upload ahead had yet to write, 2416).
+// an SM: 74 KB).  Weights may be what the kernel ahead writes (an upload, a copy that stacks them), so none is read before the wait for it,
+// and asking for the first tiles in L2 ahead of it (cp.async.bulk.prefetch.L2) is slower the more are asked for: quantiser and product of
+// 8 columns, Q4_0 4096 x 28672, with 32 / 16 / 8 / 4 / 1 / 0 tiles of a warp 22.2 / 21.3 / 20.4 / 19.6 / 19.3 / 19.3 us, 4096 x 4096 7.7 / 7.7 / 7.7 / 7.7 / 7.3 / 7.2.
 // mmq.cu copies through a shared-memory ring with a barrier per block group, works 128 rows at a time and stays the kernel for
 // more columns (16 columns here: two column tiles per weight tile are bound by instructions, 16.6 us against 13.6 at 14336 x 4096).
 // us on B200, mmq.cu / this kernel at 8 columns (K x M, weights larger than L2 in turn): Q4_0 4096 x 28672 24.6 / 16.9, 4096 x 6144
@@ -29,7 +29,6 @@
 namespace b200 {
 
 constexpr int MS_LOG_WARPS = 4, MS_WARPS = 1 << MS_LOG_WARPS, MS_THREADS = MS_WARPS * 32, MS_SMEM = 216 * 1024;
-constexpr int MS_AHEAD = 8;    // tiles of a warp that are asked for in L2 while the kernel ahead runs (at most 32: a lane each)
 constexpr int MS_SLOT = 160;   // floats of a partial tile: [column][16 rows], columns 20 apart (32 lanes, 32 banks)
 
 struct MsPlan {
@@ -79,12 +78,6 @@ __global__ void __launch_bounds__(MS_THREADS, 1) mmq_stream_kernel(TiledDims dim
         lq += go * TB;
         ld += go * 128;
     };
-    if (lane < min(left, MS_AHEAD)) {
-        const int ahead = lane / len * step * n_bg + lane % len;
-        prefetch_l2_bulk(w + (at0 + ahead) * TB, TB);
-        prefetch_l2_bulk(w + dims.qs_bytes + (at0 + ahead) * 128, 128);
-    }
-
     pdl_prologue();
 #pragma unroll
     for (int k = 0; k < RING; ++k) load(ring[k]);

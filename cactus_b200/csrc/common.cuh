@@ -73,6 +73,18 @@ static inline cudaError_t launch_pdl(void (*kernel)(P...), dim3 grid, dim3 block
 #endif
 static inline bool is_aligned(const void *p, size_t a) { return ((uintptr_t) p % a) == 0; }
 
+// ---- how a product adds its K range ---------------------------------------------------------------
+// The block groups of a row tile that are added in one go; the parts are added in K order.  That order is part of the result's last
+// bits, and a product's result is quantised again by the next one, where a last bit decides whole steps: mmq_stream.cu cuts K
+// where mmq.cu does (mmq_k_split).
+struct KSplit {
+    int ks;            // parts of ceil(n_bg / ks) block groups (no stream-K)
+    bool cluster;      // their CTAs are a cluster
+    int sk_ctas;       // > 0: stream-K over so many CTAs
+    int sk_head;       // > 0: its head/tail deal
+    int group_tiles;   // row tiles of a row group
+};
+
 // ---- ROPE and the K/V store as the end of the product that makes q, k and v ----------------------------
 // Rows 0 .. q_rows - 1 of the product are q (rotated, into dst as they lie), up to k_end k (rotated, f16 into the token's cache row),
 // then v (f16).  `angles` is what b200_rope_angles makes.  The products of up to 8 columns take it as their end: a launch less per layer and

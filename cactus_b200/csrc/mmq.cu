@@ -593,9 +593,11 @@ static int sm_count() {
 struct MmqVariant {
     int cta_tiles;   // 16-row tiles per CTA
     int cta_nt;      // 8-column tiles per CTA
-    int ctas_per_sm; // resident CTAs per SM (filled on first use)
+    int ctas_per_sm; // resident CTAs per SM
+    int sms;         // of the device
+    int clusters[9]; // resident clusters of 2 .. 8 CTAs, 0 = cannot be launched that way ([0]: asked for already, on the variant's first use)
     int (*launch)(const TiledDims &, const uint8_t *, const ActDims &, const uint8_t *, float *, int64_t, float *, int, int, const PeerDst &, cudaStream_t);
-    int (*max_clusters)(int);   // resident clusters of `ksplit` CTAs on this device (0 = cannot be launched that way)
+    int (*max_clusters)(int);
     int (*launch_streamk)(const TiledDims &, const uint8_t *, const ActDims &, const uint8_t *, float *, int64_t, void *, int, int, const PeerDst &, cudaStream_t);
     size_t streamk_slot_bytes;  // one partial tile of a CTA in the stream-K workspace
 };
@@ -660,14 +662,6 @@ template <int WTYPE, int NTW, int WN, int MT, int WM, int STAGES, int MINB, int 
 static int max_clusters_variant(int ksplit) {
     using S = MmqCfg<WTYPE, NTW, WN, MT, WM, STAGES>;
     constexpr int MODEL_SMEM = 227 * 1024 / (MODEL + 1);   // with more than this, MODEL CTAs fit and not one more
-    static int cache[64][9];   // per device and cluster size: 0 = not asked yet, -1 = none, else the count
-    static std::mutex mu;
-    int dev = 0;
-    cudaGetDevice(&dev);
-    dev &= 63;
-    if (ksplit < 2 || ksplit > 8) return 0;
-    std::lock_guard<std::mutex> lock(mu);
-    if (cache[dev][ksplit] != 0) return cache[dev][ksplit] < 0 ? 0 : cache[dev][ksplit];
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(1, 1, (unsigned) ksplit);
     cfg.blockDim = dim3(S::THREADS);
@@ -684,7 +678,6 @@ static int max_clusters_variant(int ksplit) {
         cudaGetLastError();
         n = 0;
     }
-    cache[dev][ksplit] = n > 0 ? n : -1;
     return n;
 }
 
@@ -711,6 +704,8 @@ static MmqVariant make_variant() {
         n = 1;
     }
     v.ctas_per_sm = n < MODEL ? n : MODEL;
+    v.sms = sm_count();
+    v.clusters[0] = 0;
     return v;
 }
 
@@ -749,7 +744,12 @@ static const MmqVariant &pick_variant(int64_t N) {
         return e ? atoi(e) : -1;
     }();
     const int cls = (forced_cls >= 0 && forced_cls <= 2) ? forced_cls : (N > 32 ? 2 : (N > 16 ? 1 : 0));
-    return table[dev][cls][(forced >= 0 && forced < 4) ? forced : 0];
+    MmqVariant &v = table[dev][cls][(forced >= 0 && forced < 4) ? forced : 0];
+    if (!v.clusters[0]) {   // (asking the driver takes microseconds)
+        for (int ks = 2; ks <= 8; ++ks) v.clusters[ks] = v.max_clusters(ks);
+        v.clusters[0] = 1;
+    }
+    return v;
 }
 
 // K splits: the CTA count is made to fit whole waves of resident CTAs; each split pays about three block
@@ -762,7 +762,7 @@ static int choose_ksplit(const MmqVariant &v, const TiledDims &d, int64_t n_nt, 
         return (e && atoi(e) == 0) ? 0 : 1;
     }();
     const int64_t ctas = ((d.n_rt + v.cta_tiles - 1) / v.cta_tiles) * ((n_nt + v.cta_nt - 1) / v.cta_nt);
-    const int64_t slots = (int64_t) sm_count() * v.ctas_per_sm;
+    const int64_t slots = (int64_t) v.sms * v.ctas_per_sm;
     int best = 1;
     int64_t best_cost = -1;
     *cluster = false;
@@ -777,7 +777,7 @@ static int choose_ksplit(const MmqVariant &v, const TiledDims &d, int64_t n_nt, 
             *cluster = false;
         }
         if (allow && ks >= 2 && ks <= 8) {
-            const int64_t cslots = (int64_t) v.max_clusters(ks) * ks;
+            const int64_t cslots = (int64_t) v.clusters[ks] * ks;
             if (cslots > 0) {
                 const int64_t cwaves = (ctas * ks + cslots - 1) / cslots;
                 const int64_t ccost = 2 * cwaves * (per + 3) + 1;
@@ -841,7 +841,7 @@ static int streamk_ctas(const MmqVariant &v, const TiledDims &d, const ActDims &
     *head = 0;
     if (mode == 0 || a.n_nt > v.cta_nt || d.n_rt % v.cta_tiles != 0) return 0;
     const int64_t groups = d.n_rt / v.cta_tiles, total = groups * d.n_bg;
-    const int64_t slots = (int64_t) sm_count() * v.ctas_per_sm;
+    const int64_t slots = (int64_t) v.sms * v.ctas_per_sm;
     if (total >= (1ll << 31) || groups == slots) return 0;
     if (workspace_bytes < streamk_counter_bytes(groups) + (size_t) slots * 3 * v.streamk_slot_bytes) return 0;
     if (groups < slots) {
@@ -856,7 +856,7 @@ static int streamk_ctas(const MmqVariant &v, const TiledDims &d, const ActDims &
     // 1.07 us per block group alone, 1.85 us for one of each of two), so what counts is the block groups per SM: the
     // fullest SM of the wave-quantised launch against the even share plus about eight block groups for the counter
     // reset, the parked parts and the last read.
-    const int64_t sms = sm_count();
+    const int64_t sms = v.sms;
     const int64_t per = (d.n_bg + ks - 1) / ks;
     const int64_t now = (groups * ks + sms - 1) / sms * (per + 3);
     const int64_t sk = (total + sms - 1) / sms + 8;
@@ -869,24 +869,29 @@ void launch_mmq_reduce(const float *partial, int ks, int64_t M, int64_t N, float
     launch_pdl(mmq_reduce_kernel, dim3((unsigned) ((total + 255) / 256)), dim3(256), 0, st, partial, ks, M, N, dst, dst_nb_row, PeerDst{});
 }
 
+KSplit mmq_k_split(int wtype, const TiledDims &d, const ActDims &a, bool streamk, bool workspace, size_t workspace_bytes) {
+    const MmqVariant &v = variant_for(wtype, a.N);
+    KSplit s = {};
+    s.group_tiles = v.cta_tiles;
+    s.ks = choose_ksplit(v, d, a.n_nt, &s.cluster);
+    const size_t per_split = (size_t) a.N * d.M * sizeof(float);
+    if (s.ks > 1 && !s.cluster && (!workspace || workspace_bytes < per_split * s.ks)) {
+        s.ks = workspace ? (int) std::max<size_t>(1, workspace_bytes / per_split) : 1;  // fewer splits fit: still correct, only slower
+    }
+    if (streamk && workspace) s.sk_ctas = streamk_ctas(v, d, a, s.ks, s.cluster, workspace_bytes, &s.sk_head);
+    return s;
+}
+
 int launch_mmq(int wtype, const TiledDims &d, const void *w, const ActDims &a, const void *aq, float *dst, int64_t dst_nb_row,
                void *workspace, size_t workspace_bytes, cudaStream_t st, const PeerDst &peers) {
     const MmqVariant &v = variant_for(wtype, a.N);
-    bool cluster = false;
-    int ks = choose_ksplit(v, d, a.n_nt, &cluster);
-    const size_t per_split = (size_t) a.N * d.M * sizeof(float);
-    if (ks > 1 && !cluster && (!workspace || workspace_bytes < per_split * ks)) {
-        ks = workspace ? (int) std::max<size_t>(1, workspace_bytes / per_split) : 1;  // fewer splits fit: still correct, only slower
-    }
-    if (peers.n == 0 && (peers.n_seg <= 1 || peers.n_wseg > 0) && workspace) {   // (the ranges of a row-split rank keep the plain grid)
-        int head = 0;
-        if (const int ctas = streamk_ctas(v, d, a, ks, cluster, workspace_bytes, &head))
-            return v.launch_streamk(d, (const uint8_t *) w, a, (const uint8_t *) aq, dst, dst_nb_row, workspace, ctas, head, peers, st);
-    }
-    if (int e = v.launch(d, (const uint8_t *) w, a, (const uint8_t *) aq, dst, dst_nb_row, (float *) workspace, ks, cluster ? 1 : 0, peers, st)) return e;
-    if (ks > 1 && !cluster) {
+    // (the ranges of a row-split rank keep the plain grid)
+    const KSplit s = mmq_k_split(wtype, d, a, peers.n == 0 && (peers.n_seg <= 1 || peers.n_wseg > 0), workspace != nullptr, workspace_bytes);
+    if (s.sk_ctas) return v.launch_streamk(d, (const uint8_t *) w, a, (const uint8_t *) aq, dst, dst_nb_row, workspace, s.sk_ctas, s.sk_head, peers, st);
+    if (int e = v.launch(d, (const uint8_t *) w, a, (const uint8_t *) aq, dst, dst_nb_row, (float *) workspace, s.ks, s.cluster ? 1 : 0, peers, st)) return e;
+    if (s.ks > 1 && !s.cluster) {
         const int64_t total = d.M * a.N;
-        launch_pdl(mmq_reduce_kernel, dim3((unsigned) ((total + 255) / 256)), dim3(256), 0, st, (const float *) workspace, ks, d.M, a.N, dst, dst_nb_row, peers);
+        launch_pdl(mmq_reduce_kernel, dim3((unsigned) ((total + 255) / 256)), dim3(256), 0, st, (const float *) workspace, s.ks, d.M, a.N, dst, dst_nb_row, peers);
         return check_launch("mmq_reduce");
     }
     return B200_OK;

@@ -19,8 +19,8 @@ int launch_mmvq(int wtype, const TiledDims &d, const void *w, const ActDims &a, 
                 const RopeStore *rope, cudaStream_t st);
 int launch_mmq(int wtype, const TiledDims &d, const void *w, const ActDims &a, const void *aq, float *dst, int64_t dst_nb_row,
                void *workspace, size_t workspace_bytes, cudaStream_t st, const PeerDst &peers);
-bool launch_mmq_stream(int wtype, const TiledDims &d, const void *w, const ActDims &a, const void *aq, float *dst, int64_t dst_nb_row, const RopeStore *rope, cudaStream_t st,
-                       int *rc);
+bool launch_mmq_stream(int wtype, const TiledDims &d, const void *w, const ActDims &a, const void *aq, float *dst, int64_t dst_nb_row, bool workspace, size_t workspace_bytes,
+                       const RopeStore *rope, cudaStream_t st, int *rc);
 int launch_peer_signal_wait(void *const *flags_of_rank, int rank, int g, cudaStream_t st);
 size_t mmq_workspace_bytes(int wtype, int64_t K, int64_t M, int64_t N);
 }  // namespace b200
@@ -95,8 +95,8 @@ static bool use_tc(int wtype, int64_t K, int64_t M, int64_t N) {
     return M >= 4096 && M * K >= (24 << 20);
 }
 
-// Up to 8 columns the kernel that streams tiles into registers (mmq_stream.cu): faster than the mma.sync kernel at every shape from 3
-// columns on (its head comment).  One and two columns have the dp4a kernel, whose short CTAs start and end faster; from some 32768
+// Up to 8 columns the kernel that streams tiles into registers (mmq_stream.cu): from 3 columns on where it is faster than the mma.sync
+// kernel, whose result it has to the last bit (ms_pays there).  One and two columns have the dp4a kernel, whose short CTAs start and end faster; from some 32768
 // tiles (16 rows x 128 values) on the stream decides.  us on B200, dp4a / stream at one and two columns (K x M): Q4_0 4096 x 28672
 // 19.6 / 16.0, 18.6 / 16.1; 4096 x 20480 14.1 / 12.4, 17.1 / 12.5; 8192 x 8192 12.2 / 11.8, 11.8 / 12.0; 4096 x 128256 60.0 / 51.6, 63.6 / 52.5;
 // 8192 x 4096 6.2 / 7.6, 7.3 / 7.7; 14336 x 4096 9.8 / 11.0, 10.8 / 11.0; Q8_0 2048 x 128256 49.8 / 45.9, 50.5 / 46.5; 4096 x 14336 13.8 / 14.2, 14.3 / 14.4.
@@ -186,7 +186,7 @@ static int mul_mat_prequant(int wtype, const void *w, int64_t K, int64_t M, cons
     const ActDims a = act_dims(K, N);
     if (peers.n == 0 && peers.n_seg <= 1 && use_stream(d, N)) {
         int rc = 0;
-        if (launch_mmq_stream(wtype, d, w, a, act, dst, dst_row_stride_bytes, nullptr, (cudaStream_t) stream, &rc)) return rc;
+        if (launch_mmq_stream(wtype, d, w, a, act, dst, dst_row_stride_bytes, workspace != nullptr, workspace_bytes, nullptr, (cudaStream_t) stream, &rc)) return rc;
     }
     if (N <= mmvq_max_n()) return launch_mmvq(wtype, d, w, a, act, dst, dst_row_stride_bytes, peers, nullptr, (cudaStream_t) stream);
     return launch_mmq(wtype, d, w, a, act, dst, dst_row_stride_bytes, workspace, workspace_bytes, (cudaStream_t) stream, peers);
@@ -206,7 +206,7 @@ int b200_mul_mat_qkv_rope(int wtype, const void *w, int64_t K, const void *act, 
     const RopeStore rope = {angles, slots, (__half *) k_cache, (__half *) v_cache, k_cache_nb_row, v_cache_nb_row, (int) (H * D), (int) ((H + Hkv) * D), (int) D / 2 - 1, n_dims / 2};
     if (use_stream(d, N)) {
         int rc = 0;
-        if (launch_mmq_stream(wtype, d, w, a, act, qkv, qkv_row_stride_bytes, &rope, (cudaStream_t) stream, &rc)) return rc;
+        if (launch_mmq_stream(wtype, d, w, a, act, qkv, qkv_row_stride_bytes, workspace != nullptr, workspace_bytes, &rope, (cudaStream_t) stream, &rc)) return rc;
     } else if (N <= std::min(2, mmvq_max_n())) {
         return launch_mmvq(wtype, d, w, a, act, qkv, qkv_row_stride_bytes, PeerDst{}, &rope, (cudaStream_t) stream);
     }

@@ -77,6 +77,8 @@ static inline bool is_aligned(const void *p, size_t a) { return ((uintptr_t) p %
 // The block groups of a row tile that are added in one go; the parts are added in K order.  That order is part of the result's last
 // bits, and a product's result is quantised again by the next one, where a last bit decides whole steps: mmq_stream.cu cuts K
 // where mmq.cu does (mmq_k_split).
+// From HEAD_ROWS rows on a weight is taken for an output head, whose result nothing quantises again: there the kernels may cut K as suits them.
+constexpr int64_t HEAD_ROWS = 65536;
 struct KSplit {
     int ks;            // parts of ceil(n_bg / ks) block groups (no stream-K)
     bool cluster;      // their CTAs are a cluster

@@ -36,8 +36,6 @@ namespace b200 {
 constexpr int MS_WARPS = 16, MS_THREADS = MS_WARPS * 32, MS_SMEM = 216 * 1024;
 constexpr int MS_SLOT = 160;   // floats of a partial tile: [column][16 rows], columns 20 apart (32 lanes, 32 banks)
 
-constexpr int64_t MS_FREE_ROWS = 65536;   // rows from which a weight is taken for an output head
-
 struct MsPlan {
     int ks, per;        // the K range of a row tile is ks tasks of `per` block groups (the last one shorter)
     // A stream-K deal cuts some row groups' last task once more: what is behind the first n_bg - unit block groups of all row groups, laid
@@ -278,7 +276,7 @@ bool launch_mmq_stream(int wtype, const TiledDims &d, const void *w, const ActDi
                        const RopeStore *rope, cudaStream_t st, int *rc) {
     const int64_t ctas = std::min<int64_t>(ms_sm_count(), d.n_rt), rt = (d.n_rt + ctas - 1) / ctas, act = d.n_bg * 1280, n_bg = d.n_bg;
     if (a.n_nt != 1 || d.n_rt * n_bg >= (1ll << 31) || rt * n_bg * d.tile_bytes >= (1ll << 31)) return false;
-    const bool free = a.N <= 2 || d.M >= MS_FREE_ROWS;
+    const bool free = d.M >= HEAD_ROWS;
     MsPlan p = {};
     if (free) {
         if (rope) return false;

@@ -96,13 +96,16 @@ static bool use_tc(int wtype, int64_t K, int64_t M, int64_t N) {
 }
 
 // Up to 8 columns the kernel that streams tiles into registers (mmq_stream.cu): from 3 columns on where it is faster than the mma.sync
-// kernel, whose result it has to the last bit (ms_pays there).  One and two columns have the dp4a kernel, whose short CTAs start and end faster; from some 32768
-// tiles (16 rows x 128 values) on the stream decides.  us on B200, dp4a / stream at one and two columns (K x M): Q4_0 4096 x 28672
-// 19.6 / 16.0, 18.6 / 16.1; 4096 x 20480 14.1 / 12.4, 17.1 / 12.5; 8192 x 8192 12.2 / 11.8, 11.8 / 12.0; 4096 x 128256 60.0 / 51.6, 63.6 / 52.5;
-// 8192 x 4096 6.2 / 7.6, 7.3 / 7.7; 14336 x 4096 9.8 / 11.0, 10.8 / 11.0; Q8_0 2048 x 128256 49.8 / 45.9, 50.5 / 46.5; 4096 x 14336 13.8 / 14.2, 14.3 / 14.4.
-static bool use_stream(const TiledDims &d, int64_t N) {
+// kernel, whose result it has to the last bit (ms_pays there).  At one and two columns it adds in another order than the dp4a kernel
+// (whose short CTAs start and end faster), so only what is taken for an output head streams: a layer's sums are quantised again, and with
+// 4096 x 28672 streaming the logits of one sequence of the 8B architecture moved by 1.4e-2 of their norm (16.3 us against 19.5).
+// Quantiser and product, us on B200, dp4a / stream at one and two columns (K x M): Q4_0 4096 x 128256 60.7 / 51.1, 63.5 / 52.6; 4096 x 65536 36.3 / 29.4,
+// 36.9 / 30.4; 1024 x 65536 12.2 / 11.6, 13.6 / 12.3; Q8_0 2048 x 128256 50.0 / 45.0, 50.0 / 47.1; 4096 x 128256 88.1 / 83.9, 90.7 / 85.4; 1024 x 128256
+// 31.2 / 25.9, 25.5 / 26.8.  Below 32768 tiles (16 rows x 128 values) nothing is won: Q4_0 512 x 65536 8.1, 256 x 128256 11.4, for the dp4a kernel.
+static bool use_stream(int wtype, const TiledDims &d, int64_t N) {
     if (N > 8 || mmq_sync_forced()) return false;
-    return N > mmvq_max_n() || (N <= 2 && d.n_rt * d.n_bg >= 32768);
+    if (N > 2) return N > mmvq_max_n();
+    return d.M >= HEAD_ROWS && d.n_rt * d.n_bg >= 32768 && (wtype == B200_TYPE_Q4_0 || N == 1 || d.n_bg >= 16);
 }
 
 extern "C" {
@@ -184,7 +187,7 @@ static int mul_mat_prequant(int wtype, const void *w, int64_t K, int64_t M, cons
     B200_REQUIRE(!workspace || is_aligned(workspace, 256), "workspace must be 256-byte aligned");
     const TiledDims d = tiled_dims(wtype, K, M);
     const ActDims a = act_dims(K, N);
-    if (peers.n == 0 && peers.n_seg <= 1 && use_stream(d, N)) {
+    if (peers.n == 0 && peers.n_seg <= 1 && use_stream(wtype, d, N)) {
         int rc = 0;
         if (launch_mmq_stream(wtype, d, w, a, act, dst, dst_row_stride_bytes, workspace != nullptr, workspace_bytes, nullptr, (cudaStream_t) stream, &rc)) return rc;
     }
@@ -204,7 +207,7 @@ int b200_mul_mat_qkv_rope(int wtype, const void *w, int64_t K, const void *act, 
     const TiledDims d = tiled_dims(wtype, K, M);
     const ActDims a = act_dims(K, N);
     const RopeStore rope = {angles, slots, (__half *) k_cache, (__half *) v_cache, k_cache_nb_row, v_cache_nb_row, (int) (H * D), (int) ((H + Hkv) * D), (int) D / 2 - 1, n_dims / 2};
-    if (use_stream(d, N)) {
+    if (use_stream(wtype, d, N)) {
         int rc = 0;
         if (launch_mmq_stream(wtype, d, w, a, act, qkv, qkv_row_stride_bytes, workspace != nullptr, workspace_bytes, &rope, (cudaStream_t) stream, &rc)) return rc;
     } else if (N <= std::min(2, mmvq_max_n())) {

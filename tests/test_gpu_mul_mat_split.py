@@ -33,3 +33,29 @@ def test_columns_do_not_depend_on_the_kernel(wtype, M, K):
         torch.cuda.synchronize()
         return out
     assert torch.equal(without_workspace(7), without_workspace(16)[:7])
+
+
+@pytest.mark.parametrize("wtype,M,K", [(2, 28672, 4096), (8, 16384, 4096), (2, 65504, 1024)])
+def test_one_and_two_columns_of_a_layer(wtype, M, K):
+    """A layer's product of one or two columns is the dp4a kernel's whatever its size: the rows of two parts of a row split, which only that
+    kernel stores, are the same to the last bit."""
+    import ctypes as C
+
+    from cactus_b200 import ops
+    from cactus_b200._lib import check, lib
+    from cactus_b200.engine import random_blocks
+    L = lib()
+    st = torch.cuda.current_stream().cuda_stream
+    g = torch.Generator(device="cuda").manual_seed(M + K)
+    w = ops.QWeight.from_blocks(wtype, K, M, random_blocks(wtype, M, K, g))
+    first = M // 32 * 16
+    rows, cols = (C.c_int64 * 2)(first, M - first), (C.c_int64 * 2)(0, first)
+    flags = torch.zeros(64, dtype=torch.int32, device="cuda")   # (a world of one: nobody is waited for)
+    for N in (1, 2):
+        x = torch.randn((N, K), device="cuda", generator=g)
+        act = torch.empty(L.b200_act_bytes(K, N), dtype=torch.uint8, device="cuda")
+        check(L.b200_quantize_activations(x.data_ptr(), K * 4, K, N, act.data_ptr(), act.numel(), 0, st))
+        want = torch.empty((N, M), device="cuda")
+        check(L.b200_mul_mat_q_rowsplit_stacked(wtype, w.data.data_ptr(), K, M, act.data_ptr(), N, 0, 1, (C.c_void_p * 1)(want.data_ptr()), M * 4, 2, rows, cols, None, 0,
+                                                (C.c_void_p * 1)(flags.data_ptr()), st))
+        assert torch.equal(ops.mul_mat(w, x), want), N

@@ -285,6 +285,9 @@ bool launch_mmq_stream(int wtype, const TiledDims &d, const void *w, const ActDi
         for (int ks = MS_WARPS; ks >= 1; ks /= 2) {
             const int64_t chunk = (n_bg + ks - 1) / ks, rounds = (rt * ks + MS_WARPS - 1) / MS_WARPS, cost = rounds * (chunk * 4 + 1);
             if (act + rt * ks * MS_SLOT * 4 > MS_SMEM || (best >= 0 && cost >= best)) continue;
+            // (not understood, but steep: with 63 row tiles and more to a CTA four parts take 119 us at Q8_0 4096 x 151936, 1 column, two 101; up to 55 row
+            // tiles four are as good as two or better: 4096 x 128256 84.0 / 84.2, 2048 x 102400 Q4_0 24.6 / 25.5)
+            if (ks == 4 && rt > 60) continue;
             best = cost;
             p.ks = ks;
             p.per = (int) chunk;

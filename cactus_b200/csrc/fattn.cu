@@ -808,13 +808,10 @@ static int fattn_nsplit(int64_t Nq, int64_t Hkv, int hgroups, int64_t n_kv) {
     const int64_t want = 2 * fa_sm_count();
     if (ctas >= want) return 1;
     int64_t ns = (want + ctas - 1) / ctas;
-    // At least 512 cells of the cache to a split, from 1024 cells on 128 (a token's own words are dealt out evenly, two at least): one
-    // sequence of 640 cells in 1024, 1B architecture, 825 us a step with two splits, 778 with four or more.
-    ns = std::min<int64_t>(ns, n_kv >= 1024 ? n_kv / 128 : 1);
-    // No more than a cluster has CTAs where those fill the SMs, or where a split has 256 cells then: us per decode step, uncapped / capped,
-    // 1B, three sequences of up to 2048 cells 885 / 860, 8B, four of 16000 3725 / 3671, 8B, one of 2000 in a cache of 2048 2143 / 2090; but
-    // 8B, one of 4000 in 4096 2235 / 2290, two of 8000 2614 / 2727.
-    if (ns > FA_CLUSTER_MAX && (FA_CLUSTER_MAX * ctas >= fa_sm_count() || n_kv <= 256 * FA_CLUSTER_MAX)) ns = FA_CLUSTER_MAX;
+    // At least 512 cells of the cache to a split.  Where a range is cut is part of the result's last bits, and the next product quantises the
+    // result, where a last bit decides whole int8 steps: 128 cells to a split from 1024 cells on are faster (1B architecture, one
+    // sequence of 640 cells in 1024, 681 us a step against 748) but moved the logits of every third step by 5e-3 of their norm.
+    ns = std::min<int64_t>(ns, std::max<int64_t>(1, n_kv / 512));
     return (int) std::min<int64_t>(ns, 64);
 }
 

@@ -334,10 +334,13 @@ __device__ __forceinline__ void fattn_store_out(const FattnParams &p, int64_t j,
 // and the plain one must not change with it
 // CLUSTER: the KV splits of a token and head group are a cluster of CTAs, which add their parts through each other's shared memory; see
 // launch_mma_cluster
-template <int D, bool QUANT, bool CLUSTER = false>
+// VOTED: launched beside the query-tiled kernel, mostly to return.  It has one walk, which reads the mask, where the others have a second one for
+// masks of 0 and -inf: with both the returning grid costs half a microsecond more once another kernel has run in between (16 ragged sequences,
+// 512 tokens: 121.8 us against 121.2).  A test in a single walk instead is no way out: 64 decode tokens 75.3 us, 73.2 with two walks.
+template <int D, bool QUANT, bool CLUSTER = false, bool VOTED = false>
 __global__ void __launch_bounds__(FA_THREADS, FA_MIN_CTAS) fattn_mma_kernel(FattnParams p) {
     pdl_prologue();
-    if (p.vote == 1 && fattn_tiled_chosen(p.plan)) return;   // the query-tiled kernel takes this ubatch
+    if ((VOTED || (CLUSTER && p.vote == 1)) && fattn_tiled_chosen(p.plan)) return;   // the query-tiled kernel takes this ubatch
     constexpr bool PREFETCH_V = FA_PREFETCH_V || (CLUSTER && D == 64);   // (where there are registers for it)
     constexpr int KS = D / 16;   // k-steps of the S MMA
     constexpr int NU = D / 32;   // 16-byte K pieces per lane and cell
@@ -396,7 +399,7 @@ __global__ void __launch_bounds__(FA_THREADS, FA_MIN_CTAS) fattn_mma_kernel(Fatt
     const int64_t w_begin = CLUSTER ? min(n_words, (int64_t) split * per_split) : (int64_t) split * per_split;
     const int64_t w_end = min(n_words, w_begin + per_split);
     // (a mask of nothing but 0 and -inf adds nothing in the cells that take part)
-    const __half *mrow = p.mask && p.plan[2] != 0 ? reinterpret_cast<const __half *>(p.mask + j * p.mask_nb_row) : nullptr;
+    const __half *mrow = VOTED || (p.mask && p.plan[2] != 0) ? reinterpret_cast<const __half *>(p.mask + j * p.mask_nb_row) : nullptr;
     const char *kbase = p.k + (int64_t) hk * p.k_nb_head;
     const char *vbase = p.v + (int64_t) hk * p.v_nb_head;
 
@@ -536,7 +539,7 @@ __global__ void __launch_bounds__(FA_THREADS, FA_MIN_CTAS) fattn_mma_kernel(Fatt
         __syncthreads();
     }
     };
-    if (mrow) walk(std::true_type{});
+    if (VOTED || mrow) walk(std::true_type{});
     else walk(std::false_type{});
 
     pdl_trigger();
@@ -1040,7 +1043,10 @@ static int flash_attn_impl(bool parity, int64_t D, int64_t H, int64_t Hkv, int64
         }
         return check_launch("fattn_mma");
     }
-    if (D == 128) {
+    if (p.vote == 1) {
+        if (D == 128) launch_pdl(fattn_mma_kernel<128, false, false, true>, grid, dim3(FA_THREADS), 0, st, p);
+        else launch_pdl(fattn_mma_kernel<64, false, false, true>, grid, dim3(FA_THREADS), 0, st, p);
+    } else if (D == 128) {
         if (qo) launch_pdl(fattn_mma_kernel<128, true>, grid, dim3(FA_THREADS), 0, st, p);
         else launch_pdl(fattn_mma_kernel<128, false>, grid, dim3(FA_THREADS), 0, st, p);
     } else {

@@ -35,8 +35,9 @@ def test_columns_do_not_depend_on_the_kernel(wtype, M, K):
     assert torch.equal(without_workspace(7), without_workspace(16)[:7])
 
 
-@pytest.mark.parametrize("wtype,M,K", [(2, 28672, 4096), (8, 16384, 4096), (2, 65504, 1024)])
-def test_one_and_two_columns_of_a_layer(wtype, M, K):
+# layers of 32768 tiles and more; a row tile short of an output head; a head one block group short of 32768 tiles, and one of a short K at two columns
+@pytest.mark.parametrize("wtype,M,K,Ns", [(2, 28672, 4096, (1, 2)), (8, 16384, 4096, (1, 2)), (2, 65520, 1024, (1, 2)), (2, 65536, 896, (1, 2)), (8, 65536, 1920, (2,))])
+def test_one_and_two_columns_of_a_layer(wtype, M, K, Ns):
     """A layer's product of one or two columns is the dp4a kernel's whatever its size: the rows of two parts of a row split, which only that
     kernel stores, are the same to the last bit."""
     import ctypes as C
@@ -51,7 +52,7 @@ def test_one_and_two_columns_of_a_layer(wtype, M, K):
     first = M // 32 * 16
     rows, cols = (C.c_int64 * 2)(first, M - first), (C.c_int64 * 2)(0, first)
     flags = torch.zeros(64, dtype=torch.int32, device="cuda")   # (a world of one: nobody is waited for)
-    for N in (1, 2):
+    for N in Ns:
         x = torch.randn((N, K), device="cuda", generator=g)
         act = torch.empty(L.b200_act_bytes(K, N), dtype=torch.uint8, device="cuda")
         check(L.b200_quantize_activations(x.data_ptr(), K * 4, K, N, act.data_ptr(), act.numel(), 0, st))

@@ -242,6 +242,8 @@ class LlamaEngine:
         fa_args = (cfg.head_dim, self.n_head_local, self.n_kv_head_local)
         split_kv = [L.b200_flash_attn_scratch_bytes(*fa_args, t, n_cells) > L.b200_mask_index_bytes(t, n_cells) for t in range(1, min(T, 128) + 1)]
         self.fa_quant_max_tokens = min(split_kv.index(False) if False in split_kv else len(split_kv), int(os.environ.get("B200_FA_QUANT_MAX_T", "128")))
+        if self.n_head_local * cfg.head_dim % 128:   # b200_flash_attn_ext_quant takes whole block groups only
+            self.fa_quant_max_tokens = 0
         self.fa_scratch = u8(max(L.b200_flash_attn_scratch_bytes(cfg.head_dim, self.n_head_local, self.n_kv_head_local, t, n_cells) for t in range(1, T + 1)))
         self.graphs: dict[int, torch.cuda.CUDAGraph] = {}
         self.launches_per_step: dict[int, int] = {}

@@ -238,9 +238,12 @@ class LlamaEngine:
         self.ws = u8(max(ws))
         # Where the attention cuts its KV range, what adds the splits leaves the result quantised (b200_flash_attn_ext_quant: one launch
         # less per layer, bit-identical).  Without splits the attention kernel itself would have to, at its register limit:
-        # 70.5 us for the 64-token batch against 57.5 + 2.5.  B200_FA_QUANT_MAX_T lowers the token count.
+        # 70.5 us for the 64-token batch against 57.5 + 2.5.  Nor where the query-tiled kernel is considered (B200_FA_TILE_MIN_NQ tokens and more),
+        # which has no quantised form.  B200_FA_QUANT_MAX_T lowers the token count.
         fa_args = (cfg.head_dim, self.n_head_local, self.n_kv_head_local)
-        split_kv = [L.b200_flash_attn_scratch_bytes(*fa_args, t, n_cells) > L.b200_mask_index_bytes(t, n_cells) for t in range(1, min(T, 128) + 1)]
+        tile_min = int(os.environ.get("B200_FA_TILE_MIN_NQ", "128"))
+        t_max = min(T, tile_min - 1 if tile_min > 0 and self.n_head_local // self.n_kv_head_local in (2, 4, 8, 16) else 128)
+        split_kv = [L.b200_flash_attn_scratch_bytes(*fa_args, t, n_cells) > L.b200_mask_index_bytes(t, n_cells) for t in range(1, t_max + 1)]
         self.fa_quant_max_tokens = min(split_kv.index(False) if False in split_kv else len(split_kv), int(os.environ.get("B200_FA_QUANT_MAX_T", "128")))
         if self.n_head_local * cfg.head_dim % 128:   # b200_flash_attn_ext_quant takes whole block groups only
             self.fa_quant_max_tokens = 0

@@ -45,3 +45,19 @@ def test_quantising_attention_in_the_engine(oracle, d_model, n_head, n_kv_head, 
         want = ref.decode(*ubatch)
         assert np.array_equal(ids, want.argmax(-1))
         assert (np.abs(got - want).max(axis=1) / np.abs(want).max()).max() < 3e-2
+
+
+def test_where_the_query_tiled_kernel_is_considered(oracle):
+    """From 128 tokens on the query-tiled kernel may take a prompt, which needs the attention's result in f32."""
+    from cactus_b200.engine import LlamaEngine, LlamaWeights
+    cfg = _config(256, 4, 2)
+    arrays = tiny_model(oracle, cfg)
+    engines = [LlamaEngine(LlamaWeights.from_numpy(cfg, arrays), 1024, max_tokens=128, use_graphs=False) for _ in range(2)]
+    assert engines[0].fa_quant_max_tokens == 127
+    engines[1].fa_quant_max_tokens = 0
+    tokens = np.random.default_rng(2).integers(0, cfg.vocab, 128)
+    for T in (127, 128):
+        args = (tokens[:T], np.arange(T), np.zeros(T, np.int64), np.arange(T))
+        assert np.array_equal(engines[0].decode(*args)[0], engines[1].decode(*args)[0])
+        for e in engines:
+            e.clear()

@@ -5,8 +5,6 @@
 #include <cooperative_groups.h>
 #include <math_constants.h>
 
-#include <algorithm>
-
 #include "common.cuh"
 
 namespace b200 {
@@ -76,19 +74,18 @@ __global__ void __launch_bounds__(256) set_rows_f16_kernel(const float *__restri
     reinterpret_cast<__half *>(reinterpret_cast<char *>(dst) + (int64_t) slots[r] * dst_nb_row)[c] = __float2half_rn(v);
 }
 
-// first index of the maximum of each row (ties: lowest index, as a linear scan finds it).  A cluster of 8 CTAs per row, each with an
-// eighth of it: bound by latency, the load of a thread's elements (8 x 16 bytes for a vocabulary of 128256, all on their way at
-// once) and the reduction.  16-byte loads where the row allows them.  us per launch on B200, one CTA of 1024 threads per row / this:
-// 1 x 128256 11.7 / 6.8, 64 x 128256 13.1 / 10.0.
-constexpr int ARGMAX_THREADS = 512, ARGMAX_CTAS = 8;
-__global__ void __cluster_dims__(ARGMAX_CTAS, 1, 1) __launch_bounds__(ARGMAX_THREADS) argmax_rows_kernel(const float *__restrict__ x, int64_t x_nb_row, int64_t d,
-                                                                                                        int32_t *__restrict__ out) {
+// first index of the maximum of each row (ties: lowest index, as a linear scan finds it).  Bound by latency: the load of a thread's
+// elements (16 bytes each where the row allows them) and the reduction.  A few long rows get a cluster of 8 CTAs each, which has 8 x 16 bytes of a
+// thread for a vocabulary of 128256, all on their way at once; many rows fill the SMs with a CTA each, and the cluster's barriers only cost.
+// us per launch on B200, rows beyond L2 in turn, a CTA of 1024 threads per row / a cluster: 128256 values, 1 row 5.4 / 3.4, 16 rows 10.7 / 6.4, 64 rows 11.9 /
+// 8.9, 96 rows 12.7 / 14.2, 512 rows 42.9 / 56.4; 32000 values, 1 row 2.6 / 2.5, 64 rows 4.9 / 5.0, 512 rows 13.5 / 28.8; 320 values, 64 rows 1.8 / 3.5.
+template <int CTAS, int THREADS>
+__device__ __forceinline__ void argmax_row(const float *__restrict__ x, int64_t x_nb_row, int64_t d, int32_t *__restrict__ out, int64_t r, int part) {
     const cooperative_groups::cluster_group cluster = cooperative_groups::this_cluster();
-    cluster.barrier_arrive();   // (the first CTA's shared memory may be written once it has started: the wait is below)
+    if (CTAS > 1) cluster.barrier_arrive();   // (the first CTA's shared memory may be written once it has started: the wait is below)
     pdl_prologue();
-    constexpr int WARPS = ARGMAX_THREADS / 32, ALL = ARGMAX_THREADS * ARGMAX_CTAS;
-    const int64_t r = blockIdx.y;
-    const int part = blockIdx.x, tid = threadIdx.x, me = part * ARGMAX_THREADS + tid;
+    constexpr int WARPS = THREADS / 32, ALL = THREADS * CTAS, UNROLL = CTAS > 1 ? 8 : 4;
+    const int tid = threadIdx.x, me = part * THREADS + tid;
     const float *row = reinterpret_cast<const float *>(reinterpret_cast<const char *>(x) + r * x_nb_row);
     float best = -CUDART_INF_F;
     int bi = 0x7fffffff;
@@ -96,7 +93,7 @@ __global__ void __cluster_dims__(ARGMAX_CTAS, 1, 1) __launch_bounds__(ARGMAX_THR
     if ((reinterpret_cast<uintptr_t>(row) & 15) == 0) {
         const int64_t n4 = d >> 2;
         const float4 *row4 = reinterpret_cast<const float4 *>(row);
-#pragma unroll 8
+#pragma unroll UNROLL
         for (int64_t i = me; i < n4; i += ALL) {
             const float4 v = __ldg(row4 + i);
             const int b = (int) (i << 2);
@@ -122,31 +119,41 @@ __global__ void __cluster_dims__(ARGMAX_CTAS, 1, 1) __launch_bounds__(ARGMAX_THR
     };
     __shared__ float sv[WARPS];
     __shared__ int si[WARPS];
-    __shared__ float cv[ARGMAX_CTAS];   // of the cluster's first CTA: every CTA's candidate
-    __shared__ int ci[ARGMAX_CTAS];
+    __shared__ float cv[CTAS];   // of the cluster's first CTA: every CTA's candidate
+    __shared__ int ci[CTAS];
     fold(16);
     if ((tid & 31) == 0) {
         sv[tid >> 5] = best;
         si[tid >> 5] = bi;
     }
     __syncthreads();
-    cluster.barrier_wait();
+    if (CTAS > 1) cluster.barrier_wait();
     if (tid < 32) {
         best = sv[tid & (WARPS - 1)];
         bi = si[tid & (WARPS - 1)];
         fold(WARPS / 2);
-        if (tid == 0) {
+        if (CTAS > 1 && tid == 0) {
             cluster.map_shared_rank(cv, 0)[part] = best;
             cluster.map_shared_rank(ci, 0)[part] = bi;
         }
     }
-    cluster.sync();
-    if (part == 0 && tid < 32) {
-        best = cv[tid & (ARGMAX_CTAS - 1)];
-        bi = ci[tid & (ARGMAX_CTAS - 1)];
-        fold(ARGMAX_CTAS / 2);
-        if (tid == 0) out[r] = bi == 0x7fffffff ? 0 : bi;   // nothing above -inf: a linear scan stays at index 0
+    if (CTAS > 1) {
+        cluster.sync();
+        if (tid < 32) {
+            best = cv[tid & (CTAS - 1)];
+            bi = ci[tid & (CTAS - 1)];
+            fold(CTAS / 2);
+        }
     }
+    if (part == 0 && tid == 0) out[r] = bi == 0x7fffffff ? 0 : bi;   // nothing above -inf: a linear scan stays at index 0
+}
+constexpr int ARGMAX_CTAS = 8, ARGMAX_CLUSTER_THREADS = 512, ARGMAX_THREADS = 1024;
+__global__ void __cluster_dims__(ARGMAX_CTAS, 1, 1) __launch_bounds__(ARGMAX_CLUSTER_THREADS)
+argmax_rows_cluster_kernel(const float *__restrict__ x, int64_t x_nb_row, int64_t d, int32_t *__restrict__ out) {
+    argmax_row<ARGMAX_CTAS, ARGMAX_CLUSTER_THREADS>(x, x_nb_row, d, out, blockIdx.y, blockIdx.x);
+}
+__global__ void __launch_bounds__(ARGMAX_THREADS) argmax_rows_kernel(const float *__restrict__ x, int64_t x_nb_row, int64_t d, int32_t *__restrict__ out) {
+    argmax_row<1, ARGMAX_THREADS>(x, x_nb_row, d, out, blockIdx.x, 0);
 }
 
 }  // namespace b200
@@ -190,10 +197,10 @@ int b200_set_rows_f16(const float *x, int64_t x_nb_row, const int32_t *slots, vo
 int b200_argmax_rows(const float *x, int64_t x_nb_row, int64_t d, int64_t rows, int32_t *out, b200_stream_t stream) {
     B200_REQUIRE(x && out && d > 0 && rows >= 0 && x_nb_row % 4 == 0, "bad argmax arguments");
     if (rows == 0) return B200_OK;
-    for (int64_t r0 = 0; r0 < rows; r0 += 65535) {   // (a grid has at most 65535 rows)
-        const dim3 grid(ARGMAX_CTAS, (unsigned) std::min<int64_t>(65535, rows - r0));
-        launch_pdl(argmax_rows_kernel, grid, dim3(ARGMAX_THREADS), 0, (cudaStream_t) stream, reinterpret_cast<const float *>(reinterpret_cast<const char *>(x) + r0 * x_nb_row), x_nb_row, d, out + r0);
-    }
+    // (where the two cross: argmax_row)
+    if (rows <= 64 && d >= 32768)
+        launch_pdl(argmax_rows_cluster_kernel, dim3(ARGMAX_CTAS, (unsigned) rows), dim3(ARGMAX_CLUSTER_THREADS), 0, (cudaStream_t) stream, x, x_nb_row, d, out);
+    else launch_pdl(argmax_rows_kernel, dim3((unsigned) rows), dim3(ARGMAX_THREADS), 0, (cudaStream_t) stream, x, x_nb_row, d, out);
     return check_launch("argmax_rows");
 }
 

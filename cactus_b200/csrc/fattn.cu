@@ -335,8 +335,9 @@ __device__ __forceinline__ void fattn_store_out(const FattnParams &p, int64_t j,
 // CLUSTER: the KV splits of a token and head group are a cluster of CTAs, which add their parts through each other's shared memory; see
 // launch_mma_cluster
 // VOTED: launched beside the query-tiled kernel, mostly to return.  It has one walk, which reads the mask, where the others have a second one for
-// masks of 0 and -inf: with both the returning grid costs half a microsecond more once another kernel has run in between (16 ragged sequences,
-// 512 tokens: 121.8 us against 121.2).  A test in a single walk instead is no way out: 64 decode tokens 75.3 us, 73.2 with two walks.
+// masks of 0 and -inf: with both the returning grid costs up to 0.6 us more, 0.3 in the mean of 12 processes that differed in what ran before (16 ragged
+// sequences, 512 tokens, 121.2 us; where the driver puts the code moves that by as much again).  A test in a single walk instead is no way
+// out: 64 decode tokens 75.3 us, 73.2 with two walks.
 template <int D, bool QUANT, bool CLUSTER = false, bool VOTED = false>
 __global__ void __launch_bounds__(FA_THREADS, FA_MIN_CTAS) fattn_mma_kernel(FattnParams p) {
     pdl_prologue();
@@ -622,7 +623,7 @@ __global__ void __launch_bounds__(FA_THREADS, FA_MIN_CTAS) fattn_mma_kernel(Fatt
 // clusters costs more than the combine pass: 30 sequences of the 1B architecture, 480 CTAs, 1631 us a step against 1528): no partial
 // results in memory, no second launch.  The CTAs meet twice, after their parts are in shared memory and before they leave.  Bound by
 // latency; D = 64 has the registers to ask for the next chunk's V rows early.  us per decode step on B200, combine pass / cluster: 1B, one
-// sequence 722 / 687; 1B, 16 sequences 1323 / 1222; 8B, seven sequences 2521 / 2424.  With two CTAs an SM and V rows asked for early at
+// sequence (2 splits) 761 / 741; 1B, 16 sequences 1323 / 1222; 8B, seven sequences 2612 / 2520.  With two CTAs an SM and V rows asked for early at
 // D = 128 as well, the seven sequences took 2642.
 template <int D, bool QUANT>
 static void launch_mma_cluster(dim3 grid, cudaStream_t st, FattnParams p) {

@@ -104,8 +104,11 @@ B200_API int b200_quantize_q8_0(const float *x, int64_t x_row_stride_bytes, int6
  *            private to the call until it completes: the quantised activations (b200_act_bytes) followed
  *            by the kernel workspace (b200_mul_mat_workspace_bytes: split-K partial sums or the parked tiles and
  *            arrival counters of the stream-K work split)
- * N <= 2 uses the HBM-bound dp4a kernel (B200_MMVQ_MAX_N moves the border up to 8), larger N the int8 tensor-core kernel,
- * b200_mul_mat_q with Q4_0 weights, more than 32 columns and enough work the tcgen05 kernel (B200_MMQ_TC=0: never).
+ * N <= 2 uses the dp4a kernel (B200_MMVQ_MAX_N moves the border up to 8; weights of 65536 rows and more, output heads, have a streaming
+ * int8 tensor-core kernel, whose sums are in another order), 3 <= N <= 8 that streaming kernel or the tiled int8 tensor-core one, whichever is
+ * faster for the shape, with the same result to the last bit, larger N the tiled one, b200_mul_mat_q with Q4_0 weights, more than 32 columns
+ * and enough work the tcgen05 kernel (B200_MMQ_TC=0: never).  Calls are ordered on their stream, weights included: a product may be enqueued
+ * right behind the upload or copy that writes its weights.
  * ---------------------------------------------------------------------------------------------- */
 B200_API size_t b200_act_bytes(int64_t K, int64_t N);
 B200_API size_t b200_mul_mat_workspace_bytes(int wtype, int64_t K, int64_t M, int64_t N);
@@ -139,8 +142,8 @@ B200_API int b200_mul_mat_q_prequant_multi(int wtype, int n_weights, const void 
  *
  * Limits: N <= B200_NOALLOC_MAX_N columns (the decode kernel) and K <= B200_NOALLOC_MAX_K; larger sizes are
  * refused with B200_E_INVALID.  Results are within the mul_mat tolerance of b200_mul_mat_q, and bit-identical to it
- * whenever both calls split K the same way (for 3 to 8 columns b200_mul_mat_q may split K across CTAs through its
- * workspace; this entry point has no workspace and never does).  The first call on a device looks up the
+ * whenever both calls cut K the same way (for 3 to 8 columns some cuts are taken only with the workspace that
+ * b200_mul_mat_q has; this entry point has none).  The first call on a device looks up the
  * array's device address (a one-off set-up step): make that first call outside any stream capture.  All calls
  * share the one array, which keeps whatever the last call left in it: two calls that overlap on the GPU (different
  * streams, or different threads without ordering between them) race; calls ordered on one stream are fine. */
@@ -188,9 +191,10 @@ B200_API int b200_flash_attn_ext_indexed(int64_t D, int64_t H, int64_t Hkv, int6
 /* b200_flash_attn_ext_indexed whose result is (also) left as the Q8_0-quantised activations of the mul_mat that
  * consumes it (attention output -> wo in llm_build_llama, cactus/llama-model.cpp:4517-4671): what
  * b200_quantize_activations(dst, ..., K = H * D, N = Nq, act, ...) would write, bit for bit, without the extra
- * launch.  dst may be NULL when only the quantised form is wanted.  H * D must be a multiple of 128.  Measured on B200
- * at 64 tokens x 32 heads x 128 over 57k cells it is slower than the two launches (70.5 us against 57.5 + 2.5: the
- * attention kernel sits at its register limit), so it pays only where launches, not kernel time, are the cost. */
+ * launch.  dst may be NULL when only the quantised form is wanted.  H * D must be a multiple of 128.  It pays where the KV
+ * range is cut, up to some 36 tokens on 8 KV heads: what adds the splits quantises, and LlamaEngine uses it there.  Uncut, at 64 tokens x 32
+ * heads x 128 over 57k cells, it is slower than the two launches (70.5 us against 57.5 + 2.5 on B200: the attention kernel sits at its
+ * register limit), and the query-tiled kernel is not considered. */
 B200_API int b200_flash_attn_ext_quant(int64_t D, int64_t H, int64_t Hkv, int64_t Nq, int64_t n_kv,
                                        const float *q, int64_t q_nb_tok, int64_t q_nb_head,
                                        const void *k, int64_t k_nb_cell, int64_t k_nb_head,

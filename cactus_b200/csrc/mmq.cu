@@ -798,7 +798,7 @@ static const MmqVariant &variant_for(int wtype, int64_t N) {
 
 // Up to this many activation columns the dp4a kernel (mmvq.cu) runs; its time grows with the columns (9.9, 10.9, 14.9,
 // 17.0 us for 1..4 columns of a 14336 x 4096 Q4_0 weight on B200), where the streaming tensor-core kernel (mmq_stream.cu) takes
-// 11.0 us for any count up to 8.
+// 11.5 us for any count up to 8.
 int mmvq_max_n() {
     static const int v = [] {
         const char *e = getenv("B200_MMVQ_MAX_N");

@@ -14,8 +14,8 @@ def _two_weights(wtype, K, M):
     return [random_blocks(wtype, M, K, g) for _ in range(2)], g
 
 
-# dp4a, streaming (one column: from 32768 tiles on), tiled mma.sync
-@pytest.mark.parametrize("wtype,K,M,N", [(2, 2048, 8192, 1), (2, 4096, 20480, 1), (8, 4096, 16384, 2), (2, 2048, 8192, 3), (2, 4096, 4096, 8), (8, 2048, 4096, 5), (2, 2048, 8192, 24)])
+# dp4a (layers and, Q8_0 at two columns, a short head), streaming (heads and 3 to 8 columns), tiled mma.sync
+@pytest.mark.parametrize("wtype,K,M,N", [(2, 2048, 8192, 1), (2, 4096, 20480, 1), (8, 1024, 65536, 2), (2, 1024, 65536, 1), (8, 1024, 65536, 1), (2, 1024, 65536, 2), (2, 2048, 8192, 3), (2, 4096, 4096, 8), (8, 2048, 4096, 5), (2, 2048, 8192, 24)])
 @pytest.mark.parametrize("quantiser_between", [False, True])
 def test_product_behind_an_upload(wtype, K, M, N, quantiser_between):
     from cactus_b200._lib import check, lib
@@ -56,7 +56,7 @@ def test_product_behind_an_upload(wtype, K, M, N, quantiser_between):
 @pytest.mark.parametrize("N", [1, 4])
 def test_product_behind_a_stacking_copy(N):
     from cactus_b200 import ops
-    K, M = 4096, 10240
+    K, M = 1024, 32768   # stacked: an output head's rows
     blocks, g = _two_weights(2, K, M)
     parts = [ops.QWeight.from_blocks(2, K, M, b) for b in blocks]
     x = torch.randn((N, K), device="cuda", generator=g)

@@ -336,7 +336,7 @@ __device__ __forceinline__ void fattn_store_out(const FattnParams &p, int64_t j,
 // launch_mma_cluster
 // VOTED: launched beside the query-tiled kernel, mostly to return.  It has one walk, which reads the mask, where the others have a second one for
 // masks of 0 and -inf: with both the returning grid costs up to 0.6 us more, 0.3 in the mean of 12 processes that differed in what ran before (16 ragged
-// sequences, 512 tokens, 121.2 us; where the driver puts the code moves that by as much again).  A test in a single walk instead is no way
+// sequences, 512 tokens, 121.2 us; what ran before moves that by as much again).  A test in a single walk instead is no way
 // out: 64 decode tokens 75.3 us, 73.2 with two walks.
 template <int D, bool QUANT, bool CLUSTER = false, bool VOTED = false>
 __global__ void __launch_bounds__(FA_THREADS, FA_MIN_CTAS) fattn_mma_kernel(FattnParams p) {
